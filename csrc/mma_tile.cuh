@@ -180,4 +180,53 @@ __device__ __forceinline__ void load_tile_async_256(bf16* __restrict__ dst, cons
   }
 }
 
+// ---- products whose A operand stays in registers -----------------------------------------------------------------------
+// A warp's accumulator fragment of one product, packed to bf16, is the A fragment of the next product (the layouts of m16n8k16
+// agree), so probabilities and score gradients go from one product to the next without shared memory or a barrier.
+
+// A fragments of rows 16 wr .. + 15 of a padded tile, all four 16-deep k steps.
+__device__ __forceinline__ void load_a(const bf16* __restrict__ As, uint32_t (&a)[4][4], int wr, int lane) {
+  const bf16* p = As + (16 * wr + (lane & 7) + 8 * ((lane >> 3) & 1)) * LDS + 8 * (lane >> 4);
+#pragma unroll
+  for (int ks = 0; ks < 4; ++ks) ldmatrix_x4(a[ks], p + 16 * ks);
+}
+
+// acc[16 x 8 NT] += A[16 x 16 KS] B, B(k,n) = TB ? Bs[n*LDS + k] : Bs[k*LDS + n].
+// Accumulator element acc[nt][e] of warp row block wr: row = 16 wr + lane/4 + 8*(e>>1), col = 8nt + 2*(lane%4) + (e&1).
+template <bool TB, int KS, int NT>
+__device__ __forceinline__ void mma_rows(const uint32_t (&a)[KS][4], const bf16* __restrict__ Bs, float (&acc)[NT][4], int lane) {
+  const int l8 = lane & 7, m = lane >> 3;
+  const bf16* b_ptr = TB ? Bs + (l8 + 8 * (m >> 1)) * LDS + 8 * (m & 1) : Bs + (l8 + 8 * (m & 1)) * LDS + 8 * (m >> 1);
+#pragma unroll
+  for (int ks = 0; ks < KS; ++ks) {
+#pragma unroll
+    for (int np = 0; np < NT / 2; ++np) {
+      uint32_t b[4];
+      if (TB) ldmatrix_x4(b, b_ptr + 16 * np * LDS + 16 * ks);
+      else ldmatrix_x4_trans(b, b_ptr + 16 * ks * LDS + 16 * np);
+      mma16816(acc[2 * np], a[ks], b[0], b[1]);
+      mma16816(acc[2 * np + 1], a[ks], b[2], b[3]);
+    }
+  }
+}
+
+__device__ __forceinline__ uint32_t pack_f2(float a, float b) {
+  const __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
+  return *reinterpret_cast<const uint32_t*>(&h);
+}
+__device__ __forceinline__ float lo_f(uint32_t v) { return __uint_as_float(v << 16); }
+__device__ __forceinline__ float hi_f(uint32_t v) { return __uint_as_float(v & 0xffff0000u); }
+
+// Accumulator [16 x 16 KS] -> A fragments.
+template <int KS>
+__device__ __forceinline__ void pack_a(const float (&acc)[2 * KS][4], uint32_t (&a)[KS][4]) {
+#pragma unroll
+  for (int ks = 0; ks < KS; ++ks) {
+    a[ks][0] = pack_f2(acc[2 * ks][0], acc[2 * ks][1]);
+    a[ks][1] = pack_f2(acc[2 * ks][2], acc[2 * ks][3]);
+    a[ks][2] = pack_f2(acc[2 * ks + 1][0], acc[2 * ks + 1][1]);
+    a[ks][3] = pack_f2(acc[2 * ks + 1][2], acc[2 * ks + 1][3]);
+  }
+}
+
 }  // namespace q38
