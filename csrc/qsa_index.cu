@@ -10,7 +10,7 @@
 //   qsa_indexer_bwd_q / _k  recompute the score tiles and produce d(q_idx), d(w) / d(k_idx).
 //
 // Layouts: main q [B,nq,S,64], main k [B,nkv,S,64], indexer q [B,NI,S,64], indexer k [B,S,64] (bf16); w [B,S,NI] fp32.
-#include <torch/extension.h>
+#include <ATen/ATen.h>
 #include <ATen/cuda/CUDAContext.h>
 #include <c10/cuda/CUDAGuard.h>
 
@@ -238,151 +238,242 @@ __global__ void __launch_bounds__(256) qsa_select_kernel(const float* __restrict
 
 // ---- indexer backward ------------------------------------------------------------------------------------------------------
 // dI[t,s] = dblse[t, blk(s)] * exp(I[t,s] - blse[t, blk(s)]) for s <= t;   I = sum_h w_h relu(S_h) scale
-// Score tile of (query block i, key block j): all heads contribute to `score`; relu(S_own) is kept for head `own`.
-__device__ __forceinline__ void indexer_score_tile(const bf16* __restrict__ Qs, const bf16* __restrict__ Kt, const float (&wrow)[2][NI_MAX], int NI, int own,
-                                                   float (&score)[8][4], float (&sown)[8][4], int warp, int lane) {
-  zero_acc(score);
-  for (int hh = 0; hh < NI; ++hh) {
-    float acc[8][4];
-    zero_acc(acc);
-    mma64<false, true>(Qs + hh * TILE_ELEMS, Kt, acc, warp, lane);
-#pragma unroll
-    for (int nt = 0; nt < 8; ++nt)
-#pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        const float r = fmaxf(bf16_round(acc[nt][e]), 0.f);
-        score[nt][e] += (e < 2 ? wrow[0][hh] : wrow[1][hh]) * r;
-        if (hh == own) sown[nt][e] = r;
-      }
-  }
-}
+// Both passes form the scores of all heads once per (query block, key block) pair, keep relu(S_h) (which is bf16 by definition) packed in
+// registers until dI is known, and pass dS_h to the next product as A fragments in registers.  Four sequences of 4096 with four heads: 741 -> 461 us.
 
-__device__ __forceinline__ void indexer_dI_tile(const float (&score)[8][4], const float* __restrict__ blse, const float* __restrict__ dblse, float gscale,
-                                                long long row_base, int nb, int j, bool diag, float (&dI)[8][4], int warp, int lane) {
-  const int r0 = 16 * warp + (lane >> 2), cq = 2 * (lane & 3);
-#pragma unroll
-  for (int hrow = 0; hrow < 2; ++hrow) {
-    const int row = r0 + 8 * hrow;
-    const float bl = blse[(row_base + row) * nb + j], g = dblse[(row_base + row) * nb + j] * gscale;
-#pragma unroll
-    for (int nt = 0; nt < 8; ++nt)
-#pragma unroll
-      for (int e = 0; e < 2; ++e) {
-        const int col = 8 * nt + cq + e;
-        dI[nt][2 * hrow + e] = (!diag || col <= row) ? g * __expf(score[nt][2 * hrow + e] - bl) : 0.f;
-      }
-  }
-}
-
-// Query pass, grid (nb, NI, B): d q_own(t) = sum_s dI w_own scale [S_own > 0] k(s);  d w_own(t) = sum_s dI relu(S_own) scale.
-__global__ void __launch_bounds__(128) qsa_indexer_bwd_q_kernel(const bf16* __restrict__ qi, const bf16* __restrict__ ki, const float* __restrict__ wi,
+// Query pass, grid (nb, B), eight warps: d q_h(t) = sum_s dI w_h scale [S_h > 0] k(s);  d w_h(t) = sum_s dI relu(S_h) scale.
+// Warps 0-3 hold heads 0 and 1, warps 4-7 heads 2 and 3, each warp 16 queries; the two partial scores of a tile meet in shared memory.
+// Eight 64^3 products per pair (one CTA per head had twenty), 306 us; bound by the latency of their chain, since the accumulators of two heads
+// leave eight warps per SM.  One head per warp and sixteen warps took 396 us: four times the exponentials and twice the exchange.
+__global__ void __launch_bounds__(256) qsa_indexer_bwd_q_kernel(const bf16* __restrict__ qi, const bf16* __restrict__ ki, const float* __restrict__ wi,
                                                                 const float* __restrict__ blse, const float* __restrict__ dblse, float gscale,
                                                                 bf16* __restrict__ dqi, float* __restrict__ dwi, int S, int NI, float scale) {
   extern __shared__ __align__(16) uint8_t smem_bytes[];
-  bf16* Qs = reinterpret_cast<bf16*>(smem_bytes);
+  bf16* Qs = reinterpret_cast<bf16*>(smem_bytes);          // NI tiles
   bf16* Ks = Qs + NI_MAX * TILE_ELEMS;                     // two buffers
-  bf16* Ts = Ks + 2 * TILE_ELEMS;                          // dS_own tile (bf16) as A operand
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int nb = S / 64, i = nb - 1 - blockIdx.x, own = blockIdx.y, b = blockIdx.z;   // late query blocks (longest loops) first
-  for (int hh = 0; hh < NI; ++hh) load_tile_async(Qs + hh * TILE_ELEMS, qi + (((long long)b * NI + hh) * S + (long long)i * 64) * 64, 64, tid);
+  float4* Px = reinterpret_cast<float4*>(Ks + 2 * TILE_ELEMS);     // partial scores of the two halves: [2][4 n-tiles][4 warps][32 lanes], per 32 keys
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, wr = warp & 3, grp = warp >> 2;
+  const int nb = S / 64, i = nb - 1 - blockIdx.x, b = blockIdx.y;   // late query blocks (longest loops) first
+  for (int hh = 0; hh < NI; ++hh) load_tile_async_256(Qs + hh * TILE_ELEMS, qi + (((long long)b * NI + hh) * S + (long long)i * 64) * 64, 64, tid);
   const bf16* kbase = ki + (long long)b * S * 64;
-  load_tile_async(Ks, kbase, 64, tid);
+  load_tile_async_256(Ks, kbase, 64, tid);
   cp_async_commit();
-  const int r0 = 16 * warp + (lane >> 2);
-  float wrow[2][NI_MAX];
+  const int r0 = 16 * wr + (lane >> 2), cq = 2 * (lane & 3);
+  const long long row = (long long)b * S + (long long)i * 64 + r0;
+  const int heads = NI - 2 * grp < 0 ? 0 : (NI - 2 * grp > 2 ? 2 : NI - 2 * grp);     // of this warp: 2 grp .. 2 grp + heads - 1
+  float w[2][2], dw[2][2] = {{0.f, 0.f}, {0.f, 0.f}};      // [head][row half]
 #pragma unroll
-  for (int hrow = 0; hrow < 2; ++hrow)
+  for (int x = 0; x < 2; ++x)
 #pragma unroll
-    for (int hh = 0; hh < NI_MAX; ++hh)
-      wrow[hrow][hh] = hh < NI ? wi[((long long)b * S + (long long)i * 64 + r0 + 8 * hrow) * NI + hh] * scale : 0.f;
-  const float wown[2] = {wi[((long long)b * S + (long long)i * 64 + r0) * NI + own] * scale, wi[((long long)b * S + (long long)i * 64 + r0 + 8) * NI + own] * scale};
-  float dw[2] = {0.f, 0.f};
-  float dq[8][4];
-  zero_acc(dq);
+    for (int hr = 0; hr < 2; ++hr) w[x][hr] = x < heads ? wi[(row + 8 * hr) * NI + 2 * grp + x] * scale : 0.f;
+  float dq[2][8][4];
+  zero_acc(dq[0]);
+  zero_acc(dq[1]);
+  float bl[2], g[2];
+#pragma unroll
+  for (int hr = 0; hr < 2; ++hr) { bl[hr] = blse[(row + 8 * hr) * nb]; g[hr] = dblse[(row + 8 * hr) * nb]; }
   for (int j = 0; j <= i; ++j) {
-    const int buf = j & 1;
-    if (j < i) { load_tile_async(Ks + (buf ^ 1) * TILE_ELEMS, kbase + (long long)(j + 1) * 4096, 64, tid); cp_async_commit(); cp_async_wait<1>(); }
-    else cp_async_wait<0>();
+    cp_async_wait<0>();
     __syncthreads();
-    const bf16* Kt = Ks + buf * TILE_ELEMS;
-    float score[8][4], sown[8][4], dI[8][4];
-    indexer_score_tile(Qs, Kt, wrow, NI, own, score, sown, warp, lane);
-    indexer_dI_tile(score, blse, dblse, gscale, (long long)b * S + (long long)i * 64, nb, j, j == i, dI, warp, lane);
+    if (j < i) load_tile_async_256(Ks + ((j + 1) & 1) * TILE_ELEMS, kbase + (long long)(j + 1) * 4096, 64, tid);
+    cp_async_commit();
+    const bf16* Kt = Ks + (j & 1) * TILE_ELEMS;
+    const float b0 = bl[0], b1 = bl[1], g0 = g[0] * gscale, g1 = g[1] * gscale;
+    if (j < i) {
 #pragma unroll
-    for (int nt = 0; nt < 8; ++nt)
+      for (int hr = 0; hr < 2; ++hr) { bl[hr] = blse[(row + 8 * hr) * nb + j + 1]; g[hr] = dblse[(row + 8 * hr) * nb + j + 1]; }
+    }
 #pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        dw[e >> 1] += dI[nt][e] * sown[nt][e] * scale;
-        dI[nt][e] = sown[nt][e] > 0.f ? dI[nt][e] * wown[e >> 1] : 0.f;        // dS_own
+    for (int half = 0; half < 2; ++half) {                 // 32 keys at a time
+      uint32_t r[2][2][4];                                 // relu(S_h) as A fragments
+      float score[4][4];
+      zero_acc(score);
+#pragma unroll
+      for (int x = 0; x < 2; ++x) {
+        float acc[4][4];
+        zero_acc(acc);
+        if (x < heads) {
+          uint32_t a[4][4];
+          load_a(Qs + (2 * grp + x) * TILE_ELEMS, a, wr, lane);
+          mma_rows<true, 4, 4>(a, Kt + 32 * half * LDS, acc, lane);
+        }
+#pragma unroll
+        for (int nt = 0; nt < 4; ++nt)
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            acc[nt][e] = fmaxf(bf16_round(acc[nt][e]), 0.f);
+            score[nt][e] += w[x][e >> 1] * acc[nt][e];
+          }
+        pack_a<2>(acc, r[x]);
       }
-    acc_to_smem(dI, Ts, warp, lane);
-    __syncthreads();
-    mma64<false, false>(Ts, Kt, dq, warp, lane);           // dS_own K
-    __syncthreads();
-  }
-  acc_to_global(dq, dqi + (((long long)b * NI + own) * S + (long long)i * 64) * 64, 64, warp, lane);
 #pragma unroll
-  for (int hrow = 0; hrow < 2; ++hrow) {
-    float v = dw[hrow];
-    v += __shfl_xor_sync(0xffffffffu, v, 1);
-    v += __shfl_xor_sync(0xffffffffu, v, 2);
-    if ((lane & 3) == 0) dwi[((long long)b * S + (long long)i * 64 + r0 + 8 * hrow) * NI + own] = v;
+      for (int nt = 0; nt < 4; ++nt) Px[(half * 8 + grp * 4 + nt) * 128 + wr * 32 + lane] = make_float4(score[nt][0], score[nt][1], score[nt][2], score[nt][3]);
+      // the two warps of these 16 rows meet; the buffer of this half is free again after the block barrier of the next tile
+      asm volatile("bar.sync %0, 64;" ::"r"(1 + wr) : "memory");
+#pragma unroll
+      for (int nt = 0; nt < 4; ++nt) {
+        const float4 o = Px[(half * 8 + (grp ^ 1) * 4 + nt) * 128 + wr * 32 + lane];
+        const float other[4] = {o.x, o.y, o.z, o.w};
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const int col = 32 * half + 8 * nt + cq + (e & 1);
+          const float d = (e >> 1 ? g1 : g0) * __expf(score[nt][e] + other[e] - (e >> 1 ? b1 : b0));
+          score[nt][e] = (j < i || col <= r0 + 8 * (e >> 1)) ? d : 0.f;       // dI
+        }
+      }
+#pragma unroll
+      for (int x = 0; x < 2; ++x) {
+        if (x < heads) {
+          float ds[4][4];
+#pragma unroll
+          for (int nt = 0; nt < 4; ++nt)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+              const uint32_t p = r[x][nt >> 1][(nt & 1) * 2 + (e >> 1)];
+              const float relu = (e & 1) ? hi_f(p) : lo_f(p);
+              dw[x][e >> 1] += score[nt][e] * relu * scale;
+              ds[nt][e] = relu > 0.f ? score[nt][e] * w[x][e >> 1] : 0.f;     // dS_h
+            }
+          uint32_t a[2][4];
+          pack_a<2>(ds, a);
+          mma_rows<false, 2, 8>(a, Kt + 32 * half * LDS, dq[x], lane);        // dS_h K
+        }
+      }
+    }
+  }
+  cp_async_wait<0>();
+#pragma unroll
+  for (int x = 0; x < 2; ++x) {
+    if (x < heads) {
+      const int own = 2 * grp + x;
+      acc_to_global(dq[x], dqi + (((long long)b * NI + own) * S + (long long)i * 64) * 64, 64, wr, lane);
+#pragma unroll
+      for (int hr = 0; hr < 2; ++hr) {
+        float v = dw[x][hr];
+        v += __shfl_xor_sync(0xffffffffu, v, 1);
+        v += __shfl_xor_sync(0xffffffffu, v, 2);
+        if ((lane & 3) == 0) dwi[(row + 8 * hr) * NI + own] = v;
+      }
+    }
   }
 }
 
-// Key pass, grid (nb, B): d k(s) = sum_{t >= s} sum_h dS_h[t,s] q_h(t), looping over query blocks i >= j.
+// Key pass, grid (nb, B, z), four warps of 16 keys: d k(s) = sum_{t >= s} sum_h dS_h[t,s] q_h(t).  Scores are formed transposed (K Q_h^T), so
+// dS_h^T is the A fragment of dS_h^T Q_h.  The query blocks i >= j of a key block are shared by gridDim.z CTAs (i = j + z, j + z + gridDim.z, ...),
+// whose partial gradients are added in fp32.  Eight products per pair, bound by the warp MMA rate.
 __global__ void __launch_bounds__(128) qsa_indexer_bwd_k_kernel(const bf16* __restrict__ qi, const bf16* __restrict__ ki, const float* __restrict__ wi,
                                                                 const float* __restrict__ blse, const float* __restrict__ dblse, float gscale,
                                                                 float* __restrict__ dki, int S, int NI, float scale) {
   extern __shared__ __align__(16) uint8_t smem_bytes[];
-  bf16* Ks = reinterpret_cast<bf16*>(smem_bytes);
-  bf16* Qs = Ks + TILE_ELEMS;                              // NI tiles of the current query block
-  bf16* Ts = Qs + NI_MAX * TILE_ELEMS;
+  bf16* Qs = reinterpret_cast<bf16*>(smem_bytes);          // two buffers of NI_MAX tiles
+  float* rows = reinterpret_cast<float*>(Qs + 2 * NI_MAX * TILE_ELEMS);      // two buffers of {blse[64], dblse gscale[64], w scale[NI_MAX][64]}
+  constexpr int ROWS = (2 + NI_MAX) * 64;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  // Key block j is scored by every query block i >= j: the loop is shared by gridDim.z CTAs (i = j + z, j + z + gridDim.z, ...)
-  // whose partial gradients are added in fp32.
   const int j = blockIdx.x, b = blockIdx.y, nb = S / 64;
   if (j + (int)blockIdx.z >= nb) return;
-  load_tile_async(Ks, ki + ((long long)b * S + (long long)j * 64) * 64, 64, tid);
+  load_tile_async(Qs + NI_MAX * TILE_ELEMS, ki + ((long long)b * S + (long long)j * 64) * 64, 64, tid);
   cp_async_commit();
-  const int r0 = 16 * warp + (lane >> 2);
+  auto fetch = [&](int i, int buf) {
+    for (int hh = 0; hh < NI; ++hh) load_tile_async(Qs + (buf * NI_MAX + hh) * TILE_ELEMS, qi + (((long long)b * NI + hh) * S + (long long)i * 64) * 64, 64, tid);
+    cp_async_commit();
+  };
+  // per query: this thread's share (query tid % 64) travels through registers so that its latency hides behind a whole tile
+  float v0 = 0.f, v1 = 0.f, v2 = 0.f;
+  auto fetch_rows = [&](int i) {
+    const long long t = (long long)b * S + (long long)i * 64 + (tid & 63);
+    const int hh = 2 * (tid >> 6);                         // the first 64 threads bring blse and heads 0, 1, the others dblse and heads 2, 3
+    v0 = tid < 64 ? blse[t * nb + j] : dblse[t * nb + j] * gscale;
+    v1 = hh < NI ? wi[t * NI + hh] * scale : 0.f;
+    v2 = hh + 1 < NI ? wi[t * NI + hh + 1] * scale : 0.f;
+  };
+  auto put_rows = [&](int buf) {
+    float* dst = rows + buf * ROWS + (tid & 63);
+    const int half = tid >> 6;
+    dst[64 * half] = v0;
+    dst[64 * (2 + 2 * half)] = v1;
+    dst[64 * (3 + 2 * half)] = v2;
+  };
+  const int step = gridDim.z;
+  int i = j + blockIdx.z;
+  fetch(i, 0);
+  fetch_rows(i);
+  cp_async_wait<1>();
+  __syncthreads();
+  uint32_t ak[4][4];
+  load_a(Qs + NI_MAX * TILE_ELEMS, ak, warp, lane);
+  put_rows(0);
+  const int r0 = 16 * warp + (lane >> 2), cq = 2 * (lane & 3);
   float dk[8][4];
   zero_acc(dk);
-  for (int i = j + blockIdx.z; i < nb; i += gridDim.z) {
-    __syncthreads();
-    for (int hh = 0; hh < NI; ++hh) load_tile_async(Qs + hh * TILE_ELEMS, qi + (((long long)b * NI + hh) * S + (long long)i * 64) * 64, 64, tid);
-    cp_async_commit();
+  for (int buf = 0; i < nb; i += step, buf ^= 1) {
     cp_async_wait<0>();
     __syncthreads();
-    float wrow[2][NI_MAX];
+    const bool more = i + step < nb;
+    if (more) { fetch(i + step, buf ^ 1); fetch_rows(i + step); }
+    const bf16* Qt = Qs + buf * NI_MAX * TILE_ELEMS;
+    const float* rw = rows + buf * ROWS;
+    const bool diag = i == j;
 #pragma unroll
-    for (int hrow = 0; hrow < 2; ++hrow)
+    for (int half = 0; half < 2; ++half) {                 // 32 queries at a time
+      uint32_t r[NI_MAX][2][4];
+      float score[4][4];
+      zero_acc(score);
 #pragma unroll
-      for (int hh = 0; hh < NI_MAX; ++hh)
-        wrow[hrow][hh] = hh < NI ? wi[((long long)b * S + (long long)i * 64 + r0 + 8 * hrow) * NI + hh] * scale : 0.f;
-    float score[8][4], sown[8][4], dI[8][4];
-    indexer_score_tile(Qs, Ks, wrow, NI, -1, score, sown, warp, lane);
-    indexer_dI_tile(score, blse, dblse, gscale, (long long)b * S + (long long)i * 64, nb, j, j == i, dI, warp, lane);
-    for (int hh = 0; hh < NI; ++hh) {
-      float acc[8][4];
-      zero_acc(acc);
-      mma64<false, true>(Qs + hh * TILE_ELEMS, Ks, acc, warp, lane);          // recompute S_h
+      for (int hh = 0; hh < NI_MAX; ++hh) {
+        if (hh < NI) {
+          float acc[4][4];
+          zero_acc(acc);
+          mma_rows<true, 4, 4>(ak, Qt + hh * TILE_ELEMS + 32 * half * LDS, acc, lane);
 #pragma unroll
-      for (int nt = 0; nt < 8; ++nt)
+          for (int nt = 0; nt < 4; ++nt) {
+            const float2 w = *reinterpret_cast<const float2*>(rw + 64 * (2 + hh) + 32 * half + 8 * nt + cq);
 #pragma unroll
-        for (int e = 0; e < 4; ++e) acc[nt][e] = bf16_round(acc[nt][e]) > 0.f ? dI[nt][e] * (e < 2 ? wrow[0][hh] : wrow[1][hh]) : 0.f;
-      __syncthreads();
-      acc_to_smem(acc, Ts, warp, lane);
-      __syncthreads();
-      mma64<true, false>(Ts, Qs + hh * TILE_ELEMS, dk, warp, lane);           // dS_h^T Q_h
+            for (int e = 0; e < 4; ++e) {
+              acc[nt][e] = fmaxf(bf16_round(acc[nt][e]), 0.f);
+              score[nt][e] += (e & 1 ? w.y : w.x) * acc[nt][e];
+            }
+          }
+          pack_a<2>(acc, r[hh]);
+        }
+      }
+#pragma unroll
+      for (int nt = 0; nt < 4; ++nt) {
+        const int col = 32 * half + 8 * nt + cq;           // query
+        const float2 bl = *reinterpret_cast<const float2*>(rw + col), g = *reinterpret_cast<const float2*>(rw + 64 + col);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const float d = (e & 1 ? g.y : g.x) * __expf(score[nt][e] - (e & 1 ? bl.y : bl.x));
+          score[nt][e] = (!diag || r0 + 8 * (e >> 1) <= col + (e & 1)) ? d : 0.f;       // dI
+        }
+      }
+#pragma unroll
+      for (int hh = 0; hh < NI_MAX; ++hh) {
+        if (hh < NI) {
+          float ds[4][4];
+#pragma unroll
+          for (int nt = 0; nt < 4; ++nt) {
+            const float2 w = *reinterpret_cast<const float2*>(rw + 64 * (2 + hh) + 32 * half + 8 * nt + cq);
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+              const uint32_t p = r[hh][nt >> 1][(nt & 1) * 2 + (e >> 1)];
+              ds[nt][e] = ((e & 1) ? hi_f(p) : lo_f(p)) > 0.f ? score[nt][e] * (e & 1 ? w.y : w.x) : 0.f;
+            }
+          }
+          uint32_t a[2][4];
+          pack_a<2>(ds, a);
+          mma_rows<false, 2, 8>(a, Qt + hh * TILE_ELEMS + 32 * half * LDS, dk, lane);   // dS_h^T Q_h
+        }
+      }
     }
+    if (more) put_rows(buf ^ 1);
   }
+  cp_async_wait<0>();
   float* dst = dki + ((long long)b * S + (long long)j * 64) * 64;
-  const int cq = 2 * (lane & 3);
 #pragma unroll
   for (int nt = 0; nt < 8; ++nt)
 #pragma unroll
-    for (int e = 0; e < 4; ++e) atomicAdd(dst + (r0 + 8 * (e >> 1)) * 64 + 8 * nt + cq + (e & 1), dk[nt][e]);
+    for (int x = 0; x < 2; ++x)
+      atomicAdd(reinterpret_cast<float2*>(dst + (r0 + 8 * x) * 64 + 8 * nt + cq), make_float2(dk[nt][2 * x], dk[nt][2 * x + 1]));
 }
 
 // ---- host ----------------------------------------------------------------------------------------------------------------------
@@ -465,17 +556,17 @@ std::vector<at::Tensor> qsa_indexer_bwd(const at::Tensor& qi, const at::Tensor& 
   auto dqi = at::empty_like(qi);
   auto dki32 = at::zeros(ki.sizes(), ki.options().dtype(at::kFloat));
   auto dwi = at::empty_like(wi);
-  const int smem = (NI_MAX + 3) * TILE_ELEMS * 2;
+  constexpr int smem_q = (NI_MAX + 2) * TILE_ELEMS * 2 + 16 * 128 * 16, smem_k = 2 * NI_MAX * TILE_ELEMS * 2 + 2 * (2 + NI_MAX) * 64 * 4;
   static bool cfg = false;
   if (!cfg) {
-    C10_CUDA_CHECK(cudaFuncSetAttribute(qsa_indexer_bwd_q_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    C10_CUDA_CHECK(cudaFuncSetAttribute(qsa_indexer_bwd_k_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    C10_CUDA_CHECK(cudaFuncSetAttribute(qsa_indexer_bwd_q_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_q));
+    C10_CUDA_CHECK(cudaFuncSetAttribute(qsa_indexer_bwd_k_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_k));
     cfg = true;
   }
   auto stream = at::cuda::getCurrentCUDAStream();
-  qsa_indexer_bwd_q_kernel<<<dim3(nb, NI, B), 128, smem, stream>>>((const bf16*)qi.data_ptr(), (const bf16*)ki.data_ptr(), wi.data_ptr<float>(), blse.data_ptr<float>(),
+  qsa_indexer_bwd_q_kernel<<<dim3(nb, B), 256, smem_q, stream>>>((const bf16*)qi.data_ptr(), (const bf16*)ki.data_ptr(), wi.data_ptr<float>(), blse.data_ptr<float>(),
       dblse.data_ptr<float>(), (float)gscale, (bf16*)dqi.data_ptr(), dwi.data_ptr<float>(), S, NI, (float)scale);
-  qsa_indexer_bwd_k_kernel<<<dim3(nb, B, std::min(nb, 8)), 128, smem, stream>>>((const bf16*)qi.data_ptr(), (const bf16*)ki.data_ptr(), wi.data_ptr<float>(),
+  qsa_indexer_bwd_k_kernel<<<dim3(nb, B, std::min(nb, 8)), 128, smem_k, stream>>>((const bf16*)qi.data_ptr(), (const bf16*)ki.data_ptr(), wi.data_ptr<float>(),
       blse.data_ptr<float>(), dblse.data_ptr<float>(), (float)gscale, dki32.data_ptr<float>(), S, NI, (float)scale);
   C10_CUDA_KERNEL_LAUNCH_CHECK();
   count_launch(2);
