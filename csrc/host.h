@@ -1,6 +1,6 @@
 // Host-side declarations shared by the extension's translation units.
 #pragma once
-#include <torch/extension.h>
+#include <ATen/ATen.h>
 #include <cuda.h>
 
 #include <atomic>
@@ -40,7 +40,7 @@ void muon_small_ns(const at::Tensor& src, at::Tensor& dst, int64_t rows, int64_t
 
 // qsa_prep.cu
 std::vector<at::Tensor> qsa_headprep_fwd(const at::Tensor& src, const c10::optional<at::Tensor>& w, const at::Tensor& cosv, const at::Tensor& sinv, double eps,
-                                         bool split_gate);
+                                         bool split_gate, bool round_products);
 std::vector<at::Tensor> qsa_headprep_bwd(const at::Tensor& dout, const c10::optional<at::Tensor>& dgate, const at::Tensor& src, const c10::optional<at::Tensor>& w,
                                          const at::Tensor& cosv, const at::Tensor& sinv, const at::Tensor& rstd);
 
