@@ -857,9 +857,18 @@ class Backend:
             elif os.environ.get("Q38_INDEXER_BASELINE"):
                 with torch.no_grad():
                     _, lp_blk = self.indexer_block_logprobs(indexer, x.detach(), cos, sin)
-            else:
+            elif indexer.d_ih == 64 and cos.shape[-1] == 16:
                 # no KL wanted (evaluation, or training steps that skip it): block selection only looks at the first query of each
-                # 64-token block, so only those S/64 queries are scored -> lp_blk [B, nb, nb]  (reference: modeling_qwen3_8_moe.py:1126)
+                # 64-token block, so only those S/64 queries are projected and scored -> lp_blk [B, nb, nb]  (reference: modeling_qwen3_8_moe.py:1126)
+                with torch.no_grad():
+                    xd, NI, step = x.detach(), indexer.n_ih, modeling.BLK
+                    xf, cf, sf = xd[:, ::step], cos[:, ::step], sin[:, ::step]
+                    rope = lambda t, c, s: load().qsa_headprep_fwd(t, None, c.float().contiguous(), s.float().contiguous(), 0.0, False, True)[0]
+                    qi = rope(self.linear(xf, indexer.wq.weight).view(B, S // step, NI, 64), cf, sf)
+                    ki = rope(self.linear(xd, indexer.wk.weight).view(B, S, 1, 64), cos, sin)[:, 0]
+                    wi = self.linear(xf, indexer.ww.weight).float() * NI ** -0.5
+                    lp_blk = load().qsa_first_query_lp(qi, ki, wi, indexer.d_ih ** -0.5)
+            else:
                 with torch.no_grad():
                     qi, ki, wi = indexer.project(x.detach(), cos, sin)
                     if qi.dtype == torch.bfloat16 and ki.dtype == torch.bfloat16:
