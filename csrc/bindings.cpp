@@ -49,6 +49,7 @@ TORCH_LIBRARY(q38, m) {
   m.def("gdn_gates_fwd(Tensor b_raw, Tensor a_raw, Tensor A_log, Tensor dt_bias) -> Tensor[]", &q38::gdn_gates_fwd);
   m.def("gdn_gates_bwd(Tensor dbeta, Tensor dg, Tensor b_raw, Tensor a_raw, Tensor A_log, Tensor dt_bias) -> Tensor[]", &q38::gdn_gates_bwd);
   m.def("embed_bwd(Tensor ids, Tensor dout, Tensor(a!) grad) -> ()", &q38::embed_bwd);
+  m.def("scale_bf16(Tensor x, Tensor factor) -> Tensor", &q38::scale_bf16);
   m.def("swiglu_fwd(Tensor g, Tensor u) -> Tensor", &q38::swiglu_fwd);
   m.def("swiglu_bwd(Tensor dy, Tensor g, Tensor u) -> Tensor[]", &q38::swiglu_bwd);
   m.def("sigmoid_mul_fwd(Tensor x, Tensor g) -> Tensor", &q38::sigmoid_mul_fwd);

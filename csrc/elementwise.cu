@@ -263,6 +263,34 @@ std::vector<at::Tensor> swiglu_bwd(const at::Tensor& dy, const at::Tensor& g, co
   return {dg, du};
 }
 
+// ---- y = x * factor[0] on bf16, eight elements per thread (a library product with a one-element device tensor runs element by element: 16 us
+// instead of 6 for 8192 x 576) ---------------------------------------------------------------------------------------------
+__global__ void __launch_bounds__(256) scale_bf16_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ factor, __nv_bfloat16* __restrict__ y, long long n8) {
+  const long long i = (long long)blockIdx.x * 256 + threadIdx.x;
+  if (i >= n8) return;
+  const float f = __bfloat162float(*factor);
+  float v[8];
+  unpack8(reinterpret_cast<const uint4*>(x)[i], v);
+#pragma unroll
+  for (int k = 0; k < 8; ++k) v[k] *= f;
+  reinterpret_cast<uint4*>(y)[i] = pack8(v);
+}
+
+at::Tensor scale_bf16(const at::Tensor& x, const at::Tensor& factor) {
+  TORCH_CHECK(x.is_cuda() && x.scalar_type() == at::kBFloat16 && x.is_contiguous() && x.numel() % 8 == 0 && (reinterpret_cast<uintptr_t>(x.data_ptr()) & 15) == 0 &&
+                  factor.is_cuda() && factor.scalar_type() == at::kBFloat16 && factor.numel() == 1, "scale_bf16: 16-byte aligned contiguous bf16 and a one-element bf16 factor required");
+  const c10::cuda::CUDAGuard guard(x.device());
+  auto y = at::empty_like(x);
+  const long long n8 = x.numel() / 8;
+  if (n8) {
+    scale_bf16_kernel<<<(unsigned)((n8 + 255) / 256), 256, 0, at::cuda::getCurrentCUDAStream()>>>((const __nv_bfloat16*)x.data_ptr(), (const __nv_bfloat16*)factor.data_ptr(),
+                                                                                                  (__nv_bfloat16*)y.data_ptr(), n8);
+    C10_CUDA_KERNEL_LAUNCH_CHECK();
+    count_launch();
+  }
+  return y;
+}
+
 // ---- output gate of the attention layer: y = x * bf16(sigmoid(g)), elementwise on bf16 (eight elements per thread) -------
 __global__ void __launch_bounds__(256) sigmoid_mul_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ g,
                                                                __nv_bfloat16* __restrict__ y, long long n8) {

@@ -51,6 +51,7 @@ std::vector<at::Tensor> gdn_gates_fwd(const at::Tensor& b_raw, const at::Tensor&
 std::vector<at::Tensor> gdn_gates_bwd(const at::Tensor& dbeta, const at::Tensor& dg, const at::Tensor& b_raw, const at::Tensor& a_raw, const at::Tensor& A_log,
                                       const at::Tensor& dt_bias);
 
+at::Tensor scale_bf16(const at::Tensor& x, const at::Tensor& factor);
 at::Tensor swiglu_fwd(const at::Tensor& g, const at::Tensor& u);
 std::vector<at::Tensor> swiglu_bwd(const at::Tensor& dy, const at::Tensor& g, const at::Tensor& u);
 
