@@ -5,12 +5,14 @@
 // the raw material of the distillation target of the indexer (same contract as qsa_main_block_stats in qsa_index.cu, which
 // remains the path for sequence lengths that are not a multiple of 128).
 //
-// One CTA per (128 query rows = two 64-token query blocks of one head, batch).  The query tile is loaded once; key tiles of 256
-// keys stream through a TMA ring; each group is one 128 x 256 x 64 product (four K = 16 instructions) into one of two 256-column
+// One CTA per (128 query rows = two 64-token query blocks of one head, batch).  The query tile is loaded once; key tiles of 128
+// keys stream through a TMA ring; each group is one 128 x 128 x 64 product (four K = 16 instructions) into one of two 128-column
 // TMEM accumulators, so the row statistics of group g (four epilogue warps, one query row per thread: tcgen05.ld, running max,
 // exp2, sum) overlap the MMAs of group g + 1.  The kernel is bound by the exponentials, not by the products: S^2 / 2 of them per
-// head.  Every mbarrier wait is bounded and reports through the error word.
-#include <torch/extension.h>
+// head, 169 us for 22 heads of four sequences of 4096.  Two CTAs per SM (256 TMEM columns and at most 102 registers each) keep the special-function
+// units busy while one of them starts, loads or takes maxima; one CTA with 256-key groups and 8-byte stores took 332 us, this takes 253.
+// Every mbarrier wait is bounded and reports through the error word.
+#include <ATen/ATen.h>
 #include <ATen/cuda/CUDAContext.h>
 #include <c10/cuda/CUDAGuard.h>
 
@@ -19,7 +21,7 @@
 
 namespace q38 {
 
-constexpr int QT_ROWS = 128, QT_KEYS = 256, QT_STAGES = 2, QT_THREADS = 320;     // TMA warp, MMA warp, two epilogue warpgroups
+constexpr int QT_ROWS = 128, QT_KEYS = 128, QT_STAGES = 3, QT_THREADS = 320;     // TMA warp, MMA warp, two epilogue warpgroups
 
 struct QsaTcArgs {
   float2* stats;
@@ -34,7 +36,7 @@ __device__ __forceinline__ float fast_exp2(float x) {
   return y;
 }
 
-__global__ void __launch_bounds__(QT_THREADS) qsa_block_stats_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK, QsaTcArgs p) {
+__global__ void __launch_bounds__(QT_THREADS, 2) qsa_block_stats_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK, QsaTcArgs p) {
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw = ptx::smem_u32(smem_raw);
   uint8_t* smem = smem_raw + ((1024u - (raw & 1023u)) & 1023u);
@@ -62,7 +64,7 @@ __global__ void __launch_bounds__(QT_THREADS) qsa_block_stats_tc_kernel(const __
     for (int a = 0; a < 2; ++a) { ptx::mbar_init(&acc_full[a], 1); ptx::mbar_init(&acc_empty[a], 4); }
     ptx::fence_barrier_init();
   }
-  if (warp == 1) { ptx::tmem_alloc(tmem_slot, 512); ptx::tmem_relinquish(); }
+  if (warp == 1) { ptx::tmem_alloc(tmem_slot, 2 * QT_KEYS); ptx::tmem_relinquish(); }
   ptx::tc_fence_before();
   __syncthreads();
   ptx::tc_fence_after();
@@ -111,44 +113,40 @@ __global__ void __launch_bounds__(QT_THREADS) qsa_block_stats_tc_kernel(const __
       if (!ptx::mbar_wait(&acc_full[acc], (g >> 1) & 1, 1u << 22)) { report_error(p.err, ERR_EPILOGUE_WAIT); ok = false; break; }
       ptx::tc_fence_after();
       const uint32_t t_addr = tmem_base + acc * QT_KEYS + (uint32_t(quarter * 32) << 16);
-      uint32_t nxt_lo[32], nxt_hi[32];
-      ptx::tmem_ld_32x32b_x32(t_addr, nxt_lo);
-      ptx::tmem_ld_32x32b_x32(t_addr + 32, nxt_hi);
-#pragma unroll 1
-      for (int jb4 = 0; jb4 < 4; ++jb4) {
-        const int jb = g * 4 + jb4;
-        float v[64];
-        ptx::tmem_ld_wait();
+      float4 pair = make_float4(0.f, 0.f, 0.f, 0.f);         // statistics of the group's two blocks
 #pragma unroll
-        for (int e = 0; e < 32; ++e) { v[e] = __uint_as_float(nxt_lo[e]); v[32 + e] = __uint_as_float(nxt_hi[e]); }
-        if (jb4 < 3) {                                       // the next block's columns load while this block is reduced
-          ptx::tmem_ld_32x32b_x32(t_addr + (jb4 + 1) * 64, nxt_lo);
-          ptx::tmem_ld_32x32b_x32(t_addr + (jb4 + 1) * 64 + 32, nxt_hi);
-        }
-        if (jb > own) continue;                              // a key block after the query's own block: not causal, never read
+      for (int half = 0; half < 2; ++half) {
+        const int jb = g * 2 + half;
+        if (jb > row0 / 64 + (quarter >> 1)) continue;       // a key block after this warp's query block: not causal, never read
+        uint32_t lo[32], hi[32];
+        ptx::tmem_ld_32x32b_x32(t_addr + half * 64, lo);
+        ptx::tmem_ld_32x32b_x32(t_addr + half * 64 + 32, hi);
+        ptx::tmem_ld_wait();
+        auto v = [&](int e) { return __uint_as_float(e < 32 ? lo[e & 31] : hi[e & 31]); };
         float m, sum = 0.f;
         if (jb < own) {                                      // every key of the block is visible
-          float m0 = v[0], m1 = v[1], m2 = v[2], m3 = v[3];
+          float m0 = v(0), m1 = v(1), m2 = v(2), m3 = v(3);
 #pragma unroll
-          for (int e = 4; e < 64; e += 4) { m0 = fmaxf(m0, v[e]); m1 = fmaxf(m1, v[e + 1]); m2 = fmaxf(m2, v[e + 2]); m3 = fmaxf(m3, v[e + 3]); }
+          for (int e = 4; e < 64; e += 4) { m0 = fmaxf(m0, v(e)); m1 = fmaxf(m1, v(e + 1)); m2 = fmaxf(m2, v(e + 2)); m3 = fmaxf(m3, v(e + 3)); }
           m = fmaxf(fmaxf(m0, m1), fmaxf(m2, m3));
           const float mc = m * c;
           float s0 = 0.f, s1 = 0.f, s2 = 0.f, s3 = 0.f;
 #pragma unroll
           for (int e = 0; e < 64; e += 4) {
-            s0 += fast_exp2(v[e] * c - mc); s1 += fast_exp2(v[e + 1] * c - mc); s2 += fast_exp2(v[e + 2] * c - mc); s3 += fast_exp2(v[e + 3] * c - mc);
+            s0 += fast_exp2(v(e) * c - mc); s1 += fast_exp2(v(e + 1) * c - mc); s2 += fast_exp2(v(e + 2) * c - mc); s3 += fast_exp2(v(e + 3) * c - mc);
           }
           sum = (s0 + s1) + (s2 + s3);
         } else {                                             // the diagonal block: keys up to the query's own position
           m = -INFINITY;
 #pragma unroll
-          for (int e = 0; e < 64; ++e) if (e <= tin) m = fmaxf(m, v[e]);
+          for (int e = 0; e < 64; ++e) if (e <= tin) m = fmaxf(m, v(e));
           const float mc = m * c;
 #pragma unroll
-          for (int e = 0; e < 64; ++e) if (e <= tin) sum += fast_exp2(v[e] * c - mc);
+          for (int e = 0; e < 64; ++e) if (e <= tin) sum += fast_exp2(v(e) * c - mc);
         }
-        out_row[jb] = make_float2(m * p.scale, sum);
+        if (half == 0) { pair.x = m * p.scale; pair.y = sum; } else { pair.z = m * p.scale; pair.w = sum; }
       }
+      *reinterpret_cast<float4*>(out_row + g * 2) = pair;    // S / 64 is even: 16-byte aligned; entries past the own block are never read
       ptx::tc_fence_before();
       __syncwarp();
       if (lane == 0) ptx::mbar_arrive(&acc_empty[acc]);
@@ -156,7 +154,7 @@ __global__ void __launch_bounds__(QT_THREADS) qsa_block_stats_tc_kernel(const __
   }
   ptx::tc_fence_before();
   __syncthreads();
-  if (warp == 1) ptx::tmem_dealloc(tmem_base, 512);
+  if (warp == 1) ptx::tmem_dealloc(tmem_base, 2 * QT_KEYS);
 }
 
 // q [B, nq, S, 64], k [B, nkv, S, 64] bf16 contiguous, S a multiple of 128 -> stats [B, nq, S, S / 64] float2 (as a [.., 2] fp32 tensor).
