@@ -117,7 +117,7 @@ TORCH_LIBRARY(q38, m) {
   m.def("conv_silu_bwd(Tensor x, Tensor w, Tensor dy) -> Tensor[]");
   m.def("gdn_prep_fwd(Tensor q, Tensor k, Tensor v, Tensor g, Tensor beta) -> Tensor[]");
   m.def("gdn_prep_bwd(Tensor q, Tensor k, Tensor v, Tensor g, Tensor beta, Tensor Tm, Tensor dw, Tensor du, Tensor dP, Tensor dqg, Tensor dkg, Tensor dd) -> Tensor[]");
-  m.def("gdn_scan_fwd(Tensor w, Tensor u, Tensor P, Tensor qg, Tensor kg, Tensor dch, int B, int H) -> Tensor[]");
+  m.def("gdn_scan_fwd(Tensor w, Tensor u, Tensor P, Tensor qg, Tensor kg, Tensor dch, int B, int H, Tensor? err=None, bool save=True) -> Tensor[]");
   m.def("gdn_scan_bwd(Tensor w, Tensor P, Tensor qg, Tensor kg, Tensor dch, Tensor vnew, Tensor states, Tensor dout, int B, int H) -> Tensor[]");
   m.def("moe_route_fwd(Tensor logits, int k) -> Tensor[]");
   m.def("moe_route_bwd(Tensor probs, Tensor top_idx, Tensor top_w, Tensor d_top_w, Tensor? d_prob_sum) -> Tensor");

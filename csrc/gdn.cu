@@ -9,85 +9,144 @@
 // with q, k L2-normalised and q scaled by 64^-1/2.
 //
 // Kernels
-//   gdn_scan_fwd   one CTA per (batch, value head): the sequential pass over chunks.  The fp32 state lives in the
-//                  accumulator registers of eight warps (16 k-rows x 32 v-columns each); every product is a 64x64x64
-//                  bf16 mma.sync with fp32 accumulation; chunk operands are prefetched with cp.async one chunk ahead.
-//                  The chain per chunk is latency bound (three dependent products), which is why this pass uses
+//   gdn_scan_fwd   the sequential pass over chunks, one chain of warps per 16 value columns of a (batch, value head) pair (gdn_tile.cuh).
+//                  The fp32 state lives in the warp's accumulator registers; the operand tiles come by TMA, several chunks ahead.
+//                  The chain per chunk is latency bound (two dependent products), which is why this pass uses
 //                  register-resident warp MMAs instead of the TMEM round trips of tcgen05.
 //   gdn_scan_bwd   the reverse pass: dS' -> (dw, du, dP, dqg, dkg, dd) per chunk and dS.
-#include <torch/extension.h>
+#include <ATen/ATen.h>
 #include <ATen/cuda/CUDAContext.h>
 #include <c10/cuda/CUDAGuard.h>
 
 #include "common.cuh"
 #include "host.h"
+#include "gdn_tile.cuh"
 #include "mma_tile.cuh"
 
 namespace q38 {
 
 // ---------------------------------------------------------------------------------------------------------------------
 // Forward scan.  Chunk operands w,u,P,qg,kg: [BH, NT, 64, 64] bf16; dch: [BH, NT] fp32.
-// Outputs: o [B, S, H, 64] bf16 (token-major), vnew [BH, NT, 64, 64] bf16, states [BH, NT, 64, 64] bf16 (chunk-start S).
+// Outputs: o [B, S, H, 64] bf16 (token-major) and, when the backward pass will want them, vnew [BH, NT, 64, 64] bf16 and
+// states [BH, NT, 64, 64] bf16 (chunk-start S).
+//
+// Roles: warps 0..W-1 carry the chain (v_new and the new state, two products per chunk), warps W..2W-1 turn the packed state and v_new
+// that a chain warp leaves in shared memory into o and do all stores (two products), two more warps keep the operand tiles coming.
+// One warp alone on its scheduler can neither hide its own latencies nor overlap its halves, and the chain is what the pass waits for (some 600
+// instructions per 16 columns and chunk, six cycles each; neither memory nor the MMA rate).  84 pairs of 64 chunks: 112 us, 81 without the
+// tensors saved for the backward; 142 us with one warp for both roles, 160 us with eight warps per product and three block barriers per
+// chunk.  39 pairs of 128 chunks (one prompt of 8192): 123 us, before 320.
 // ---------------------------------------------------------------------------------------------------------------------
-__global__ void __launch_bounds__(256) gdn_scan_fwd_kernel(const bf16* __restrict__ w, const bf16* __restrict__ u, const bf16* __restrict__ P,
-                                                           const bf16* __restrict__ qg, const bf16* __restrict__ kg, const float* __restrict__ dch,
-                                                           bf16* __restrict__ o, bf16* __restrict__ vnew, bf16* __restrict__ states, int NT, int H) {
-  extern __shared__ __align__(16) uint8_t smem_bytes[];
-  bf16* sm = reinterpret_cast<bf16*>(smem_bytes);
-  // two buffers of five operand tiles, then the bf16 copies of S and v_new
-  bf16* Sb = sm + 10 * TILE_ELEMS;
-  bf16* Vn = Sb + TILE_ELEMS;
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+constexpr int SCAN_U = 4;                                                // slices of u in flight per chain warp
+template <int W> struct ScanSmem {
+  static constexpr int XCHG = 2 * 4096;                                  // two slots of {S, v_new} fragments
+  static constexpr int PAIR = SCAN_U * gdn::SLICE_BYTES + XCHG + gdn::SLICE_BYTES;
+  static constexpr int TILES = (gdn::CHAIN_STAGES + gdn::SIDE_STAGES) * 2 * gdn::TILE_BYTES;
+  static constexpr int BARS = 2 * gdn::CHAIN_STAGES + 2 * gdn::SIDE_STAGES + 4 * W;
+  static constexpr int BYTES = TILES + W * PAIR + BARS * 8;
+};
+
+template <int W>
+__global__ void __launch_bounds__(64 * W + 64) gdn_scan_fwd_kernel(const __grid_constant__ gdn::Maps4 maps, const bf16* __restrict__ u, const float* __restrict__ dch,
+                                                                   bf16* __restrict__ o, bf16* __restrict__ vnew, bf16* __restrict__ states, int NT, int H,
+                                                                   int* __restrict__ err) {
+  using namespace gdn;
+  using L = ScanSmem<W>;
+  extern __shared__ __align__(1024) uint8_t scan_smem[];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int bh = blockIdx.x, b = bh / H, hv = bh % H;
-  const long long tile = 64 * 64;
-  const bf16* srcs[5] = {w + (long long)bh * NT * tile, u + (long long)bh * NT * tile, P + (long long)bh * NT * tile,
-                         qg + (long long)bh * NT * tile, kg + (long long)bh * NT * tile};
-  auto prefetch = [&](int c, int buf) {
-#pragma unroll
-    for (int t = 0; t < 5; ++t) load_tile_async_256(sm + (buf * 5 + t) * TILE_ELEMS, srcs[t] + (long long)c * tile, 64, tid);
-    cp_async_commit();
-  };
-  // eight warps: warp w keeps rows 16 (w & 3).. and v-columns 32 (w >> 2).. of the fp32 state in registers
-  float S[4][4];
-  zero_acc(S);
-  prefetch(0, 0);
-  for (int c = 0; c < NT; ++c) {
-    const int buf = c & 1;
-    if (c + 1 < NT) { prefetch(c + 1, buf ^ 1); cp_async_wait<1>(); } else { cp_async_wait<0>(); }
-    acc_to_smem_h(S, Sb, warp, lane);
-    acc_to_global_h(S, states + ((long long)bh * NT + c) * tile, 64, warp, lane);
-    __syncthreads();                                   // operand tiles of chunk c and Sb are visible
-    const bf16* Wt = sm + (buf * 5 + 0) * TILE_ELEMS;
-    const bf16* Ut = Wt + TILE_ELEMS;
-    const bf16* Pt = Ut + TILE_ELEMS;
-    const bf16* Qt = Pt + TILE_ELEMS;
-    const bf16* Kt = Qt + TILE_ELEMS;
-    float acc[4][4];
-    zero_acc(acc);
-    mma64h<false, false>(Wt, Sb, acc, warp, lane);     // w S
-    {
-      const int r = 16 * (warp & 3) + (lane >> 2), c0 = 32 * (warp >> 2) + 2 * (lane & 3);
-#pragma unroll
-      for (int nt = 0; nt < 4; ++nt) {
-        const __nv_bfloat162 u0 = *reinterpret_cast<const __nv_bfloat162*>(Ut + r * LDS + 8 * nt + c0);
-        const __nv_bfloat162 u1 = *reinterpret_cast<const __nv_bfloat162*>(Ut + (r + 8) * LDS + 8 * nt + c0);
-        acc[nt][0] = __low2float(u0) - acc[nt][0]; acc[nt][1] = __high2float(u0) - acc[nt][1];
-        acc[nt][2] = __low2float(u1) - acc[nt][2]; acc[nt][3] = __high2float(u1) - acc[nt][3];
-      }
+  uint64_t* bars = reinterpret_cast<uint64_t*>(scan_smem + L::TILES + W * L::PAIR);
+  const Ring<CHAIN_STAGES> chain{scan_smem, bars, bars + CHAIN_STAGES};
+  const Ring<SIDE_STAGES> side{scan_smem + CHAIN_STAGES * 2 * TILE_BYTES, bars + 2 * CHAIN_STAGES, bars + 2 * CHAIN_STAGES + SIDE_STAGES};
+  uint64_t* xbars = bars + 2 * CHAIN_STAGES + 2 * SIDE_STAGES;           // per pair: two full, two empty
+  if (threadIdx.x == 0) {
+    chain.init(W);
+    side.init(W);
+    for (int i = 0; i < 4 * W; ++i) ptx::mbar_init(&xbars[i], 1);
+    ptx::fence_barrier_init();
+  }
+  __syncthreads();
+  if (warp >= 2 * W) {
+    if (lane == 0) {
+      const bool ok = warp == 2 * W ? chain.produce(&maps.m[0], &maps.m[1], bh * NT, NT, 1) : side.produce(&maps.m[2], &maps.m[3], bh * NT, NT, 1);
+      if (!ok) report_error(err, ERR_MMA_WAIT);
     }
-    acc_to_smem_h(acc, Vn, warp, lane);                // v_new (bf16) for the two products below
-    acc_to_global_h(acc, vnew + ((long long)bh * NT + c) * tile, 64, warp, lane);
-    float out[4][4];
-    zero_acc(out);
-    mma64h<false, false>(Qt, Sb, out, warp, lane);     // qg S
-    __syncthreads();                                   // Vn complete
-    mma64h<false, false>(Pt, Vn, out, warp, lane);     // + P v_new
-    acc_to_global_h(out, o + (((long long)b * NT * 64 + (long long)c * 64) * H + hv) * 64, (long long)H * 64, warp, lane);
-    const float d = dch[(long long)bh * NT + c];
+    return;
+  }
+  const int pair = warp % W, col = 16 * (blockIdx.y * W + pair);
+  const uint32_t slices = ptx::smem_u32(scan_smem) + L::TILES + pair * L::PAIR, xchg = slices + SCAN_U * SLICE_BYTES, out_slice = xchg + L::XCHG;
+  uint64_t *xfull = xbars + 4 * pair, *xempty = xfull + 2;
+  const long long base = (long long)bh * NT * 4096;
+  if (warp < W) {
+    for (int c = 0; c < SCAN_U - 1; ++c) {
+      if (c < NT) slice_load_async(slices + c * SLICE_BYTES, u + base + (long long)c * 4096 + col, 64, lane);
+      cp_async_commit();
+    }
+    float S[8][4];
+    zero_acc(S);
+    float d_next = dch[(long long)bh * NT];
+    for (int c = 0; c < NT; ++c) {
+      if (c + SCAN_U - 1 < NT) slice_load_async(slices + ((c + SCAN_U - 1) % SCAN_U) * SLICE_BYTES, u + base + (long long)(c + SCAN_U - 1) * 4096 + col, 64, lane);
+      cp_async_commit();
+      const float d = d_next;
+      d_next = dch[(long long)bh * NT + (c + 1 < NT ? c + 1 : c)];
+      uint32_t aS[4][4], av[4][4];
+      float acc[8][4];
+      pack_a<4>(S, aS);
+      bool ok = c < 2 || ptx::mbar_wait(&xempty[c & 1], ((c >> 1) & 1) ^ 1);
+      frags_put(xchg + (c & 1) * 4096, aS, lane);
+      cp_async_wait<SCAN_U - 1>();
+      __syncwarp();
+      slice_read_t(slices + (c % SCAN_U) * SLICE_BYTES, av, lane);       // u^T
+      ok = ptx::mbar_wait(chain.full + c % CHAIN_STAGES, (c / CHAIN_STAGES) & 1) && ok;
+      if (!__all_sync(0xffffffffu, ok)) { if (lane == 0) report_error(err, ERR_TMA_WAIT); break; }
+      const uint32_t wt = chain.tile(c), kt = wt + TILE_BYTES;
+      zero_acc(acc);
+      mma64<false>(aS, wt, acc, lane);                                   // (w S)^T
 #pragma unroll
-    for (int nt = 0; nt < 4; ++nt) { S[nt][0] *= d; S[nt][1] *= d; S[nt][2] *= d; S[nt][3] *= d; }
-    mma64h<true, false>(Kt, Vn, S, warp, lane);        // + kg^T v_new
-    __syncthreads();                                   // everyone is done with Sb, Vn and this buffer
+      for (int ks = 0; ks < 4; ++ks) {
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          float* x = &acc[2 * ks + (e >> 1)][2 * (e & 1)];
+          x[0] = lo_f(av[ks][e]) - x[0];
+          x[1] = hi_f(av[ks][e]) - x[1];
+        }
+      }
+      pack_a<4>(acc, av);                                                // v_new^T
+      frags_put(xchg + (c & 1) * 4096 + 2048, av, lane);
+      __syncwarp();
+      if (lane == 0) ptx::mbar_arrive(&xfull[c & 1]);
+#pragma unroll
+      for (int nt = 0; nt < 8; ++nt) { S[nt][0] *= d; S[nt][1] *= d; S[nt][2] *= d; S[nt][3] *= d; }
+      mma64<true>(av, kt, S, lane);                                      // + (kg^T v_new)^T
+      __syncwarp();
+      if (lane == 0) ptx::mbar_arrive(chain.empty + c % CHAIN_STAGES);
+    }
+    cp_async_wait<0>();
+  } else {
+    for (int c = 0; c < NT; ++c) {
+      bool ok = ptx::mbar_wait(&xfull[c & 1], (c >> 1) & 1);
+      ok = ptx::mbar_wait(side.full + c % SIDE_STAGES, (c / SIDE_STAGES) & 1) && ok;
+      if (!__all_sync(0xffffffffu, ok)) { if (lane == 0) report_error(err, ERR_TMA_WAIT); break; }
+      uint32_t aS[4][4], av[4][4];
+      float acc[8][4];
+      frags_get(xchg + (c & 1) * 4096, aS, lane);
+      frags_get(xchg + (c & 1) * 4096 + 2048, av, lane);
+      __syncwarp();
+      if (lane == 0) ptx::mbar_arrive(&xempty[c & 1]);
+      const uint32_t qt = side.tile(c), pt = qt + TILE_BYTES;
+      zero_acc(acc);
+      mma64<false>(aS, qt, acc, lane);                                   // (qg S)^T
+      mma64<false>(av, pt, acc, lane);                                   // + (P v_new)^T
+      __syncwarp();
+      if (lane == 0) ptx::mbar_arrive(side.empty + c % SIDE_STAGES);
+      if (states != nullptr) {
+        slice_store_t(out_slice, aS, states + base + (long long)c * 4096 + col, 64, lane);
+        slice_store_t(out_slice, av, vnew + base + (long long)c * 4096 + col, 64, lane);
+      }
+      pack_a<4>(acc, aS);
+      slice_store_t(out_slice, aS, o + (((long long)b * NT * 64 + (long long)c * 64) * H + hv) * 64 + col, (long long)H * 64, lane);
+    }
   }
 }
 
@@ -198,21 +257,39 @@ static void check_tiles(const at::Tensor& t, int64_t BH, int64_t NT, const char*
   TORCH_CHECK(t.is_cuda() && t.scalar_type() == at::kBFloat16 && t.is_contiguous() && t.numel() == BH * NT * 64 * 64, name, ": contiguous bf16 [BH,NT,64,64] required");
 }
 
-// Returns {o [B,S,H,64], vnew [BH,NT,64,64], states [BH,NT,64,64]}
+static gdn::Maps4 tile_maps(const at::Tensor& a, const at::Tensor& b, const at::Tensor& c, const at::Tensor& d) {
+  const at::Tensor* t[4] = {&a, &b, &c, &d};
+  gdn::Maps4 maps;
+  for (int i = 0; i < 4; ++i) maps.m[i] = make_tmap_box(t[i]->data_ptr(), 2, 64, t[i]->numel() / 64, 1, 64, 0, 64, 128);
+  return maps;
+}
+
+// Returns {o [B,S,H,64], vnew [BH,NT,64,64], states [BH,NT,64,64]}; without `save` (no backward pass will follow) the last two are empty.
 std::vector<at::Tensor> gdn_scan_fwd(const at::Tensor& w, const at::Tensor& u, const at::Tensor& P, const at::Tensor& qg, const at::Tensor& kg,
-                                     const at::Tensor& dch, int64_t B, int64_t H) {
+                                     const at::Tensor& dch, int64_t B, int64_t H, const c10::optional<at::Tensor>& err, bool save) {
   const c10::cuda::CUDAGuard guard(w.device());
   const int64_t BH = B * H, NT = w.numel() / (BH * 64 * 64);
   check_tiles(w, BH, NT, "w"); check_tiles(u, BH, NT, "u"); check_tiles(P, BH, NT, "P"); check_tiles(qg, BH, NT, "qg"); check_tiles(kg, BH, NT, "kg");
   TORCH_CHECK(dch.scalar_type() == at::kFloat && dch.is_contiguous() && dch.numel() == BH * NT, "gdn_scan_fwd: dch must be fp32 [BH,NT]");
   auto o = at::empty({B, NT * 64, H, 64}, w.options());
-  auto vnew = at::empty({BH, NT, 64, 64}, w.options()), states = at::empty({BH, NT, 64, 64}, w.options());
-  const int smem = 12 * TILE_ELEMS * 2;
-  static bool configured = false;
-  if (!configured) { C10_CUDA_CHECK(cudaFuncSetAttribute(gdn_scan_fwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem)); configured = true; }
-  gdn_scan_fwd_kernel<<<(int)BH, 256, smem, at::cuda::getCurrentCUDAStream()>>>(
-      (const bf16*)w.data_ptr(), (const bf16*)u.data_ptr(), (const bf16*)P.data_ptr(), (const bf16*)qg.data_ptr(), (const bf16*)kg.data_ptr(),
-      dch.data_ptr<float>(), (bf16*)o.data_ptr(), (bf16*)vnew.data_ptr(), (bf16*)states.data_ptr(), (int)NT, (int)H);
+  const std::vector<int64_t> kept = save ? std::vector<int64_t>{BH, NT, 64, 64} : std::vector<int64_t>{0};
+  auto vnew = at::empty(kept, w.options()), states = at::empty(kept, w.options());
+  if (NT == 0 || BH == 0) return {o, vnew, states};
+  const auto maps = tile_maps(w, kg, qg, P);
+  auto launch = [&](auto warps) {
+    constexpr int W = decltype(warps)::value;
+    constexpr int smem = ScanSmem<W>::BYTES;
+    static bool configured = false;
+    if (!configured) { C10_CUDA_CHECK(cudaFuncSetAttribute(gdn_scan_fwd_kernel<W>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem)); configured = true; }
+    gdn_scan_fwd_kernel<W><<<dim3((int)BH, 4 / W), 64 * W + 64, smem, at::cuda::getCurrentCUDAStream()>>>(
+        maps, (const bf16*)u.data_ptr(), dch.data_ptr<float>(), (bf16*)o.data_ptr(), save ? (bf16*)vnew.data_ptr() : nullptr,
+        save ? (bf16*)states.data_ptr() : nullptr, (int)NT, (int)H, err.has_value() ? err->data_ptr<int>() : nullptr);
+  };
+  switch (gdn::scan_pairs(BH)) {
+    case 1: launch(std::integral_constant<int, 1>()); break;
+    case 2: launch(std::integral_constant<int, 2>()); break;
+    default: launch(std::integral_constant<int, 4>());
+  }
   C10_CUDA_KERNEL_LAUNCH_CHECK();
   count_launch();
   return {o, vnew, states};

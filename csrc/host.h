@@ -110,7 +110,7 @@ void moe_grouped_dswiglu_p(const at::Tensor& dy, const at::Tensor& w_down, const
 
 // gdn.cu
 std::vector<at::Tensor> gdn_scan_fwd(const at::Tensor& w, const at::Tensor& u, const at::Tensor& P, const at::Tensor& qg, const at::Tensor& kg,
-                                     const at::Tensor& dch, int64_t B, int64_t H);
+                                     const at::Tensor& dch, int64_t B, int64_t H, const c10::optional<at::Tensor>& err, bool save);
 std::vector<at::Tensor> gdn_scan_bwd(const at::Tensor& w, const at::Tensor& P, const at::Tensor& qg, const at::Tensor& kg, const at::Tensor& dch,
                                      const at::Tensor& vnew, const at::Tensor& states, const at::Tensor& dout, int64_t B, int64_t H);
 

@@ -357,7 +357,7 @@ class _GdnScan(torch.autograd.Function):
     def forward(ctx, w, u, P, qg, kg, carry, B, H):
         w, u, P, qg, kg = (t.to(torch.bfloat16).contiguous() for t in (w, u, P, qg, kg))
         carry = carry.float().contiguous()
-        o, vnew, states = load().gdn_scan_fwd(w, u, P, qg, kg, carry, B, H)
+        o, vnew, states = load().gdn_scan_fwd(w, u, P, qg, kg, carry, B, H, error_flag(w.device))
         ctx.save_for_backward(w, P, qg, kg, carry, vnew, states)
         ctx.dims = (B, H)
         return o
@@ -386,7 +386,8 @@ class _DeltaRule(torch.autograd.Function):
         v = qkv[..., 2 * Hk * 64:].unflatten(-1, (Hv, 64))
         g, beta = g.float().contiguous(), beta.to(torch.bfloat16).contiguous()
         w, u, P, qg, kg, Tm, carry, _gc = ops.gdn_prep_fwd(q, k, v, g, beta)
-        o, vnew, states = ops.gdn_scan_fwd(w, u, P, qg, kg, carry, B, Hv)
+        # without a backward pass neither the chunk states nor v_new are written
+        o, vnew, states = ops.gdn_scan_fwd(w, u, P, qg, kg, carry, B, Hv, error_flag(qkv.device), any(ctx.needs_input_grad))
         ctx.save_for_backward(qkv, g, beta, Tm, w, P, qg, kg, carry, vnew, states)
         ctx.heads = (Hk, Hv)
         return o
