@@ -116,7 +116,8 @@ TORCH_LIBRARY(q38, m) {
   m.def("conv_silu_fwd(Tensor x, Tensor w) -> Tensor");
   m.def("conv_silu_bwd(Tensor x, Tensor w, Tensor dy) -> Tensor[]");
   m.def("gdn_prep_fwd(Tensor q, Tensor k, Tensor v, Tensor g, Tensor beta) -> Tensor[]");
-  m.def("gdn_prep_bwd(Tensor q, Tensor k, Tensor v, Tensor g, Tensor beta, Tensor Tm, Tensor dw, Tensor du, Tensor dP, Tensor dqg, Tensor dkg, Tensor dd) -> Tensor[]");
+  m.def("gdn_prep_bwd(Tensor q, Tensor k, Tensor v, Tensor g, Tensor beta, Tensor Tm, Tensor w, Tensor u, Tensor vnew, Tensor states, Tensor dout, Tensor du, Tensor dstate, Tensor dd) -> Tensor[]");
+  m.def("gdn_chain_bwd(Tensor w, Tensor P, Tensor qg, Tensor kg, Tensor dch, Tensor states, Tensor dout, int B, int H, Tensor? err=None) -> Tensor[]");
   m.def("gdn_scan_fwd(Tensor w, Tensor u, Tensor P, Tensor qg, Tensor kg, Tensor dch, int B, int H, Tensor? err=None, bool save=True) -> Tensor[]");
   m.def("gdn_scan_bwd(Tensor w, Tensor P, Tensor qg, Tensor kg, Tensor dch, Tensor vnew, Tensor states, Tensor dout, int B, int H) -> Tensor[]");
   m.def("moe_route_fwd(Tensor logits, int k) -> Tensor[]");
@@ -164,6 +165,7 @@ TORCH_LIBRARY_IMPL(q38, CUDA, m) {
   m.impl("conv_silu_bwd", &q38::conv_silu_bwd);
   m.impl("gdn_prep_fwd", &q38::gdn_prep_fwd);
   m.impl("gdn_prep_bwd", &q38::gdn_prep_bwd);
+  m.impl("gdn_chain_bwd", &q38::gdn_chain_bwd);
   m.impl("gdn_scan_fwd", &q38::gdn_scan_fwd);
   m.impl("gdn_scan_bwd", &q38::gdn_scan_bwd);
   m.impl("moe_route_fwd", &q38::moe_route_fwd);

@@ -497,251 +497,306 @@ __global__ void __launch_bounds__(128) gdn_prep_fwd_kernel(const bf16* __restric
   acc_to_global(acc, u_out + tile_off, 64, warp, lane);
 }
 
-// Row sums of a fragment-distributed 64x64 quantity into a shared [64] array (all four warps contribute distinct rows).
-__device__ __forceinline__ void frag_row_add(const float (&val)[8][4], float* __restrict__ dst, int warp, int lane, float sign = 1.f) {
-  float lo = 0.f, hi = 0.f;
-#pragma unroll
-  for (int nt = 0; nt < 8; ++nt) { lo += val[nt][0] + val[nt][1]; hi += val[nt][2] + val[nt][3]; }
-  lo += __shfl_xor_sync(0xffffffffu, lo, 1); lo += __shfl_xor_sync(0xffffffffu, lo, 2);
-  hi += __shfl_xor_sync(0xffffffffu, hi, 1); hi += __shfl_xor_sync(0xffffffffu, hi, 2);
-  if ((lane & 3) == 0) {
-    const int r = 16 * warp + (lane >> 2);
-    atomicAdd(&dst[r], sign * lo);
-    atomicAdd(&dst[r + 8], sign * hi);
-  }
-}
-// Column sums (over all 64 rows: across lanes of a warp, then across warps through shared atomics).
-__device__ __forceinline__ void frag_col_add(const float (&val)[8][4], float* __restrict__ dst, int lane, float sign = 1.f) {
-#pragma unroll
-  for (int nt = 0; nt < 8; ++nt) {
-    float c0 = val[nt][0] + val[nt][2], c1 = val[nt][1] + val[nt][3];
-#pragma unroll
-    for (int o = 4; o < 32; o <<= 1) { c0 += __shfl_xor_sync(0xffffffffu, c0, o); c1 += __shfl_xor_sync(0xffffffffu, c1, o); }
-    if ((lane >> 2) == 0) {
-      atomicAdd(&dst[8 * nt + 2 * (lane & 3)], sign * c0);
-      atomicAdd(&dst[8 * nt + 2 * (lane & 3) + 1], sign * c1);
-    }
-  }
-}
-// One CTA per (chunk, batch, key head); loops over the value heads that share the key head so dq/dk need no atomics.
-__global__ void __launch_bounds__(128) gdn_prep_bwd_kernel(const bf16* __restrict__ q, const bf16* __restrict__ k, const bf16* __restrict__ v,
-                                                           const float* __restrict__ g, const bf16* __restrict__ beta, const bf16* __restrict__ Tm_in,
-                                                           const bf16* __restrict__ dw, const bf16* __restrict__ du, const bf16* __restrict__ dP,
-                                                           const bf16* __restrict__ dqg, const bf16* __restrict__ dkg, const float* __restrict__ dd,
-                                                           bf16* __restrict__ dq, bf16* __restrict__ dk, bf16* __restrict__ dv,
-                                                           float* __restrict__ dg, float* __restrict__ dbeta, int S, int Hk, int Hv,
-                                                           long long qk_ld, long long v_ld, long long dqk_ld, long long dv_ld) {
+// Gradients of the chunk operands and of everything the preparation computed, chunk-parallel.  One CTA of eight warps per (chunk,
+// batch, key head), looping over the value heads that share the key head so dq/dk need no atomics.
+//
+// From the reverse scan (dv_new = du and the state gradient dS' at the chunk's end) it forms
+//     dw = -du S^T    dP = dO v_new^T    dqg = dO S^T    dkg = v_new dS'^T
+// and with A = Tm^T dw = d(beta e^gc k), B = Tm^T du = d(beta v) the gradient of the triangular system is dM = -(A w^T + B u^T),
+// because Tm (beta e^gc k) and Tm (beta v) are w and u themselves: two independent products instead of a chain of four.
+// The gate and beta gradients are sums over rows and columns of products such as dP_ij Gamma_ij (q_i.k_j); with H = dP Gamma they equal
+// q_i.(H K)_i and k_j.(H^T Q)_j, row dots of products that dq and dk need anyway, so k.k and q.k are not formed again and
+// every row sum stays in two registers per thread until the end of the head.  (The sums cancel pairwise between rows and columns as
+// before, since both sides read the same rounded H.)
+// Bound by the shared-memory round trips of its twelve dependent 64^3 products (70 % of that pipe); eight warps with half-width accumulators and
+// two CTAs per SM (at most 128 registers, 112 KB of tiles) hide part of them, and the next head's eight tiles load while this head's last
+// products run.  5376 chunks: 241 us; the kernel that took dw, dP, dqg, dkg from the scan, four warps and sixteen row or column sums, 337.
+__global__ void __launch_bounds__(256, 2) gdn_prep_bwd_kernel(const bf16* __restrict__ q, const bf16* __restrict__ k, const bf16* __restrict__ v,
+                                                              const float* __restrict__ g, const bf16* __restrict__ beta, const bf16* __restrict__ Tm_in,
+                                                              const bf16* __restrict__ w_in, const bf16* __restrict__ u_in, const bf16* __restrict__ vnew,
+                                                              const bf16* __restrict__ states, const bf16* __restrict__ dout, const bf16* __restrict__ du,
+                                                              const bf16* __restrict__ dstate, const float* __restrict__ dd,
+                                                              bf16* __restrict__ dq, bf16* __restrict__ dk, bf16* __restrict__ dv,
+                                                              float* __restrict__ dg, float* __restrict__ dbeta, int S, int Hk, int Hv,
+                                                              long long qk_ld, long long v_ld, long long dqk_ld, long long dv_ld) {
   extern __shared__ __align__(16) uint8_t smem_bytes[];
   bf16* sm = reinterpret_cast<bf16*>(smem_bytes);
-  PrepSmem s;
-  s.Qn = sm; s.Kn = sm + TILE_ELEMS; s.KBG = sm + 2 * TILE_ELEMS; s.VB = sm + 3 * TILE_ELEMS; s.Tm = sm + 4 * TILE_ELEMS;
-  bf16* dWs = sm + 5 * TILE_ELEMS;
-  bf16* dUs = sm + 6 * TILE_ELEMS;
-  bf16* T1 = sm + 7 * TILE_ELEMS;
-  bf16* T2 = sm + 8 * TILE_ELEMS;
-  float* fl = reinterpret_cast<float*>(sm + 9 * TILE_ELEMS);
-  s.gc = fl; s.beta = fl + 64; s.rq = fl + 128; s.rk = fl + 192;
-  float* dgc = fl + 256;      // [64]
-  float* dbt = fl + 320;      // [64]
-  float* dgl = fl + 384;      // [1] gradient of gc_last from kg and the carry
+  bf16 *Qn = sm, *Kn = sm + TILE_ELEMS, *St = sm + 2 * TILE_ELEMS, *Do = sm + 3 * TILE_ELEMS, *Vn = sm + 4 * TILE_ELEMS, *Ds = sm + 5 * TILE_ELEMS;
+  bf16 *Du = sm + 6 * TILE_ELEMS, *Tm = sm + 7 * TILE_ELEMS, *Wt = sm + 8 * TILE_ELEMS, *Ut = sm + 9 * TILE_ELEMS, *X1 = sm + 10 * TILE_ELEMS, *X2 = sm + 11 * TILE_ELEMS;
+  float* fl = reinterpret_cast<float*>(sm + 12 * TILE_ELEMS);
+  float *gc = fl, *bet = fl + 64, *eg = fl + 128, *el = fl + 192, *rqs = fl + 256, *rks = fl + 320;
+  float *redg = fl + 384, *redb = fl + 512;                  // [2 column halves][64 rows]
+  float* redk = fl + 640;                                    // [8 warps]
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int c = blockIdx.x, NT = gridDim.x, rep = Hv / Hk;
   const int b = blockIdx.y / Hk, hk = blockIdx.y % Hk;
   const long long tok0 = (long long)b * S + (long long)c * 64;
-  prep_load_qk(s, q + tok0 * qk_ld + hk * 64, k + tok0 * qk_ld + hk * 64, qk_ld, tid);
-  float dQn[8][4], dKn[8][4];
+  const int r0 = 16 * (warp & 3) + (lane >> 2), ch = warp >> 2, c0 = 32 * ch + 2 * (lane & 3);
+  auto load_head = [&](int hv) {
+    const long long off = ((long long)(b * Hv + hv) * NT + c) * 4096;
+    load_tile_async_256(St, states + off, 64, tid);
+    load_tile_async_256(Do, dout + (tok0 * Hv + hv) * 64, (long long)Hv * 64, tid);
+    load_tile_async_256(Vn, vnew + off, 64, tid);
+    load_tile_async_256(Ds, dstate + off, 64, tid);
+    load_tile_async_256(Du, du + off, 64, tid);
+    cp_async_commit();
+    load_tile_async_256(Tm, Tm_in + off, 64, tid);
+    load_tile_async_256(Wt, w_in + off, 64, tid);
+    load_tile_async_256(Ut, u_in + off, 64, tid);
+    cp_async_commit();
+  };
+  // gates of one head: two log decays per lane of warp 0, one beta per thread of warps 1 and 2
+  float g0 = 0.f, g1 = 0.f;
+  auto fetch_gates = [&](int hv) {
+    if (tid < 32) { g0 = g[(tok0 + 2 * tid) * Hv + hv]; g1 = g[(tok0 + 2 * tid + 1) * Hv + hv]; }
+    else if (tid < 96) g0 = __bfloat162float(beta[(tok0 + tid - 32) * Hv + hv]);
+  };
+  load_head(hk * rep);
+  fetch_gates(hk * rep);
+  {
+    // normalised q and k rows: four threads per token
+    const int tok = tid >> 2, part = tid & 3;
+    const long long src = (tok0 + tok) * qk_ld + hk * 64 + part * 16;
+    float qv[16], kv[16], sq = 0.f, sk = 0.f;
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      const uint4 rawq = reinterpret_cast<const uint4*>(q + src)[i], rawk = reinterpret_cast<const uint4*>(k + src)[i];
+      const uint32_t wq[4] = {rawq.x, rawq.y, rawq.z, rawq.w}, wk[4] = {rawk.x, rawk.y, rawk.z, rawk.w};
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        qv[8 * i + 2 * j] = lo_f(wq[j]); qv[8 * i + 2 * j + 1] = hi_f(wq[j]);
+        kv[8 * i + 2 * j] = lo_f(wk[j]); kv[8 * i + 2 * j + 1] = hi_f(wk[j]);
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < 16; ++i) { sq += qv[i] * qv[i]; sk += kv[i] * kv[i]; }
+    sq += __shfl_xor_sync(0xffffffffu, sq, 1); sq += __shfl_xor_sync(0xffffffffu, sq, 2);
+    sk += __shfl_xor_sync(0xffffffffu, sk, 1); sk += __shfl_xor_sync(0xffffffffu, sk, 2);
+    const float rq = rsqrtf(sq + 1e-6f), rk = rsqrtf(sk + 1e-6f);
+    if (part == 0) { rqs[tok] = rq; rks[tok] = rk; }
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      *reinterpret_cast<uint32_t*>(Qn + tok * LDS + part * 16 + 2 * i) = pack_f2(qv[2 * i] * (rq * 0.125f), qv[2 * i + 1] * (rq * 0.125f));
+      *reinterpret_cast<uint32_t*>(Kn + tok * LDS + part * 16 + 2 * i) = pack_f2(kv[2 * i] * rk, kv[2 * i + 1] * rk);
+    }
+  }
+  float dQn[4][4], dKn[4][4];
   zero_acc(dQn);
   zero_acc(dKn);
+  // row dot of a half-width accumulator with a tile, added to the two per-row registers
+  auto row_dot = [&](const float (&acc)[4][4], const bf16* tile, float& lo, float& hi) {
+    lo = hi = 0.f;
+#pragma unroll
+    for (int nt = 0; nt < 4; ++nt) {
+      const uint32_t x = *reinterpret_cast<const uint32_t*>(tile + r0 * LDS + 8 * nt + c0), y = *reinterpret_cast<const uint32_t*>(tile + (r0 + 8) * LDS + 8 * nt + c0);
+      lo += acc[nt][0] * lo_f(x) + acc[nt][1] * hi_f(x);
+      hi += acc[nt][2] * lo_f(y) + acc[nt][3] * hi_f(y);
+    }
+  };
+  auto add_rows = [&](float (&dst)[4][4], const float (&acc)[4][4], float slo, float shi) {
+#pragma unroll
+    for (int nt = 0; nt < 4; ++nt) { dst[nt][0] += slo * acc[nt][0]; dst[nt][1] += slo * acc[nt][1]; dst[nt][2] += shi * acc[nt][2]; dst[nt][3] += shi * acc[nt][3]; }
+  };
   for (int r = 0; r < rep; ++r) {
     const int hv = hk * rep + r, bh = b * Hv + hv;
-    const long long tile_off = ((long long)bh * NT + c) * 4096;
-    __syncthreads();                                        // previous head is done with every shared buffer
-    prep_load_gates(s, g + tok0 * Hv + hv, beta + tok0 * Hv + hv, Hv, tid);
-    if (tid < 64) { dgc[tid] = 0.f; dbt[tid] = 0.f; }
-    if (tid == 0) dgl[0] = 0.f;
-    load_tile_async(s.Tm, Tm_in + tile_off, 64, tid);
-    load_tile_async(dWs, dw + tile_off, 64, tid);
-    load_tile_async(dUs, du + tile_off, 64, tid);
-    cp_async_commit();
-    __syncthreads();
-    {
-      const int tok = tid >> 1, half = tid & 1;
-      const float gct = s.gc[tok], bt = s.beta[tok];
-      float row[32];
+    if (tid < 32) {
+      float run = g0 + g1;
 #pragma unroll
-      for (int i = 0; i < 16; ++i) {
-        const __nv_bfloat162 h = *reinterpret_cast<const __nv_bfloat162*>(s.Kn + tok * LDS + half * 32 + 2 * i);
-        row[2 * i] = __low2float(h); row[2 * i + 1] = __high2float(h);
+      for (int o = 1; o < 32; o <<= 1) { const float up = __shfl_up_sync(0xffffffffu, run, o); if (tid >= o) run += up; }
+      const float last = __shfl_sync(0xffffffffu, run, 31), first = run - g1;
+      gc[2 * tid] = first; gc[2 * tid + 1] = run;
+      eg[2 * tid] = __expf(first); eg[2 * tid + 1] = __expf(run);
+      el[2 * tid] = __expf(last - first); el[2 * tid + 1] = __expf(last - run);
+    } else if (tid < 96) {
+      bet[tid - 32] = g0;
+    }
+    uint32_t vv[4][2];                                       // this thread's fragment of v
+    const bf16* vsrc = v + tok0 * v_ld + hv * 64;
+#pragma unroll
+    for (int nt = 0; nt < 4; ++nt) {
+      vv[nt][0] = *reinterpret_cast<const uint32_t*>(vsrc + (long long)r0 * v_ld + 8 * nt + c0);
+      vv[nt][1] = *reinterpret_cast<const uint32_t*>(vsrc + (long long)(r0 + 8) * v_ld + 8 * nt + c0);
+    }
+    if (r + 1 < rep) fetch_gates(hv + 1);
+    cp_async_wait<1>();
+    __syncthreads();                                         // gates and the first five tiles (and, the first time, Qn and Kn)
+    const float glo = gc[r0], ghi = gc[r0 + 8], blo = bet[r0], bhi = bet[r0 + 8], elo = eg[r0], ehi = eg[r0 + 8];
+    float dglo = 0.f, dghi = 0.f, dblo = 0.f, dbhi = 0.f, ksum = 0.f, lo, hi;
+    float acc[4][4];
+    // ---- dw = -du S^T ----
+    zero_acc(acc);
+    mma64h<false, true>(Du, St, acc, warp, lane);
+#pragma unroll
+    for (int nt = 0; nt < 4; ++nt) { acc[nt][0] = -acc[nt][0]; acc[nt][1] = -acc[nt][1]; acc[nt][2] = -acc[nt][2]; acc[nt][3] = -acc[nt][3]; }
+    acc_to_smem_h(acc, X1, warp, lane);
+    // ---- H = dP Gamma on and below the diagonal, dP = dO v_new^T ----
+    zero_acc(acc);
+    mma64h<false, true>(Do, Vn, acc, warp, lane);
+#pragma unroll
+    for (int nt = 0; nt < 4; ++nt) {
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const int row = r0 + 8 * (e >> 1), cc = 8 * nt + c0 + (e & 1);
+        acc[nt][e] = cc <= row ? acc[nt][e] * __expf((e >> 1 ? ghi : glo) - gc[cc]) : 0.f;
       }
-      store_half_row_smem(s.KBG, tid, row, bt * __expf(gct));
-      load_half_row(v + tok0 * v_ld + hv * 64, v_ld, tid, row);
-      store_half_row_smem(s.VB, tid, row, bt);
+    }
+    acc_to_smem_h(acc, X2, warp, lane);
+    // ---- qg = qn e^gc ; dqg = dO S^T ----
+    zero_acc(acc);
+    mma64h<false, true>(Do, St, acc, warp, lane);
+    add_rows(dQn, acc, elo, ehi);
+    row_dot(acc, Qn, lo, hi);
+    dglo += lo * elo; dghi += hi * ehi;
+    // ---- kg = kn e^(gl - gc) ; dkg = v_new dS'^T ----
+    zero_acc(acc);
+    mma64h<false, true>(Vn, Ds, acc, warp, lane);
+    {
+      const float flo = el[r0], fhi = el[r0 + 8];
+      add_rows(dKn, acc, flo, fhi);
+      row_dot(acc, Kn, lo, hi);
+      lo *= flo; hi *= fhi;
+      dglo -= lo; dghi -= hi;
+      ksum = lo + hi;
     }
     cp_async_wait<0>();
-    __syncthreads();
-    const float gl = s.gc[63];
-    float acc[8][4], t[8][4];
-    // ---- d(KBG) = Tm^T dW: contributes to dk, dbeta, dgc ----
+    __syncthreads();                                         // X1, X2 complete, Tm / w / u landed; St, Do, Vn, Ds are free
+    // ---- A = Tm^T dw, the gradient of beta e^gc kn ----
     zero_acc(acc);
-    mma64<true, false>(s.Tm, dWs, acc, warp, lane);
-    frag_from_smem(s.Kn, t, warp, lane);
-    {
-      float tb[8][4], tg[8][4];
-      FRAG_LOOP(nt, e, row, col) {
-        const float E = __expf(s.gc[row]);
-        tb[nt][e] = acc[nt][e] * E * t[nt][e];                       // d beta_i
-        tg[nt][e] = tb[nt][e] * s.beta[row];                          // d gc_i  (= dKBG . kbg)
-        dKn[nt][e] += acc[nt][e] * s.beta[row] * E;
-      }
-      frag_row_add(tb, dbt, warp, lane);
-      frag_row_add(tg, dgc, warp, lane);
+    mma64h<true, false>(Tm, X1, acc, warp, lane);
+    acc_to_smem_h(acc, St, warp, lane);
+    add_rows(dKn, acc, blo * elo, bhi * ehi);
+    row_dot(acc, Kn, lo, hi);
+    lo *= elo; hi *= ehi;
+    dblo += lo; dbhi += hi;
+    dglo += lo * blo; dghi += hi * bhi;
+    // ---- B = Tm^T du, the gradient of beta v ----
+    zero_acc(acc);
+    mma64h<true, false>(Tm, Du, acc, warp, lane);
+    acc_to_smem_h(acc, Do, warp, lane);
+#pragma unroll
+    for (int nt = 0; nt < 4; ++nt) {
+      dblo += acc[nt][0] * lo_f(vv[nt][0]) + acc[nt][1] * hi_f(vv[nt][0]);
+      dbhi += acc[nt][2] * lo_f(vv[nt][1]) + acc[nt][3] * hi_f(vv[nt][1]);
+      acc[nt][0] *= blo; acc[nt][1] *= blo; acc[nt][2] *= bhi; acc[nt][3] *= bhi;
     }
-    // ---- d(VB) = Tm^T dU: dv and dbeta ----
+    acc_to_smem_h(acc, Vn, warp, lane);                      // dv, on its way to global memory
+    // ---- P: dqn += H Kn, dkn += H^T Qn ----
     zero_acc(acc);
-    mma64<true, false>(s.Tm, dUs, acc, warp, lane);
+    mma64h<false, false>(X2, Kn, acc, warp, lane);
+    add_rows(dQn, acc, 1.f, 1.f);
+    row_dot(acc, Qn, lo, hi);
+    dglo += lo; dghi += hi;
+    zero_acc(acc);
+    mma64h<true, false>(X2, Qn, acc, warp, lane);
+    add_rows(dKn, acc, 1.f, 1.f);
+    row_dot(acc, Kn, lo, hi);
+    dglo -= lo; dghi -= hi;
+    __syncthreads();                                         // A, B and dv complete; X1, X2 are free
     {
-      float tb[8][4];
-      const bf16* vsrc = v + tok0 * v_ld + hv * 64;
       bf16* dvdst = dv + tok0 * dv_ld + hv * 64;
-      const int r0 = 16 * warp + (lane >> 2), cq = 2 * (lane & 3);
 #pragma unroll
-      for (int nt = 0; nt < 8; ++nt) {
+      for (int i = 0; i < 2; ++i) {
+        const int chunk = tid + 256 * i, row = chunk >> 3, col = (chunk & 7) * 8;
+        *reinterpret_cast<uint4*>(dvdst + (long long)row * dv_ld + col) = *reinterpret_cast<const uint4*>(Vn + row * LDS + col);
+      }
+    }
+    // ---- dM = -(A w^T + B u^T); L_ij = beta_i (kn_i.kn_j) Gamma_ij (j < i) ----
+    // The tile holds beta_i dL_ij Gamma_ij; beta is floored so that a row with beta = 0 still yields its beta gradient by the division
+    // below (what the floor adds elsewhere is 1e-18 of dL).
+    const float flo = fmaxf(blo, 8.6736174e-19f), fhi = fmaxf(bhi, 8.6736174e-19f);
+    zero_acc(acc);
+    mma64h<false, true>(St, Wt, acc, warp, lane);
+    mma64h<false, true>(Do, Ut, acc, warp, lane);
 #pragma unroll
-        for (int hrow = 0; hrow < 2; ++hrow) {
-          const int row = r0 + 8 * hrow;
-          const __nv_bfloat162 vv = *reinterpret_cast<const __nv_bfloat162*>(vsrc + (long long)row * v_ld + 8 * nt + cq);
-          const float a0 = acc[nt][2 * hrow], a1 = acc[nt][2 * hrow + 1];
-          tb[nt][2 * hrow] = a0 * __low2float(vv);
-          tb[nt][2 * hrow + 1] = a1 * __high2float(vv);
-          *reinterpret_cast<__nv_bfloat162*>(dvdst + (long long)row * dv_ld + 8 * nt + cq) = __floats2bfloat162_rn(a0 * s.beta[row], a1 * s.beta[row]);
-        }
+    for (int nt = 0; nt < 4; ++nt) {
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const int row = r0 + 8 * (e >> 1), cc = 8 * nt + c0 + (e & 1);
+        acc[nt][e] = cc < row ? -acc[nt][e] * __expf((e >> 1 ? ghi : glo) - gc[cc]) * (e >> 1 ? fhi : flo) : 0.f;
       }
-      frag_row_add(tb, dbt, warp, lane);
     }
-    // ---- dTm = dW KBG^T + dU VB^T ;  dM = -Tm^T dTm Tm^T ----
+    acc_to_smem_h(acc, X1, warp, lane);
+    __syncthreads();                                         // X1 complete; every loaded tile is free
+    if (r + 1 < rep) load_head(hv + 1);
     zero_acc(acc);
-    mma64<false, true>(dWs, s.KBG, acc, warp, lane);
-    mma64<false, true>(dUs, s.VB, acc, warp, lane);
-    acc_to_smem(acc, T1, warp, lane);
-    __syncthreads();
+    mma64h<false, false>(X1, Kn, acc, warp, lane);           // dA1 Kn
+    add_rows(dKn, acc, 1.f, 1.f);
+    row_dot(acc, Kn, lo, hi);
+    dblo += lo / flo; dbhi += hi / fhi;
+    dglo += lo; dghi += hi;
     zero_acc(acc);
-    mma64<false, true>(T1, s.Tm, acc, warp, lane);           // dTm Tm^T
-    acc_to_smem(acc, T2, warp, lane);
-    __syncthreads();
-    zero_acc(acc);
-    mma64<true, false>(s.Tm, T2, acc, warp, lane);           // Tm^T (dTm Tm^T)  = -dM
-    // ---- L_ij = beta_i A1_ij Gamma_ij (j < i) ----
-    zero_acc(t);
-    mma64<false, true>(s.Kn, s.Kn, t, warp, lane);           // A1
-    {
-      float tb[8][4], tg[8][4], da[8][4];
-      FRAG_LOOP(nt, e, row, col) {
-        const bool low = col < row;
-        const float G = low ? -acc[nt][e] * __expf(s.gc[row] - s.gc[col]) : 0.f;      // dL_ij Gamma_ij
-        tb[nt][e] = G * t[nt][e];                                                    // d beta_i
-        tg[nt][e] = tb[nt][e] * s.beta[row];                                         // dL_ij L_ij
-        da[nt][e] = G * s.beta[row];                                                 // dA1_ij
-      }
-      frag_row_add(tb, dbt, warp, lane);
-      frag_row_add(tg, dgc, warp, lane);
-      frag_col_add(tg, dgc, lane, -1.f);
-      __syncthreads();                                        // T1 no longer read
-      acc_to_smem(da, T1, warp, lane);
+    mma64h<true, false>(X1, Kn, acc, warp, lane);            // dA1^T Kn
+    add_rows(dKn, acc, 1.f, 1.f);
+    row_dot(acc, Kn, lo, hi);
+    dglo -= lo; dghi -= hi;
+    // ---- gates out: dg = reverse cumsum of dgc (gc_last also collects kg's row sums and the carry term) ----
+    auto quad = [](float x) { x += __shfl_xor_sync(0xffffffffu, x, 1); return x + __shfl_xor_sync(0xffffffffu, x, 2); };
+    dglo = quad(dglo); dghi = quad(dghi); dblo = quad(dblo); dbhi = quad(dbhi);
+    ksum = warp_sum(ksum);
+    if ((lane & 3) == 0) {
+      redg[64 * ch + r0] = dglo; redg[64 * ch + r0 + 8] = dghi;
+      redb[64 * ch + r0] = dblo; redb[64 * ch + r0 + 8] = dbhi;
     }
+    if (lane == 0) redk[warp] = ksum;
     __syncthreads();
-    mma64<false, false>(T1, s.Kn, dKn, warp, lane);          // dA1 Kn
-    mma64<true, false>(T1, s.Kn, dKn, warp, lane);           // dA1^T Kn
-    // ---- P_ij = (q_i.k_j) Gamma_ij (j <= i) ----
-    zero_acc(t);
-    mma64<false, true>(s.Qn, s.Kn, t, warp, lane);
-    frag_from_global(dP + tile_off, acc, warp, lane);
-    {
-      float tg[8][4], hh[8][4];
-      FRAG_LOOP(nt, e, row, col) {
-        const float gam = col <= row ? __expf(s.gc[row] - s.gc[col]) : 0.f;
-        hh[nt][e] = acc[nt][e] * gam;                                                  // dP_ij Gamma_ij
-        tg[nt][e] = hh[nt][e] * t[nt][e];                                              // dP_ij P_ij
-      }
-      frag_row_add(tg, dgc, warp, lane);
-      frag_col_add(tg, dgc, lane, -1.f);
-      __syncthreads();                                        // T2 no longer read
-      acc_to_smem(hh, T2, warp, lane);
-    }
-    __syncthreads();
-    mma64<false, false>(T2, s.Kn, dQn, warp, lane);          // H Kn
-    mma64<true, false>(T2, s.Qn, dKn, warp, lane);           // H^T Qn
-    // ---- qg = qn e^gc ;  kg = kn e^(gl - gc) ;  carry = e^gl ----
-    frag_from_global(dqg + tile_off, acc, warp, lane);
-    frag_from_smem(s.Qn, t, warp, lane);
-    {
-      float tg[8][4];
-      FRAG_LOOP(nt, e, row, col) {
-        const float E = __expf(s.gc[row]);
-        tg[nt][e] = acc[nt][e] * t[nt][e] * E;
-        dQn[nt][e] += acc[nt][e] * E;
-      }
-      frag_row_add(tg, dgc, warp, lane);
-    }
-    frag_from_global(dkg + tile_off, acc, warp, lane);
-    frag_from_smem(s.Kn, t, warp, lane);
-    {
-      float tg[8][4];
-      float total = 0.f;
-      FRAG_LOOP(nt, e, row, col) {
-        const float E = __expf(gl - s.gc[row]);
-        tg[nt][e] = acc[nt][e] * t[nt][e] * E;
-        total += tg[nt][e];
-        dKn[nt][e] += acc[nt][e] * E;
-      }
-      frag_row_add(tg, dgc, warp, lane, -1.f);
-      total = warp_sum(total);
-      if (lane == 0) atomicAdd(dgl, total);
-    }
-    __syncthreads();
-    // ---- gates out: dg = reverse cumsum of dgc (gc_last also collects dgl and the carry term) ----
     if (tid < 32) {
-      float d0 = dgc[2 * tid], d1 = dgc[2 * tid + 1];
-      if (tid == 31) d1 += dgl[0] + dd[(long long)bh * NT + c] * __expf(gl);
+      float d0 = redg[2 * tid] + redg[64 + 2 * tid], d1 = redg[2 * tid + 1] + redg[65 + 2 * tid];
+      const float4 p = reinterpret_cast<const float4*>(dd)[(long long)bh * NT + c];
+      if (tid == 31) {
+        float gl = ((p.x + p.y) + (p.z + p.w)) * eg[63];
+        for (int i = 0; i < 8; ++i) gl += redk[i];
+        d1 += gl;
+      }
       float run = d0 + d1;
 #pragma unroll
       for (int o = 1; o < 32; o <<= 1) { const float dn = __shfl_down_sync(0xffffffffu, run, o); if (tid + o < 32) run += dn; }
       dg[(tok0 + 2 * tid) * Hv + hv] = run;
       dg[(tok0 + 2 * tid + 1) * Hv + hv] = run - d0;
     } else if (tid < 96) {
-      dbeta[(tok0 + tid - 32) * Hv + hv] = dbt[tid - 32];
+      dbeta[(tok0 + tid - 32) * Hv + hv] = redb[tid - 32] + redb[32 + tid];
     }
+    __syncthreads();                                         // the gate arrays may be replaced
   }
   // ---- L2-norm backward: qn = 0.125 rq q, kn = rk k ----
   {
-    const bf16* qsrc = q + tok0 * qk_ld + hk * 64;
-    const bf16* ksrc = k + tok0 * qk_ld + hk * 64;
-    bf16* dqdst = dq + tok0 * dqk_ld + hk * 64;
-    bf16* dkdst = dk + tok0 * dqk_ld + hk * 64;
-    const long long ld = qk_ld, dld = dqk_ld;
-    const int r0 = 16 * warp + (lane >> 2), cq = 2 * (lane & 3);
+    float qh[4][4], kh[4][4], dotq[2] = {0.f, 0.f}, dotk[2] = {0.f, 0.f};
 #pragma unroll
-    for (int hrow = 0; hrow < 2; ++hrow) {
-      const int row = r0 + 8 * hrow;
-      const float rq = s.rq[row], rk = s.rk[row];
-      float qh[16], kh[16], dotq = 0.f, dotk = 0.f;
+    for (int half = 0; half < 2; ++half) {
+      const int row = r0 + 8 * half;
+      const long long src = (tok0 + row) * qk_ld + hk * 64 + c0;
+      const float rq = rqs[row], rk = rks[row];
 #pragma unroll
-      for (int nt = 0; nt < 8; ++nt) {
-        const __nv_bfloat162 qq = *reinterpret_cast<const __nv_bfloat162*>(qsrc + row * ld + 8 * nt + cq);
-        const __nv_bfloat162 kk = *reinterpret_cast<const __nv_bfloat162*>(ksrc + row * ld + 8 * nt + cq);
-        qh[2 * nt] = __low2float(qq) * rq; qh[2 * nt + 1] = __high2float(qq) * rq;
-        kh[2 * nt] = __low2float(kk) * rk; kh[2 * nt + 1] = __high2float(kk) * rk;
-        dotq += 0.125f * (dQn[nt][2 * hrow] * qh[2 * nt] + dQn[nt][2 * hrow + 1] * qh[2 * nt + 1]);
-        dotk += dKn[nt][2 * hrow] * kh[2 * nt] + dKn[nt][2 * hrow + 1] * kh[2 * nt + 1];
+      for (int nt = 0; nt < 4; ++nt) {
+        const uint32_t qq = *reinterpret_cast<const uint32_t*>(q + src + 8 * nt), kk = *reinterpret_cast<const uint32_t*>(k + src + 8 * nt);
+        qh[nt][2 * half] = lo_f(qq) * rq; qh[nt][2 * half + 1] = hi_f(qq) * rq;
+        kh[nt][2 * half] = lo_f(kk) * rk; kh[nt][2 * half + 1] = hi_f(kk) * rk;
+        dotq[half] += 0.125f * (dQn[nt][2 * half] * qh[nt][2 * half] + dQn[nt][2 * half + 1] * qh[nt][2 * half + 1]);
+        dotk[half] += dKn[nt][2 * half] * kh[nt][2 * half] + dKn[nt][2 * half + 1] * kh[nt][2 * half + 1];
       }
-      dotq += __shfl_xor_sync(0xffffffffu, dotq, 1); dotq += __shfl_xor_sync(0xffffffffu, dotq, 2);
-      dotk += __shfl_xor_sync(0xffffffffu, dotk, 1); dotk += __shfl_xor_sync(0xffffffffu, dotk, 2);
+      dotq[half] += __shfl_xor_sync(0xffffffffu, dotq[half], 1); dotq[half] += __shfl_xor_sync(0xffffffffu, dotq[half], 2);
+      dotk[half] += __shfl_xor_sync(0xffffffffu, dotk[half], 1); dotk[half] += __shfl_xor_sync(0xffffffffu, dotk[half], 2);
+      if ((lane & 3) == 0) { redg[64 * ch + row] = dotq[half]; redb[64 * ch + row] = dotk[half]; }
+    }
+    __syncthreads();
 #pragma unroll
-      for (int nt = 0; nt < 8; ++nt) {
-        *reinterpret_cast<__nv_bfloat162*>(dqdst + row * dld + 8 * nt + cq) =
-            __floats2bfloat162_rn(rq * (0.125f * dQn[nt][2 * hrow] - qh[2 * nt] * dotq), rq * (0.125f * dQn[nt][2 * hrow + 1] - qh[2 * nt + 1] * dotq));
-        *reinterpret_cast<__nv_bfloat162*>(dkdst + row * dld + 8 * nt + cq) =
-            __floats2bfloat162_rn(rk * (dKn[nt][2 * hrow] - kh[2 * nt] * dotk), rk * (dKn[nt][2 * hrow + 1] - kh[2 * nt + 1] * dotk));
+    for (int half = 0; half < 2; ++half) {
+      const int row = r0 + 8 * half;
+      const float rq = rqs[row], rk = rks[row], sq = redg[row] + redg[64 + row], sk = redb[row] + redb[64 + row];
+#pragma unroll
+      for (int nt = 0; nt < 4; ++nt) {
+        *reinterpret_cast<uint32_t*>(X1 + row * LDS + 8 * nt + c0) =
+            pack_f2(rq * (0.125f * dQn[nt][2 * half] - qh[nt][2 * half] * sq), rq * (0.125f * dQn[nt][2 * half + 1] - qh[nt][2 * half + 1] * sq));
+        *reinterpret_cast<uint32_t*>(X2 + row * LDS + 8 * nt + c0) =
+            pack_f2(rk * (dKn[nt][2 * half] - kh[nt][2 * half] * sk), rk * (dKn[nt][2 * half + 1] - kh[nt][2 * half + 1] * sk));
       }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      const int chunk = tid + 256 * i, row = chunk >> 3, col = (chunk & 7) * 8;
+      const long long dst = (tok0 + row) * dqk_ld + hk * 64 + col;
+      *reinterpret_cast<uint4*>(dq + dst) = *reinterpret_cast<const uint4*>(X1 + row * LDS + col);
+      *reinterpret_cast<uint4*>(dk + dst) = *reinterpret_cast<const uint4*>(X2 + row * LDS + col);
     }
   }
 }
@@ -779,27 +834,28 @@ std::vector<at::Tensor> gdn_prep_fwd(const at::Tensor& q, const at::Tensor& k, c
 
 // Returns {dqkv packed bf16 [B,S,(2 Hk + Hv) 64] holding dq | dk | dv per token, dg, dbeta (fp32 [B,S,Hv])}
 std::vector<at::Tensor> gdn_prep_bwd(const at::Tensor& q, const at::Tensor& k, const at::Tensor& v, const at::Tensor& g, const at::Tensor& beta,
-                                     const at::Tensor& Tm, const at::Tensor& dw, const at::Tensor& du, const at::Tensor& dP, const at::Tensor& dqg,
-                                     const at::Tensor& dkg, const at::Tensor& dd) {
+                                     const at::Tensor& Tm, const at::Tensor& w, const at::Tensor& u, const at::Tensor& vnew, const at::Tensor& states,
+                                     const at::Tensor& dout, const at::Tensor& du, const at::Tensor& dstate, const at::Tensor& dd) {
   const c10::cuda::CUDAGuard guard(q.device());
   const int64_t B = q.size(0), S = q.size(1), Hk = q.size(2), Hv = v.size(2), NT = S / 64, BH = B * Hv;
-  check_tiles(Tm, BH, NT, "Tm"); check_tiles(dw, BH, NT, "dw"); check_tiles(du, BH, NT, "du"); check_tiles(dP, BH, NT, "dP");
-  check_tiles(dqg, BH, NT, "dqg"); check_tiles(dkg, BH, NT, "dkg");
-  TORCH_CHECK(dd.scalar_type() == at::kFloat && dd.is_contiguous() && dd.numel() == BH * NT, "gdn_prep_bwd: dd must be fp32 [BH,NT]");
+  check_tiles(Tm, BH, NT, "Tm"); check_tiles(w, BH, NT, "w"); check_tiles(u, BH, NT, "u"); check_tiles(vnew, BH, NT, "vnew");
+  check_tiles(states, BH, NT, "states"); check_tiles(dout, BH, NT, "do"); check_tiles(du, BH, NT, "du"); check_tiles(dstate, BH, NT, "dstate");
+  TORCH_CHECK(dd.scalar_type() == at::kFloat && dd.is_contiguous() && dd.numel() == BH * NT * 4, "gdn_prep_bwd: dd must be fp32 [BH,NT,4]");
+  TORCH_CHECK(q.stride(1) == k.stride(1) && q.stride(1) % 8 == 0 && v.stride(1) % 2 == 0, "gdn_prep_bwd: q, k, v must be the strided views the forward took");
   const int64_t packed = (2 * Hk + Hv) * 64;
   auto dqkv = at::empty({B, S, packed}, q.options());
   bf16* dq_ptr = (bf16*)dqkv.data_ptr();
   bf16* dk_ptr = dq_ptr + Hk * 64;
   bf16* dv_ptr = dq_ptr + 2 * Hk * 64;
   auto dg = at::empty({B, S, Hv}, q.options().dtype(at::kFloat)), dbeta = at::empty({B, S, Hv}, q.options().dtype(at::kFloat));
-  const int smem = 9 * TILE_ELEMS * 2 + 400 * 4;
+  constexpr int smem = 12 * TILE_ELEMS * 2 + 648 * 4;
   static bool configured = false;
   if (!configured) { C10_CUDA_CHECK(cudaFuncSetAttribute(gdn_prep_bwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem)); configured = true; }
-  gdn_prep_bwd_kernel<<<dim3((int)NT, (int)(B * Hk)), 128, smem, at::cuda::getCurrentCUDAStream()>>>(
+  gdn_prep_bwd_kernel<<<dim3((int)NT, (int)(B * Hk)), 256, smem, at::cuda::getCurrentCUDAStream()>>>(
       (const bf16*)q.data_ptr(), (const bf16*)k.data_ptr(), (const bf16*)v.data_ptr(), g.data_ptr<float>(), (const bf16*)beta.data_ptr(),
-      (const bf16*)Tm.data_ptr(), (const bf16*)dw.data_ptr(), (const bf16*)du.data_ptr(), (const bf16*)dP.data_ptr(), (const bf16*)dqg.data_ptr(),
-      (const bf16*)dkg.data_ptr(), dd.data_ptr<float>(), dq_ptr, dk_ptr, dv_ptr, dg.data_ptr<float>(),
-      dbeta.data_ptr<float>(), (int)S, (int)Hk, (int)Hv, (long long)q.stride(1), (long long)v.stride(1), (long long)packed, (long long)packed);
+      (const bf16*)Tm.data_ptr(), (const bf16*)w.data_ptr(), (const bf16*)u.data_ptr(), (const bf16*)vnew.data_ptr(), (const bf16*)states.data_ptr(),
+      (const bf16*)dout.data_ptr(), (const bf16*)du.data_ptr(), (const bf16*)dstate.data_ptr(), dd.data_ptr<float>(), dq_ptr, dk_ptr, dv_ptr,
+      dg.data_ptr<float>(), dbeta.data_ptr<float>(), (int)S, (int)Hk, (int)Hv, (long long)q.stride(1), (long long)v.stride(1), (long long)packed, (long long)packed);
   C10_CUDA_KERNEL_LAUNCH_CHECK();
   count_launch();
   return {dqkv, dg, dbeta};

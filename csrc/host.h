@@ -116,8 +116,11 @@ std::vector<at::Tensor> gdn_scan_bwd(const at::Tensor& w, const at::Tensor& P, c
 
 std::vector<at::Tensor> gdn_prep_fwd(const at::Tensor& q, const at::Tensor& k, const at::Tensor& v, const at::Tensor& g, const at::Tensor& beta);
 std::vector<at::Tensor> gdn_prep_bwd(const at::Tensor& q, const at::Tensor& k, const at::Tensor& v, const at::Tensor& g, const at::Tensor& beta,
-                                     const at::Tensor& Tm, const at::Tensor& dw, const at::Tensor& du, const at::Tensor& dP, const at::Tensor& dqg,
-                                     const at::Tensor& dkg, const at::Tensor& dd);
+                                     const at::Tensor& Tm, const at::Tensor& w, const at::Tensor& u, const at::Tensor& vnew, const at::Tensor& states,
+                                     const at::Tensor& dout, const at::Tensor& du, const at::Tensor& dstate, const at::Tensor& dd);
+// gdn_chain.cu
+std::vector<at::Tensor> gdn_chain_bwd(const at::Tensor& w, const at::Tensor& P, const at::Tensor& qg, const at::Tensor& kg, const at::Tensor& dch,
+                                      const at::Tensor& states, const at::Tensor& dout, int64_t B, int64_t H, const c10::optional<at::Tensor>& err);
 // qsa_index.cu
 at::Tensor qsa_main_block_stats(const at::Tensor& q, const at::Tensor& k, double scale);
 at::Tensor qsa_indexer_fwd(const at::Tensor& qi, const at::Tensor& ki, const at::Tensor& wi, double scale);

@@ -143,7 +143,9 @@ def load_megatron_function(path, expected_sha256=MEGATRON_SHA256):
 
 
 def delta_rule_kernel_products(source=None):
-    """64x64x64 tensor-core products per (chunk, value head) issued by each delta-rule kernel, counted from the kernel source."""
+    """64x64x64 tensor-core products per (chunk, value head) issued by each delta-rule kernel, counted from the kernel source.  A training step
+    runs `gdn_chain_bwd_kernel` (csrc/gdn_chain.cu, four products) in the place of `gdn_scan_bwd_kernel`, which serves operands that come
+    from the PyTorch specification; the products it leaves out are among the twelve of `gdn_prep_bwd_kernel`."""
     text = Path(source or Path(__file__).resolve().parents[2] / "csrc" / "gdn.cu").read_text()
     kernels = re.split(r"__global__ void[^\n]*?\b(gdn_\w+_kernel)\(", text)
     counts = {}

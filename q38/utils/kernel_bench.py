@@ -143,12 +143,14 @@ def bench_gdn(rows, shape, T, iters, pk, seq=4096):
     t = timeit(lambda: lib.gdn_scan_fwd(w, u, P, qg, kg, carry, B, Hv), iters)
     report(rows, f"gdn_scan_fwd B={B} Hv={Hv}", t, flops=chunks * 4 * 2.0 * 64 ** 3, bytes_=chunks * 8 * 8192.0, pk=pk)
     o, vnew, states = lib.gdn_scan_fwd(w, u, P, qg, kg, carry, B, Hv)
+    t = timeit(lambda: lib.gdn_scan_fwd(w, u, P, qg, kg, carry, B, Hv, None, False), iters)
+    report(rows, f"gdn_scan_fwd, inference B={B} Hv={Hv}", t, flops=chunks * 4 * 2.0 * 64 ** 3, bytes_=chunks * 6 * 8192.0, pk=pk)
     do = torch.randn_like(o)
-    t = timeit(lambda: lib.gdn_scan_bwd(w, P, qg, kg, carry, vnew, states, do, B, Hv), iters)
-    report(rows, f"gdn_scan_bwd B={B} Hv={Hv}", t, flops=chunks * 9 * 2.0 * 64 ** 3, bytes_=chunks * 12 * 8192.0, pk=pk)
-    dw, du, dP, dqg, dkg, dd = lib.gdn_scan_bwd(w, P, qg, kg, carry, vnew, states, do, B, Hv)
-    t = timeit(lambda: lib.gdn_prep_bwd(q, k, v, g, beta, Tm, dw, du, dP, dqg, dkg, dd), iters)
-    report(rows, f"gdn_prep_bwd B={B} Hv={Hv}", t, flops=chunks * 14 * 2.0 * 64 ** 3, bytes_=chunks * 6 * 8192.0 + 4.0 * qkv.numel(), pk=pk)
+    t = timeit(lambda: lib.gdn_chain_bwd(w, P, qg, kg, carry, states, do, B, Hv), iters)
+    report(rows, f"gdn_chain_bwd B={B} Hv={Hv}", t, flops=chunks * 4 * 2.0 * 64 ** 3, bytes_=chunks * 8 * 8192.0, pk=pk)
+    du, dstate, dd = lib.gdn_chain_bwd(w, P, qg, kg, carry, states, do, B, Hv)
+    t = timeit(lambda: lib.gdn_prep_bwd(q, k, v, g, beta, Tm, w, u, vnew, states, do, du, dstate, dd), iters)
+    report(rows, f"gdn_prep_bwd B={B} Hv={Hv}", t, flops=chunks * 12 * 2.0 * 64 ** 3, bytes_=chunks * 8 * 8192.0 + 4.0 * qkv.numel(), pk=pk)
 
 
 def bench_qsa(rows, shape, T, iters, pk, seq=4096):

@@ -43,3 +43,46 @@ def test_scan_forward(ops, B, H, NT):
         # bf16 operands of every product (2^-9 each) carried along the chunks: three roundings of 2e-3 (rms) and their propagation
         assert rel(states[:, c], S) < 1e-2 and rel(vnew[:, c], v) < 1e-2 and rel(o[:, 64 * c:64 * c + 64], out) < 1e-2, c
         S = d[:, c, None, None].double() * S + f[4][:, c].transpose(-1, -2) @ v
+
+
+def recurrence(qkv, g, beta, Hk, Hv):
+    B, S, _ = qkv.shape
+    q, k, v = qkv.split([64 * Hk, 64 * Hk, 64 * Hv], -1)
+    unit = lambda t: t * torch.rsqrt((t * t).sum(-1, keepdim=True) + 1e-6)
+    q = (unit(q.reshape(B, S, Hk, 64)) / 8).repeat_interleave(Hv // Hk, 2)
+    k = unit(k.reshape(B, S, Hk, 64)).repeat_interleave(Hv // Hk, 2)
+    v = v.reshape(B, S, Hv, 64)
+    state, outs = qkv.new_zeros(B, Hv, 64, 64), []
+    for t in range(S):
+        state = state * g[:, t].exp()[..., None, None]
+        fresh = (v[:, t] - torch.einsum("bhkv,bhk->bhv", state, k[:, t])) * beta[:, t][..., None]
+        state = state + k[:, t][..., None] * fresh[..., None, :]
+        outs.append(torch.einsum("bhkv,bhk->bhv", state, q[:, t]))
+    return torch.stack(outs, 1)
+
+
+# one and three value heads per key head; one chunk, an odd number of chunks; heads that forget at once and heads that keep everything
+# (the reverse scan runs one warp per CTA up to 37 pairs, then two)
+@pytest.mark.parametrize("B,S,Hk,Hv", [(1, 64, 1, 1), (2, 192, 2, 6), (1, 320, 13, 39)])
+@pytest.mark.parametrize("decay", [0.0, 0.05, 20.0])
+def test_delta_rule_gradients(ops, B, S, Hk, Hv, decay):
+    from q38.ops.backend import _DeltaRule
+    gen = torch.Generator(device="cuda").manual_seed(S + Hv)
+    qkv = torch.randn(B, S, (2 * Hk + Hv) * 64, device="cuda", generator=gen).to(torch.bfloat16).requires_grad_()
+    g = (-decay * torch.rand(B, S, Hv, device="cuda", generator=gen)).requires_grad_()
+    beta = torch.rand(B, S, Hv, device="cuda", generator=gen).to(torch.bfloat16)
+    beta[:, ::7] = 0                                           # tokens that write nothing still have a beta gradient
+    beta.requires_grad_()
+    do = torch.randn(B, S, Hv, 64, device="cuda", generator=gen).to(torch.bfloat16)
+    o = _DeltaRule.apply(qkv, g, beta, Hk, Hv)
+    o.backward(do)
+    ops.check_errors()
+    ref = [t.detach().double().requires_grad_() for t in (qkv, g, beta)]
+    ro = recurrence(*ref, Hk, Hv)
+    ro.backward(do.double())
+    # bf16 chunk operands (2e-3 rms each); the gate gradients are differences of row and column sums of those products
+    assert rel(o, ro.detach()) < 1.5e-2 and rel(qkv.grad, ref[0].grad) < 2e-2 and rel(beta.grad, ref[2].grad) < 2e-2
+    if decay:
+        assert rel(g.grad, ref[1].grad) < 2.5e-2
+    zero = beta.detach() == 0
+    assert rel(beta.grad[zero], ref[2].grad[zero]) < 2e-2
