@@ -115,7 +115,7 @@ TORCH_LIBRARY(q38, m) {
   m.def("ce_inplace(Tensor(a!) logits, Tensor target) -> Tensor", [](at::Tensor& l, const at::Tensor& t) { return q38::ce_inplace(l, t); });
   m.def("conv_silu_fwd(Tensor x, Tensor w) -> Tensor");
   m.def("conv_silu_bwd(Tensor x, Tensor w, Tensor dy) -> Tensor[]");
-  m.def("gdn_prep_fwd(Tensor q, Tensor k, Tensor v, Tensor g, Tensor beta) -> Tensor[]");
+  m.def("gdn_prep_fwd(Tensor q, Tensor k, Tensor v, Tensor g, Tensor beta, bool save=True) -> Tensor[]");
   m.def("gdn_prep_bwd(Tensor q, Tensor k, Tensor v, Tensor g, Tensor beta, Tensor Tm, Tensor w, Tensor u, Tensor vnew, Tensor states, Tensor dout, Tensor du, Tensor dstate, Tensor dd) -> Tensor[]");
   m.def("gdn_chain_bwd(Tensor w, Tensor P, Tensor qg, Tensor kg, Tensor dch, Tensor states, Tensor dout, int B, int H, Tensor? err=None) -> Tensor[]");
   m.def("gdn_scan_fwd(Tensor w, Tensor u, Tensor P, Tensor qg, Tensor kg, Tensor dch, int B, int H, Tensor? err=None, bool save=True) -> Tensor[]");

@@ -326,175 +326,221 @@ std::vector<at::Tensor> gdn_scan_bwd(const at::Tensor& w, const at::Tensor& P, c
 // =====================================================================================================================
 namespace q38 {
 
-#define FRAG_LOOP(nt, e, row, col)                                             \
-  _Pragma("unroll") for (int nt = 0; nt < 8; ++nt)                              \
-  _Pragma("unroll") for (int e = 0; e < 4; ++e)                                 \
-    if (const int row = 16 * warp + (lane >> 2) + 8 * (e >> 1); true)           \
-      if (const int col = 8 * nt + 2 * (lane & 3) + (e & 1); true)
-
-// Loads 64 tokens x 64 dims of one head (token stride `ld` elements) and returns, per token row, the reciprocal norm.
-// Thread layout: token = tid / 2, half = tid % 2 (32 dims each).
-__device__ __forceinline__ void load_half_row(const bf16* __restrict__ src, long long ld, int tid, float (&vals)[32]) {
-  const int tok = tid >> 1, half = tid & 1;
-  const uint4* p = reinterpret_cast<const uint4*>(src + (long long)tok * ld + half * 32);
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const uint4 raw = p[i];
-    const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&raw);
-#pragma unroll
-    for (int j = 0; j < 4; ++j) { vals[i * 8 + 2 * j] = __low2float(h[j]); vals[i * 8 + 2 * j + 1] = __high2float(h[j]); }
-  }
-}
-
-__device__ __forceinline__ void store_half_row_smem(bf16* __restrict__ tile, int tid, const float (&vals)[32], float scale) {
-  const int tok = tid >> 1, half = tid & 1;
-#pragma unroll
-  for (int i = 0; i < 16; ++i)
-    *reinterpret_cast<__nv_bfloat162*>(tile + tok * LDS + half * 32 + 2 * i) = __floats2bfloat162_rn(vals[2 * i] * scale, vals[2 * i + 1] * scale);
-}
-
-__device__ __forceinline__ void store_half_row_global(bf16* __restrict__ dst, int tid, const float (&vals)[32], float scale) {
-  const int tok = tid >> 1, half = tid & 1;
-  uint4* p = reinterpret_cast<uint4*>(dst + tok * 64 + half * 32);
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    uint32_t wds[4];
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      __nv_bfloat162 h = __floats2bfloat162_rn(vals[i * 8 + 2 * j] * scale, vals[i * 8 + 2 * j + 1] * scale);
-      wds[j] = *reinterpret_cast<uint32_t*>(&h);
-    }
-    p[i] = make_uint4(wds[0], wds[1], wds[2], wds[3]);
-  }
-}
-
-// Shared prologue of the preparation kernels: normalised q/k tiles, gc, beta, reciprocal norms in shared memory.
-struct PrepSmem {
-  bf16 *Qn, *Kn, *KBG, *VB, *Tm;
-  float *gc, *beta, *rq, *rk;
-};
-
-__device__ __forceinline__ void prep_load_qk(const PrepSmem& s, const bf16* __restrict__ q, const bf16* __restrict__ k, long long ld_qk, int tid) {
-  float qv[32], kv[32];
-  load_half_row(q, ld_qk, tid, qv);
-  load_half_row(k, ld_qk, tid, kv);
-  float sq = 0.f, sk = 0.f;
-#pragma unroll
-  for (int i = 0; i < 32; ++i) { sq += qv[i] * qv[i]; sk += kv[i] * kv[i]; }
-  sq += __shfl_xor_sync(0xffffffffu, sq, 1);
-  sk += __shfl_xor_sync(0xffffffffu, sk, 1);
-  const float rq = rsqrtf(sq + 1e-6f), rk = rsqrtf(sk + 1e-6f);
-  if ((tid & 1) == 0) { s.rq[tid >> 1] = rq; s.rk[tid >> 1] = rk; }
-  store_half_row_smem(s.Qn, tid, qv, rq * 0.125f);
-  store_half_row_smem(s.Kn, tid, kv, rk);
-}
-
-// gc = inclusive cumsum of g over the chunk (warp 0, two tokens per lane); beta copied to shared memory.
-__device__ __forceinline__ void prep_load_gates(const PrepSmem& s, const float* __restrict__ g, const bf16* __restrict__ beta, long long ld, int tid) {
-  if (tid < 32) {
-    const float g0 = g[(long long)(2 * tid) * ld], g1 = g[(long long)(2 * tid + 1) * ld];
-    float run = g0 + g1;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) { const float up = __shfl_up_sync(0xffffffffu, run, o); if (tid >= o) run += up; }
-    s.gc[2 * tid] = run - g1;
-    s.gc[2 * tid + 1] = run;
-  } else if (tid < 96) {
-    s.beta[tid - 32] = __bfloat162float(beta[(long long)(tid - 32) * ld]);
-  }
-}
-
-// q,k: [B,S,Hk,64]; v: [B,S,Hv,64]; g fp32 / beta bf16: [B,S,Hv].  Tiles out: [B*Hv, NT, 64, 64] bf16.
-__global__ void __launch_bounds__(128) gdn_prep_fwd_kernel(const bf16* __restrict__ q, const bf16* __restrict__ k, const bf16* __restrict__ v,
-                                                           const float* __restrict__ g, const bf16* __restrict__ beta, bf16* __restrict__ w_out,
-                                                           bf16* __restrict__ u_out, bf16* __restrict__ P_out, bf16* __restrict__ qg_out,
-                                                           bf16* __restrict__ kg_out, bf16* __restrict__ Tm_out, float* __restrict__ carry,
-                                                           float* __restrict__ gc_out, int S, int Hk, int Hv, long long qk_ld, long long v_ld) {
+// q,k: [B,S,Hk,64]; v: [B,S,Hv,64]; g fp32 / beta bf16: [B,S,Hv].  Tiles out: [B*Hv, NT, 64, 64] bf16 (Tm only for a backward pass).
+// One CTA of four warps per (chunk, batch, value head), four per SM.  Every global access is a 16-byte piece of a 128-byte row.
+// (I + L)^-1 is found by forward substitution in fp32, in blocks of eight rows: a warp owns blocks `warp` and `warp + 4`, one column (and from
+// row 32 on a second one) per lane; the owner of a block solves it and leaves its rows in place of L's, then every warp subtracts them from
+// its later blocks.  A row's dot product runs as four ascending chains (j mod 4), as it would in one pass, so the blocks do not change a bit.
+// With one warp per 32 columns and all rows unrolled the other warps waited at the barrier for 2500 serial instructions that the
+// instruction cache did not hold: 169 us for 5376 chunks of a 16384-token layer (207 us with one thread per column of all rows), now 146.
+__global__ void __launch_bounds__(128, 4) gdn_prep_fwd_kernel(const bf16* __restrict__ q, const bf16* __restrict__ k, const bf16* __restrict__ v,
+                                                              const float* __restrict__ g, const bf16* __restrict__ beta, bf16* __restrict__ w_out,
+                                                              bf16* __restrict__ u_out, bf16* __restrict__ P_out, bf16* __restrict__ qg_out,
+                                                              bf16* __restrict__ kg_out, bf16* __restrict__ Tm_out, float* __restrict__ carry,
+                                                              float* __restrict__ gc_out, int S, int Hk, int Hv, long long qk_ld, long long v_ld) {
   extern __shared__ __align__(16) uint8_t smem_bytes[];
   bf16* sm = reinterpret_cast<bf16*>(smem_bytes);
-  PrepSmem s;
-  s.Qn = sm; s.Kn = sm + TILE_ELEMS; s.KBG = sm + 2 * TILE_ELEMS; s.VB = sm + 3 * TILE_ELEMS; s.Tm = sm + 4 * TILE_ELEMS;
-  constexpr int LSTRIDE = 68;                                        // rows 16-byte aligned for float4 reads
-  float* L = reinterpret_cast<float*>(sm + 5 * TILE_ELEMS);          // [64][68]
-  s.gc = L + 64 * LSTRIDE; s.beta = s.gc + 64; s.rq = s.beta + 64; s.rk = s.rq + 64;
+  bf16 *Qn = sm, *Kn = sm + TILE_ELEMS, *KBG = sm + 2 * TILE_ELEMS, *VB = sm + 3 * TILE_ELEMS, *Tm = sm + 4 * TILE_ELEMS;
+  constexpr int LD = 68;                                             // fp32 rows, 16-byte aligned
+  float* L = reinterpret_cast<float*>(sm);                           // [64][68], over Qn and Kn once they are used up
+  float *gc = reinterpret_cast<float*>(sm + 5 * TILE_ELEMS), *bet = gc + 64, *eg = bet + 64, *el = eg + 64;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int c = blockIdx.x, bh = blockIdx.y, b = bh / Hv, hv = bh % Hv, hk = hv / (Hv / Hk);
   const int NT = gridDim.x;
   const long long tok0 = (long long)b * S + (long long)c * 64;
   const long long tile_off = ((long long)bh * NT + c) * 4096;
-  prep_load_qk(s, q + tok0 * qk_ld + hk * 64, k + tok0 * qk_ld + hk * 64, qk_ld, tid);
-  prep_load_gates(s, g + tok0 * Hv + hv, beta + tok0 * Hv + hv, Hv, tid);
-  __syncthreads();
-  {
-    // qg, kg to global; KBG and VB to shared memory (thread = token half-row)
-    const int tok = tid >> 1, half = tid & 1;
-    const float gct = s.gc[tok], gl = s.gc[63], bt = s.beta[tok];
-    float row[32];
+  const int piece = 8 * (tid & 7), tok_t = tid >> 3;                 // this thread's 8 dims of tokens tok_t + 16 i
+  if (tid < 32) {
+    // gc = inclusive cumsum of g over the chunk, two tokens per lane
+    const float g0 = g[(tok0 + 2 * tid) * Hv + hv], g1 = g[(tok0 + 2 * tid + 1) * Hv + hv];
+    float run = g0 + g1;
 #pragma unroll
-    for (int i = 0; i < 16; ++i) {
-      const __nv_bfloat162 h = *reinterpret_cast<const __nv_bfloat162*>(s.Qn + tok * LDS + half * 32 + 2 * i);
-      row[2 * i] = __low2float(h); row[2 * i + 1] = __high2float(h);
-    }
-    store_half_row_global(qg_out + tile_off, tid, row, __expf(gct));
-#pragma unroll
-    for (int i = 0; i < 16; ++i) {
-      const __nv_bfloat162 h = *reinterpret_cast<const __nv_bfloat162*>(s.Kn + tok * LDS + half * 32 + 2 * i);
-      row[2 * i] = __low2float(h); row[2 * i + 1] = __high2float(h);
-    }
-    store_half_row_global(kg_out + tile_off, tid, row, __expf(gl - gct));
-    store_half_row_smem(s.KBG, tid, row, bt * __expf(gct));
-    load_half_row(v + tok0 * v_ld + hv * 64, v_ld, tid, row);
-    store_half_row_smem(s.VB, tid, row, bt);
-    if (tid == 0) carry[(long long)bh * NT + c] = __expf(gl);
-    if (tid < 64) gc_out[((long long)bh * NT + c) * 64 + tid] = s.gc[tid];
+    for (int o = 1; o < 32; o <<= 1) { const float up = __shfl_up_sync(0xffffffffu, run, o); if (tid >= o) run += up; }
+    const float last = __shfl_sync(0xffffffffu, run, 31), first = run - g1;
+    gc[2 * tid] = first; gc[2 * tid + 1] = run;
+    eg[2 * tid] = __expf(first); eg[2 * tid + 1] = __expf(run);
+    el[2 * tid] = __expf(last - first); el[2 * tid + 1] = __expf(last - run);
+    if (tid == 0) carry[(long long)bh * NT + c] = __expf(last);
+  } else if (tid < 96) {
+    bet[tid - 32] = __bfloat162float(beta[(tok0 + tid - 32) * Hv + hv]);
   }
-  float acc[8][4];
-  zero_acc(acc);
-  mma64<false, true>(s.Kn, s.Kn, acc, warp, lane);                    // k_i . k_j
-  FRAG_LOOP(nt, e, row, col) { L[row * LSTRIDE + col] = col < row ? s.beta[row] * acc[nt][e] * __expf(s.gc[row] - s.gc[col]) : 0.f; }
-  zero_acc(acc);
-  mma64<false, true>(s.Qn, s.Kn, acc, warp, lane);                    // q_i . k_j
-  FRAG_LOOP(nt, e, row, col) { acc[nt][e] = col <= row ? acc[nt][e] * __expf(s.gc[row] - s.gc[col]) : 0.f; }
-  acc_to_global(acc, P_out + tile_off, 64, warp, lane);
-  __syncthreads();
-  if (tid < 64) {
-    // column `tid` of (I + L)^-1 by forward substitution; L[i][j] reads are warp broadcasts, four at a time.  The dot product of
-    // row i runs as four independent chains so that its length, not the FMA latency times i, bounds the step.
-    float x[64];
+  uint32_t qn[4][4], kn[4][4];
+  uint4 vr[4];
 #pragma unroll
-    for (int i = 0; i < 64; ++i) {
-      float a0 = (i == tid) ? 1.f : 0.f, a1 = 0.f, a2 = 0.f, a3 = 0.f;
-      const float4* Lrow = reinterpret_cast<const float4*>(L + i * LSTRIDE);
+  for (int i = 0; i < 4; ++i) {
+    const long long tok = tok0 + tok_t + 16 * i;
+    const uint4 qr = *reinterpret_cast<const uint4*>(q + tok * qk_ld + hk * 64 + piece), kr = *reinterpret_cast<const uint4*>(k + tok * qk_ld + hk * 64 + piece);
+    vr[i] = *reinterpret_cast<const uint4*>(v + tok * v_ld + hv * 64 + piece);
+    qn[i][0] = qr.x; qn[i][1] = qr.y; qn[i][2] = qr.z; qn[i][3] = qr.w;
+    kn[i][0] = kr.x; kn[i][1] = kr.y; kn[i][2] = kr.z; kn[i][3] = kr.w;
+  }
+  {
+    // squared norms: each half row is one ascending chain of 32 terms, handed from lane to lane; then the two halves are added
+    float sq[4] = {0.f, 0.f, 0.f, 0.f}, sk[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
-      for (int j4 = 0; j4 < (i + 3) / 4; ++j4) {
-        const float4 l = Lrow[j4];                      // entries at or right of the diagonal are zero
-        a0 -= l.x * x[4 * j4];
-        if (4 * j4 + 1 < i) a1 -= l.y * x[4 * j4 + 1];
-        if (4 * j4 + 2 < i) a2 -= l.z * x[4 * j4 + 2];
-        if (4 * j4 + 3 < i) a3 -= l.w * x[4 * j4 + 3];
+    for (int step = 0; step < 4; ++step) {
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        if (step > 0) {
+          const float uq = __shfl_up_sync(0xffffffffu, sq[i], 1), uk = __shfl_up_sync(0xffffffffu, sk[i], 1);
+          if ((tid & 3) == step) { sq[i] = uq; sk[i] = uk; }
+        }
+        if ((tid & 3) == step) {
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            sq[i] = fmaf(lo_f(qn[i][j]), lo_f(qn[i][j]), sq[i]); sq[i] = fmaf(hi_f(qn[i][j]), hi_f(qn[i][j]), sq[i]);
+            sk[i] = fmaf(lo_f(kn[i][j]), lo_f(kn[i][j]), sk[i]); sk[i] = fmaf(hi_f(kn[i][j]), hi_f(kn[i][j]), sk[i]);
+          }
+        }
       }
-      x[i] = (a0 + a1) + (a2 + a3);
     }
 #pragma unroll
-    for (int i = 0; i < 64; ++i) s.Tm[i * LDS + tid] = __float2bfloat16_rn(x[i]);
+    for (int i = 0; i < 4; ++i) {
+      float a = __shfl_sync(0xffffffffu, sq[i], (tid & 31) | 3), d = __shfl_sync(0xffffffffu, sk[i], (tid & 31) | 3);
+      a += __shfl_xor_sync(0xffffffffu, a, 4);
+      d += __shfl_xor_sync(0xffffffffu, d, 4);
+      const float rq = rsqrtf(a + 1e-6f) * 0.125f, rk = rsqrtf(d + 1e-6f);
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        qn[i][j] = pack_f2(lo_f(qn[i][j]) * rq, hi_f(qn[i][j]) * rq);
+        kn[i][j] = pack_f2(lo_f(kn[i][j]) * rk, hi_f(kn[i][j]) * rk);
+      }
+      const int at = (tok_t + 16 * i) * LDS + piece;
+      *reinterpret_cast<uint4*>(Qn + at) = make_uint4(qn[i][0], qn[i][1], qn[i][2], qn[i][3]);
+      *reinterpret_cast<uint4*>(Kn + at) = make_uint4(kn[i][0], kn[i][1], kn[i][2], kn[i][3]);
+    }
   }
   __syncthreads();
-  {
-    // Tm tile to global for the backward pass
-    const int tok = tid >> 1, half = tid & 1;
-    float row[32];
+  auto scaled = [](const uint32_t (&x)[4], float s) {
+    return make_uint4(pack_f2(lo_f(x[0]) * s, hi_f(x[0]) * s), pack_f2(lo_f(x[1]) * s, hi_f(x[1]) * s),
+                      pack_f2(lo_f(x[2]) * s, hi_f(x[2]) * s), pack_f2(lo_f(x[3]) * s, hi_f(x[3]) * s));
+  };
 #pragma unroll
-    for (int i = 0; i < 16; ++i) {
-      const __nv_bfloat162 h = *reinterpret_cast<const __nv_bfloat162*>(s.Tm + tok * LDS + half * 32 + 2 * i);
-      row[2 * i] = __low2float(h); row[2 * i + 1] = __high2float(h);
-    }
-    store_half_row_global(Tm_out + tile_off, tid, row, 1.f);
+  for (int i = 0; i < 4; ++i) {
+    // qg, kg to global memory; KBG and VB to shared memory
+    const int tok = tok_t + 16 * i;
+    const float E = eg[tok], bt = bet[tok];
+    const uint32_t vw[4] = {vr[i].x, vr[i].y, vr[i].z, vr[i].w};
+    *reinterpret_cast<uint4*>(qg_out + tile_off + tok * 64 + piece) = scaled(qn[i], E);
+    *reinterpret_cast<uint4*>(kg_out + tile_off + tok * 64 + piece) = scaled(kn[i], el[tok]);
+    *reinterpret_cast<uint4*>(KBG + tok * LDS + piece) = scaled(kn[i], bt * E);
+    *reinterpret_cast<uint4*>(VB + tok * LDS + piece) = scaled(vw, bt);
   }
+  if (tid < 64) gc_out[((long long)bh * NT + c) * 64 + tid] = gc[tid];
+  const int r0 = 16 * warp + (lane >> 2), cq = 2 * (lane & 3);
+  float acc[8][4], kk[8][4];
+  {
+    const float glo = gc[r0], ghi = gc[r0 + 8], blo = bet[r0], bhi = bet[r0 + 8];
+    zero_acc(kk);
+    mma64<false, true>(Kn, Kn, kk, warp, lane);                        // k_i . k_j
+    zero_acc(acc);
+    mma64<false, true>(Qn, Kn, acc, warp, lane);                       // q_i . k_j
+    __syncthreads();                                                   // Qn and Kn are used up
+#pragma unroll
+    for (int nt = 0; nt < 8; ++nt) {
+      const int cc = 8 * nt + cq;
+      const float2 gj = *reinterpret_cast<const float2*>(gc + cc);
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const int row = r0 + 8 * (e >> 1), cl = cc + (e & 1);
+        const float gam = __expf((e >> 1 ? ghi : glo) - (e & 1 ? gj.y : gj.x));
+        kk[nt][e] = cl < row ? (e >> 1 ? bhi : blo) * kk[nt][e] * gam : 0.f;
+        acc[nt][e] = cl <= row ? acc[nt][e] * gam : 0.f;
+      }
+      *reinterpret_cast<float2*>(L + r0 * LD + cc) = make_float2(kk[nt][0], kk[nt][1]);
+      *reinterpret_cast<float2*>(L + (r0 + 8) * LD + cc) = make_float2(kk[nt][2], kk[nt][3]);
+    }
+    acc_to_smem(acc, Tm, warp, lane);                                  // P, on its way to global memory
+  }
+  auto store_tile = [&](const bf16* tile, bf16* dst) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int row = tok_t + 16 * i;
+      *reinterpret_cast<uint4*>(dst + row * 64 + piece) = *reinterpret_cast<const uint4*>(tile + row * LDS + piece);
+    }
+  };
+  __syncthreads();                                                     // L and P complete
+  store_tile(Tm, P_out + tile_off);
+  __syncthreads();                                                     // P has left Tm
+  {
+    // rows 8 t + r minus block s of the finished rows, for columns lane (and lane + 32)
+    auto update = [&](auto& a, int t, int sblk) {
+      constexpr int NC = sizeof(a) / sizeof(a[0]);
+      float x[NC][8];
+#pragma unroll
+      for (int j = 0; j < 8; ++j)
+#pragma unroll
+        for (int n = 0; n < NC; ++n) x[n][j] = L[(8 * sblk + j) * LD + 32 * n + lane];
+#pragma unroll
+      for (int r = 0; r < 8; ++r) {
+        const float4 l0 = *reinterpret_cast<const float4*>(L + (8 * t + r) * LD + 8 * sblk), l1 = *reinterpret_cast<const float4*>(L + (8 * t + r) * LD + 8 * sblk + 4);
+#pragma unroll
+        for (int n = 0; n < NC; ++n) {
+          a[n][r][0] -= l0.x * x[n][0]; a[n][r][1] -= l0.y * x[n][1]; a[n][r][2] -= l0.z * x[n][2]; a[n][r][3] -= l0.w * x[n][3];
+          a[n][r][0] -= l1.x * x[n][4]; a[n][r][1] -= l1.y * x[n][5]; a[n][r][2] -= l1.z * x[n][6]; a[n][r][3] -= l1.w * x[n][7];
+        }
+      }
+    };
+    // the block's own triangle; its rows replace L's, which nobody reads any more
+    auto solve = [&](auto& a, int t) {
+      constexpr int NC = sizeof(a) / sizeof(a[0]);
+      float x[NC][8];
+#pragma unroll
+      for (int r = 0; r < 8; ++r) {
+        const float4 l0 = *reinterpret_cast<const float4*>(L + (8 * t + r) * LD + 8 * t), l1 = *reinterpret_cast<const float4*>(L + (8 * t + r) * LD + 8 * t + 4);
+        const float l[8] = {l0.x, l0.y, l0.z, l0.w, l1.x, l1.y, l1.z, l1.w};
+#pragma unroll
+        for (int n = 0; n < NC; ++n) {
+#pragma unroll
+          for (int j = 0; j < r; ++j) a[n][r][j & 3] -= l[j] * x[n][j];
+          x[n][r] = (a[n][r][0] + a[n][r][1]) + (a[n][r][2] + a[n][r][3]);
+        }
+      }
+      __syncwarp();                                                    // every lane has read the rows
+#pragma unroll
+      for (int r = 0; r < 8; ++r) {
+#pragma unroll
+        for (int n = 0; n < 2; ++n) {
+          if (n < NC) L[(8 * t + r) * LD + 32 * n + lane] = x[n < NC ? n : 0][r];
+          Tm[(8 * t + r) * LDS + 32 * n + lane] = __float2bfloat16_rn(n < NC ? x[n < NC ? n : 0][r] : 0.f);
+        }
+      }
+    };
+    float low[1][8][4], high[2][8][4];                                 // chains of block `warp` (columns 0..31) and block `warp + 4` (both halves)
+#pragma unroll
+    for (int r = 0; r < 8; ++r) {
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        low[0][r][e] = e == 0 && 8 * warp + r == lane ? 1.f : 0.f;
+        high[0][r][e] = 0.f;
+        high[1][r][e] = low[0][r][e];
+      }
+    }
+#pragma unroll 1
+    for (int sblk = 0; sblk < 4; ++sblk) {
+      if (warp == sblk) solve(low, sblk);
+      __syncthreads();
+      if (warp > sblk) update(low, warp, sblk);
+      update(reinterpret_cast<float(&)[1][8][4]>(high), warp + 4, sblk);        // columns 32..63 of the first half are zero
+    }
+#pragma unroll 1
+    for (int sblk = 4; sblk < 8; ++sblk) {
+      if (warp == sblk - 4) solve(high, sblk);
+      __syncthreads();
+      if (warp > sblk - 4) update(high, warp + 4, sblk);
+    }
+  }
+  __syncthreads();
+  if (Tm_out != nullptr) store_tile(Tm, Tm_out + tile_off);
   zero_acc(acc);
-  mma64<false, false>(s.Tm, s.KBG, acc, warp, lane);
-  acc_to_global(acc, w_out + tile_off, 64, warp, lane);
+  mma64<false, false>(Tm, KBG, acc, warp, lane);
+  acc_to_smem(acc, Qn, warp, lane);
   zero_acc(acc);
-  mma64<false, false>(s.Tm, s.VB, acc, warp, lane);
-  acc_to_global(acc, u_out + tile_off, 64, warp, lane);
+  mma64<false, false>(Tm, VB, acc, warp, lane);
+  acc_to_smem(acc, Kn, warp, lane);
+  __syncthreads();
+  store_tile(Qn, w_out + tile_off);
+  store_tile(Kn, u_out + tile_off);
 }
 
 // Gradients of the chunk operands and of everything the preparation computed, chunk-parallel.  One CTA of eight warps per (chunk,
@@ -802,8 +848,8 @@ __global__ void __launch_bounds__(256, 2) gdn_prep_bwd_kernel(const bf16* __rest
 }
 
 // ---- host ----------------------------------------------------------------------------------------------------------------
-// Returns {w, u, P, qg, kg, Tm (bf16 tiles [B*Hv,NT,64,64]), carry [B*Hv,NT] fp32, gc [B*Hv,NT,64] fp32}
-std::vector<at::Tensor> gdn_prep_fwd(const at::Tensor& q, const at::Tensor& k, const at::Tensor& v, const at::Tensor& g, const at::Tensor& beta) {
+// Returns {w, u, P, qg, kg, Tm (bf16 tiles [B*Hv,NT,64,64]; Tm empty without `save`), carry [B*Hv,NT] fp32, gc [B*Hv,NT,64] fp32}
+std::vector<at::Tensor> gdn_prep_fwd(const at::Tensor& q, const at::Tensor& k, const at::Tensor& v, const at::Tensor& g, const at::Tensor& beta, bool save) {
   auto token_major = [](const at::Tensor& t) {
     return t.dim() == 4 && t.size(3) == 64 && t.stride(3) == 1 && t.stride(2) == 64 && t.stride(0) == t.size(1) * t.stride(1) && t.stride(1) % 8 == 0 &&
            (reinterpret_cast<uintptr_t>(t.data_ptr()) & 15) == 0;
@@ -817,16 +863,17 @@ std::vector<at::Tensor> gdn_prep_fwd(const at::Tensor& q, const at::Tensor& k, c
   const int64_t NT = S / 64, BH = B * Hv;
   auto opts = q.options();
   std::vector<at::Tensor> out;
-  for (int i = 0; i < 6; ++i) out.push_back(at::empty({BH, NT, 64, 64}, opts));
+  for (int i = 0; i < 5; ++i) out.push_back(at::empty({BH, NT, 64, 64}, opts));
+  out.push_back(save ? at::empty({BH, NT, 64, 64}, opts) : at::empty({0}, opts));
   out.push_back(at::empty({BH, NT}, opts.dtype(at::kFloat)));
   out.push_back(at::empty({BH, NT, 64}, opts.dtype(at::kFloat)));
-  const int smem = 5 * TILE_ELEMS * 2 + (64 * 68 + 256) * 4;
+  constexpr int smem = 5 * TILE_ELEMS * 2 + 256 * 4;
   static bool configured = false;
   if (!configured) { C10_CUDA_CHECK(cudaFuncSetAttribute(gdn_prep_fwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem)); configured = true; }
   gdn_prep_fwd_kernel<<<dim3((int)NT, (int)BH), 128, smem, at::cuda::getCurrentCUDAStream()>>>(
       (const bf16*)q.data_ptr(), (const bf16*)k.data_ptr(), (const bf16*)v.data_ptr(), g.data_ptr<float>(), (const bf16*)beta.data_ptr(),
       (bf16*)out[0].data_ptr(), (bf16*)out[1].data_ptr(), (bf16*)out[2].data_ptr(), (bf16*)out[3].data_ptr(), (bf16*)out[4].data_ptr(),
-      (bf16*)out[5].data_ptr(), out[6].data_ptr<float>(), out[7].data_ptr<float>(), (int)S, (int)Hk, (int)Hv, (long long)q.stride(1), (long long)v.stride(1));
+      save ? (bf16*)out[5].data_ptr() : nullptr, out[6].data_ptr<float>(), out[7].data_ptr<float>(), (int)S, (int)Hk, (int)Hv, (long long)q.stride(1), (long long)v.stride(1));
   C10_CUDA_KERNEL_LAUNCH_CHECK();
   count_launch();
   return out;

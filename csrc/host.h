@@ -114,7 +114,7 @@ std::vector<at::Tensor> gdn_scan_fwd(const at::Tensor& w, const at::Tensor& u, c
 std::vector<at::Tensor> gdn_scan_bwd(const at::Tensor& w, const at::Tensor& P, const at::Tensor& qg, const at::Tensor& kg, const at::Tensor& dch,
                                      const at::Tensor& vnew, const at::Tensor& states, const at::Tensor& dout, int64_t B, int64_t H);
 
-std::vector<at::Tensor> gdn_prep_fwd(const at::Tensor& q, const at::Tensor& k, const at::Tensor& v, const at::Tensor& g, const at::Tensor& beta);
+std::vector<at::Tensor> gdn_prep_fwd(const at::Tensor& q, const at::Tensor& k, const at::Tensor& v, const at::Tensor& g, const at::Tensor& beta, bool save);
 std::vector<at::Tensor> gdn_prep_bwd(const at::Tensor& q, const at::Tensor& k, const at::Tensor& v, const at::Tensor& g, const at::Tensor& beta,
                                      const at::Tensor& Tm, const at::Tensor& w, const at::Tensor& u, const at::Tensor& vnew, const at::Tensor& states,
                                      const at::Tensor& dout, const at::Tensor& du, const at::Tensor& dstate, const at::Tensor& dd);

@@ -385,8 +385,8 @@ class _DeltaRule(torch.autograd.Function):
         k = qkv[..., Hk * 64:2 * Hk * 64].unflatten(-1, (Hk, 64))
         v = qkv[..., 2 * Hk * 64:].unflatten(-1, (Hv, 64))
         g, beta = g.float().contiguous(), beta.to(torch.bfloat16).contiguous()
-        save = any(ctx.needs_input_grad)          # without a backward pass neither the chunk states nor v_new are written
-        w, u, P, qg, kg, Tm, carry, _gc = ops.gdn_prep_fwd(q, k, v, g, beta)
+        save = any(ctx.needs_input_grad)          # without a backward pass neither Tm nor the chunk states nor v_new are written
+        w, u, P, qg, kg, Tm, carry, _gc = ops.gdn_prep_fwd(q, k, v, g, beta, save)
         o, vnew, states = ops.gdn_scan_fwd(w, u, P, qg, kg, carry, B, Hv, error_flag(qkv.device), save)
         ctx.save_for_backward(qkv, g, beta, Tm, w, u, P, qg, kg, carry, vnew, states)
         ctx.heads = (Hk, Hv)
