@@ -11,7 +11,7 @@
 //                  dxin, and the parameter gradients (B, biases, alphas, norm weight)
 //   mhc_pre_bwd_c  dX_n = G_n + c1 X_n + pre_n dxin + sum_m res[m,n] dX'_m   with G = dL_raw . A from a GEMM
 // Coefficient row layout: [0,4) pre, [4,8) post, [8,24) res (row m, column n).  n_branch is fixed at 4.
-#include <torch/extension.h>
+#include <ATen/ATen.h>
 #include <ATen/cuda/CUDAContext.h>
 #include <c10/cuda/CUDAGuard.h>
 
@@ -51,42 +51,84 @@ __device__ __forceinline__ float sinkhorn_fwd(float logit, int iters, float* Y, 
   return p;
 }
 
-// Forward + backward with a compile-time iteration count: the loops unroll completely, so the saved iterates live in
-// registers instead of a per-thread local-memory array.  Lanes 0..15 (lane = 4 m + n); returns d(logit) given d(result).
-template <int ITERS>
-__device__ __forceinline__ float sinkhorn_fwd_bwd_unrolled(float logit, float dres) {
-  float Y[2 * ITERS], S[2 * ITERS];
-  float mx = logit;
+// The same on one thread per token: p[4 m + n] in registers, sums in the order the shuffles above give them, so the results are the same bits.
+// Twenty iterations are 40 dependent sum-and-divide steps; on sixteen lanes with two shuffles per sum they kept a warp busy for longer than its
+// token's memory traffic, here 16384 tokens are 512 independent warps: 4 us forward, 8 us backward, and the kernels that held the chains went from 52
+// to 41 us and from 61 to 33 us (hidden size 576).
+constexpr int SK = 32;                       // threads per CTA
+__device__ __forceinline__ float sinkhorn_start(const float (&logit)[16], float (&p)[16]) {
+  float mx = logit[0];
 #pragma unroll
-  for (int o = 8; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0x0000ffffu, mx, o));
-  const float p0 = __expf(logit - mx);
-  float p = p0;
+  for (int i = 1; i < 16; ++i) mx = fmaxf(mx, logit[i]);
 #pragma unroll
-  for (int it = 0; it < ITERS; ++it) {
-    float s = p + __shfl_xor_sync(0x0000ffffu, p, 1);
-    s += __shfl_xor_sync(0x0000ffffu, s, 2);
-    s = fmaxf(s, 1e-9f);
-    p = p / s;
-    Y[2 * it] = p; S[2 * it] = s;
-    float c = p + __shfl_xor_sync(0x0000ffffu, p, 4);
-    c += __shfl_xor_sync(0x0000ffffu, c, 8);
-    c = fmaxf(c, 1e-9f);
-    p = p / c;
-    Y[2 * it + 1] = p; S[2 * it + 1] = c;
+  for (int i = 0; i < 16; ++i) p[i] = __expf(logit[i] - mx);
+  return mx;
+}
+// One half step over the four groups p[g * GS + k * KS]: divides each by its sum, which `keep` receives.
+template <int GS, int KS, typename F> __device__ __forceinline__ void sinkhorn_half(float (&p)[16], F keep) {
+#pragma unroll
+  for (int g = 0; g < 4; ++g) {
+    const float s = fmaxf((p[g * GS] + p[g * GS + KS]) + (p[g * GS + 2 * KS] + p[g * GS + 3 * KS]), 1e-9f);
+    keep(g, s);
+#pragma unroll
+    for (int k = 0; k < 4; ++k) p[g * GS + k * KS] = p[g * GS + k * KS] / s;
   }
-  float d = dres;
+}
+
+// coef[t, 8..24): logits in, doubly normalised residual mix out.
+__global__ void __launch_bounds__(SK) mhc_sinkhorn_fwd_kernel(float* __restrict__ coef, int T, int iters) {
+  const int t = blockIdx.x * SK + threadIdx.x;
+  if (t >= T) return;
+  float4* row = reinterpret_cast<float4*>(coef + (size_t)t * NCOEF + 8);
+  float logit[16], p[16];
 #pragma unroll
-  for (int it = ITERS - 1; it >= 0; --it) {
-    float t = d * Y[2 * it + 1];
-    t += __shfl_xor_sync(0x0000ffffu, t, 4);
-    t += __shfl_xor_sync(0x0000ffffu, t, 8);
-    d = (d - t) / S[2 * it + 1];
-    t = d * Y[2 * it];
-    t += __shfl_xor_sync(0x0000ffffu, t, 1);
-    t += __shfl_xor_sync(0x0000ffffu, t, 2);
-    d = (d - t) / S[2 * it];
+  for (int m = 0; m < 4; ++m) { const float4 v = row[m]; logit[4 * m] = v.x; logit[4 * m + 1] = v.y; logit[4 * m + 2] = v.z; logit[4 * m + 3] = v.w; }
+  sinkhorn_start(logit, p);
+  auto drop = [](int, float) {};
+#pragma unroll 1
+  for (int it = 0; it < iters; ++it) { sinkhorn_half<4, 1>(p, drop); sinkhorn_half<1, 4>(p, drop); }
+#pragma unroll
+  for (int m = 0; m < 4; ++m) row[m] = make_float4(p[4 * m], p[4 * m + 1], p[4 * m + 2], p[4 * m + 3]);
+}
+
+// dcoef[t, 8..24): d(residual mix) in, d(logits) out.  Only the divisors are kept; the iterates follow from them backwards (p before a division is
+// p after it times the divisor), and y = p / sum(p)  =>  dp = (dy - sum(dy * y)) / s.
+__global__ void __launch_bounds__(SK) mhc_sinkhorn_bwd_kernel(const float* __restrict__ zsave, MhcParams P, float* __restrict__ dcoef, int T, int iters) {
+  extern __shared__ float divisors[];        // [iters][8][SK]
+  const int t = blockIdx.x * SK + threadIdx.x;
+  if (t >= T) return;
+  float logit[16], p[16], p0[16], d[16];
+  const float a2 = P.alphas[2];
+#pragma unroll
+  for (int i = 0; i < 16; ++i) { logit[i] = P.b_res[i] + a2 * zsave[(size_t)t * NCOEF + 8 + i]; d[i] = dcoef[(size_t)t * NCOEF + 8 + i]; }
+  sinkhorn_start(logit, p0);
+#pragma unroll
+  for (int i = 0; i < 16; ++i) p[i] = p0[i];
+  float* sv = divisors + threadIdx.x;
+#pragma unroll 1
+  for (int it = 0; it < iters; ++it) {
+    sinkhorn_half<4, 1>(p, [&](int g, float s) { sv[(8 * it + g) * SK] = s; });
+    sinkhorn_half<1, 4>(p, [&](int g, float s) { sv[(8 * it + 4 + g) * SK] = s; });
   }
-  return d * p0;
+  auto back = [&](auto group, auto step, const float* s4) {
+    constexpr int GS = decltype(group)::value, KS = decltype(step)::value;
+#pragma unroll
+    for (int g = 0; g < 4; ++g) {
+      const float s = s4[g * SK];
+      float dot = 0.f;
+#pragma unroll
+      for (int k = 0; k < 4; ++k) dot += d[g * GS + k * KS] * p[g * GS + k * KS];
+#pragma unroll
+      for (int k = 0; k < 4; ++k) { d[g * GS + k * KS] = (d[g * GS + k * KS] - dot) / s; p[g * GS + k * KS] *= s; }
+    }
+  };
+#pragma unroll 1
+  for (int it = iters - 1; it >= 0; --it) {
+    back(std::integral_constant<int, 1>(), std::integral_constant<int, 4>(), sv + (8 * it + 4) * SK);
+    back(std::integral_constant<int, 4>(), std::integral_constant<int, 1>(), sv + 8 * it * SK);
+  }
+#pragma unroll
+  for (int i = 0; i < 16; ++i) dcoef[(size_t)t * NCOEF + 8 + i] = d[i] * p0[i];     // the shift by the maximum cancels in the normalisations
 }
 
 // d(logit) given d(result); y = p / sum(p)  =>  dp = (dy - sum(dy * y)) / s
@@ -429,7 +471,7 @@ __global__ void __launch_bounds__(32 * RW, 4) mhc_coef_fwd_rows_kernel(const flo
                                                                        const float* __restrict__ norm_w, OutT* __restrict__ xout,
                                                                        float* __restrict__ coef, float* __restrict__ zsave,
                                                                        float* __restrict__ inv_save, float* __restrict__ rstd_save, int T, int h,
-                                                                       int r, int iters, float norm_eps) {
+                                                                       int r, float norm_eps) {
   extern __shared__ float sm[];
   const int RP = r + 1;
   float* Bs = sm;                               // [24][r + 1]
@@ -461,10 +503,8 @@ __global__ void __launch_bounds__(32 * RW, 4) mhc_coef_fwd_rows_kernel(const flo
     if (lane < 4) c = sigmoidf_(P.b_pre[lane] + P.alphas[0] * z);
     else if (lane < 8) c = 2.f * sigmoidf_(P.b_post[lane - 4] + P.alphas[1] * z);
     const float zr = __shfl_sync(0xffffffffu, z, (lane & 15) + 8);
-    float res = 0.f;
-    if (lane < 16) res = sinkhorn_fwd(P.b_res[lane] + P.alphas[2] * zr, iters, nullptr, nullptr, false);
     if (lane < 8) coef[(size_t)t * NCOEF + lane] = c;
-    if (lane < 16) coef[(size_t)t * NCOEF + 8 + lane] = res;
+    if (lane < 16) coef[(size_t)t * NCOEF + 8 + lane] = P.b_res[lane] + P.alphas[2] * zr;      // logits; mhc_sinkhorn_fwd_kernel normalises them
     const float p0 = __shfl_sync(0xffffffffu, c, 0), p1 = __shfl_sync(0xffffffffu, c, 1), p2 = __shfl_sync(0xffffffffu, c, 2),
                 p3 = __shfl_sync(0xffffffffu, c, 3);
     float4 v[NQ];
@@ -492,13 +532,14 @@ __global__ void __launch_bounds__(32 * RW, 4) mhc_coef_fwd_rows_kernel(const flo
   }
 }
 
-// Part A of the pre backward on register rows, in two kernels.
+// Part A of the pre backward on register rows, in four kernels.
 //   mhc_pre_bwd_rows_kernel   streaming part: norm backward (dxin), dpre_n = <dxin, X_n> (written to dcoef[0,4)), d(norm weight)
 //                             accumulated per lane across the warp's tokens.  No long dependent chain, so the loads of the next
 //                             token are issued while the current one is reduced.
-//   mhc_coef_bwd_kernel       per-token coefficient backward on [T,24] data only (sigmoid / Sinkhorn / tanh backward, dL_raw,
+//   mhc_sinkhorn_bwd_kernel   d(logits) of the residual mix, one token per thread.
+//   mhc_coef_bwd_kernel       per-token coefficient backward on [T,24] data only (sigmoid / tanh backward, dL_raw,
 //                             c1, bias and alpha gradients); it writes dlin [T,24], and dB = dlin^T (inv L_raw) is formed by
-//                             mhc_dB_kernel.  Few registers, so enough warps are resident to hide the Sinkhorn chain.
+//                             mhc_dB_kernel.
 template <typename GT, int NQ>
 __global__ void __launch_bounds__(32 * RW, 3) mhc_pre_bwd_rows_kernel(const GT* __restrict__ dxout, const float* __restrict__ X,
                                                                       const float* __restrict__ norm_w, const float* __restrict__ coef,
@@ -582,7 +623,7 @@ constexpr int CW = 8;      // warps per CTA of the coefficient backward
 __global__ void __launch_bounds__(32 * CW) mhc_coef_bwd_kernel(const float* __restrict__ Lraw, MhcParams P, const float* __restrict__ coef,
                                                                const float* __restrict__ zsave, const float* __restrict__ inv_save,
                                                                const float* __restrict__ dcoef, float* __restrict__ dLraw, float* __restrict__ c1_out,
-                                                               float* __restrict__ dlin_out, float* __restrict__ dbias, int T, int h, int r, int iters) {
+                                                               float* __restrict__ dlin_out, float* __restrict__ dbias, int T, int h, int r) {
   extern __shared__ float sm[];
   const int RP = r + 1;
   float* Bs = sm;                      // [24][r + 1]
@@ -601,23 +642,7 @@ __global__ void __launch_bounds__(32 * CW) mhc_coef_bwd_kernel(const float* __re
     float dlogit = 0.f;
     if (lane < 4) dlogit = dc * cv * (1.f - cv);
     else if (lane < 8) dlogit = dc * cv * (1.f - 0.5f * cv);                  // post = 2 sigmoid
-    float dres_logit = 0.f;
-    {
-      const float zr = __shfl_sync(0xffffffffu, z, (lane & 15) + 8);
-      const float dres = __shfl_sync(0xffffffffu, dc, (lane & 15) + 8);
-      if (lane < 16) {
-        const float logit = P.b_res[lane] + P.alphas[2] * zr;
-        if (iters == 20) {                                  // the presets' iteration count: register-resident variant
-          dres_logit = sinkhorn_fwd_bwd_unrolled<20>(logit, dres);
-        } else {
-          float Y[2 * MAX_SINKHORN], S[2 * MAX_SINKHORN];
-          sinkhorn_fwd(logit, iters, Y, S, true);
-          dres_logit = sinkhorn_bwd(dres, logit, iters, Y, S);
-        }
-      }
-    }
-    const float moved = __shfl_sync(0xffffffffu, dres_logit, (lane + 24) & 31);   // lane j gets lane j - 8
-    if (lane >= 8 && lane < NCOEF) dlogit = moved;
+    else dlogit = dc;                                                         // already d(logit) of the residual mix
     if (lane < NCOEF) { db += dlogit; da += dlogit * z; }
     const float dlin = lane < NCOEF ? dlogit * alpha * (1.f - z * z) : 0.f;
     if (lane < NCOEF) dlin_out[(size_t)t * NCOEF + lane] = dlin;
@@ -689,14 +714,15 @@ std::vector<at::Tensor> mhc_coef_fwd(const at::Tensor& X, const at::Tensor& Lraw
     const size_t smem = NCOEF * (r + 1) * sizeof(float);
     const int grid = std::min((T + RW - 1) / RW, 4 * kNumSMs);
 #define Q38_ROWS(OutT, NQ) mhc_coef_fwd_rows_kernel<OutT, NQ><<<grid, 32 * RW, smem, stream>>>(X.data_ptr<float>(), Lraw.data_ptr<float>(), P, norm_w.data_ptr<float>(), \
-      (OutT*)xout.data_ptr(), coef.data_ptr<float>(), z.data_ptr<float>(), inv.data_ptr<float>(), rstd.data_ptr<float>(), T, h, r, (int)iters, (float)norm_eps)
+      (OutT*)xout.data_ptr(), coef.data_ptr<float>(), z.data_ptr<float>(), inv.data_ptr<float>(), rstd.data_ptr<float>(), T, h, r, (float)norm_eps)
 #define Q38_ROWS_NQ(OutT) switch (nq) { case 1: Q38_ROWS(OutT, 1); break; case 2: Q38_ROWS(OutT, 2); break; case 3: Q38_ROWS(OutT, 3); break; case 4: Q38_ROWS(OutT, 4); break; \
       case 5: Q38_ROWS(OutT, 5); break; case 6: Q38_ROWS(OutT, 6); break; default: Q38_ROWS(OutT, 8); break; }
     if (out_bf16) Q38_ROWS_NQ(__nv_bfloat16) else Q38_ROWS_NQ(float)
 #undef Q38_ROWS_NQ
 #undef Q38_ROWS
+    mhc_sinkhorn_fwd_kernel<<<(T + SK - 1) / SK, SK, 0, stream>>>(coef.data_ptr<float>(), T, (int)iters);
     C10_CUDA_KERNEL_LAUNCH_CHECK();
-    count_launch();
+    count_launch(2);
     return {xout, coef, z, inv, rstd};
   }
   const size_t smem = (NCOEF * r + WARPS * h) * sizeof(float);
@@ -784,9 +810,12 @@ std::vector<at::Tensor> mhc_pre_bwd_a(const at::Tensor& dxout, const at::Tensor&
 #undef Q38_ROWS
     C10_CUDA_KERNEL_LAUNCH_CHECK();
     count_launch();
+    mhc_sinkhorn_bwd_kernel<<<(T + SK - 1) / SK, SK, 8 * SK * iters * sizeof(float), stream>>>(z.data_ptr<float>(), P, dcoef.data_ptr<float>(), T, (int)iters);
+    C10_CUDA_KERNEL_LAUNCH_CHECK();
+    count_launch();
     mhc_coef_bwd_kernel<<<std::min((T + CW - 1) / CW, 8 * kNumSMs), 32 * CW, (NCOEF * (r + 1) + 32) * sizeof(float), stream>>>(
         Lraw.data_ptr<float>(), P, coef.data_ptr<float>(), z.data_ptr<float>(), inv.data_ptr<float>(), dcoef.data_ptr<float>(), dLraw.data_ptr<float>(),
-        c1.data_ptr<float>(), dlin.data_ptr<float>(), dbias.data_ptr<float>(), T, h, r, (int)iters);
+        c1.data_ptr<float>(), dlin.data_ptr<float>(), dbias.data_ptr<float>(), T, h, r);
     C10_CUDA_KERNEL_LAUNCH_CHECK();
     count_launch();
     mhc_dB_kernel<<<(T + DB_TOK - 1) / DB_TOK, 256, DB_TOK * (NCOEF + r) * sizeof(float), stream>>>(dlin.data_ptr<float>(), Lraw.data_ptr<float>(), inv.data_ptr<float>(),
