@@ -93,8 +93,9 @@ __global__ void __launch_bounds__(128) qsa_main_block_stats_kernel(const bf16* _
 
 // ---- indexer forward ---------------------------------------------------------------------------------------------------
 // grid (nb, B).  blse[b, t, j] for j <= block(t); entries j > block(t) are left untouched (the caller pre-fills them).
-__global__ void __launch_bounds__(128) qsa_indexer_fwd_kernel(const bf16* __restrict__ qi, const bf16* __restrict__ ki, const float* __restrict__ wi,
-                                                              float* __restrict__ blse, int S, int NI, float scale) {
+// The query fragments of all heads stay in registers, the next key block is fetched while the current one is scored, one barrier per block.
+__global__ void __launch_bounds__(128, 3) qsa_indexer_fwd_kernel(const bf16* __restrict__ qi, const bf16* __restrict__ ki, const float* __restrict__ wi,
+                                                                 float* __restrict__ blse, int S, int NI, float scale) {
   extern __shared__ __align__(16) uint8_t smem_bytes[];
   bf16* Qs = reinterpret_cast<bf16*>(smem_bytes);          // NI tiles
   bf16* Ks = Qs + NI_MAX * TILE_ELEMS;                     // two buffers
@@ -111,23 +112,35 @@ __global__ void __launch_bounds__(128) qsa_indexer_fwd_kernel(const bf16* __rest
   float wrow[2][NI_MAX];
 #pragma unroll
   for (int hrow = 0; hrow < 2; ++hrow)
-    for (int hh = 0; hh < NI; ++hh) wrow[hrow][hh] = wi[((long long)b * S + (long long)i * 64 + r0 + 8 * hrow) * NI + hh] * scale;
+#pragma unroll
+    for (int hh = 0; hh < NI_MAX; ++hh) wrow[hrow][hh] = hh < NI ? wi[((long long)b * S + (long long)i * 64 + r0 + 8 * hrow) * NI + hh] * scale : 0.f;
+  cp_async_wait<0>();
+  __syncthreads();
+  uint32_t aq[NI_MAX][4][4];
+#pragma unroll
+  for (int hh = 0; hh < NI_MAX; ++hh) if (hh < NI) load_a(Qs + hh * TILE_ELEMS, aq[hh], warp, lane);
   int buf = 0;
   for (int j = blockIdx.z; j <= i; j += jstep, buf ^= 1) {
-    if (j + jstep <= i) { load_tile_async(Ks + (buf ^ 1) * TILE_ELEMS, kbase + (long long)(j + jstep) * 4096, 64, tid); cp_async_commit(); cp_async_wait<1>(); }
-    else cp_async_wait<0>();
-    __syncthreads();
+    cp_async_wait<0>();
+    __syncthreads();                                       // this key block is visible; the other buffer's readers are done
+    if (j + jstep <= i) load_tile_async(Ks + (buf ^ 1) * TILE_ELEMS, kbase + (long long)(j + jstep) * 4096, 64, tid);
+    cp_async_commit();
     float score[8][4];
     zero_acc(score);
-    for (int hh = 0; hh < NI; ++hh) {
-      float acc[8][4];
-      zero_acc(acc);
-      mma64<false, true>(Qs + hh * TILE_ELEMS, Ks + buf * TILE_ELEMS, acc, warp, lane);
 #pragma unroll
-      for (int nt = 0; nt < 8; ++nt) {
-        // the reference rounds q.k to bf16 before the relu (its matmul output dtype)
-        score[nt][0] += wrow[0][hh] * fmaxf(bf16_round(acc[nt][0]), 0.f); score[nt][1] += wrow[0][hh] * fmaxf(bf16_round(acc[nt][1]), 0.f);
-        score[nt][2] += wrow[1][hh] * fmaxf(bf16_round(acc[nt][2]), 0.f); score[nt][3] += wrow[1][hh] * fmaxf(bf16_round(acc[nt][3]), 0.f);
+    for (int hh = 0; hh < NI_MAX; ++hh) {
+      if (hh < NI) {
+#pragma unroll
+        for (int half = 0; half < 2; ++half) {
+          float acc[4][4];
+          zero_acc(acc);
+          mma_rows<true, 4, 4>(aq[hh], Ks + buf * TILE_ELEMS + 32 * half * LDS, acc, lane);
+#pragma unroll
+          for (int nt = 0; nt < 4; ++nt)
+#pragma unroll
+            for (int e = 0; e < 4; ++e)                    // the reference rounds q.k to bf16 before the relu (its matmul output dtype)
+              score[4 * half + nt][e] += wrow[e >> 1][hh] * fmaxf(bf16_round(acc[nt][e]), 0.f);
+        }
       }
     }
     float mx[2], sm[2];
@@ -139,8 +152,8 @@ __global__ void __launch_bounds__(128) qsa_indexer_fwd_kernel(const bf16* __rest
         blse[((long long)b * S + t) * nb + j] = mx[hrow] + __logf(sm[hrow]);
       }
     }
-    __syncthreads();
   }
+  cp_async_wait<0>();
 }
 
 // ---- combine: target mass, lp_blk, KL --------------------------------------------------------------------------------
@@ -239,24 +252,27 @@ __global__ void __launch_bounds__(256) qsa_select_kernel(const float* __restrict
 // ---- indexer backward ------------------------------------------------------------------------------------------------------
 // dI[t,s] = dblse[t, blk(s)] * exp(I[t,s] - blse[t, blk(s)]) for s <= t;   I = sum_h w_h relu(S_h) scale
 // Both passes form the scores of all heads once per (query block, key block) pair, keep relu(S_h) (which is bf16 by definition) packed in
-// registers until dI is known, and pass dS_h to the next product as A fragments in registers.  Four sequences of 4096 with four heads: 741 -> 461 us.
+// registers until dI is known, and pass dS_h to the next product as A fragments in registers.  Four sequences of 4096 with four heads: 741 -> 417 us.
 
-// Query pass, grid (nb, B), eight warps: d q_h(t) = sum_s dI w_h scale [S_h > 0] k(s);  d w_h(t) = sum_s dI relu(S_h) scale.
+// Query pass, grid (nb, B, z), eight warps: d q_h(t) = sum_s dI w_h scale [S_h > 0] k(s);  d w_h(t) = sum_s dI relu(S_h) scale.
 // Warps 0-3 hold heads 0 and 1, warps 4-7 heads 2 and 3, each warp 16 queries; the two partial scores of a tile meet in shared memory.
-// Eight 64^3 products per pair (one CTA per head had twenty), 306 us; bound by the latency of their chain, since the accumulators of two heads
-// leave eight warps per SM.  One head per warp and sixteen warps took 396 us: four times the exponentials and twice the exchange.
-__global__ void __launch_bounds__(256) qsa_indexer_bwd_q_kernel(const bf16* __restrict__ qi, const bf16* __restrict__ ki, const float* __restrict__ wi,
-                                                                const float* __restrict__ blse, const float* __restrict__ dblse, float gscale,
-                                                                bf16* __restrict__ dqi, float* __restrict__ dwi, int S, int NI, float scale) {
+// Eight 64^3 products per pair (one CTA per head had twenty).  Bound by the latency of their chain: a tile costs a CTA four times its issue slots, and
+// the last query block has 64 tiles.  So tiles are taken in quarters of 16 keys, which keeps two CTAs on an SM (128 registers), and the key
+// blocks j <= i of a query block are shared by gridDim.z CTAs (j = z, z + gridDim.z, ...) whose partial gradients are added in fp32.  About 255 us;
+// one CTA of eight warps per query block and SM took 306, sixteen warps with one head per four of them 396 (four times the exponentials).
+__global__ void __launch_bounds__(256, 2) qsa_indexer_bwd_q_kernel(const bf16* __restrict__ qi, const bf16* __restrict__ ki, const float* __restrict__ wi,
+                                                                   const float* __restrict__ blse, const float* __restrict__ dblse, float gscale,
+                                                                   float* __restrict__ dqi, float* __restrict__ dwi, int S, int NI, float scale) {
   extern __shared__ __align__(16) uint8_t smem_bytes[];
   bf16* Qs = reinterpret_cast<bf16*>(smem_bytes);          // NI tiles
   bf16* Ks = Qs + NI_MAX * TILE_ELEMS;                     // two buffers
-  float4* Px = reinterpret_cast<float4*>(Ks + 2 * TILE_ELEMS);     // partial scores of the two halves: [2][4 n-tiles][4 warps][32 lanes], per 32 keys
+  float4* Px = reinterpret_cast<float4*>(Ks + 2 * TILE_ELEMS);     // partial scores per 16 keys: [4 quarters][2 groups][2 n-tiles][4 warps][32 lanes]
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, wr = warp & 3, grp = warp >> 2;
-  const int nb = S / 64, i = nb - 1 - blockIdx.x, b = blockIdx.y;   // late query blocks (longest loops) first
+  const int nb = S / 64, i = nb - 1 - blockIdx.x, b = blockIdx.y, step = gridDim.z;   // late query blocks (longest loops) first
+  if ((int)blockIdx.z > i) return;
   for (int hh = 0; hh < NI; ++hh) load_tile_async_256(Qs + hh * TILE_ELEMS, qi + (((long long)b * NI + hh) * S + (long long)i * 64) * 64, 64, tid);
   const bf16* kbase = ki + (long long)b * S * 64;
-  load_tile_async_256(Ks, kbase, 64, tid);
+  load_tile_async_256(Ks, kbase + (long long)blockIdx.z * 4096, 64, tid);
   cp_async_commit();
   const int r0 = 16 * wr + (lane >> 2), cq = 2 * (lane & 3);
   const long long row = (long long)b * S + (long long)i * 64 + r0;
@@ -271,52 +287,51 @@ __global__ void __launch_bounds__(256) qsa_indexer_bwd_q_kernel(const bf16* __re
   zero_acc(dq[1]);
   float bl[2], g[2];
 #pragma unroll
-  for (int hr = 0; hr < 2; ++hr) { bl[hr] = blse[(row + 8 * hr) * nb]; g[hr] = dblse[(row + 8 * hr) * nb]; }
-  for (int j = 0; j <= i; ++j) {
+  for (int hr = 0; hr < 2; ++hr) { bl[hr] = blse[(row + 8 * hr) * nb + blockIdx.z]; g[hr] = dblse[(row + 8 * hr) * nb + blockIdx.z]; }
+  for (int j = blockIdx.z, buf = 0; j <= i; j += step, buf ^= 1) {
     cp_async_wait<0>();
     __syncthreads();
-    if (j < i) load_tile_async_256(Ks + ((j + 1) & 1) * TILE_ELEMS, kbase + (long long)(j + 1) * 4096, 64, tid);
+    const bool more = j + step <= i;
+    if (more) load_tile_async_256(Ks + (buf ^ 1) * TILE_ELEMS, kbase + (long long)(j + step) * 4096, 64, tid);
     cp_async_commit();
-    const bf16* Kt = Ks + (j & 1) * TILE_ELEMS;
+    const bf16* Kt = Ks + buf * TILE_ELEMS;
     const float b0 = bl[0], b1 = bl[1], g0 = g[0] * gscale, g1 = g[1] * gscale;
-    if (j < i) {
+    if (more) {
 #pragma unroll
-      for (int hr = 0; hr < 2; ++hr) { bl[hr] = blse[(row + 8 * hr) * nb + j + 1]; g[hr] = dblse[(row + 8 * hr) * nb + j + 1]; }
+      for (int hr = 0; hr < 2; ++hr) { bl[hr] = blse[(row + 8 * hr) * nb + j + step]; g[hr] = dblse[(row + 8 * hr) * nb + j + step]; }
     }
 #pragma unroll
-    for (int half = 0; half < 2; ++half) {                 // 32 keys at a time
-      uint32_t r[2][2][4];                                 // relu(S_h) as A fragments
-      float score[4][4];
-      zero_acc(score);
+    for (int part = 0; part < 4; ++part) {                 // 16 keys at a time
+      uint32_t r[2][1][4];                                 // relu(S_h) as A fragments
+      float score[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
 #pragma unroll
       for (int x = 0; x < 2; ++x) {
-        float acc[4][4];
-        zero_acc(acc);
+        float acc[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
         if (x < heads) {
           uint32_t a[4][4];
           load_a(Qs + (2 * grp + x) * TILE_ELEMS, a, wr, lane);
-          mma_rows<true, 4, 4>(a, Kt + 32 * half * LDS, acc, lane);
+          mma_rows<true, 4, 2>(a, Kt + 16 * part * LDS, acc, lane);
         }
 #pragma unroll
-        for (int nt = 0; nt < 4; ++nt)
+        for (int nt = 0; nt < 2; ++nt)
 #pragma unroll
           for (int e = 0; e < 4; ++e) {
             acc[nt][e] = fmaxf(bf16_round(acc[nt][e]), 0.f);
             score[nt][e] += w[x][e >> 1] * acc[nt][e];
           }
-        pack_a<2>(acc, r[x]);
+        pack_a<1>(acc, r[x]);
       }
 #pragma unroll
-      for (int nt = 0; nt < 4; ++nt) Px[(half * 8 + grp * 4 + nt) * 128 + wr * 32 + lane] = make_float4(score[nt][0], score[nt][1], score[nt][2], score[nt][3]);
-      // the two warps of these 16 rows meet; the buffer of this half is free again after the block barrier of the next tile
+      for (int nt = 0; nt < 2; ++nt) Px[((part * 2 + grp) * 2 + nt) * 128 + wr * 32 + lane] = make_float4(score[nt][0], score[nt][1], score[nt][2], score[nt][3]);
+      // the two warps of these 16 rows meet; this quarter's buffer is free again after the block barrier of the next tile
       asm volatile("bar.sync %0, 64;" ::"r"(1 + wr) : "memory");
 #pragma unroll
-      for (int nt = 0; nt < 4; ++nt) {
-        const float4 o = Px[(half * 8 + (grp ^ 1) * 4 + nt) * 128 + wr * 32 + lane];
+      for (int nt = 0; nt < 2; ++nt) {
+        const float4 o = Px[((part * 2 + (grp ^ 1)) * 2 + nt) * 128 + wr * 32 + lane];
         const float other[4] = {o.x, o.y, o.z, o.w};
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
-          const int col = 32 * half + 8 * nt + cq + (e & 1);
+          const int col = 16 * part + 8 * nt + cq + (e & 1);
           const float d = (e >> 1 ? g1 : g0) * __expf(score[nt][e] + other[e] - (e >> 1 ? b1 : b0));
           score[nt][e] = (j < i || col <= r0 + 8 * (e >> 1)) ? d : 0.f;       // dI
         }
@@ -324,19 +339,19 @@ __global__ void __launch_bounds__(256) qsa_indexer_bwd_q_kernel(const bf16* __re
 #pragma unroll
       for (int x = 0; x < 2; ++x) {
         if (x < heads) {
-          float ds[4][4];
+          float ds[2][4];
 #pragma unroll
-          for (int nt = 0; nt < 4; ++nt)
+          for (int nt = 0; nt < 2; ++nt)
 #pragma unroll
             for (int e = 0; e < 4; ++e) {
-              const uint32_t p = r[x][nt >> 1][(nt & 1) * 2 + (e >> 1)];
+              const uint32_t p = r[x][0][nt * 2 + (e >> 1)];
               const float relu = (e & 1) ? hi_f(p) : lo_f(p);
               dw[x][e >> 1] += score[nt][e] * relu * scale;
               ds[nt][e] = relu > 0.f ? score[nt][e] * w[x][e >> 1] : 0.f;     // dS_h
             }
-          uint32_t a[2][4];
-          pack_a<2>(ds, a);
-          mma_rows<false, 2, 8>(a, Kt + 32 * half * LDS, dq[x], lane);        // dS_h K
+          uint32_t a[1][4];
+          pack_a<1>(ds, a);
+          mma_rows<false, 1, 8>(a, Kt + 16 * part * LDS, dq[x], lane);        // dS_h K
         }
       }
     }
@@ -346,13 +361,18 @@ __global__ void __launch_bounds__(256) qsa_indexer_bwd_q_kernel(const bf16* __re
   for (int x = 0; x < 2; ++x) {
     if (x < heads) {
       const int own = 2 * grp + x;
-      acc_to_global(dq[x], dqi + (((long long)b * NI + own) * S + (long long)i * 64) * 64, 64, wr, lane);
+      float* dst = dqi + (((long long)b * NI + own) * S + (long long)i * 64) * 64;
+#pragma unroll
+      for (int nt = 0; nt < 8; ++nt)
+#pragma unroll
+        for (int hr = 0; hr < 2; ++hr)
+          atomicAdd(reinterpret_cast<float2*>(dst + (r0 + 8 * hr) * 64 + 8 * nt + cq), make_float2(dq[x][nt][2 * hr], dq[x][nt][2 * hr + 1]));
 #pragma unroll
       for (int hr = 0; hr < 2; ++hr) {
         float v = dw[x][hr];
         v += __shfl_xor_sync(0xffffffffu, v, 1);
         v += __shfl_xor_sync(0xffffffffu, v, 2);
-        if ((lane & 3) == 0) dwi[(row + 8 * hr) * NI + own] = v;
+        if ((lane & 3) == 0) atomicAdd(&dwi[(row + 8 * hr) * NI + own], v);
       }
     }
   }
@@ -553,9 +573,9 @@ std::vector<at::Tensor> qsa_indexer_bwd(const at::Tensor& qi, const at::Tensor& 
                                         double gscale, double scale) {
   const c10::cuda::CUDAGuard guard(qi.device());
   const int B = qi.size(0), NI = qi.size(1), S = qi.size(2), nb = S / 64;
-  auto dqi = at::empty_like(qi);
+  auto dqi32 = at::zeros(qi.sizes(), qi.options().dtype(at::kFloat));
   auto dki32 = at::zeros(ki.sizes(), ki.options().dtype(at::kFloat));
-  auto dwi = at::empty_like(wi);
+  auto dwi = at::zeros_like(wi);
   constexpr int smem_q = (NI_MAX + 2) * TILE_ELEMS * 2 + 16 * 128 * 16, smem_k = 2 * NI_MAX * TILE_ELEMS * 2 + 2 * (2 + NI_MAX) * 64 * 4;
   static bool cfg = false;
   if (!cfg) {
@@ -564,13 +584,13 @@ std::vector<at::Tensor> qsa_indexer_bwd(const at::Tensor& qi, const at::Tensor& 
     cfg = true;
   }
   auto stream = at::cuda::getCurrentCUDAStream();
-  qsa_indexer_bwd_q_kernel<<<dim3(nb, B), 256, smem_q, stream>>>((const bf16*)qi.data_ptr(), (const bf16*)ki.data_ptr(), wi.data_ptr<float>(), blse.data_ptr<float>(),
-      dblse.data_ptr<float>(), (float)gscale, (bf16*)dqi.data_ptr(), dwi.data_ptr<float>(), S, NI, (float)scale);
+  qsa_indexer_bwd_q_kernel<<<dim3(nb, B, std::min(nb, 4)), 256, smem_q, stream>>>((const bf16*)qi.data_ptr(), (const bf16*)ki.data_ptr(), wi.data_ptr<float>(), blse.data_ptr<float>(),
+      dblse.data_ptr<float>(), (float)gscale, dqi32.data_ptr<float>(), dwi.data_ptr<float>(), S, NI, (float)scale);
   qsa_indexer_bwd_k_kernel<<<dim3(nb, B, std::min(nb, 8)), 128, smem_k, stream>>>((const bf16*)qi.data_ptr(), (const bf16*)ki.data_ptr(), wi.data_ptr<float>(),
       blse.data_ptr<float>(), dblse.data_ptr<float>(), (float)gscale, dki32.data_ptr<float>(), S, NI, (float)scale);
   C10_CUDA_KERNEL_LAUNCH_CHECK();
   count_launch(2);
-  return {dqi, dki32.to(at::kBFloat16), dwi};
+  return {dqi32.to(at::kBFloat16), dki32.to(at::kBFloat16), dwi};
 }
 
 }  // namespace q38
