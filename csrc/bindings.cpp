@@ -40,6 +40,21 @@ TORCH_LIBRARY(q38, m) {
         [](const at::Tensor& src, at::Tensor& dst, int64_t rows, int64_t cols, int64_t steps, c10::optional<at::Tensor> err) {
           q38::muon_small_ns(src, dst, rows, cols, steps, err);
         });
+  // 2-D operands (batch 1): the views and, without an output, its allocation are made here instead of in four Python calls
+  m.def("gemm2d(Tensor a, Tensor b, bool a_mn_major, bool b_mn_major, float alpha, bool fp32, Tensor err) -> Tensor",
+        [](const at::Tensor& a, const at::Tensor& b, bool amn, bool bmn, double alpha, bool fp32, at::Tensor err) {
+          TORCH_CHECK(a.dim() == 2 && b.dim() == 2, "gemm2d: 2-D operands required");
+          auto c = at::empty({a.size(amn ? 1 : 0), b.size(bmn ? 1 : 0)}, a.options().dtype(fp32 ? at::kFloat : at::kBFloat16));
+          auto c3 = c.unsqueeze(0);
+          q38::gemm_bf16_persistent(a.unsqueeze(0), b.unsqueeze(0), c3, amn, bmn, alpha, false, err, -1);
+          return c;
+        });
+  m.def("gemm2d_out(Tensor a, Tensor b, Tensor(a!) c, bool a_mn_major, bool b_mn_major, float alpha, bool accumulate, Tensor(b!) err, int splits) -> ()",
+        [](const at::Tensor& a, const at::Tensor& b, at::Tensor& c, bool amn, bool bmn, double alpha, bool acc, at::Tensor& err, int64_t splits) {
+          TORCH_CHECK(a.dim() == 2 && b.dim() == 2 && c.dim() == 2, "gemm2d_out: 2-D tensors required");
+          auto c3 = c.unsqueeze(0);
+          q38::gemm_bf16_persistent(a.unsqueeze(0), b.unsqueeze(0), c3, amn, bmn, alpha, acc, err, splits);
+        });
   m.def("cast_shadow_except(Tensor params, Tensor(a!) shadow, int skip_start, int skip_count, Tensor? err) -> ()",
         [](const at::Tensor& p, at::Tensor& sh, int64_t s0, int64_t n, c10::optional<at::Tensor> err) { q38::cast_shadow_except(p, sh, s0, n, err); });
   m.def("qsa_headprep_fwd(Tensor src, Tensor? w, Tensor cos, Tensor sin, float eps, bool split_gate, bool round_products=False) -> Tensor[]", &q38::qsa_headprep_fwd);
@@ -117,6 +132,8 @@ TORCH_LIBRARY(q38, m) {
   m.def("conv_silu_bwd(Tensor x, Tensor w, Tensor dy) -> Tensor[]");
   m.def("gdn_prep_fwd(Tensor q, Tensor k, Tensor v, Tensor g, Tensor beta, bool save=True) -> Tensor[]");
   m.def("gdn_prep_bwd(Tensor q, Tensor k, Tensor v, Tensor g, Tensor beta, Tensor Tm, Tensor w, Tensor u, Tensor vnew, Tensor states, Tensor dout, Tensor du, Tensor dstate, Tensor dd) -> Tensor[]");
+  m.def("gdn_rule_fwd(Tensor qkv, Tensor g, Tensor beta, int Hk, int Hv, Tensor? err, bool save) -> Tensor[]");
+  m.def("gdn_rule_bwd(Tensor qkv, Tensor g, Tensor beta, Tensor[] saved, Tensor dout, int Hk, int Hv, Tensor? err) -> Tensor[]");
   m.def("gdn_chain_bwd(Tensor w, Tensor P, Tensor qg, Tensor kg, Tensor dch, Tensor states, Tensor dout, int B, int H, Tensor? err=None) -> Tensor[]");
   m.def("gdn_scan_fwd(Tensor w, Tensor u, Tensor P, Tensor qg, Tensor kg, Tensor dch, int B, int H, Tensor? err=None, bool save=True) -> Tensor[]");
   m.def("gdn_scan_bwd(Tensor w, Tensor P, Tensor qg, Tensor kg, Tensor dch, Tensor vnew, Tensor states, Tensor dout, int B, int H) -> Tensor[]");
@@ -166,6 +183,8 @@ TORCH_LIBRARY_IMPL(q38, CUDA, m) {
   m.impl("gdn_prep_fwd", &q38::gdn_prep_fwd);
   m.impl("gdn_prep_bwd", &q38::gdn_prep_bwd);
   m.impl("gdn_chain_bwd", &q38::gdn_chain_bwd);
+  m.impl("gdn_rule_fwd", &q38::gdn_rule_fwd);
+  m.impl("gdn_rule_bwd", &q38::gdn_rule_bwd);
   m.impl("gdn_scan_fwd", &q38::gdn_scan_fwd);
   m.impl("gdn_scan_bwd", &q38::gdn_scan_bwd);
   m.impl("moe_route_fwd", &q38::moe_route_fwd);

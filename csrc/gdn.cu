@@ -18,6 +18,8 @@
 #include <ATen/cuda/CUDAContext.h>
 #include <c10/cuda/CUDAGuard.h>
 
+#include <array>
+
 #include "common.cuh"
 #include "host.h"
 #include "gdn_tile.cuh"
@@ -906,6 +908,31 @@ std::vector<at::Tensor> gdn_prep_bwd(const at::Tensor& q, const at::Tensor& k, c
   C10_CUDA_KERNEL_LAUNCH_CHECK();
   count_launch();
   return {dqkv, dg, dbeta};
+}
+
+// The whole rule on a packed ``qkv [B,S,(2 Hk + Hv) 64]`` tensor (q | k | v per token): the strided views are made here, one call per pass.
+static std::array<at::Tensor, 3> split_qkv(const at::Tensor& qkv, int64_t Hk, int64_t Hv) {
+  TORCH_CHECK(qkv.dim() == 3 && qkv.is_contiguous() && qkv.size(2) == (2 * Hk + Hv) * 64, "gdn_rule: contiguous [B,S,(2 Hk + Hv) 64] required");
+  const int64_t B = qkv.size(0), S = qkv.size(1), C = qkv.size(2), at0 = qkv.storage_offset();
+  auto heads = [&](int64_t first, int64_t n) { return qkv.as_strided({B, S, n, 64}, {S * C, C, 64, 1}, at0 + first * 64); };
+  return {heads(0, Hk), heads(Hk, Hk), heads(2 * Hk, Hv)};
+}
+
+// Returns {o, w, u, P, qg, kg, Tm, carry, vnew, states}: the output and what gdn_rule_bwd takes as `saved`.
+std::vector<at::Tensor> gdn_rule_fwd(const at::Tensor& qkv, const at::Tensor& g, const at::Tensor& beta, int64_t Hk, int64_t Hv, const c10::optional<at::Tensor>& err, bool save) {
+  const auto x = split_qkv(qkv, Hk, Hv);
+  auto p = gdn_prep_fwd(x[0], x[1], x[2], g, beta, save);
+  auto s = gdn_scan_fwd(p[0], p[1], p[2], p[3], p[4], p[6], qkv.size(0), Hv, err, save);
+  return {s[0], p[0], p[1], p[2], p[3], p[4], p[5], p[6], s[1], s[2]};
+}
+
+// saved = {w, u, P, qg, kg, Tm, carry, vnew, states}.  Returns {dqkv, dg, dbeta}.
+std::vector<at::Tensor> gdn_rule_bwd(const at::Tensor& qkv, const at::Tensor& g, const at::Tensor& beta, at::TensorList saved, const at::Tensor& dout, int64_t Hk, int64_t Hv,
+                                     const c10::optional<at::Tensor>& err) {
+  TORCH_CHECK(saved.size() == 9, "gdn_rule_bwd: nine saved tensors required");
+  const auto x = split_qkv(qkv, Hk, Hv);
+  auto c = gdn_chain_bwd(saved[0], saved[2], saved[3], saved[4], saved[6], saved[8], dout, qkv.size(0), Hv, err);
+  return gdn_prep_bwd(x[0], x[1], x[2], g, beta, saved[5], saved[0], saved[1], saved[7], saved[8], dout, c[0], c[1], c[2]);
 }
 
 }  // namespace q38

@@ -118,6 +118,9 @@ std::vector<at::Tensor> gdn_prep_fwd(const at::Tensor& q, const at::Tensor& k, c
 std::vector<at::Tensor> gdn_prep_bwd(const at::Tensor& q, const at::Tensor& k, const at::Tensor& v, const at::Tensor& g, const at::Tensor& beta,
                                      const at::Tensor& Tm, const at::Tensor& w, const at::Tensor& u, const at::Tensor& vnew, const at::Tensor& states,
                                      const at::Tensor& dout, const at::Tensor& du, const at::Tensor& dstate, const at::Tensor& dd);
+std::vector<at::Tensor> gdn_rule_fwd(const at::Tensor& qkv, const at::Tensor& g, const at::Tensor& beta, int64_t Hk, int64_t Hv, const c10::optional<at::Tensor>& err, bool save);
+std::vector<at::Tensor> gdn_rule_bwd(const at::Tensor& qkv, const at::Tensor& g, const at::Tensor& beta, at::TensorList saved, const at::Tensor& dout, int64_t Hk, int64_t Hv,
+                                     const c10::optional<at::Tensor>& err);
 // gdn_chain.cu
 std::vector<at::Tensor> gdn_chain_bwd(const at::Tensor& w, const at::Tensor& P, const at::Tensor& qg, const at::Tensor& kg, const at::Tensor& dch,
                                       const at::Tensor& states, const at::Tensor& dout, int64_t B, int64_t H, const c10::optional<at::Tensor>& err);

@@ -35,11 +35,12 @@ def load():
 
 def error_flag(device=None):
     """Per-device int32 word into which kernels record a bounded-wait timeout or a failed self-check."""
-    device = torch.device("cuda", torch.cuda.current_device()) if device is None else torch.device(device)
-    key = device.index
-    if key not in _error_flags:
-        _error_flags[key] = torch.zeros(1, dtype=torch.int32, device=device)
-    return _error_flags[key]
+    if type(device) is not torch.device or device.index is None:
+        device = torch.device("cuda", torch.cuda.current_device()) if device is None else torch.device(device)
+    flag = _error_flags.get(device.index)
+    if flag is None:
+        flag = _error_flags[device.index] = torch.zeros(1, dtype=torch.int32, device=device)
+    return flag
 
 
 ERROR_NAMES = {1: "TMA stage never arrived", 2: "tensor core never released a stage", 3: "accumulator never became ready",
@@ -78,6 +79,13 @@ def gemm(a, b, out=None, a_mn_major=False, b_mn_major=False, alpha=1.0, accumula
     sums are added atomically (the summation order, hence the last bits, then vary from run to run)."""
     ops = load()
     squeeze = a.dim() == 2
+    if squeeze and PERSISTENT_GEMM and addend is None and b.dim() == 2 and (out is None or out.dim() == 2) and (out is not None or not accumulate):
+        if out is None:                       # the common products: views and output are made in one native call
+            if out_dtype in (torch.bfloat16, torch.float32):
+                return ops.gemm2d(a, b, a_mn_major, b_mn_major, float(alpha), out_dtype == torch.float32, error_flag(a.device))
+        else:
+            ops.gemm2d_out(a, b, out, a_mn_major, b_mn_major, float(alpha), bool(accumulate), error_flag(a.device), int(splits))
+            return out
     if squeeze:
         a, b = a.unsqueeze(0), b.unsqueeze(0)
     M = a.shape[2] if a_mn_major else a.shape[1]

@@ -379,31 +379,17 @@ class _DeltaRule(torch.autograd.Function):
     @staticmethod
     def forward(ctx, qkv, g, beta, Hk, Hv):
         ops = load()
-        qkv = qkv.contiguous()
-        B, S, _ = qkv.shape
-        q = qkv[..., :Hk * 64].unflatten(-1, (Hk, 64))
-        k = qkv[..., Hk * 64:2 * Hk * 64].unflatten(-1, (Hk, 64))
-        v = qkv[..., 2 * Hk * 64:].unflatten(-1, (Hv, 64))
-        g, beta = g.float().contiguous(), beta.to(torch.bfloat16).contiguous()
-        save = any(ctx.needs_input_grad)          # without a backward pass neither Tm nor the chunk states nor v_new are written
-        w, u, P, qg, kg, Tm, carry, _gc = ops.gdn_prep_fwd(q, k, v, g, beta, save)
-        o, vnew, states = ops.gdn_scan_fwd(w, u, P, qg, kg, carry, B, Hv, error_flag(qkv.device), save)
-        ctx.save_for_backward(qkv, g, beta, Tm, w, u, P, qg, kg, carry, vnew, states)
+        qkv, g, beta = qkv.contiguous(), g.float().contiguous(), beta.to(torch.bfloat16).contiguous()
+        # without a backward pass neither Tm nor the chunk states nor v_new are written
+        o, *saved = ops.gdn_rule_fwd(qkv, g, beta, Hk, Hv, error_flag(qkv.device), any(ctx.needs_input_grad))
+        ctx.save_for_backward(qkv, g, beta, *saved)
         ctx.heads = (Hk, Hv)
         return o
 
     @staticmethod
     def backward(ctx, do):
-        ops = load()
-        qkv, g, beta, Tm, w, u, P, qg, kg, carry, vnew, states = ctx.saved_tensors
-        Hk, Hv = ctx.heads
-        B = qkv.shape[0]
-        q = qkv[..., :Hk * 64].unflatten(-1, (Hk, 64))
-        k = qkv[..., Hk * 64:2 * Hk * 64].unflatten(-1, (Hk, 64))
-        v = qkv[..., 2 * Hk * 64:].unflatten(-1, (Hv, 64))
-        do = do.to(torch.bfloat16).contiguous()
-        du, dstate, dd = ops.gdn_chain_bwd(w, P, qg, kg, carry, states, do, B, Hv, error_flag(qkv.device))
-        dqkv, dg, dbeta = ops.gdn_prep_bwd(q, k, v, g, beta, Tm, w, u, vnew, states, do, du, dstate, dd)
+        qkv, g, beta, *saved = ctx.saved_tensors
+        dqkv, dg, dbeta = load().gdn_rule_bwd(qkv, g, beta, saved, do.to(torch.bfloat16).contiguous(), *ctx.heads, error_flag(qkv.device))
         return dqkv, dg, dbeta, None, None
 
 
