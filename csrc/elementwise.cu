@@ -162,18 +162,25 @@ __global__ void __launch_bounds__(256) gated_rmsnorm_bwd_kernel(const __nv_bfloa
   const long long first = ((long long)blockIdx.x * 256 + threadIdx.x) >> 3;
   // every 8-lane group walks rows first, first + stride, ...; the loop bound is uniform per warp up to the last iteration,
   // where finished groups keep shuffling on zeros
+  // the next row's three pieces are in flight while the current one is evaluated (344064 rows: 55 -> 44 us; the bytes need 34)
+  uint4 nx, ng, nd;
+  auto fetch = [&](long long row) {
+    nx = ng = nd = make_uint4(0, 0, 0, 0);
+    if (row < rows) {
+      nx = reinterpret_cast<const uint4*>(x + row * 64)[sub];
+      ng = reinterpret_cast<const uint4*>(gate + row * 64)[sub];
+      nd = reinterpret_cast<const uint4*>(dy + row * 64)[sub];
+    }
+  };
+  fetch(first);
   for (long long base = first - (threadIdx.x >> 3 & 3); base < rows; base += stride) {
     const long long row = base + (threadIdx.x >> 3 & 3);
     const bool live = row < rows;
     float xv[8], gv[8], dv[8];
-    if (live) {
-      unpack8(reinterpret_cast<const uint4*>(x + row * 64)[sub], xv);
-      unpack8(reinterpret_cast<const uint4*>(gate + row * 64)[sub], gv);
-      unpack8(reinterpret_cast<const uint4*>(dy + row * 64)[sub], dv);
-    } else {
-#pragma unroll
-      for (int i = 0; i < 8; ++i) xv[i] = gv[i] = dv[i] = 0.f;
-    }
+    unpack8(nx, xv);
+    unpack8(ng, gv);
+    unpack8(nd, dv);
+    fetch(row + stride);
     float ss = 0.f;
 #pragma unroll
     for (int i = 0; i < 8; ++i) ss += xv[i] * xv[i];
@@ -200,7 +207,11 @@ __global__ void __launch_bounds__(256) gated_rmsnorm_bwd_kernel(const __nv_bfloa
     }
   }
 #pragma unroll
-  for (int i = 0; i < 8; ++i) atomicAdd(&dw_acc[8 * sub + i], dwv[i]);
+  for (int i = 0; i < 8; ++i) {
+    dwv[i] += __shfl_xor_sync(0xffffffffu, dwv[i], 8);
+    dwv[i] += __shfl_xor_sync(0xffffffffu, dwv[i], 16);
+    if ((threadIdx.x & 31) < 8) atomicAdd(&dw_acc[8 * sub + i], dwv[i]);
+  }
   __syncthreads();
   if (threadIdx.x < 64) atomicAdd(&dw[threadIdx.x], dw_acc[threadIdx.x]);
 }
