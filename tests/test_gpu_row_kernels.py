@@ -1,0 +1,77 @@
+"""Row kernels of the expert block, the head preparation and the loss at the edges of their pieces, against PyTorch."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def lib():
+    from q38 import ops
+    ops.install()
+    return ops.load()
+
+
+# one pair, one block of 1024 pairs and one more, enough blocks that the scan's sixteen segments hold one and two of them
+@pytest.mark.parametrize("T,k,E", [(1, 1, 1), (1024, 1, 3), (205, 5, 64), (16 * 1024, 1, 64), (4 * 1024 + 1, 4, 7)])
+def test_sort_and_row_sums(lib, T, k, E):
+    gen = torch.Generator(device="cuda").manual_seed(T)
+    top = torch.randint(0, E, (T, k), device="cuda", generator=gen, dtype=torch.int32)
+    perm, inv, offsets, sched = lib.moe_sort(top, E, None)
+    order = torch.sort(top.flatten().long(), stable=True).indices
+    assert torch.equal(perm.long(), order) and torch.equal(inv.long()[order], torch.arange(T * k, device="cuda"))
+    counts = torch.bincount(top.flatten().long(), minlength=E)
+    assert torch.equal(offsets.long(), torch.cat([counts.new_zeros(1), counts.cumsum(0)]))
+    tiles = [(e, int(offsets[e]) + r, min(128, int(counts[e]) - r)) for e in range(E) for r in range(0, int(counts[e]), 128)]
+    got = sched[1:].view(-1, 3)
+    assert int(sched[0]) == len(tiles) and got[:len(tiles)].tolist() == [list(t) for t in tiles] and not got[len(tiles):, 2].any()
+    for h in (8, 36, 264):                                     # one 16-byte piece, no whole pieces, more pieces than a warp
+        rows = torch.randn(T * k, h, device="cuda", generator=gen).to(torch.bfloat16)
+        w = torch.rand(T, k, device="cuda", generator=gen)
+        pairs = rows[inv.long()].view(T, k, h)
+        want, plain = torch.zeros(T, h, device="cuda"), torch.zeros(T, h, device="cuda")
+        for j in range(k):                                     # slot order, each weighted row rounded to bf16 first
+            want += (pairs[:, j].float() * w[:, j, None]).to(torch.bfloat16).float()
+            plain += pairs[:, j].float()
+        assert torch.equal(lib.moe_combine_fwd(rows, inv, w), want.to(torch.bfloat16))
+        assert torch.equal(lib.moe_unpermute_sum(rows, inv, T, k), plain.to(torch.bfloat16))
+
+
+@pytest.mark.parametrize("B,S,H", [(1, 1, 1), (2, 3, 5), (1, 1000, 2)])
+def test_rotary_with_rounded_products(lib, B, S, H):
+    from q38.models import modeling
+    gen = torch.Generator(device="cuda").manual_seed(S)
+    x = torch.randn(B, S, H, 64, device="cuda", generator=gen).to(torch.bfloat16)
+    cos, sin = modeling.rope_tables(torch.arange(S, device="cuda")[None], 16, 1e7, torch.float32)
+    out = lib.qsa_headprep_fwd(x, None, cos, sin, 0.0, False, True)[0]
+    assert torch.equal(out, modeling.apply_rope(x.transpose(1, 2), cos, sin))
+    shifted = torch.empty(x.numel() + 1, device="cuda", dtype=torch.bfloat16)[1:].view_as(x).copy_(x)      # contiguous, but not on 16 bytes
+    assert torch.equal(lib.qsa_headprep_fwd(shifted, None, cos, sin, 0.0, False, True)[0], out)
+
+
+@pytest.mark.parametrize("n", [8, 2048, 2056])
+def test_scale(lib, n):
+    from q38.ops.backend import scale_bf16
+    x = torch.randn(n, device="cuda").to(torch.bfloat16)
+    f = torch.tensor(0.37, device="cuda").to(torch.bfloat16)
+    assert torch.equal(scale_bf16(x, f), x * f) and torch.equal(scale_bf16(x[1:], f), x[1:] * f)
+
+
+@pytest.mark.parametrize("rows", [0, 1, 8192, 8193])
+def test_loss_over_chunk_edges(lib, rows):
+    from q38.models import modeling
+    V, h = 128, 64
+    gen = torch.Generator(device="cuda").manual_seed(rows)
+    hid = torch.randn(rows, h, device="cuda", generator=gen).to(torch.bfloat16).requires_grad_()
+    w = (torch.randn(V, h, device="cuda", generator=gen) / 4).requires_grad_()
+    tgt = torch.randint(0, V, (rows,), device="cuda", generator=gen)
+    loss = modeling.get_backend().linear_cross_entropy(w, hid, tgt, "sum")
+    loss.backward()
+    hr, wr = hid.detach().double().requires_grad_(), w.detach().to(torch.bfloat16).double().requires_grad_()
+    ref = torch.nn.functional.cross_entropy(hr @ wr.t(), tgt, reduction="sum")
+    ref.backward()
+    assert hid.grad.shape == hid.shape
+    if rows:
+        # logits of rms 2 rounded to bf16 (3e-3, so the probabilities move by 0.3 %), then their bf16 gradients and the bf16 outputs (2e-3 rms each)
+        rel = lambda a, b: ((a.double() - b).norm() / b.norm()).item()
+        assert abs(loss.item() - ref.item()) < 5e-3 * abs(ref.item()) + 5e-2 and rel(hid.grad, hr.grad) < 2e-2 and rel(w.grad, wr.grad) < 2e-2
