@@ -10,10 +10,6 @@ constexpr int C64 = 64, LDS = 72;                 // 64x64 bf16 tiles padded to 
 constexpr int TILE_ELEMS = C64 * LDS;
 using bf16 = __nv_bfloat16;
 
-__device__ __forceinline__ uint32_t pack2(bf16 a, bf16 b) {
-  return (uint32_t)__bfloat16_as_ushort(a) | ((uint32_t)__bfloat16_as_ushort(b) << 16);
-}
-
 __device__ __forceinline__ void mma16816(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
   asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
                : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
@@ -97,27 +93,6 @@ __device__ __forceinline__ void load_tile_async(bf16* __restrict__ dst, const bf
 }
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int N> __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
-
-
-// Fragment of a dense [64,64] bf16 tile in global memory.
-__device__ __forceinline__ void frag_from_global(const bf16* __restrict__ src, float (&dst)[8][4], int warp, int lane) {
-  const int r = 16 * warp + (lane >> 2), cq = 2 * (lane & 3);
-#pragma unroll
-  for (int nt = 0; nt < 8; ++nt) {
-    const __nv_bfloat162 a = *reinterpret_cast<const __nv_bfloat162*>(src + r * 64 + 8 * nt + cq);
-    const __nv_bfloat162 b2 = *reinterpret_cast<const __nv_bfloat162*>(src + (r + 8) * 64 + 8 * nt + cq);
-    dst[nt][0] = __low2float(a); dst[nt][1] = __high2float(a); dst[nt][2] = __low2float(b2); dst[nt][3] = __high2float(b2);
-  }
-}
-__device__ __forceinline__ void frag_from_smem(const bf16* __restrict__ src, float (&dst)[8][4], int warp, int lane) {
-  const int r = 16 * warp + (lane >> 2), cq = 2 * (lane & 3);
-#pragma unroll
-  for (int nt = 0; nt < 8; ++nt) {
-    const __nv_bfloat162 a = *reinterpret_cast<const __nv_bfloat162*>(src + r * LDS + 8 * nt + cq);
-    const __nv_bfloat162 b2 = *reinterpret_cast<const __nv_bfloat162*>(src + (r + 8) * LDS + 8 * nt + cq);
-    dst[nt][0] = __low2float(a); dst[nt][1] = __high2float(a); dst[nt][2] = __low2float(b2); dst[nt][3] = __high2float(b2);
-  }
-}
 
 // ---- half-width variants for CTAs of eight warps -----------------------------------------------------------------------
 // Warp w owns rows 16 (w & 3) .. +15 and columns 32 (w >> 2) .. +31 of the 64x64 output: twice the warps of mma64 work on
