@@ -69,7 +69,7 @@ __global__ void __launch_bounds__(32 * W) gdn_chain_bwd_kernel(const __grid_cons
     d_next = dch[(long long)bh * NT + (c > 0 ? c - 1 : 0)];
     cp_async_wait<1>();
     __syncwarp();
-    if (!ptx::mbar_wait(&full[stage], phase)) { dead = 1; if (lane == 0) report_error(err, ERR_TMA_WAIT); }
+    if (!ptx::mbar_wait_warp(&full[stage], phase)) { dead = 1; if (lane == 0) report_error(err, ERR_TMA_WAIT); }
     const uint32_t wt = tiles + stage * 4 * TILE_BYTES, pt = wt + TILE_BYTES, qt = pt + TILE_BYTES, kt = qt + TILE_BYTES;
     const uint32_t mine = pairs + (i & 1) * 2 * SLICE_BYTES;
     if (!dead) {

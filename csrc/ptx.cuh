@@ -42,6 +42,11 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, uint32
   }
   return false;
 }
+// The same for a whole warp: every lane gets the same verdict, so that instructions which need all lanes (ldmatrix, mma.sync, shuffles)
+// may follow under it.  Each lane polls for itself and could otherwise run out one poll before the barrier completes for its neighbour.
+__device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, uint32_t limit = (1u << 22)) {
+  return __all_sync(0xffffffffu, mbar_wait(bar, parity, limit));
+}
 
 // ---- TMA ----------------------------------------------------------------------------------------------------
 __device__ __forceinline__ void prefetch_tensormap(const CUtensorMap* m) {
