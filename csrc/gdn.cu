@@ -749,9 +749,10 @@ __global__ void __launch_bounds__(256, 2) gdn_prep_bwd_kernel(const bf16* __rest
       }
     }
     // ---- dM = -(A w^T + B u^T); L_ij = beta_i (kn_i.kn_j) Gamma_ij (j < i) ----
-    // The tile holds beta_i dL_ij Gamma_ij; beta is floored so that a row with beta = 0 still yields its beta gradient by the division
-    // below (what the floor adds elsewhere is 1e-18 of dL).
-    const float flo = fmaxf(blo, 8.6736174e-19f), fhi = fmaxf(bhi, 8.6736174e-19f);
+    // The tile holds beta_i dL_ij Gamma_ij; the magnitude of beta is floored so that a row with beta = 0 still yields its beta gradient by the
+    // division below (what the floor adds elsewhere is 1e-18 of dL).  Its sign stays, and a NaN stays one.
+    auto floored = [](float x) { return fabsf(x) < 8.6736174e-19f ? copysignf(8.6736174e-19f, x) : x; };
+    const float flo = floored(blo), fhi = floored(bhi);
     zero_acc(acc);
     mma64h<false, true>(St, Wt, acc, warp, lane);
     mma64h<false, true>(Do, Ut, acc, warp, lane);

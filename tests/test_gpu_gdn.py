@@ -86,3 +86,24 @@ def test_delta_rule_gradients(ops, B, S, Hk, Hv, decay):
         assert rel(g.grad, ref[1].grad) < 2.5e-2
     zero = beta.detach() == 0
     assert rel(beta.grad[zero], ref[2].grad[zero]) < 2e-2
+
+
+def test_delta_rule_gradients_with_negative_beta(ops):
+    """The rule is defined for any beta; a sigmoid never gives a negative one, a caller of the rule may."""
+    from q38.ops.backend import _DeltaRule
+    B, S, Hk, Hv = 1, 192, 2, 6
+    gen = torch.Generator(device="cuda").manual_seed(3)
+    qkv = torch.randn(B, S, (2 * Hk + Hv) * 64, device="cuda", generator=gen).to(torch.bfloat16).requires_grad_()
+    g = (-0.1 * torch.rand(B, S, Hv, device="cuda", generator=gen)).requires_grad_()
+    beta = (torch.rand(B, S, Hv, device="cuda", generator=gen) - 0.5).to(torch.bfloat16)
+    beta[:, ::7] = 0
+    beta.requires_grad_()
+    do = torch.randn(B, S, Hv, 64, device="cuda", generator=gen).to(torch.bfloat16)
+    _DeltaRule.apply(qkv, g, beta, Hk, Hv).backward(do)
+    ops.check_errors()
+    ref = [t.detach().double().requires_grad_() for t in (qkv, g, beta)]
+    recurrence(*ref, Hk, Hv).backward(do.double())
+    # the bounds of the positive case: bf16 chunk operands, 2e-3 rms each
+    assert rel(qkv.grad, ref[0].grad) < 2e-2 and rel(beta.grad, ref[2].grad) < 2e-2 and rel(g.grad, ref[1].grad) < 2.5e-2
+    for part in (beta.detach() < 0, beta.detach() == 0):
+        assert rel(beta.grad[part], ref[2].grad[part]) < 2e-2
