@@ -91,44 +91,56 @@ __global__ void __launch_bounds__(SK) mhc_sinkhorn_fwd_kernel(float* __restrict_
   for (int m = 0; m < 4; ++m) row[m] = make_float4(p[4 * m], p[4 * m + 1], p[4 * m + 2], p[4 * m + 3]);
 }
 
-// dcoef[t, 8..24): d(residual mix) in, d(logits) out.  Only the divisors are kept; the iterates follow from them backwards (p before a division is
-// p after it times the divisor), and y = p / sum(p)  =>  dp = (dy - sum(dy * y)) / s.
+// dcoef[t, 8..24): d(residual mix) in, d(logits) out; y = p / sum(p)  =>  dp = (dy - sum(dy * y)) / s.  The iterate at the start of every
+// iteration is kept (64 bytes a token; five CTAs fit an SM at the presets' 20 iterations), its half steps are done again on the way back, so
+// every y is the one of the forward.  Going back by p *= s from the divisors alone costs 20 KB instead of 40 and rounds p forty times: the same
+// error on logits of ordinary spread, a hundred times as much on a token in a thousand whose logits span sixty.
 __global__ void __launch_bounds__(SK) mhc_sinkhorn_bwd_kernel(const float* __restrict__ zsave, MhcParams P, float* __restrict__ dcoef, int T, int iters) {
-  extern __shared__ float divisors[];        // [iters][8][SK]
+  extern __shared__ float iterates[];        // [iters][16][SK]
   const int t = blockIdx.x * SK + threadIdx.x;
   if (t >= T) return;
-  float logit[16], p[16], p0[16], d[16];
+  float logit[16], p[16], d[16];
   const float a2 = P.alphas[2];
 #pragma unroll
   for (int i = 0; i < 16; ++i) { logit[i] = P.b_res[i] + a2 * zsave[(size_t)t * NCOEF + 8 + i]; d[i] = dcoef[(size_t)t * NCOEF + 8 + i]; }
-  sinkhorn_start(logit, p0);
-#pragma unroll
-  for (int i = 0; i < 16; ++i) p[i] = p0[i];
-  float* sv = divisors + threadIdx.x;
+  sinkhorn_start(logit, p);
+  float* sv = iterates + threadIdx.x;
+  auto drop = [](int, float) {};
 #pragma unroll 1
   for (int it = 0; it < iters; ++it) {
-    sinkhorn_half<4, 1>(p, [&](int g, float s) { sv[(8 * it + g) * SK] = s; });
-    sinkhorn_half<1, 4>(p, [&](int g, float s) { sv[(8 * it + 4 + g) * SK] = s; });
+#pragma unroll
+    for (int i = 0; i < 16; ++i) sv[(16 * it + i) * SK] = p[i];
+    sinkhorn_half<4, 1>(p, drop);
+    sinkhorn_half<1, 4>(p, drop);
   }
-  auto back = [&](auto group, auto step, const float* s4) {
+  auto back = [&](auto group, auto step, const float (&y)[16], const float (&s)[4]) {
     constexpr int GS = decltype(group)::value, KS = decltype(step)::value;
 #pragma unroll
     for (int g = 0; g < 4; ++g) {
-      const float s = s4[g * SK];
-      float dot = 0.f;
+      float e[4];
 #pragma unroll
-      for (int k = 0; k < 4; ++k) dot += d[g * GS + k * KS] * p[g * GS + k * KS];
+      for (int k = 0; k < 4; ++k) e[k] = d[g * GS + k * KS] * y[g * GS + k * KS];
+      const float dot = (e[0] + e[1]) + (e[2] + e[3]);
 #pragma unroll
-      for (int k = 0; k < 4; ++k) { d[g * GS + k * KS] = (d[g * GS + k * KS] - dot) / s; p[g * GS + k * KS] *= s; }
+      for (int k = 0; k < 4; ++k) d[g * GS + k * KS] = (d[g * GS + k * KS] - dot) / s[g];
     }
   };
 #pragma unroll 1
   for (int it = iters - 1; it >= 0; --it) {
-    back(std::integral_constant<int, 1>(), std::integral_constant<int, 4>(), sv + (8 * it + 4) * SK);
-    back(std::integral_constant<int, 4>(), std::integral_constant<int, 1>(), sv + 8 * it * SK);
-  }
+    float mid[16], rows[4], cols[4];
 #pragma unroll
-  for (int i = 0; i < 16; ++i) dcoef[(size_t)t * NCOEF + 8 + i] = d[i] * p0[i];     // the shift by the maximum cancels in the normalisations
+    for (int i = 0; i < 16; ++i) mid[i] = sv[(16 * it + i) * SK];
+    sinkhorn_half<4, 1>(mid, [&](int g, float s) { rows[g] = s; });
+    float end[16];
+#pragma unroll
+    for (int i = 0; i < 16; ++i) end[i] = mid[i];
+    sinkhorn_half<1, 4>(end, [&](int g, float s) { cols[g] = s; });
+    back(std::integral_constant<int, 1>(), std::integral_constant<int, 4>(), end, cols);
+    back(std::integral_constant<int, 4>(), std::integral_constant<int, 1>(), mid, rows);
+  }
+  sinkhorn_start(logit, p);
+#pragma unroll
+  for (int i = 0; i < 16; ++i) dcoef[(size_t)t * NCOEF + 8 + i] = d[i] * p[i];     // the shift by the maximum cancels in the normalisations
 }
 
 // d(logit) given d(result); y = p / sum(p)  =>  dp = (dy - sum(dy * y)) / s
@@ -810,7 +822,12 @@ std::vector<at::Tensor> mhc_pre_bwd_a(const at::Tensor& dxout, const at::Tensor&
 #undef Q38_ROWS
     C10_CUDA_KERNEL_LAUNCH_CHECK();
     count_launch();
-    mhc_sinkhorn_bwd_kernel<<<(T + SK - 1) / SK, SK, 8 * SK * iters * sizeof(float), stream>>>(z.data_ptr<float>(), P, dcoef.data_ptr<float>(), T, (int)iters);
+    static bool configured = false;
+    if (!configured) {
+      C10_CUDA_CHECK(cudaFuncSetAttribute(mhc_sinkhorn_bwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 16 * SK * MAX_SINKHORN * (int)sizeof(float)));
+      configured = true;
+    }
+    mhc_sinkhorn_bwd_kernel<<<(T + SK - 1) / SK, SK, 16 * SK * iters * sizeof(float), stream>>>(z.data_ptr<float>(), P, dcoef.data_ptr<float>(), T, (int)iters);
     C10_CUDA_KERNEL_LAUNCH_CHECK();
     count_launch();
     mhc_coef_bwd_kernel<<<std::min((T + CW - 1) / CW, 8 * kNumSMs), 32 * CW, (NCOEF * (r + 1) + 32) * sizeof(float), stream>>>(

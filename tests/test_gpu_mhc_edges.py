@@ -50,3 +50,41 @@ def test_coefficients_and_gradients(T, iters):
     assert rel(Y, Yr.detach()) < 5e-3 and rel(X.grad, Xr.grad) < 1e-2
     for name in ("b_res", "b_pre", "b_post"):
         assert rel(dict(mhc.named_parameters())[name].grad, ref[name].grad) < 2e-2, name
+
+
+def sinkhorn_gradient(logits, d, iters):
+    """d(logits) of the iterated row and column normalisation, from kept iterates, in the dtype of the arguments."""
+    p0 = p = torch.exp(logits - logits.amax((-2, -1), keepdim=True))
+    kept = []
+    for _ in range(iters):
+        for dim in (-1, -2):
+            s = p.sum(dim, keepdim=True).clamp(min=1e-9)
+            p = p / s
+            kept.append((p, s, dim))
+    for y, s, dim in reversed(kept):
+        d = (d - (d * y).sum(dim, keepdim=True)) / s
+    return d * p0
+
+
+def test_sinkhorn_gradient_of_widely_spread_logits():
+    """Logits that span eighty: the gradient is as good as iterates kept in 32 bits give it.  Iterates rebuilt on the way back are not."""
+    from q38 import ops
+    ops.install()
+    T, h, iters, a2 = 65536, 64, 20, 64.0
+    gen = torch.Generator(device="cuda").manual_seed(0)
+    z = (torch.randn(T, 24, device="cuda", generator=gen) * (20 / a2)).clamp(-0.9, 0.9)
+    dcoef = torch.randn(T, 24, device="cuda", generator=gen)
+    dcoef[:, :8] = 0
+    zeros = lambda *s: torch.zeros(*s, device="cuda")
+    alphas = torch.tensor([0.0, 0.0, a2], device="cuda")
+    logits, d = (a2 * z[:, 8:]).view(T, 4, 4), dcoef[:, 8:].clone().view(T, 4, 4)
+    # with an identity as the second projection and unit norms, dL_raw is d(logits) alphas (1 - z^2) of every token
+    dL = ops.load().mhc_pre_bwd_a(zeros(T, h), zeros(T, 4, h), zeros(T, 24), torch.eye(24, device="cuda"), zeros(4), zeros(4), zeros(16), alphas, zeros(h),
+                                  zeros(T, 24), z, zeros(T) + 1, zeros(T) + 1, dcoef, iters)[0]
+    ref = sinkhorn_gradient(logits.double(), d.double(), iters) * (a2 * (1 - z[:, 8:].double() ** 2)).view(T, 4, 4)
+    err = lambda x: (x.double().view(T, 16) - ref.view(T, 16)).norm(dim=1) / ref.view(T, 16).norm(dim=1)
+    good = err(sinkhorn_gradient(logits, d, iters) * (a2 * (1 - z[:, 8:] ** 2)).view(T, 4, 4)) < 1e-5
+    assert good.float().mean() > 0.95
+    got = err(dL[:, 8:])[good]
+    # 1e-5 of the 32-bit formula, times up to twenty for the kernel's approximate exponential (some 60 units in the last place at -80) and divisions
+    assert got.max() < 2e-4 and got.mean() < 3e-6, (got.max().item(), got.mean().item())
