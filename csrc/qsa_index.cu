@@ -258,7 +258,8 @@ __global__ void __launch_bounds__(256) qsa_select_kernel(const float* __restrict
 // Warps 0-3 hold heads 0 and 1, warps 4-7 heads 2 and 3, each warp 16 queries; the two partial scores of a tile meet in shared memory.
 // Eight 64^3 products per pair (one CTA per head had twenty).  Bound by the latency of their chain: a tile costs a CTA four times its issue slots, and
 // the last query block has 64 tiles.  So tiles are taken in quarters of 16 keys, which keeps two CTAs on an SM (128 registers), and the key
-// blocks j <= i of a query block are shared by gridDim.z CTAs (j = z, z + gridDim.z, ...) whose partial gradients are added in fp32.  About 255 us;
+// blocks j <= i of a query block are shared by gridDim.z CTAs (j = z, z + gridDim.z, ...).  Each leaves its partial gradients in its own slice of
+// dqi [z,B,NI,S,64] and dwi [z,B,S,NI], which the kernel below adds in ascending z: no atomics, the same bits in every run.  About 255 us;
 // one CTA of eight warps per query block and SM took 306, sixteen warps with one head per four of them 396 (four times the exponentials).
 __global__ void __launch_bounds__(256, 2) qsa_indexer_bwd_q_kernel(const bf16* __restrict__ qi, const bf16* __restrict__ ki, const float* __restrict__ wi,
                                                                    const float* __restrict__ blse, const float* __restrict__ dblse, float gscale,
@@ -361,20 +362,43 @@ __global__ void __launch_bounds__(256, 2) qsa_indexer_bwd_q_kernel(const bf16* _
   for (int x = 0; x < 2; ++x) {
     if (x < heads) {
       const int own = 2 * grp + x;
-      float* dst = dqi + (((long long)b * NI + own) * S + (long long)i * 64) * 64;
+      float* dst = dqi + ((((long long)blockIdx.z * gridDim.y + b) * NI + own) * S + (long long)i * 64) * 64;
 #pragma unroll
       for (int nt = 0; nt < 8; ++nt)
 #pragma unroll
         for (int hr = 0; hr < 2; ++hr)
-          atomicAdd(reinterpret_cast<float2*>(dst + (r0 + 8 * hr) * 64 + 8 * nt + cq), make_float2(dq[x][nt][2 * hr], dq[x][nt][2 * hr + 1]));
+          *reinterpret_cast<float2*>(dst + (r0 + 8 * hr) * 64 + 8 * nt + cq) = make_float2(dq[x][nt][2 * hr], dq[x][nt][2 * hr + 1]);
 #pragma unroll
       for (int hr = 0; hr < 2; ++hr) {
         float v = dw[x][hr];
         v += __shfl_xor_sync(0xffffffffu, v, 1);
         v += __shfl_xor_sync(0xffffffffu, v, 2);
-        if ((lane & 3) == 0) atomicAdd(&dwi[(row + 8 * hr) * NI + own], v);
+        if ((lane & 3) == 0) dwi[((long long)blockIdx.z * gridDim.y * S + row + 8 * hr) * NI + own] = v;
       }
     }
+  }
+}
+
+// The query pass' partial gradients added up: query block i has min(i + 1, Z) of them.  One thread per eight dims of a row; the
+// first of a row's eight threads also takes its head weight.
+__global__ void __launch_bounds__(256) qsa_indexer_sum_q_kernel(const float* __restrict__ part, const float* __restrict__ dw_part, bf16* __restrict__ dqi,
+                                                                float* __restrict__ dwi, int B, int NI, int S, int Z) {
+  const long long id = (long long)blockIdx.x * 256 + threadIdx.x, rows = (long long)B * NI * S, row = id >> 3;
+  if (row >= rows) return;
+  const int s = (int)(row % S), n = min(s / 64 + 1, Z);
+  float v[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+  for (int z = 0; z < n; ++z) {
+    const float4* src = reinterpret_cast<const float4*>(part + (z * rows * 8 + id) * 8);
+    const float4 a = src[0], c = src[1];
+    v[0] += a.x; v[1] += a.y; v[2] += a.z; v[3] += a.w;
+    v[4] += c.x; v[5] += c.y; v[6] += c.z; v[7] += c.w;
+  }
+  reinterpret_cast<uint4*>(dqi)[id] = make_uint4(pack_f2(v[0], v[1]), pack_f2(v[2], v[3]), pack_f2(v[4], v[5]), pack_f2(v[6], v[7]));
+  if ((id & 7) == 0) {
+    const long long bh = row / S, at = ((bh / NI) * S + s) * NI + bh % NI;
+    float w = 0.f;
+    for (int z = 0; z < n; ++z) w += dw_part[z * rows + at];
+    dwi[at] = w;
   }
 }
 
@@ -573,9 +597,11 @@ std::vector<at::Tensor> qsa_indexer_bwd(const at::Tensor& qi, const at::Tensor& 
                                         double gscale, double scale) {
   const c10::cuda::CUDAGuard guard(qi.device());
   const int B = qi.size(0), NI = qi.size(1), S = qi.size(2), nb = S / 64;
-  auto dqi32 = at::zeros(qi.sizes(), qi.options().dtype(at::kFloat));
-  auto dki32 = at::zeros(ki.sizes(), ki.options().dtype(at::kFloat));
-  auto dwi = at::zeros_like(wi);
+  const int Z = std::min(nb, 4);
+  auto f32 = qi.options().dtype(at::kFloat);
+  auto part = at::empty({Z, B, NI, S, 64}, f32), dw_part = at::empty({Z, B, S, NI}, f32);
+  auto dqi = at::empty(qi.sizes(), qi.options()), dwi = at::empty(wi.sizes(), wi.options());
+  auto dki32 = at::zeros(ki.sizes(), f32);
   constexpr int smem_q = (NI_MAX + 2) * TILE_ELEMS * 2 + 16 * 128 * 16, smem_k = 2 * NI_MAX * TILE_ELEMS * 2 + 2 * (2 + NI_MAX) * 64 * 4;
   static bool cfg = false;
   if (!cfg) {
@@ -584,13 +610,15 @@ std::vector<at::Tensor> qsa_indexer_bwd(const at::Tensor& qi, const at::Tensor& 
     cfg = true;
   }
   auto stream = at::cuda::getCurrentCUDAStream();
-  qsa_indexer_bwd_q_kernel<<<dim3(nb, B, std::min(nb, 4)), 256, smem_q, stream>>>((const bf16*)qi.data_ptr(), (const bf16*)ki.data_ptr(), wi.data_ptr<float>(), blse.data_ptr<float>(),
-      dblse.data_ptr<float>(), (float)gscale, dqi32.data_ptr<float>(), dwi.data_ptr<float>(), S, NI, (float)scale);
+  qsa_indexer_bwd_q_kernel<<<dim3(nb, B, Z), 256, smem_q, stream>>>((const bf16*)qi.data_ptr(), (const bf16*)ki.data_ptr(), wi.data_ptr<float>(), blse.data_ptr<float>(),
+      dblse.data_ptr<float>(), (float)gscale, part.data_ptr<float>(), dw_part.data_ptr<float>(), S, NI, (float)scale);
+  qsa_indexer_sum_q_kernel<<<(unsigned)(((long long)B * NI * S * 8 + 255) / 256), 256, 0, stream>>>(part.data_ptr<float>(), dw_part.data_ptr<float>(), (bf16*)dqi.data_ptr(),
+      dwi.data_ptr<float>(), B, NI, S, Z);
   qsa_indexer_bwd_k_kernel<<<dim3(nb, B, std::min(nb, 8)), 128, smem_k, stream>>>((const bf16*)qi.data_ptr(), (const bf16*)ki.data_ptr(), wi.data_ptr<float>(),
       blse.data_ptr<float>(), dblse.data_ptr<float>(), (float)gscale, dki32.data_ptr<float>(), S, NI, (float)scale);
   C10_CUDA_KERNEL_LAUNCH_CHECK();
-  count_launch(2);
-  return {dqi32.to(at::kBFloat16), dki32.to(at::kBFloat16), dwi};
+  count_launch(3);
+  return {dqi, dki32.to(at::kBFloat16), dwi};
 }
 
 }  // namespace q38

@@ -674,7 +674,7 @@ class Backend:
         self.layouts = dict(nt=True, nn=True, tn=True)       # which GEMM operand layouts passed the self-check
         # True: chunk operands come from the PyTorch specification and only the scan runs in the CUDA kernel (debug aid)
         self.hybrid_delta_rule = bool(int(os.environ.get("Q38_GDN_HYBRID", "0")))
-        # True: no atomically accumulated split-K; weight gradients are then bitwise reproducible from run to run
+        # True: no atomically accumulated split-K in the weight gradients (the accumulations of other kernels stay as they are)
         self.deterministic = bool(int(os.environ.get("Q38_DETERMINISTIC", "0")))
         self.ep = None            # an `ExpertParallel` context when the experts are split over ranks
         self.selection_override = None   # optional iterator of (count, index) pairs that replaces the block selection (tests)

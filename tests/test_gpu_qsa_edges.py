@@ -39,6 +39,23 @@ def test_indexer_backward(ops, NI, B, nb):
     assert rel(dqi, q.grad) < 2e-2 and rel(dki, k.grad) < 2e-2 and rel(dwi, w.grad) < 2e-2
 
 
+# query blocks with one to four shares of their key blocks
+def test_indexer_query_gradients_have_the_same_bits_in_every_run(ops):
+    B, NI, nb = 4, 4, 24
+    S = 64 * nb
+    gen = torch.Generator(device="cuda").manual_seed(0)
+    qi = torch.randn(B, NI, S, 64, device="cuda", generator=gen).to(torch.bfloat16)
+    ki = torch.randn(B, S, 64, device="cuda", generator=gen).to(torch.bfloat16)
+    wi = torch.randn(B, S, NI, device="cuda", generator=gen) / 2
+    lib = ops.load()
+    blse = lib.qsa_indexer_fwd(qi, ki, wi, 0.125)
+    dblse = torch.randn(B, S, nb, device="cuda", generator=gen)
+    first = lib.qsa_indexer_bwd(qi, ki, wi, blse, dblse, 0.5, 0.125)
+    for _ in range(20):
+        again = lib.qsa_indexer_bwd(qi, ki, wi, blse, dblse, 0.5, 0.125)
+        assert torch.equal(again[0], first[0]) and torch.equal(again[2], first[2])
+
+
 # the own block alone, a list with gaps, every block (dense); the second half of a 64-row tile is what the half-tile loops reach last
 @pytest.mark.parametrize("B,nb,nq,nkv,pick", [(1, 1, 2, 1, "dense"), (1, 5, 6, 2, "own"), (2, 7, 4, 2, "gaps"), (1, 33, 2, 1, "dense")])
 def test_block_attention(ops, B, nb, nq, nkv, pick):
