@@ -595,8 +595,13 @@ std::vector<at::Tensor> qsa_select(const at::Tensor& lp_blk, int64_t budget) {
 // Returns {dqi [B,NI,S,64] bf16, dki [B,S,64] bf16, dwi [B,S,NI] fp32}; gscale multiplies dblse (upstream grad / token count).
 std::vector<at::Tensor> qsa_indexer_bwd(const at::Tensor& qi, const at::Tensor& ki, const at::Tensor& wi, const at::Tensor& blse, const at::Tensor& dblse,
                                         double gscale, double scale) {
+  check4(qi, "qsa_indexer_bwd q"); check4(ki, "qsa_indexer_bwd k");
   const c10::cuda::CUDAGuard guard(qi.device());
+  TORCH_CHECK(qi.dim() == 4 && qi.size(1) <= NI_MAX && qi.size(2) % 64 == 0, "qsa_indexer_bwd: at most 4 indexer heads and whole blocks of 64 tokens");
   const int B = qi.size(0), NI = qi.size(1), S = qi.size(2), nb = S / 64;
+  TORCH_CHECK(ki.numel() == (int64_t)B * S * 64, "qsa_indexer_bwd: k must be [B,S,64]");
+  auto rows = [&](const at::Tensor& t, int64_t n) { return t.is_cuda() && t.scalar_type() == at::kFloat && t.is_contiguous() && t.numel() == (int64_t)B * S * n; };
+  TORCH_CHECK(rows(wi, NI) && rows(blse, nb) && rows(dblse, nb), "qsa_indexer_bwd: contiguous fp32 w [B,S,heads], blse and dblse [B,S,blocks] required");
   const int Z = std::min(nb, 4);
   auto f32 = qi.options().dtype(at::kFloat);
   auto part = at::empty({Z, B, NI, S, 64}, f32), dw_part = at::empty({Z, B, S, NI}, f32);

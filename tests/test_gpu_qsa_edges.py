@@ -56,6 +56,22 @@ def test_indexer_query_gradients_have_the_same_bits_in_every_run(ops):
         assert torch.equal(again[0], first[0]) and torch.equal(again[2], first[2])
 
 
+def test_indexer_backward_refuses_what_its_tiles_do_not_hold(ops):
+    B, S, nb = 1, 128, 2
+    lib = ops.load()
+    make = lambda NI: (torch.zeros(B, NI, S, 64, device="cuda", dtype=torch.bfloat16), torch.zeros(B, S, 64, device="cuda", dtype=torch.bfloat16),
+                       torch.zeros(B, S, NI, device="cuda"), torch.zeros(B, S, nb, device="cuda"), torch.zeros(B, S, nb, device="cuda"))
+    lib.qsa_indexer_bwd(*make(4), 1.0, 0.125)
+    with pytest.raises(RuntimeError, match="at most 4 indexer heads"):
+        lib.qsa_indexer_bwd(*make(5), 1.0, 0.125)
+    for at, bad in ((1, lambda t: t.float()), (2, lambda t: t.double()), (2, lambda t: t[..., :1].expand_as(t)), (3, lambda t: t[..., :1]),
+                    (4, lambda t: t.transpose(1, 2).contiguous().transpose(1, 2))):
+        args = list(make(4))
+        args[at] = bad(args[at])
+        with pytest.raises(RuntimeError, match="required"):
+            lib.qsa_indexer_bwd(*args, 1.0, 0.125)
+
+
 # the own block alone, a list with gaps, every block (dense); the second half of a 64-row tile is what the half-tile loops reach last
 @pytest.mark.parametrize("B,nb,nq,nkv,pick", [(1, 1, 2, 1, "dense"), (1, 5, 6, 2, "own"), (2, 7, 4, 2, "gaps"), (1, 33, 2, 1, "dense")])
 def test_block_attention(ops, B, nb, nq, nkv, pick):
