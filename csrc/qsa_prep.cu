@@ -163,8 +163,9 @@ __global__ void __launch_bounds__(32 * HP_WARPS) qsa_headprep_bwd_kernel(const b
 // Enough CTAs to fill the chip several times over, few enough that a warp handles many rows (the backward adds one weight gradient per CTA).
 static unsigned headprep_grid(long long rows) { return (unsigned)std::max<long long>(1, std::min<long long>((rows + 4 * HP_WARPS - 1) / (4 * HP_WARPS), kNumSMs * 8)); }
 
-// The kernels read 16-byte pieces; a contiguous view that starts elsewhere is copied first.
-static at::Tensor aligned16(const at::Tensor& t) { return (reinterpret_cast<uintptr_t>(t.data_ptr()) & 15) == 0 ? t : t.clone(); }
+// The kernels read 16-byte pieces; a contiguous view that starts elsewhere is copied first.  Other strides go on to the checks as they are (a copy
+// would make them contiguous).
+static at::Tensor aligned16(const at::Tensor& t) { return (reinterpret_cast<uintptr_t>(t.data_ptr()) & 15) == 0 || !t.is_contiguous() ? t : t.clone(); }
 
 static void check_tables(const at::Tensor& cosv, const at::Tensor& sinv, int B, int S) {
   TORCH_CHECK(cosv.scalar_type() == at::kFloat && sinv.scalar_type() == at::kFloat && cosv.is_contiguous() && sinv.is_contiguous() && cosv.dim() == 3 &&

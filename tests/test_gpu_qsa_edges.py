@@ -122,3 +122,23 @@ def test_conv_silu(ops, C, S):
     yr.backward(dy.double())
     # the convolution output is bf16 before the activation, and so are y and dx
     assert rel(y, yr.detach()) < 6e-3 and rel(dx, xr.grad) < 6e-3 and rel(dw, wr.grad) < 6e-3
+
+
+def test_head_preparation_of_views(ops):
+    """A contiguous view may start anywhere; other strides are refused wherever they start."""
+    B, S, H = 1, 64, 3
+    gen = torch.Generator(device="cuda").manual_seed(0)
+    flat = torch.randn(B * S * H * 64 + 8, device="cuda", generator=gen).to(torch.bfloat16)
+    cos, sin = (f(torch.rand(1, S, 8, device="cuda", generator=gen)).repeat(1, 1, 2) for f in (torch.cos, torch.sin))
+    lib = ops.load()
+    for first in (0, 1, 2, 8):
+        view = flat[first:first + B * S * H * 64].view(B, S, H, 64)
+        out = lib.qsa_headprep_fwd(view, None, cos, sin, 0.0, False)
+        again = lib.qsa_headprep_fwd(view.clone(), None, cos, sin, 0.0, False)
+        assert torch.equal(out[0], again[0])
+    wide = torch.zeros(B, S, H, 72, device="cuda", dtype=torch.bfloat16)
+    for first in (0, 1):
+        with pytest.raises(RuntimeError, match="contiguous bf16"):
+            lib.qsa_headprep_fwd(wide[..., first:first + 64], None, cos, sin, 0.0, False)
+        with pytest.raises(RuntimeError, match="bad inputs"):
+            lib.qsa_headprep_bwd(torch.zeros(B, H, S, 64, device="cuda", dtype=torch.bfloat16), None, wide[..., first:first + 64], None, cos, sin, torch.zeros(0, S, H, device="cuda"))
