@@ -41,8 +41,8 @@ TORCH_LIBRARY(q38, m) {
           q38::muon_small_ns(src, dst, rows, cols, steps, err);
         });
   // 2-D operands (batch 1): the views and, without an output, its allocation are made here instead of in four Python calls
-  m.def("gemm2d(Tensor a, Tensor b, bool a_mn_major, bool b_mn_major, float alpha, bool fp32, Tensor err) -> Tensor",
-        [](const at::Tensor& a, const at::Tensor& b, bool amn, bool bmn, double alpha, bool fp32, at::Tensor err) {
+  m.def("gemm2d(Tensor a, Tensor b, bool a_mn_major, bool b_mn_major, float alpha, bool fp32, Tensor(a!) err) -> Tensor",
+        [](const at::Tensor& a, const at::Tensor& b, bool amn, bool bmn, double alpha, bool fp32, at::Tensor& err) {
           TORCH_CHECK(a.dim() == 2 && b.dim() == 2, "gemm2d: 2-D operands required");
           auto c = at::empty({a.size(amn ? 1 : 0), b.size(bmn ? 1 : 0)}, a.options().dtype(fp32 ? at::kFloat : at::kBFloat16));
           auto c3 = c.unsqueeze(0);
@@ -132,10 +132,10 @@ TORCH_LIBRARY(q38, m) {
   m.def("conv_silu_bwd(Tensor x, Tensor w, Tensor dy) -> Tensor[]");
   m.def("gdn_prep_fwd(Tensor q, Tensor k, Tensor v, Tensor g, Tensor beta, bool save=True) -> Tensor[]");
   m.def("gdn_prep_bwd(Tensor q, Tensor k, Tensor v, Tensor g, Tensor beta, Tensor Tm, Tensor w, Tensor u, Tensor vnew, Tensor states, Tensor dout, Tensor du, Tensor dstate, Tensor dd) -> Tensor[]");
-  m.def("gdn_rule_fwd(Tensor qkv, Tensor g, Tensor beta, int Hk, int Hv, Tensor? err, bool save) -> Tensor[]");
-  m.def("gdn_rule_bwd(Tensor qkv, Tensor g, Tensor beta, Tensor[] saved, Tensor dout, int Hk, int Hv, Tensor? err) -> Tensor[]");
-  m.def("gdn_chain_bwd(Tensor w, Tensor P, Tensor qg, Tensor kg, Tensor dch, Tensor states, Tensor dout, int B, int H, Tensor? err=None) -> Tensor[]");
-  m.def("gdn_scan_fwd(Tensor w, Tensor u, Tensor P, Tensor qg, Tensor kg, Tensor dch, int B, int H, Tensor? err=None, bool save=True) -> Tensor[]");
+  m.def("gdn_rule_fwd(Tensor qkv, Tensor g, Tensor beta, int Hk, int Hv, Tensor(a!)? err, bool save) -> Tensor[]");
+  m.def("gdn_rule_bwd(Tensor qkv, Tensor g, Tensor beta, Tensor[] saved, Tensor dout, int Hk, int Hv, Tensor(a!)? err) -> Tensor[]");
+  m.def("gdn_chain_bwd(Tensor w, Tensor P, Tensor qg, Tensor kg, Tensor dch, Tensor states, Tensor dout, int B, int H, Tensor(a!)? err=None) -> Tensor[]");
+  m.def("gdn_scan_fwd(Tensor w, Tensor u, Tensor P, Tensor qg, Tensor kg, Tensor dch, int B, int H, Tensor(a!)? err=None, bool save=True) -> Tensor[]");
   m.def("gdn_scan_bwd(Tensor w, Tensor P, Tensor qg, Tensor kg, Tensor dch, Tensor vnew, Tensor states, Tensor dout, int B, int H) -> Tensor[]");
   m.def("moe_route_fwd(Tensor logits, int k) -> Tensor[]");
   m.def("moe_route_bwd(Tensor probs, Tensor top_idx, Tensor top_w, Tensor d_top_w, Tensor? d_prob_sum) -> Tensor");

@@ -22,3 +22,10 @@ def test_bounded_waits_are_voted_before_warp_instructions(name):
         product = code.find("mma64<", m.end())
         voted = m.group(1) or "__all_sync(" in code[m.end():product]
         assert voted, code[m.start():m.start() + 120]
+
+
+@pytest.mark.parametrize("op", ["gemm2d", "gemm2d_out", "gdn_rule_fwd", "gdn_rule_bwd", "gdn_chain_bwd", "gdn_scan_fwd"])
+def test_error_word_is_declared_as_written(op):
+    """These kernels store into the device's error word when a wait runs out, so their schemas say that the argument is mutated."""
+    schema = re.search(r'm\.def\("' + op + r"\(([^\"]*)\) ->", code_of("bindings.cpp")).group(1)
+    assert re.search(r"Tensor\([a-z]!\)\??\s+err\b", schema), schema
