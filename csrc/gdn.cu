@@ -556,9 +556,9 @@ __global__ void __launch_bounds__(128, 4) gdn_prep_fwd_kernel(const bf16* __rest
 // q_i.(H K)_i and k_j.(H^T Q)_j, row dots of products that dq and dk need anyway, so k.k and q.k are not formed again and
 // every row sum stays in two registers per thread until the end of the head.  (The sums cancel pairwise between rows and columns as
 // before, since both sides read the same rounded H.)
-// Bound by the shared-memory round trips of its twelve dependent 64^3 products (70 % of that pipe); eight warps with half-width accumulators and
+// Bound by the shared-memory round trips of its thirteen 64^3 products, most of them dependent (70 % of that pipe); eight warps with half-width accumulators and
 // two CTAs per SM (at most 128 registers, 112 KB of tiles) hide part of them, and the next head's eight tiles load while this head's last
-// products run.  5376 chunks: 241 us; the kernel that took dw, dP, dqg, dkg from the scan, four warps and sixteen row or column sums, 337.
+// products run.  5376 chunks: 230 us; the kernel that took dw, dP, dqg, dkg from the scan, four warps and sixteen row or column sums, 337.
 __global__ void __launch_bounds__(256, 2) gdn_prep_bwd_kernel(const bf16* __restrict__ q, const bf16* __restrict__ k, const bf16* __restrict__ v,
                                                               const float* __restrict__ g, const bf16* __restrict__ beta, const bf16* __restrict__ Tm_in,
                                                               const bf16* __restrict__ w_in, const bf16* __restrict__ u_in, const bf16* __restrict__ vnew,
@@ -749,10 +749,15 @@ __global__ void __launch_bounds__(256, 2) gdn_prep_bwd_kernel(const bf16* __rest
       }
     }
     // ---- dM = -(A w^T + B u^T); L_ij = beta_i (kn_i.kn_j) Gamma_ij (j < i) ----
-    // The tile holds beta_i dL_ij Gamma_ij; the magnitude of beta is floored so that a row with beta = 0 still yields its beta gradient by the
-    // division below (what the floor adds elsewhere is 1e-18 of dL).  Its sign stays, and a NaN stays one.
-    auto floored = [](float x) { return fabsf(x) < 8.6736174e-19f ? copysignf(8.6736174e-19f, x) : x; };
-    const float flo = floored(blo), fhi = floored(bhi);
+    // beta's own gradient, sum_j dL_ij (kn_i.kn_j) Gamma_ij, is taken from the fp32 fragments.  (As a row dot with the rounded tile, like the gates,
+    // it would need a division by beta and came out 0.3 to 0.9 % further from the 64-bit gradient.)
+    float kk[4][4];
+    {
+      uint32_t ak[4][4];
+      load_a(Kn, ak, warp & 3, lane);
+      zero_acc(kk);
+      mma_rows<true, 4, 4>(ak, Kn + 32 * ch * LDS, kk, lane);
+    }
     zero_acc(acc);
     mma64h<false, true>(St, Wt, acc, warp, lane);
     mma64h<false, true>(Do, Ut, acc, warp, lane);
@@ -761,7 +766,9 @@ __global__ void __launch_bounds__(256, 2) gdn_prep_bwd_kernel(const bf16* __rest
 #pragma unroll
       for (int e = 0; e < 4; ++e) {
         const int row = r0 + 8 * (e >> 1), cc = 8 * nt + c0 + (e & 1);
-        acc[nt][e] = cc < row ? -acc[nt][e] * __expf((e >> 1 ? ghi : glo) - gc[cc]) * (e >> 1 ? fhi : flo) : 0.f;
+        const float dl = cc < row ? -acc[nt][e] * __expf((e >> 1 ? ghi : glo) - gc[cc]) : 0.f;
+        (e >> 1 ? dbhi : dblo) += dl * kk[nt][e];
+        acc[nt][e] = dl * (e >> 1 ? bhi : blo);
       }
     }
     acc_to_smem_h(acc, X1, warp, lane);
@@ -771,7 +778,6 @@ __global__ void __launch_bounds__(256, 2) gdn_prep_bwd_kernel(const bf16* __rest
     mma64h<false, false>(X1, Kn, acc, warp, lane);           // dA1 Kn
     add_rows(dKn, acc, 1.f, 1.f);
     row_dot(acc, Kn, lo, hi);
-    dblo += lo / flo; dbhi += hi / fhi;
     dglo += lo; dghi += hi;
     zero_acc(acc);
     mma64h<true, false>(X1, Kn, acc, warp, lane);            // dA1^T Kn

@@ -150,7 +150,7 @@ def bench_gdn(rows, shape, T, iters, pk, seq=4096):
     report(rows, f"gdn_chain_bwd B={B} Hv={Hv}", t, flops=chunks * 4 * 2.0 * 64 ** 3, bytes_=chunks * 8 * 8192.0, pk=pk)
     du, dstate, dd = lib.gdn_chain_bwd(w, P, qg, kg, carry, states, do, B, Hv)
     t = timeit(lambda: lib.gdn_prep_bwd(q, k, v, g, beta, Tm, w, u, vnew, states, do, du, dstate, dd), iters)
-    report(rows, f"gdn_prep_bwd B={B} Hv={Hv}", t, flops=chunks * 12 * 2.0 * 64 ** 3, bytes_=chunks * 8 * 8192.0 + 4.0 * qkv.numel(), pk=pk)
+    report(rows, f"gdn_prep_bwd B={B} Hv={Hv}", t, flops=chunks * 13 * 2.0 * 64 ** 3, bytes_=chunks * 8 * 8192.0 + 4.0 * qkv.numel(), pk=pk)
 
 
 def bench_qsa(rows, shape, T, iters, pk, seq=4096):

@@ -107,3 +107,25 @@ def test_delta_rule_gradients_with_negative_beta(ops):
     assert rel(qkv.grad, ref[0].grad) < 2e-2 and rel(beta.grad, ref[2].grad) < 2e-2 and rel(g.grad, ref[1].grad) < 2.5e-2
     for part in (beta.detach() < 0, beta.detach() == 0):
         assert rel(beta.grad[part], ref[2].grad[part]) < 2e-2
+
+
+def test_beta_gradient_is_summed_in_32_bits(ops):
+    """Every factor is exact in bf16 and only the gradient of the triangular system, an integer of up to sixteen bits, is not: beta's gradient comes
+    from its fp32 form.  Only token 0 writes (beta = 0 elsewhere) and only token 63 has an upstream gradient."""
+    gen = torch.Generator(device="cuda").manual_seed(5)
+    sign = lambda *s: torch.randint(0, 2, s, device="cuda", generator=gen).float() * 2 - 1
+    q, k, v = sign(1, 64, 64), sign(1, 64, 64), torch.zeros(1, 64, 64, device="cuda")
+    v[:, 0] = torch.randint(-15, 16, (64,), device="cuda", generator=gen).float()
+    qkv = torch.cat([q, k, v], -1).to(torch.bfloat16)
+    g, beta = torch.zeros(1, 64, 1, device="cuda"), torch.zeros(1, 64, 1, device="cuda", dtype=torch.bfloat16)
+    beta[:, 0] = 0.5
+    do = torch.zeros(1, 64, 1, 64, device="cuda", dtype=torch.bfloat16)
+    do[:, 63] = sign(1, 64).to(torch.bfloat16)
+    lib = ops.load()
+    _, *saved = lib.gdn_rule_fwd(qkv, g, beta, 1, 1, ops.error_flag(), True)
+    dbeta = lib.gdn_rule_bwd(qkv, g, beta, saved, do, 1, 1, ops.error_flag())[2]
+    ops.check_errors()
+    ref = [t.double().requires_grad_() for t in (qkv, g, beta)]
+    recurrence(*ref, 1, 1).backward(do.double())
+    # rounded to bf16 before the sum it is 1e-3 off; what is left is the 1e-6 in the norms against 64 and fp32 sums
+    assert rel(dbeta[:, 1:], ref[2].grad[:, 1:]) < 1e-5
