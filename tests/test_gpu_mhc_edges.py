@@ -66,13 +66,15 @@ def sinkhorn_gradient(logits, d, iters):
     return d * p0
 
 
-def test_sinkhorn_gradient_of_widely_spread_logits():
-    """Logits that span eighty: the gradient is as good as iterates kept in 32 bits give it.  Iterates rebuilt on the way back are not."""
+# residual logits that span some 25 and some 70
+@pytest.mark.parametrize("spread,mean,tail", [(4, 3.0e-7, 2.5e-6), (12, 6.5e-7, 1.0e-5)])
+def test_sinkhorn_gradient_per_token(spread, mean, tail):
+    """The gradient is as good as iterates kept in 32 bits give it; iterates rebuilt on the way back are a quarter to a third worse."""
     from q38 import ops
     ops.install()
     T, h, iters, a2 = 65536, 64, 20, 64.0
     gen = torch.Generator(device="cuda").manual_seed(0)
-    z = (torch.randn(T, 24, device="cuda", generator=gen) * (20 / a2)).clamp(-0.9, 0.9)
+    z = (torch.randn(T, 24, device="cuda", generator=gen) * (spread / a2)).clamp(-0.9, 0.9)
     dcoef = torch.randn(T, 24, device="cuda", generator=gen)
     dcoef[:, :8] = 0
     zeros = lambda *s: torch.zeros(*s, device="cuda")
@@ -81,10 +83,12 @@ def test_sinkhorn_gradient_of_widely_spread_logits():
     # with an identity as the second projection and unit norms, dL_raw is d(logits) alphas (1 - z^2) of every token
     dL = ops.load().mhc_pre_bwd_a(zeros(T, h), zeros(T, 4, h), zeros(T, 24), torch.eye(24, device="cuda"), zeros(4), zeros(4), zeros(16), alphas, zeros(h),
                                   zeros(T, 24), z, zeros(T) + 1, zeros(T) + 1, dcoef, iters)[0]
-    ref = sinkhorn_gradient(logits.double(), d.double(), iters) * (a2 * (1 - z[:, 8:].double() ** 2)).view(T, 4, 4)
+    factor = (a2 * (1 - z[:, 8:].double() ** 2)).view(T, 4, 4)
+    ref = sinkhorn_gradient(logits.double(), d.double(), iters) * factor
     err = lambda x: (x.double().view(T, 16) - ref.view(T, 16)).norm(dim=1) / ref.view(T, 16).norm(dim=1)
-    good = err(sinkhorn_gradient(logits, d, iters) * (a2 * (1 - z[:, 8:] ** 2)).view(T, 4, 4)) < 1e-5
-    assert good.float().mean() > 0.95
+    good = err(sinkhorn_gradient(logits, d, iters) * factor.float()) < 1e-5       # some tokens' gradients are ill-conditioned in any 32-bit arithmetic
+    assert good.float().mean() > 0.999
     got = err(dL[:, 8:])[good]
-    # 1e-5 of the 32-bit formula, times up to twenty for the kernel's approximate exponential (some 60 units in the last place at -80) and divisions
-    assert got.max() < 2e-4 and got.mean() < 3e-6, (got.max().item(), got.mean().item())
+    # forty divisions of 2^-23 each way and an exponential of 2^-22: with kept iterates 2.6e-7 and 5.8e-7 in the mean, 1.5e-6 and 6.8e-6 for one token in
+    # a thousand; with rebuilt ones 3.5e-7 and 7.4e-7, 1.6e-6 and 1.5e-5
+    assert got.mean() < mean and got.quantile(0.999) < tail, (got.mean().item(), got.quantile(0.999).item())
