@@ -142,17 +142,32 @@ def load_megatron_function(path, expected_sha256=MEGATRON_SHA256):
     return scope["num_floating_point_operations"]
 
 
-def delta_rule_kernel_products(source=None):
-    """64x64x64 tensor-core products per (chunk, value head) issued by each delta-rule kernel, counted from the kernel source.  A training step
-    runs `gdn_chain_bwd_kernel` (csrc/gdn_chain.cu, four products) in the place of `gdn_scan_bwd_kernel`, which serves operands that come
-    from the PyTorch specification; the products it leaves out are among the twelve of `gdn_prep_bwd_kernel`."""
-    text = Path(source or Path(__file__).resolve().parents[2] / "csrc" / "gdn.cu").read_text()
-    kernels = re.split(r"__global__ void[^\n]*?\b(gdn_\w+_kernel)\(", text)
+CSRC = Path(__file__).resolve().parents[2] / "csrc"
+TRAINING_KERNELS = ("gdn_prep_fwd_kernel", "gdn_scan_fwd_kernel", "gdn_chain_bwd_kernel", "gdn_prep_bwd_kernel")
+
+
+def _count_products(path, call):
+    kernels = re.split(r"__global__ void[^\n]*?\b(gdn_\w+_kernel)\(", Path(path).read_text())
     counts = {}
     for name, body in zip(kernels[1::2], kernels[2::2]):
         code = "\n".join(line.split("//")[0] for line in body.splitlines())
-        counts[name] = len(re.findall(r"\bmma64h?<", code))
+        counts[name] = len(re.findall(call, code))
     return counts
+
+
+def delta_rule_kernel_products(source=None):
+    """64x64x64 tensor-core products of two shared-memory tiles per (chunk, value head) in each kernel of csrc/gdn.cu, counted from the source.
+    `gdn_scan_bwd_kernel` serves operands that come from the PyTorch specification; a training step does not run it."""
+    return _count_products(source or CSRC / "gdn.cu", r"\bmma64h?<")
+
+
+def delta_rule_training_products():
+    """The products of the four kernels that a training step runs, in both source files.  A product whose first operand is in registers
+    (`mma_rows`) counts like the others: k.k, formed once more for beta's gradient, is the thirteenth of the preparation backward."""
+    counts = {}
+    for name in ("gdn.cu", "gdn_chain.cu"):
+        counts.update(_count_products(CSRC / name, r"\b(?:mma64h?|mma_rows)<"))
+    return {name: counts[name] for name in TRAINING_KERNELS}
 
 
 def audit_backbone(c, seq, megatron=None):
@@ -194,16 +209,19 @@ def backbone_report(seq=8192, vocab=10112, megatron_source=None):
                    megatron_reaccounted_budget_fraction=tokens * row["megatron_train_flops_per_token"] / p["compute"] - 1)
         archived.append(row)
     family = [audit_backbone(model_config(make_isoflops.shape_for(hidden), vocab, seq).to_dict(), seq, megatron) for hidden in make_isoflops.WIDTHS]
-    products = delta_rule_kernel_products()
+    products = delta_rule_training_products()
     per_token = {name: n * 2 * 64 * 64 * 64 / 64 for name, n in products.items()}
     return dict(reference=dict(commit=MEGATRON_COMMIT, url=MEGATRON_URL, sha256=MEGATRON_SHA256, original_function_evaluated=megatron is not None),
                 scope=dict(seq=seq, vocab=vocab, physical_kernel_flops=False),
                 archived_configs=archived, canonical_family=family,
-                delta_rule_kernels=dict(products_64x64x64_per_chunk_and_value_head=products, gemm_flops_per_token_and_value_head=per_token,
+                delta_rule_kernels=dict(products_64x64x64_per_chunk_and_value_head=delta_rule_kernel_products(),
+                                        training_products_64x64x64_per_chunk_and_value_head=products, gemm_flops_per_token_and_value_head=per_token,
                                         training_total_per_token_and_value_head=sum(per_token.values()),
                                         convention_training_per_token_and_value_head=3 * 8 * 64 * 64,
                                         note="partial ledger: tensor-core products only (the triangular solve, gating, norms and "
-                                             "reductions are vector work); the convention charges the recurrent form"),
+                                             "reductions are vector work); the convention charges the recurrent form; the first table counts "
+                                             "tile products in csrc/gdn.cu, of which gdn_scan_bwd_kernel is not part of a training step, the "
+                                             "second and the operation counts those of the kernels that a training step runs"),
                 failures=[f for row in archived + family for f in row["failures"]])
 
 
@@ -223,7 +241,7 @@ def main(argv=None):
             print(f"{row['shape']:12} ledger={row['train_flops_per_token']:13,d} megatron={row['megatron_train_flops_per_token']:13,d} "
                   f"router/gate={row['over_megatron_fraction']:+.3%}")
         print(f"checked {len(report['archived_configs'])} archived configs and {len(report['canonical_family'])} widths; "
-              f"delta-rule kernel products {report['delta_rule_kernels']['products_64x64x64_per_chunk_and_value_head']}; failures: {len(report['failures'])}")
+              f"delta-rule products of a training step {report['delta_rule_kernels']['training_products_64x64x64_per_chunk_and_value_head']}; failures: {len(report['failures'])}")
         return 1 if report["failures"] else 0
     a.seq = a.seq or 4096
     bad = 0

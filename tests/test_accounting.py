@@ -134,6 +134,19 @@ def test_backbone_ledger_equals_the_pinned_megatron_formula(tmp_path):
     assert audit_flops.main(["--backbone", "--output", str(tmp_path / "audit.json")]) == 0
 
 
+def test_delta_rule_ledger_counts_the_kernels_of_a_training_step():
+    """The total is that of the four kernels which gdn_rule_fwd and gdn_rule_bwd launch, in whichever file they are."""
+    import re
+    from q38.utils import audit_flops
+    ledger = audit_flops.backbone_report()["delta_rule_kernels"]
+    assert ledger["training_products_64x64x64_per_chunk_and_value_head"] == {
+        "gdn_prep_fwd_kernel": 4, "gdn_scan_fwd_kernel": 4, "gdn_chain_bwd_kernel": 4, "gdn_prep_bwd_kernel": 13}
+    assert ledger["training_total_per_token_and_value_head"] == sum(ledger["gemm_flops_per_token_and_value_head"].values()) == 25 * 2 * 64 ** 3 / 64
+    source = (audit_flops.CSRC / "gdn.cu").read_text()
+    calls = set(re.findall(r"\b(gdn_\w+)\(", "".join(re.findall(r"gdn_rule_(?:fwd|bwd)\([^;]*?\{\n(.*?)\n\}", source, re.S))))
+    assert {c + "_kernel" for c in calls} == set(audit_flops.TRAINING_KERNELS)
+
+
 def test_launcher_builds_loopback_torchrun_command():
     from q38.launch import command
     single = command("q38.train", 1, 29500, ["--preset", "q38_c1"])
