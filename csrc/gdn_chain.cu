@@ -5,7 +5,7 @@
 // Like the forward scan (gdn_tile.cuh) this never mixes value columns, so a warp owns 16 of them, keeps dS'^T in its accumulator
 // registers and needs no block barrier in the chain.  The products that sum over value columns (dw, dP, dqg, dkg) depend on the chain only
 // through dS' and dv_new, which this kernel stores; the preparation backward forms them chunk-parallel over the whole chip.
-// 84 pairs of 64 chunks: 133 us, where the pass that formed everything took 270.  Bound by the latency of the chain; a second warp per slice
+// 84 pairs of 64 chunks: 130 us (1 pair 82, 156 pairs 246), where the pass that formed everything took 270.  Bound by the latency of the chain; a second warp per slice
 // for the products that do not wait for it took 143 us with a whole pair per SM (the 14 KB that the two exchange per chunk cost more).
 #include <ATen/ATen.h>
 #include <ATen/cuda/CUDAContext.h>
@@ -55,8 +55,22 @@ __global__ void __launch_bounds__(32 * W) gdn_chain_bwd_kernel(const __grid_cons
   float dS[8][4];
   zero_acc(dS);
   float d_next = dch[(long long)bh * NT + NT - 1];
-  int dead = 0, stage = 0, phase = 0;
-  for (int i = 0; i < NT; ++i) {
+  int stage = 0, phase = 0;
+  // A chunk's tiles are waited for before the barrier that ends the chunk before it, which exchanges the verdict: a lane whose wait ran out (the
+  // lanes poll for themselves) neither leaves its warp's collective instructions nor the barrier, the CTA leaves together.  It also takes the
+  // wait off the start of the chain: with a vote and a branch in front of the products 84 pairs took 138 us, with each lane's own branch 133.
+  bool late = !ptx::mbar_wait(&full[0], 0);
+  for (int i = 0; ; ++i) {
+    if (__syncthreads_or(late)) {                            // a tile never came: let the copies in flight land (bounded), then leave
+      if (threadIdx.x == 0) report_error(err, ERR_TMA_WAIT);
+      for (int j = 1; j < STAGES - 1 && i + j < NT; ++j) {
+        if (++stage == STAGES) { stage = 0; phase ^= 1; }
+        ptx::mbar_wait(&full[stage], phase);
+      }
+      cp_async_wait<0>();
+      return;
+    }
+    if (i == NT) break;
     const int c = NT - 1 - i;
     {  // refill the stage that the chunk before left
       const int n = i + STAGES - 1, ns = stage == 0 ? STAGES - 1 : stage - 1;
@@ -69,52 +83,41 @@ __global__ void __launch_bounds__(32 * W) gdn_chain_bwd_kernel(const __grid_cons
     d_next = dch[(long long)bh * NT + (c > 0 ? c - 1 : 0)];
     cp_async_wait<1>();
     __syncwarp();
-    if (!ptx::mbar_wait_warp(&full[stage], phase)) { dead = 1; if (lane == 0) report_error(err, ERR_TMA_WAIT); }
     const uint32_t wt = tiles + stage * 4 * TILE_BYTES, pt = wt + TILE_BYTES, qt = pt + TILE_BYTES, kt = qt + TILE_BYTES;
     const uint32_t mine = pairs + (i & 1) * 2 * SLICE_BYTES;
-    if (!dead) {
-      uint32_t aD[4][4], aS[4][4], av[4][4];
-      float acc[8][4], part = 0.f;
-      slice_read_t(mine, aD, lane);                          // dO^T
-      slice_read_t(mine + SLICE_BYTES, av, lane);            // S^T, in accumulator order
+    uint32_t aD[4][4], aS[4][4], av[4][4];
+    float acc[8][4], part = 0.f;
+    slice_read_t(mine, aD, lane);                          // dO^T
+    slice_read_t(mine + SLICE_BYTES, av, lane);            // S^T, in accumulator order
 #pragma unroll
-      for (int ks = 0; ks < 4; ++ks) {
+    for (int ks = 0; ks < 4; ++ks) {
 #pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          const float* x = &dS[2 * ks + (e >> 1)][2 * (e & 1)];
-          part += x[0] * lo_f(av[ks][e]) + x[1] * hi_f(av[ks][e]);
-        }
+      for (int e = 0; e < 4; ++e) {
+        const float* x = &dS[2 * ks + (e >> 1)][2 * (e & 1)];
+        part += x[0] * lo_f(av[ks][e]) + x[1] * hi_f(av[ks][e]);
       }
-      pack_a<4>(dS, aS);
-      zero_acc(acc);
-      mma64<true>(aD, pt, acc, lane);                        // (P^T dO)^T
-      mma64<false>(aS, kt, acc, lane);                       // + (kg dS')^T
-      pack_a<4>(acc, av);
-#pragma unroll
-      for (int nt = 0; nt < 8; ++nt) { dS[nt][0] *= d; dS[nt][1] *= d; dS[nt][2] *= d; dS[nt][3] *= d; }
-      mma64<true>(aD, qt, dS, lane);                         // + (qg^T dO)^T
-      uint32_t neg[4][4];
-#pragma unroll
-      for (int ks = 0; ks < 4; ++ks) {
-#pragma unroll
-        for (int e = 0; e < 4; ++e) neg[ks][e] = av[ks][e] ^ 0x80008000u;
-      }
-      mma64<true>(neg, wt, dS, lane);                        // - (w^T dv_new)^T
-      slice_store_t(mine, aS, dstate + base + (long long)c * 4096 + col, 64, lane);
-      slice_store_t(mine + SLICE_BYTES, av, du + base + (long long)c * 4096 + col, 64, lane);
-      part = warp_sum(part);
-      if (lane == 0) dd[((long long)bh * NT + c) * 4 + slice] = part;
     }
-    dead = __syncthreads_or(dead);                           // everyone is done with this stage
+    pack_a<4>(dS, aS);
+    zero_acc(acc);
+    mma64<true>(aD, pt, acc, lane);                        // (P^T dO)^T
+    mma64<false>(aS, kt, acc, lane);                       // + (kg dS')^T
+    pack_a<4>(acc, av);
+#pragma unroll
+    for (int nt = 0; nt < 8; ++nt) { dS[nt][0] *= d; dS[nt][1] *= d; dS[nt][2] *= d; dS[nt][3] *= d; }
+    mma64<true>(aD, qt, dS, lane);                         // + (qg^T dO)^T
+    uint32_t neg[4][4];
+#pragma unroll
+    for (int ks = 0; ks < 4; ++ks) {
+#pragma unroll
+      for (int e = 0; e < 4; ++e) neg[ks][e] = av[ks][e] ^ 0x80008000u;
+    }
+    mma64<true>(neg, wt, dS, lane);                        // - (w^T dv_new)^T
+    slice_store_t(mine, aS, dstate + base + (long long)c * 4096 + col, 64, lane);
+    slice_store_t(mine + SLICE_BYTES, av, du + base + (long long)c * 4096 + col, 64, lane);
+    part = warp_sum(part);
+    if (lane == 0) dd[((long long)bh * NT + c) * 4 + slice] = part;
     if (++stage == STAGES) { stage = 0; phase ^= 1; }
-    if (dead) {                                              // a tile never came: let the copies in flight land (bounded), then leave
-      for (int j = 1; j < STAGES && i + j < NT; ++j) {
-        ptx::mbar_wait(&full[stage], phase);
-        if (++stage == STAGES) { stage = 0; phase ^= 1; }
-      }
-      cp_async_wait<0>();
-      return;
-    }
+    late = i + 1 < NT && !ptx::mbar_wait(&full[stage], phase);
   }
 }
 
