@@ -124,7 +124,7 @@ __global__ void __launch_bounds__(GEMM_THREADS) gemm_bf16_kernel(const __grid_co
   } else {
     const int quarter = warp & 3;             // TMEM lanes this warp may read
     const int row = m0 + quarter * 32 + lane;
-    bool ok = ptx::mbar_wait(acc_ready, 0, 1u << 22);
+    bool ok = ptx::mbar_wait_warp(acc_ready, 0, 1u << 22);
     if (!ok) report_error(p.err, ERR_EPILOGUE_WAIT);
     ptx::tc_fence_after();
     if (ok) {

@@ -177,7 +177,7 @@ __global__ void __launch_bounds__(G2_THREADS) gemm_pair_kernel(const __grid_cons
       int bz, m0, n0;
       decode(w, bz, m0, n0);
       const int acc = tile & 1;
-      if (!ptx::mbar_wait(&acc_full[acc], (tile >> 1) & 1, 1u << 22)) { report_error(p.err, ERR_EPILOGUE_WAIT); ok = false; break; }
+      if (!ptx::mbar_wait_warp(&acc_full[acc], (tile >> 1) & 1, 1u << 22)) { report_error(p.err, ERR_EPILOGUE_WAIT); ok = false; break; }
       ptx::tc_fence_after();
       const int row0 = m0 + (int)rank * G2_BM + quarter * 32;
       const uint32_t t_addr = tmem_base + acc * G2_ACC_COLS + (uint32_t(quarter * 32) << 16);

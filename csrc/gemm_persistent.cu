@@ -144,7 +144,7 @@ __global__ void __launch_bounds__(P_THREADS) gemm_persistent_kernel(const __grid
       int bz, m0, n0, kb_begin, num_kb;
       decode(w, bz, m0, n0, kb_begin, num_kb);
       const int acc = tile & 1;
-      if (!ptx::mbar_wait(&acc_full[acc], (tile >> 1) & 1, 1u << 22)) { report_error(p.err, ERR_EPILOGUE_WAIT); ok = false; break; }
+      if (!ptx::mbar_wait_warp(&acc_full[acc], (tile >> 1) & 1, 1u << 22)) { report_error(p.err, ERR_EPILOGUE_WAIT); ok = false; break; }
       ptx::tc_fence_after();
       const int row = m0 + quarter * 32 + lane;
       OutT* c_row = reinterpret_cast<OutT*>(p.C) + bz * p.c_batch_stride + (long long)row * p.ldc;

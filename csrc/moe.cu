@@ -445,7 +445,7 @@ __global__ void __launch_bounds__(G_THREADS) grouped_gemm_kernel(const __grid_co
     bool ok = true;
     for (int kb = 0; kb < num_kb && ok; ++kb) {
       const int s = kb % p.stages, round = kb / p.stages;
-      if (!ptx::mbar_wait(&full[s], round & 1, 1u << 20)) { if (lane == 0) report_error(p.err, ERR_TMA_WAIT); ok = false; break; }
+      if (!ptx::mbar_wait_warp(&full[s], round & 1, 1u << 20)) { if (lane == 0) report_error(p.err, ERR_TMA_WAIT); ok = false; break; }
       uint8_t* a_tile = smem + s * STAGE_BYTES;
       if (EPI == EPI_WGRAD) {
         const int valid = rows_valid - kb * G_BK;          // rows of this K block that belong to the expert
@@ -482,7 +482,7 @@ __global__ void __launch_bounds__(G_THREADS) grouped_gemm_kernel(const __grid_co
   } else {
     const int quarter = warp & 3;
     const int r_local = quarter * 32 + lane;
-    bool ok = ptx::mbar_wait(acc_ready, 0, 1u << 22);
+    bool ok = ptx::mbar_wait_warp(acc_ready, 0, 1u << 22);
     if (!ok) report_error(p.err, ERR_EPILOGUE_WAIT);
     ptx::tc_fence_after();
     if (ok) {

@@ -144,12 +144,12 @@ __global__ void __launch_bounds__(PG_THREADS) grouped_persistent_kernel(const __
       const PGWork k = decode(w);
       if (k.num_kb == 0) continue;
       const int acc = item & 1;
-      if (!ptx::mbar_wait(&acc_empty[acc], ((item >> 1) & 1) ^ 1, 1u << 22)) { if (lane == 0) report_error(p.err, ERR_EPILOGUE_WAIT); ok = false; break; }
+      if (!ptx::mbar_wait_warp(&acc_empty[acc], ((item >> 1) & 1) ^ 1, 1u << 22)) { if (lane == 0) report_error(p.err, ERR_EPILOGUE_WAIT); ok = false; break; }
       ptx::tc_fence_after();
       const uint32_t d_tmem = tmem_base + acc * PG_ACC_COLS;
       for (int kb = 0; kb < k.num_kb; ++kb, ++it) {
         const int s = it % PG_STAGES;
-        if (!ptx::mbar_wait(&full[s], (it / PG_STAGES) & 1, 1u << 20)) { if (lane == 0) report_error(p.err, ERR_TMA_WAIT); ok = false; break; }
+        if (!ptx::mbar_wait_warp(&full[s], (it / PG_STAGES) & 1, 1u << 20)) { if (lane == 0) report_error(p.err, ERR_TMA_WAIT); ok = false; break; }
         uint8_t* a_tile = smem + s * STAGE_BYTES;
         if (EPI == PE_WGRAD) {
           const int valid = k.rows - kb * PG_BK;            // K rows of this block that belong to the expert
@@ -210,7 +210,7 @@ __global__ void __launch_bounds__(PG_THREADS) grouped_persistent_kernel(const __
           }
         };
         fetch(n0 + 16 * group, cur);
-        if (!ptx::mbar_wait(&acc_full[acc], (item >> 1) & 1, 1u << 22)) { report_error(p.err, ERR_EPILOGUE_WAIT); ok = false; break; }
+        if (!ptx::mbar_wait_warp(&acc_full[acc], (item >> 1) & 1, 1u << 22)) { report_error(p.err, ERR_EPILOGUE_WAIT); ok = false; break; }
         ptx::tc_fence_after();
         for (int c0 = 16 * group; c0 < p.bn; c0 += 32) {
           uint32_t r[16];
@@ -241,7 +241,7 @@ __global__ void __launch_bounds__(PG_THREADS) grouped_persistent_kernel(const __
         ++item;
         continue;
       }
-      if (!ptx::mbar_wait(&acc_full[acc], (item >> 1) & 1, 1u << 22)) { report_error(p.err, ERR_EPILOGUE_WAIT); ok = false; break; }
+      if (!ptx::mbar_wait_warp(&acc_full[acc], (item >> 1) & 1, 1u << 22)) { report_error(p.err, ERR_EPILOGUE_WAIT); ok = false; break; }
       ptx::tc_fence_after();
       const bool live = r_local < rows;
       const long long row = k.row0 + r_local;

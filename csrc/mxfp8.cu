@@ -255,7 +255,7 @@ __global__ void __launch_bounds__(MX_THREADS) mxfp8_grouped_gemm_kernel(const __
     }
   } else {
     const int quarter = warp & 3, r_local = quarter * 32 + lane;
-    const bool ok = ptx::mbar_wait(acc_ready, 0, 1u << 22);
+    const bool ok = ptx::mbar_wait_warp(acc_ready, 0, 1u << 22);
     if (!ok) report_error(p.err, ERR_EPILOGUE_WAIT);
     ptx::tc_fence_after();
     if (ok) {

@@ -110,7 +110,7 @@ __global__ void __launch_bounds__(QT_THREADS, 2) qsa_block_stats_tc_kernel(const
     bool ok = true;
     for (int g = wg; g < groups && ok; g += 2) {
       const int acc = g & 1;
-      if (!ptx::mbar_wait(&acc_full[acc], (g >> 1) & 1, 1u << 22)) { report_error(p.err, ERR_EPILOGUE_WAIT); ok = false; break; }
+      if (!ptx::mbar_wait_warp(&acc_full[acc], (g >> 1) & 1, 1u << 22)) { report_error(p.err, ERR_EPILOGUE_WAIT); ok = false; break; }
       ptx::tc_fence_after();
       const uint32_t t_addr = tmem_base + acc * QT_KEYS + (uint32_t(quarter * 32) << 16);
       float4 pair = make_float4(0.f, 0.f, 0.f, 0.f);         // statistics of the group's two blocks

@@ -12,16 +12,46 @@ def code_of(name):
 
 
 @pytest.mark.parametrize("name", ["gdn.cu", "gdn_chain.cu"])
-def test_bounded_waits_are_voted_before_warp_instructions(name):
-    """Every lane of a scan's warp polls the barrier for itself.  Where the verdict decides whether the warp goes on to ldmatrix / mma.sync, it must
-    be the warp's, not the lane's: lanes that disagree at the limit would leave those instructions and the block barrier behind them half attended."""
+def test_no_lane_leaves_its_warp_between_a_wait_and_a_product(name):
+    """Every lane of a scan's warp polls the barrier for itself.  Lanes that disagree at the limit must not part before ldmatrix / mma.sync, which
+    would run half attended: the warp votes or a block barrier exchanges the verdict before anything branches on it."""
     code = code_of(name)
-    used = [m for m in re.finditer(r"(?:=|\|\||&&|if \(!)\s*ptx::mbar_wait(_warp)?\(", code)]
+    used = [m for m in re.finditer(r"(?:=|\|\||&&|if \()\s*!?ptx::mbar_wait(_warp)?\(", code)]
     assert used, "no waits found"
     for m in used:
         product = code.find("mma64<", m.end())
-        voted = m.group(1) or "__all_sync(" in code[m.end():product]
-        assert voted, code[m.start():m.start() + 120]
+        if product < 0:                                        # the wait ends a loop whose next round begins with the product
+            loop = code.rfind("\n  for (", 0, m.start())
+            between = code[m.end():code.find("\n}", m.end())] + code[loop:code.find("mma64<", loop)]
+        else:
+            between = code[m.end():product]
+        vote = re.search(r"__all_sync\(|__syncthreads_or\(", between)
+        parted = re.search(r"if \(!?(?:dead|late|ok)\b|break;|return;", between)
+        assert m.group(1) or vote and not (parted and parted.start() < vote.start()), code[m.start():m.start() + 120]
+
+
+def enclosing_headers(code, at):
+    """Text in front of every brace that is open at position `at`."""
+    heads, start = [], 0
+    for i, ch in enumerate(code[:at]):
+        if ch == "{":
+            heads.append(code[start:i])
+            start = i + 1
+        elif ch == "}":
+            heads.pop()
+            start = i + 1
+        elif ch == ";":
+            start = i + 1
+    return heads
+
+
+@pytest.mark.parametrize("name", ["gemm.cu", "gemm_pair.cu", "gemm_persistent.cu", "moe.cu", "moe_persistent.cu", "mxfp8.cu", "qsa_tc.cu"])
+def test_waits_of_whole_warps_are_voted(name):
+    """The same for the warps that read accumulators (tcgen05.ld needs all lanes): a wait whose verdict belongs to one lane stands in a part
+    that one elected lane executes; everywhere else the warp votes."""
+    code = code_of(name)
+    for m in re.finditer(r"ptx::mbar_wait\(", code):
+        assert any("elect_one()" in head for head in enclosing_headers(code, m.start())), code[m.start():m.start() + 100]
 
 
 @pytest.mark.parametrize("op", ["gemm2d", "gemm2d_out", "gdn_rule_fwd", "gdn_rule_bwd", "gdn_chain_bwd", "gdn_scan_fwd"])
