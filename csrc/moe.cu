@@ -795,7 +795,7 @@ at::Tensor moe_gather(const at::Tensor& x, const at::Tensor& perm, int64_t k) {
 // 16-byte pieces apply: whole pieces per row, aligned storage, at most MAX_TOPK slots.
 static bool row_pieces(int h, int64_t k, std::initializer_list<const void*> ptrs) {
   for (const void* p : ptrs) if (reinterpret_cast<uintptr_t>(p) & 15) return false;
-  return h % 8 == 0 && k <= MAX_TOPK;
+  return h > 0 && h % 8 == 0 && k <= MAX_TOPK;
 }
 
 at::Tensor moe_combine_fwd(const at::Tensor& y_sorted, const at::Tensor& inv_perm, const at::Tensor& top_w) {

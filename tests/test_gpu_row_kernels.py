@@ -37,6 +37,14 @@ def test_sort_and_row_sums(lib, T, k, E):
         assert torch.equal(lib.moe_unpermute_sum(rows, inv, T, k), plain.to(torch.bfloat16))
 
 
+def test_row_sums_of_empty_rows(lib):
+    top = torch.tensor([[0, 1], [1, 0]], device="cuda", dtype=torch.int32)
+    inv = lib.moe_sort(top, 2, None)[1]
+    rows = torch.zeros(4, 0, device="cuda", dtype=torch.bfloat16)
+    assert lib.moe_combine_fwd(rows, inv, torch.ones(2, 2, device="cuda")).shape == (2, 0)
+    assert lib.moe_unpermute_sum(rows, inv, 2, 2).shape == (2, 0)
+
+
 @pytest.mark.parametrize("B,S,H", [(1, 1, 1), (2, 3, 5), (1, 1000, 2)])
 def test_rotary_with_rounded_products(lib, B, S, H):
     from q38.models import modeling
