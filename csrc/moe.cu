@@ -28,14 +28,23 @@ constexpr int MAX_TOPK = 8;
 
 // One warp per token, E <= 64 (two logits per lane).  probs = softmax(logits) in fp32, top-k, renormalise, round the
 // weights to bf16 (the logits' dtype).  Also accumulates assignment counts and probability sums for the balancing loss.
+// Both are the same bits in every run: they are added as whole numbers, the CTAs' probability sums as multiples of 2^-36 (64 bits hold 2^27
+// tokens), and the CTA that finishes last turns them into floats with one rounding.  16384 tokens: 25.6 us, 23 with float atomics and one more zero fill.
+struct RouteSums {
+  unsigned long long prob[64], not_finite;             // multiples of 2^-36; experts with a sum that has no such form, one bit each
+  unsigned int count[64], done;                        // assignments; CTAs that have added theirs
+};
 __global__ void __launch_bounds__(256) moe_route_fwd_kernel(const __nv_bfloat16* __restrict__ logits, int T, int E, int K,
                                                             float* __restrict__ top_w, int* __restrict__ top_idx,
                                                             float* __restrict__ probs_out, float* __restrict__ counts,
-                                                            float* __restrict__ prob_sum) {
-  __shared__ float s_cnt[64], s_ps[64];
-  if (threadIdx.x < 64) { s_cnt[threadIdx.x] = 0.f; s_ps[threadIdx.x] = 0.f; }
-  __syncthreads();
+                                                            RouteSums* __restrict__ sums, float* __restrict__ prob_sum) {
+  __shared__ float s_ps[8][64];
+  __shared__ unsigned int s_cnt[64];
+  __shared__ bool last;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if (threadIdx.x < 64) s_cnt[threadIdx.x] = 0;
+  s_ps[warp][lane] = s_ps[warp][lane + 32] = 0.f;
+  __syncthreads();
   const int t = blockIdx.x * 8 + warp;
   if (t < T) {
     const int e0 = lane, e1 = lane + 32;
@@ -45,8 +54,8 @@ __global__ void __launch_bounds__(256) moe_route_fwd_kernel(const __nv_bfloat16*
     float p0 = e0 < E ? __expf(l0 - mx) : 0.f, p1 = e1 < E ? __expf(l1 - mx) : 0.f;
     const float denom = warp_sum(p0 + p1);
     p0 /= denom; p1 /= denom;
-    if (e0 < E) { probs_out[(size_t)t * E + e0] = p0; atomicAdd(&s_ps[e0], p0); }
-    if (e1 < E) { probs_out[(size_t)t * E + e1] = p1; atomicAdd(&s_ps[e1], p1); }
+    if (e0 < E) { probs_out[(size_t)t * E + e0] = p0; s_ps[warp][e0] = p0; }
+    if (e1 < E) { probs_out[(size_t)t * E + e1] = p1; s_ps[warp][e1] = p1; }
     float a0 = e0 < E ? p0 : -1.f, a1 = e1 < E ? p1 : -1.f;
     float sel_p[MAX_TOPK]; int sel_e[MAX_TOPK];
     float total = 0.f;
@@ -68,12 +77,31 @@ __global__ void __launch_bounds__(256) moe_route_fwd_kernel(const __nv_bfloat16*
       for (int j = 0; j < K; ++j) {
         top_w[(size_t)t * K + j] = bf16_round(sel_p[j] / total);
         top_idx[(size_t)t * K + j] = sel_e[j];
-        atomicAdd(&s_cnt[sel_e[j]], 1.f);
+        atomicAdd(&s_cnt[sel_e[j]], 1u);
       }
     }
   }
   __syncthreads();
-  if (threadIdx.x < E) { atomicAdd(&counts[threadIdx.x], s_cnt[threadIdx.x]); atomicAdd(&prob_sum[threadIdx.x], s_ps[threadIdx.x]); }
+  if (threadIdx.x < E) {
+    const int e = threadIdx.x;
+    float v = 0.f;
+#pragma unroll
+    for (int w = 0; w < 8; ++w) v += s_ps[w][e];
+    if (v <= 8.5f) atomicAdd(&sums->prob[e], (unsigned long long)__float2ll_rn(v * 68719476736.f));
+    else atomicOr(&sums->not_finite, 1ull << e);
+    atomicAdd(&sums->count[e], s_cnt[e]);
+    __threadfence();
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) last = atomicAdd(&sums->done, 1u) == gridDim.x - 1;
+  __syncthreads();
+  if (last && threadIdx.x < E) {
+    __threadfence();
+    const int e = threadIdx.x;
+    counts[e] = (float)__ldcg(&sums->count[e]);
+    const bool bad = (__ldcg(&sums->not_finite) >> e) & 1ull;
+    prob_sum[e] = bad ? __int_as_float(0x7fc00000) : __ull2float_rn(__ldcg(&sums->prob[e])) * 1.4551915228366852e-11f;
+  }
 }
 
 // dlogits = probs * (dp - <dp, probs>),  dp_e = dprob_sum_e + [e selected as slot j] (dw_j - <dw, w>) / s
@@ -236,7 +264,7 @@ __global__ void __launch_bounds__(256) moe_gather_kernel(const __nv_bfloat16* __
   for (int i = lane; i < h / 8; i += 32) dst[i] = src[i];
 }
 
-// out[t,:] = sum_j w[t,j] * bf16(y_sorted[inv_perm[t*k+j], :])  (+ extra[t,:] * extra_scale[t])   fixed slot order, no atomics
+// out[t,:] = sum_j rows[inv_perm[t*k+j],:], or with weights sum_j bf16(w[t,j] rows[inv_perm[t*k+j],:]); fixed slot order, no atomics.
 // Row sums over the K slots in 16-byte pieces (h a multiple of 8, aligned rows): one thread per (token, piece), its K loads in flight together,
 // summed in slot order.  16384 x 5 x 576: 35 -> 27 us weighted, 32 -> 21 us plain, against 4-byte pieces one slot at a time; the bytes need 17.
 template <bool WEIGHTED>
@@ -274,7 +302,7 @@ __global__ void __launch_bounds__(256) moe_slot_sum_kernel(const __nv_bfloat16* 
   reinterpret_cast<uint4*>(out)[id] = make_uint4(o[0], o[1], o[2], o[3]);
 }
 
-// Any row length, 4-byte pieces.
+// The weighted sum for any row length, 4-byte pieces.
 __global__ void __launch_bounds__(256) moe_combine_fwd_kernel(const __nv_bfloat16* __restrict__ y_sorted, const int* __restrict__ inv_perm,
                                                               const float* __restrict__ top_w, int T, int K, int h,
                                                               __nv_bfloat16* __restrict__ out) {
@@ -739,10 +767,12 @@ std::vector<at::Tensor> moe_route_fwd(const at::Tensor& logits, int64_t k) {
   const int T = logits.size(0), E = logits.size(1);
   TORCH_CHECK(E <= 64 && k <= MAX_TOPK && k <= E, "moe_route_fwd: at most 64 experts and top-8");
   auto f32 = logits.options().dtype(at::kFloat);
-  auto top_w = at::empty({T, k}, f32), probs = at::empty({T, E}, f32), counts = at::zeros({E}, f32), psum = at::zeros({E}, f32);
+  auto top_w = at::empty({T, k}, f32), probs = at::empty({T, E}, f32);
+  auto sums = at::zeros({(int64_t)sizeof(RouteSums)}, logits.options().dtype(at::kByte));
+  auto counts = T ? at::empty({E}, f32) : at::zeros({E}, f32), psum = T ? at::empty({E}, f32) : at::zeros({E}, f32);
   auto top_idx = at::empty({T, k}, logits.options().dtype(at::kInt));
   if (T) moe_route_fwd_kernel<<<(T + 7) / 8, 256, 0, at::cuda::getCurrentCUDAStream()>>>((const __nv_bfloat16*)logits.data_ptr(), T, E, (int)k, top_w.data_ptr<float>(),
-      top_idx.data_ptr<int>(), probs.data_ptr<float>(), counts.data_ptr<float>(), psum.data_ptr<float>());
+      top_idx.data_ptr<int>(), probs.data_ptr<float>(), counts.data_ptr<float>(), reinterpret_cast<RouteSums*>(sums.data_ptr()), psum.data_ptr<float>());
   C10_CUDA_KERNEL_LAUNCH_CHECK();
   count_launch();
   return {top_w, top_idx, probs, counts, psum};

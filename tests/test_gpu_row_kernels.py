@@ -37,6 +37,26 @@ def test_sort_and_row_sums(lib, T, k, E):
         assert torch.equal(lib.moe_unpermute_sum(rows, inv, T, k), plain.to(torch.bfloat16))
 
 
+# one CTA of eight tokens, a ragged second one, more CTAs than fit the chip at once
+@pytest.mark.parametrize("T,E,k", [(1, 1, 1), (9, 64, 8), (16384, 64, 5), (5000, 33, 2)])
+def test_router_sums(lib, T, E, k):
+    gen = torch.Generator(device="cuda").manual_seed(T)
+    logits = (2 * torch.randn(T, E, device="cuda", generator=gen)).to(torch.bfloat16)
+    _, idx, probs, counts, prob_sum = lib.moe_route_fwd(logits, k)
+    assert torch.equal(counts, torch.bincount(idx.flatten().long(), minlength=E).float())
+    want = logits.double().softmax(-1)
+    # an approximate exponential and quotient (2^-21); a sum has seven roundings within a CTA, 2^-37 per CTA and one rounding at the end
+    assert ((probs.double() - want).norm() / want.norm()).item() < 1e-6
+    assert ((prob_sum.double() - probs.double().sum(0)).norm() / want.sum(0).norm()).item() < 3e-7
+    for _ in range(20):
+        again = lib.moe_route_fwd(logits, k)
+        assert torch.equal(again[4], prob_sum) and torch.equal(again[3], counts)
+    logits[T // 2, 0] = float("nan")
+    assert lib.moe_route_fwd(logits, k)[4].isnan().all()
+    empty = lib.moe_route_fwd(logits[:0], k)
+    assert not empty[3].any() and not empty[4].any()
+
+
 def test_row_sums_of_empty_rows(lib):
     top = torch.tensor([[0, 1], [1, 0]], device="cuda", dtype=torch.int32)
     inv = lib.moe_sort(top, 2, None)[1]
