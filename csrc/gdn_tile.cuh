@@ -72,7 +72,7 @@ __device__ __forceinline__ void slice_store_t(uint32_t base, const uint32_t (&a)
   }
 }
 
-// The four shared operand tiles of chunk `c` into one stage.
+// The four shared operand tiles of the chunk that starts at `row` into one stage.
 struct Maps4 { CUtensorMap m[4]; };
 __device__ __forceinline__ void load_stage(const Maps4& maps, uint8_t* stage, uint64_t* bar, int row) {
   ptx::mbar_expect_tx(bar, 4 * TILE_BYTES);
@@ -122,7 +122,9 @@ template <int N> struct Ring {
 inline int scan_warps(int64_t BH) { return 4 * BH <= kNumSMs ? 1 : 2; }
 
 // Column slices (a chain warp and its output warp each) per CTA of the forward scan: as few as keep every CTA on an SM of its own, because
-// the slices of a CTA share its schedulers and MMA pipes, while every further CTA of a pair reads the four operand tiles once more.
+// the slices of a CTA share its schedulers and MMA pipes, while every further CTA of a pair reads the four operand tiles once more.  Beyond 148
+// pairs whole pairs share an SM one after the other (188 KB each): 156 pairs of 64 chunks take 218 us and 296 take 225, where
+// the pass with block barriers took 302 and 306; 400 pairs 328 against 454.
 inline int scan_pairs(int64_t BH) { return 4 * BH <= kNumSMs ? 1 : 2 * BH <= kNumSMs ? 2 : 4; }
 
 }  // namespace gdn

@@ -145,7 +145,7 @@ __global__ void __launch_bounds__(128, 3) qsa_attn_bwd_q_kernel(const bf16* __re
                                                                 const unsigned char* __restrict__ sel, bf16* __restrict__ dq, float* __restrict__ Dout,
                                                                 int S, int nq, int nkv, float scale) {
   extern __shared__ __align__(16) uint8_t smem_bytes[];
-  bf16* KV = reinterpret_cast<bf16*>(smem_bytes);          // two buffers of {K, V}; a third pair for the prologue's q and o
+  bf16* KV = reinterpret_cast<bf16*>(smem_bytes);          // two buffers of {K, V} and one tile; at the start buffer 1 holds q and dO, the tile holds o
   unsigned short* list = reinterpret_cast<unsigned short*>(KV + 5 * TILE_ELEMS);
   __shared__ int count;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;

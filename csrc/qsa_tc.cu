@@ -78,7 +78,7 @@ __global__ void __launch_bounds__(QT_THREADS, 2) qsa_block_stats_tc_kernel(const
         const int s = g % QT_STAGES, round = g / QT_STAGES;
         if (!ptx::mbar_wait(&k_empty[s], (round & 1) ^ 1, 1u << 20)) { report_error(p.err, ERR_MMA_WAIT); break; }
         ptx::mbar_expect_tx(&k_full[s], K_BYTES);
-        ptx::tma_load_3d(k_ring + s * K_BYTES, &tmK, &k_full[s], 0, g * QT_KEYS, k_batch);     // rows past S are zero-filled
+        ptx::tma_load_3d(k_ring + s * K_BYTES, &tmK, &k_full[s], 0, g * QT_KEYS, k_batch);     // S is a whole number of groups
       }
     }
   } else if (warp == 1) {

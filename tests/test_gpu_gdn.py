@@ -24,8 +24,8 @@ def chunk_operands(BH, NT, seed):
     return [x.to(torch.bfloat16) for x in (w, u, P, qg, kg)] + [torch.rand(BH, NT, device="cuda", generator=gen)]
 
 
-# 1 and 37 pairs: four CTAs per pair; 38 and 74: two; 75: one; chunk counts below, at and above the three and four pipeline stages
-@pytest.mark.parametrize("B,H", [(1, 1), (1, 37), (2, 19), (2, 37), (5, 15)])
+# 1 and 37 pairs: four CTAs per pair; 38 and 74: two; 75: one; 156: more pairs than SMs; chunk counts below, at and above the three and four pipeline stages
+@pytest.mark.parametrize("B,H", [(1, 1), (1, 37), (2, 19), (2, 37), (5, 15), (4, 39)])
 @pytest.mark.parametrize("NT", [1, 2, 3, 4, 5, 9])
 def test_scan_forward(ops, B, H, NT):
     BH = B * H
