@@ -88,7 +88,7 @@ TORCH_LIBRARY(q38, m) {
   m.def("qsa_select(Tensor lp_blk, int budget) -> Tensor[]");
   m.def("qsa_indexer_bwd(Tensor qi, Tensor ki, Tensor wi, Tensor blse, Tensor dblse, float gscale, float scale) -> Tensor[]");
   m.def("qsa_attn_fwd(Tensor q, Tensor k, Tensor v, Tensor? count, Tensor? index, float scale) -> Tensor[]");
-  m.def("qsa_attn_bwd(Tensor q, Tensor k, Tensor v, Tensor o, Tensor dout, Tensor lse, Tensor sel, float scale) -> Tensor[]");
+  m.def("qsa_attn_bwd(Tensor q, Tensor k, Tensor v, Tensor o, Tensor dout, Tensor lse, Tensor sel, float scale, Tensor(a!)? err=None) -> Tensor[]");
   m.def("ep_publish_counts(Tensor offsets, int rank, int[] peer_counts) -> ()",
         [](const at::Tensor& o, int64_t rank, std::vector<int64_t> peers) { q38::ep_publish_counts(o, rank, peers); });
   m.def("ep_plan(Tensor counts_all, int rank, int world, int capacity, Tensor(a!) err) -> Tensor[]",

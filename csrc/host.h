@@ -133,11 +133,11 @@ std::vector<at::Tensor> qsa_indexer_bwd(const at::Tensor& qi, const at::Tensor& 
                                         double gscale, double scale);
 // qsa_tc.cu
 at::Tensor qsa_block_stats_tc(const at::Tensor& q, const at::Tensor& k, double scale, at::Tensor& err);
-// qsa_attn.cu
+// qsa_attn.cu, qsa_attn_bwd.cu
 std::vector<at::Tensor> qsa_attn_fwd(const at::Tensor& q, const at::Tensor& k, const at::Tensor& v, const c10::optional<at::Tensor>& count,
                                      const c10::optional<at::Tensor>& index, double scale);
 std::vector<at::Tensor> qsa_attn_bwd(const at::Tensor& q, const at::Tensor& k, const at::Tensor& v, const at::Tensor& o, const at::Tensor& dout,
-                                     const at::Tensor& lse, const at::Tensor& sel, double scale);
+                                     const at::Tensor& lse, const at::Tensor& sel, double scale, const c10::optional<at::Tensor>& err);
 // ep.cu
 void ep_publish_counts(const at::Tensor& offsets, int64_t rank, std::vector<int64_t> peer_counts);
 std::vector<at::Tensor> ep_plan(const at::Tensor& counts_all, int64_t rank, int64_t world, int64_t capacity, at::Tensor& err);

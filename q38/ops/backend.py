@@ -558,7 +558,7 @@ class _BlockAttention(torch.autograd.Function):
     @staticmethod
     def backward(ctx, do):
         q, k, v, o, lse, sel = ctx.saved_tensors
-        dq, dk, dv = load().qsa_attn_bwd(q, k, v, o, do.to(torch.bfloat16).contiguous(), lse, sel, ctx.scale)
+        dq, dk, dv = load().qsa_attn_bwd(q, k, v, o, do.to(torch.bfloat16).contiguous(), lse, sel, ctx.scale, error_flag(q.device))
         return dq, dk, dv, None, None, None
 
 

@@ -1,0 +1,21 @@
+"""Attention and indexer kernels on the tcgen05 path at the edges of their tiles, against the same sums in 64 bits."""
+import pytest
+import torch
+
+from test_gpu_qsa_edges import ops, rel, test_block_attention as block_attention  # noqa: F401
+from test_kernel_sources import test_waits_of_whole_warps_are_voted as waits_are_voted
+
+gpu = pytest.mark.gpu
+
+
+# one and an odd number of heads per group (a half-empty tile of the dQ pass; an odd last (query block, head) pair of the dK / dV pass), one tile, fewer
+# tiles than a part has, and key blocks split over several parts of unequal length
+@gpu
+@pytest.mark.parametrize("B,nb,nq,nkv,pick", [(1, 1, 1, 1, "dense"), (1, 1, 3, 1, "dense"), (2, 9, 11, 1, "gaps"), (1, 21, 10, 2, "dense"), (1, 24, 22, 2, "gaps")])
+def test_block_attention_tiles(ops, B, nb, nq, nkv, pick):  # noqa: F811
+    block_attention(ops, B, nb, nq, nkv, pick)
+
+
+@pytest.mark.parametrize("name", ["qsa_attn_bwd.cu"])
+def test_waits_of_whole_warps(name):
+    waits_are_voted(name)
