@@ -20,8 +20,9 @@
 #include <ATen/cuda/CUDAContext.h>
 #include <c10/cuda/CUDAGuard.h>
 
-#include "ptx.cuh"
+#include "f32x2.cuh"
 #include "host.h"
+#include "ptx.cuh"
 #include "qsa_blocks.cuh"
 
 namespace q38 {
@@ -44,14 +45,6 @@ struct BwdArgs {
   float scale;
   int* err;
 };
-
-// Pairs of fp32 in one 64-bit register: one instruction for two elements.
-__device__ __forceinline__ uint64_t pair2(float a, float b) { uint64_t r; asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b)); return r; }
-__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) { uint64_t r; asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c)); return r; }
-__device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b) { uint64_t r; asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b)); return r; }
-__device__ __forceinline__ float2 unpair(uint64_t a) { float2 f; asm("mov.b64 {%0, %1}, %2;" : "=f"(f.x), "=f"(f.y) : "l"(a)); return f; }
-__device__ __forceinline__ uint32_t bf16_pair(float2 f) { const __nv_bfloat162 h = __floats2bfloat162_rn(f.x, f.y); return *reinterpret_cast<const uint32_t*>(&h); }
-__device__ __forceinline__ float exp2_approx(float x) { float y; asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x)); return y; }
 
 // 32 scores and probability gradients of one row -> packed P and dS.  DIAG: keys after `last` (the query's own position) get zero; `key0` is
 // the first of the 32.

@@ -7,7 +7,7 @@
 //   qsa_kl_combine        per token: target P[t,b] (head-averaged block mass), lp_blk[t,b] = bLSE - logsumexp_b bLSE,
 //                         KL_t = sum_b P (log P - lp_blk) and the gradient seed (exp(lp_blk) - P).
 //   qsa_select            per query block: top-k key blocks from the first query's lp_blk (own block forced, future excluded).
-//   qsa_indexer_bwd_q / _k  recompute the score tiles and produce d(q_idx), d(w) / d(k_idx).
+// The backward pass of the scores is in qsa_index_bwd.cu.
 //
 // Layouts: main q [B,nq,S,64], main k [B,nkv,S,64], indexer q [B,NI,S,64], indexer k [B,S,64] (bf16); w [B,S,NI] fp32.
 #include <ATen/ATen.h>
@@ -249,277 +249,6 @@ __global__ void __launch_bounds__(256) qsa_select_kernel(const float* __restrict
   if (lane == 0) count[b * nb + j] = (j + 1 < k) ? j + 1 : k;
 }
 
-// ---- indexer backward ------------------------------------------------------------------------------------------------------
-// dI[t,s] = dblse[t, blk(s)] * exp(I[t,s] - blse[t, blk(s)]) for s <= t;   I = sum_h w_h relu(S_h) scale
-// Both passes form the scores of all heads once per (query block, key block) pair, keep relu(S_h) (which is bf16 by definition) packed in
-// registers until dI is known, and pass dS_h to the next product as A fragments in registers.  Four sequences of 4096 with four heads: 741 -> 413 us.
-
-// Query pass, grid (nb, B, z), eight warps: d q_h(t) = sum_s dI w_h scale [S_h > 0] k(s);  d w_h(t) = sum_s dI relu(S_h) scale.
-// Warps 0-3 hold heads 0 and 1, warps 4-7 heads 2 and 3, each warp 16 queries; the two partial scores of a tile meet in shared memory.
-// Eight 64^3 products per pair (one CTA per head had twenty).  Bound by the latency of their chain: a tile costs a CTA four times its issue slots, and
-// the last query block has 64 tiles.  So tiles are taken in quarters of 16 keys, which keeps two CTAs on an SM (128 registers), and the key
-// blocks j <= i of a query block are shared by gridDim.z CTAs (j = z, z + gridDim.z, ...).  Each leaves its partial gradients in its own slice of
-// dqi [z,B,NI,S,64] and dwi [z,B,S,NI], which the kernel below adds in ascending z: no atomics, the same bits in every run.  About 255 us;
-// one CTA of eight warps per query block and SM took 306, sixteen warps with one head per four of them 396 (four times the exponentials).
-__global__ void __launch_bounds__(256, 2) qsa_indexer_bwd_q_kernel(const bf16* __restrict__ qi, const bf16* __restrict__ ki, const float* __restrict__ wi,
-                                                                   const float* __restrict__ blse, const float* __restrict__ dblse, float gscale,
-                                                                   float* __restrict__ dqi, float* __restrict__ dwi, int S, int NI, float scale) {
-  extern __shared__ __align__(16) uint8_t smem_bytes[];
-  bf16* Qs = reinterpret_cast<bf16*>(smem_bytes);          // NI tiles
-  bf16* Ks = Qs + NI_MAX * TILE_ELEMS;                     // two buffers
-  float4* Px = reinterpret_cast<float4*>(Ks + 2 * TILE_ELEMS);     // partial scores per 16 keys: [4 quarters][2 groups][2 n-tiles][4 warps][32 lanes]
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, wr = warp & 3, grp = warp >> 2;
-  const int nb = S / 64, i = nb - 1 - blockIdx.x, b = blockIdx.y, step = gridDim.z;   // late query blocks (longest loops) first
-  if ((int)blockIdx.z > i) return;
-  for (int hh = 0; hh < NI; ++hh) load_tile_async_256(Qs + hh * TILE_ELEMS, qi + (((long long)b * NI + hh) * S + (long long)i * 64) * 64, 64, tid);
-  const bf16* kbase = ki + (long long)b * S * 64;
-  load_tile_async_256(Ks, kbase + (long long)blockIdx.z * 4096, 64, tid);
-  cp_async_commit();
-  const int r0 = 16 * wr + (lane >> 2), cq = 2 * (lane & 3);
-  const long long row = (long long)b * S + (long long)i * 64 + r0;
-  const int heads = NI - 2 * grp < 0 ? 0 : (NI - 2 * grp > 2 ? 2 : NI - 2 * grp);     // of this warp: 2 grp .. 2 grp + heads - 1
-  float w[2][2], dw[2][2] = {{0.f, 0.f}, {0.f, 0.f}};      // [head][row half]
-#pragma unroll
-  for (int x = 0; x < 2; ++x)
-#pragma unroll
-    for (int hr = 0; hr < 2; ++hr) w[x][hr] = x < heads ? wi[(row + 8 * hr) * NI + 2 * grp + x] * scale : 0.f;
-  float dq[2][8][4];
-  zero_acc(dq[0]);
-  zero_acc(dq[1]);
-  float bl[2], g[2];
-#pragma unroll
-  for (int hr = 0; hr < 2; ++hr) { bl[hr] = blse[(row + 8 * hr) * nb + blockIdx.z]; g[hr] = dblse[(row + 8 * hr) * nb + blockIdx.z]; }
-  for (int j = blockIdx.z, buf = 0; j <= i; j += step, buf ^= 1) {
-    cp_async_wait<0>();
-    __syncthreads();
-    const bool more = j + step <= i;
-    if (more) load_tile_async_256(Ks + (buf ^ 1) * TILE_ELEMS, kbase + (long long)(j + step) * 4096, 64, tid);
-    cp_async_commit();
-    const bf16* Kt = Ks + buf * TILE_ELEMS;
-    const float b0 = bl[0], b1 = bl[1], g0 = g[0] * gscale, g1 = g[1] * gscale;
-    if (more) {
-#pragma unroll
-      for (int hr = 0; hr < 2; ++hr) { bl[hr] = blse[(row + 8 * hr) * nb + j + step]; g[hr] = dblse[(row + 8 * hr) * nb + j + step]; }
-    }
-#pragma unroll
-    for (int part = 0; part < 4; ++part) {                 // 16 keys at a time
-      uint32_t r[2][1][4];                                 // relu(S_h) as A fragments
-      float score[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
-#pragma unroll
-      for (int x = 0; x < 2; ++x) {
-        float acc[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
-        if (x < heads) {
-          uint32_t a[4][4];
-          load_a(Qs + (2 * grp + x) * TILE_ELEMS, a, wr, lane);
-          mma_rows<true, 4, 2>(a, Kt + 16 * part * LDS, acc, lane);
-        }
-#pragma unroll
-        for (int nt = 0; nt < 2; ++nt)
-#pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            acc[nt][e] = fmaxf(bf16_round(acc[nt][e]), 0.f);
-            score[nt][e] += w[x][e >> 1] * acc[nt][e];
-          }
-        pack_a<1>(acc, r[x]);
-      }
-#pragma unroll
-      for (int nt = 0; nt < 2; ++nt) Px[((part * 2 + grp) * 2 + nt) * 128 + wr * 32 + lane] = make_float4(score[nt][0], score[nt][1], score[nt][2], score[nt][3]);
-      // the two warps of these 16 rows meet; this quarter's buffer is free again after the block barrier of the next tile
-      asm volatile("bar.sync %0, 64;" ::"r"(1 + wr) : "memory");
-#pragma unroll
-      for (int nt = 0; nt < 2; ++nt) {
-        const float4 o = Px[((part * 2 + (grp ^ 1)) * 2 + nt) * 128 + wr * 32 + lane];
-        const float other[4] = {o.x, o.y, o.z, o.w};
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          const int col = 16 * part + 8 * nt + cq + (e & 1);
-          const float d = (e >> 1 ? g1 : g0) * __expf(score[nt][e] + other[e] - (e >> 1 ? b1 : b0));
-          score[nt][e] = (j < i || col <= r0 + 8 * (e >> 1)) ? d : 0.f;       // dI
-        }
-      }
-#pragma unroll
-      for (int x = 0; x < 2; ++x) {
-        if (x < heads) {
-          float ds[2][4];
-#pragma unroll
-          for (int nt = 0; nt < 2; ++nt)
-#pragma unroll
-            for (int e = 0; e < 4; ++e) {
-              const uint32_t p = r[x][0][nt * 2 + (e >> 1)];
-              const float relu = (e & 1) ? hi_f(p) : lo_f(p);
-              dw[x][e >> 1] += score[nt][e] * relu * scale;
-              ds[nt][e] = relu > 0.f ? score[nt][e] * w[x][e >> 1] : 0.f;     // dS_h
-            }
-          uint32_t a[1][4];
-          pack_a<1>(ds, a);
-          mma_rows<false, 1, 8>(a, Kt + 16 * part * LDS, dq[x], lane);        // dS_h K
-        }
-      }
-    }
-  }
-  cp_async_wait<0>();
-#pragma unroll
-  for (int x = 0; x < 2; ++x) {
-    if (x < heads) {
-      const int own = 2 * grp + x;
-      float* dst = dqi + ((((long long)blockIdx.z * gridDim.y + b) * NI + own) * S + (long long)i * 64) * 64;
-#pragma unroll
-      for (int nt = 0; nt < 8; ++nt)
-#pragma unroll
-        for (int hr = 0; hr < 2; ++hr)
-          *reinterpret_cast<float2*>(dst + (r0 + 8 * hr) * 64 + 8 * nt + cq) = make_float2(dq[x][nt][2 * hr], dq[x][nt][2 * hr + 1]);
-#pragma unroll
-      for (int hr = 0; hr < 2; ++hr) {
-        float v = dw[x][hr];
-        v += __shfl_xor_sync(0xffffffffu, v, 1);
-        v += __shfl_xor_sync(0xffffffffu, v, 2);
-        if ((lane & 3) == 0) dwi[((long long)blockIdx.z * gridDim.y * S + row + 8 * hr) * NI + own] = v;
-      }
-    }
-  }
-}
-
-// The query pass' partial gradients added up: query block i has min(i + 1, Z) of them.  One thread per eight dims of a row; the
-// first of a row's eight threads also takes its head weight.
-__global__ void __launch_bounds__(256) qsa_indexer_sum_q_kernel(const float* __restrict__ part, const float* __restrict__ dw_part, bf16* __restrict__ dqi,
-                                                                float* __restrict__ dwi, int B, int NI, int S, int Z) {
-  const long long id = (long long)blockIdx.x * 256 + threadIdx.x, rows = (long long)B * NI * S, row = id >> 3;
-  if (row >= rows) return;
-  const int s = (int)(row % S), n = min(s / 64 + 1, Z);
-  float v[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-  for (int z = 0; z < n; ++z) {
-    const float4* src = reinterpret_cast<const float4*>(part + (z * rows * 8 + id) * 8);
-    const float4 a = src[0], c = src[1];
-    v[0] += a.x; v[1] += a.y; v[2] += a.z; v[3] += a.w;
-    v[4] += c.x; v[5] += c.y; v[6] += c.z; v[7] += c.w;
-  }
-  reinterpret_cast<uint4*>(dqi)[id] = make_uint4(pack_f2(v[0], v[1]), pack_f2(v[2], v[3]), pack_f2(v[4], v[5]), pack_f2(v[6], v[7]));
-  if ((id & 7) == 0) {
-    const long long bh = row / S, at = ((bh / NI) * S + s) * NI + bh % NI;
-    float w = 0.f;
-    for (int z = 0; z < n; ++z) w += dw_part[z * rows + at];
-    dwi[at] = w;
-  }
-}
-
-// Key pass, grid (nb, B, z), four warps of 16 keys: d k(s) = sum_{t >= s} sum_h dS_h[t,s] q_h(t).  Scores are formed transposed (K Q_h^T), so
-// dS_h^T is the A fragment of dS_h^T Q_h.  The query blocks i >= j of a key block are shared by gridDim.z CTAs (i = j + z, j + z + gridDim.z, ...),
-// whose partial gradients are added in fp32.  Eight products per pair, bound by the warp MMA rate.
-__global__ void __launch_bounds__(128) qsa_indexer_bwd_k_kernel(const bf16* __restrict__ qi, const bf16* __restrict__ ki, const float* __restrict__ wi,
-                                                                const float* __restrict__ blse, const float* __restrict__ dblse, float gscale,
-                                                                float* __restrict__ dki, int S, int NI, float scale) {
-  extern __shared__ __align__(16) uint8_t smem_bytes[];
-  bf16* Qs = reinterpret_cast<bf16*>(smem_bytes);          // two buffers of NI_MAX tiles
-  float* rows = reinterpret_cast<float*>(Qs + 2 * NI_MAX * TILE_ELEMS);      // two buffers of {blse[64], dblse gscale[64], w scale[NI_MAX][64]}
-  constexpr int ROWS = (2 + NI_MAX) * 64;
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int j = blockIdx.x, b = blockIdx.y, nb = S / 64;
-  if (j + (int)blockIdx.z >= nb) return;
-  load_tile_async(Qs + NI_MAX * TILE_ELEMS, ki + ((long long)b * S + (long long)j * 64) * 64, 64, tid);
-  cp_async_commit();
-  auto fetch = [&](int i, int buf) {
-    for (int hh = 0; hh < NI; ++hh) load_tile_async(Qs + (buf * NI_MAX + hh) * TILE_ELEMS, qi + (((long long)b * NI + hh) * S + (long long)i * 64) * 64, 64, tid);
-    cp_async_commit();
-  };
-  // per query: this thread's share (query tid % 64) travels through registers so that its latency hides behind a whole tile
-  float v0 = 0.f, v1 = 0.f, v2 = 0.f;
-  auto fetch_rows = [&](int i) {
-    const long long t = (long long)b * S + (long long)i * 64 + (tid & 63);
-    const int hh = 2 * (tid >> 6);                         // the first 64 threads bring blse and heads 0, 1, the others dblse and heads 2, 3
-    v0 = tid < 64 ? blse[t * nb + j] : dblse[t * nb + j] * gscale;
-    v1 = hh < NI ? wi[t * NI + hh] * scale : 0.f;
-    v2 = hh + 1 < NI ? wi[t * NI + hh + 1] * scale : 0.f;
-  };
-  auto put_rows = [&](int buf) {
-    float* dst = rows + buf * ROWS + (tid & 63);
-    const int half = tid >> 6;
-    dst[64 * half] = v0;
-    dst[64 * (2 + 2 * half)] = v1;
-    dst[64 * (3 + 2 * half)] = v2;
-  };
-  const int step = gridDim.z;
-  int i = j + blockIdx.z;
-  fetch(i, 0);
-  fetch_rows(i);
-  cp_async_wait<1>();
-  __syncthreads();
-  uint32_t ak[4][4];
-  load_a(Qs + NI_MAX * TILE_ELEMS, ak, warp, lane);
-  put_rows(0);
-  const int r0 = 16 * warp + (lane >> 2), cq = 2 * (lane & 3);
-  float dk[8][4];
-  zero_acc(dk);
-  for (int buf = 0; i < nb; i += step, buf ^= 1) {
-    cp_async_wait<0>();
-    __syncthreads();
-    const bool more = i + step < nb;
-    if (more) { fetch(i + step, buf ^ 1); fetch_rows(i + step); }
-    const bf16* Qt = Qs + buf * NI_MAX * TILE_ELEMS;
-    const float* rw = rows + buf * ROWS;
-    const bool diag = i == j;
-#pragma unroll
-    for (int half = 0; half < 2; ++half) {                 // 32 queries at a time
-      uint32_t r[NI_MAX][2][4];
-      float score[4][4];
-      zero_acc(score);
-#pragma unroll
-      for (int hh = 0; hh < NI_MAX; ++hh) {
-        if (hh < NI) {
-          float acc[4][4];
-          zero_acc(acc);
-          mma_rows<true, 4, 4>(ak, Qt + hh * TILE_ELEMS + 32 * half * LDS, acc, lane);
-#pragma unroll
-          for (int nt = 0; nt < 4; ++nt) {
-            const float2 w = *reinterpret_cast<const float2*>(rw + 64 * (2 + hh) + 32 * half + 8 * nt + cq);
-#pragma unroll
-            for (int e = 0; e < 4; ++e) {
-              acc[nt][e] = fmaxf(bf16_round(acc[nt][e]), 0.f);
-              score[nt][e] += (e & 1 ? w.y : w.x) * acc[nt][e];
-            }
-          }
-          pack_a<2>(acc, r[hh]);
-        }
-      }
-#pragma unroll
-      for (int nt = 0; nt < 4; ++nt) {
-        const int col = 32 * half + 8 * nt + cq;           // query
-        const float2 bl = *reinterpret_cast<const float2*>(rw + col), g = *reinterpret_cast<const float2*>(rw + 64 + col);
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          const float d = (e & 1 ? g.y : g.x) * __expf(score[nt][e] - (e & 1 ? bl.y : bl.x));
-          score[nt][e] = (!diag || r0 + 8 * (e >> 1) <= col + (e & 1)) ? d : 0.f;       // dI
-        }
-      }
-#pragma unroll
-      for (int hh = 0; hh < NI_MAX; ++hh) {
-        if (hh < NI) {
-          float ds[4][4];
-#pragma unroll
-          for (int nt = 0; nt < 4; ++nt) {
-            const float2 w = *reinterpret_cast<const float2*>(rw + 64 * (2 + hh) + 32 * half + 8 * nt + cq);
-#pragma unroll
-            for (int e = 0; e < 4; ++e) {
-              const uint32_t p = r[hh][nt >> 1][(nt & 1) * 2 + (e >> 1)];
-              ds[nt][e] = ((e & 1) ? hi_f(p) : lo_f(p)) > 0.f ? score[nt][e] * (e & 1 ? w.y : w.x) : 0.f;
-            }
-          }
-          uint32_t a[2][4];
-          pack_a<2>(ds, a);
-          mma_rows<false, 2, 8>(a, Qt + hh * TILE_ELEMS + 32 * half * LDS, dk, lane);   // dS_h^T Q_h
-        }
-      }
-    }
-    if (more) put_rows(buf ^ 1);
-  }
-  cp_async_wait<0>();
-  float* dst = dki + ((long long)b * S + (long long)j * 64) * 64;
-#pragma unroll
-  for (int nt = 0; nt < 8; ++nt)
-#pragma unroll
-    for (int x = 0; x < 2; ++x)
-      atomicAdd(reinterpret_cast<float2*>(dst + (r0 + 8 * x) * 64 + 8 * nt + cq), make_float2(dk[nt][2 * x], dk[nt][2 * x + 1]));
-}
-
 // ---- host ----------------------------------------------------------------------------------------------------------------------
 static void check4(const at::Tensor& t, const char* name) {
   TORCH_CHECK(t.is_cuda() && t.scalar_type() == at::kBFloat16 && t.is_contiguous() && t.size(-1) == 64, name, ": contiguous bf16 [...,64] required");
@@ -590,40 +319,6 @@ std::vector<at::Tensor> qsa_select(const at::Tensor& lp_blk, int64_t budget) {
   C10_CUDA_KERNEL_LAUNCH_CHECK();
   count_launch();
   return {count, index};
-}
-
-// Returns {dqi [B,NI,S,64] bf16, dki [B,S,64] bf16, dwi [B,S,NI] fp32}; gscale multiplies dblse (upstream grad / token count).
-std::vector<at::Tensor> qsa_indexer_bwd(const at::Tensor& qi, const at::Tensor& ki, const at::Tensor& wi, const at::Tensor& blse, const at::Tensor& dblse,
-                                        double gscale, double scale) {
-  check4(qi, "qsa_indexer_bwd q"); check4(ki, "qsa_indexer_bwd k");
-  const c10::cuda::CUDAGuard guard(qi.device());
-  TORCH_CHECK(qi.dim() == 4 && qi.size(1) <= NI_MAX && qi.size(2) % 64 == 0, "qsa_indexer_bwd: at most 4 indexer heads and whole blocks of 64 tokens");
-  const int B = qi.size(0), NI = qi.size(1), S = qi.size(2), nb = S / 64;
-  TORCH_CHECK(ki.numel() == (int64_t)B * S * 64, "qsa_indexer_bwd: k must be [B,S,64]");
-  auto rows = [&](const at::Tensor& t, int64_t n) { return t.is_cuda() && t.scalar_type() == at::kFloat && t.is_contiguous() && t.numel() == (int64_t)B * S * n; };
-  TORCH_CHECK(rows(wi, NI) && rows(blse, nb) && rows(dblse, nb), "qsa_indexer_bwd: contiguous fp32 w [B,S,heads], blse and dblse [B,S,blocks] required");
-  const int Z = std::min(nb, 4);
-  auto f32 = qi.options().dtype(at::kFloat);
-  auto part = at::empty({Z, B, NI, S, 64}, f32), dw_part = at::empty({Z, B, S, NI}, f32);
-  auto dqi = at::empty(qi.sizes(), qi.options()), dwi = at::empty(wi.sizes(), wi.options());
-  auto dki32 = at::zeros(ki.sizes(), f32);
-  constexpr int smem_q = (NI_MAX + 2) * TILE_ELEMS * 2 + 16 * 128 * 16, smem_k = 2 * NI_MAX * TILE_ELEMS * 2 + 2 * (2 + NI_MAX) * 64 * 4;
-  static bool cfg = false;
-  if (!cfg) {
-    C10_CUDA_CHECK(cudaFuncSetAttribute(qsa_indexer_bwd_q_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_q));
-    C10_CUDA_CHECK(cudaFuncSetAttribute(qsa_indexer_bwd_k_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_k));
-    cfg = true;
-  }
-  auto stream = at::cuda::getCurrentCUDAStream();
-  qsa_indexer_bwd_q_kernel<<<dim3(nb, B, Z), 256, smem_q, stream>>>((const bf16*)qi.data_ptr(), (const bf16*)ki.data_ptr(), wi.data_ptr<float>(), blse.data_ptr<float>(),
-      dblse.data_ptr<float>(), (float)gscale, part.data_ptr<float>(), dw_part.data_ptr<float>(), S, NI, (float)scale);
-  qsa_indexer_sum_q_kernel<<<(unsigned)(((long long)B * NI * S * 8 + 255) / 256), 256, 0, stream>>>(part.data_ptr<float>(), dw_part.data_ptr<float>(), (bf16*)dqi.data_ptr(),
-      dwi.data_ptr<float>(), B, NI, S, Z);
-  qsa_indexer_bwd_k_kernel<<<dim3(nb, B, std::min(nb, 8)), 128, smem_k, stream>>>((const bf16*)qi.data_ptr(), (const bf16*)ki.data_ptr(), wi.data_ptr<float>(),
-      blse.data_ptr<float>(), dblse.data_ptr<float>(), (float)gscale, dki32.data_ptr<float>(), S, NI, (float)scale);
-  C10_CUDA_KERNEL_LAUNCH_CHECK();
-  count_launch(3);
-  return {dqi, dki32.to(at::kBFloat16), dwi};
 }
 
 }  // namespace q38

@@ -415,7 +415,7 @@ class _IndexerKL(torch.autograd.Function):
     def backward(ctx, dkl, _lp):
         qi, ki, wi, blse, dblse = ctx.saved_tensors
         tokens = qi.shape[0] * qi.shape[2]
-        dqi, dki, dwi = load().qsa_indexer_bwd(qi, ki, wi, blse, dblse, 1.0 / tokens, ctx.idx_scale)
+        dqi, dki, dwi = load().qsa_indexer_bwd(qi, ki, wi, blse, dblse, 1.0 / tokens, ctx.idx_scale, error_flag(qi.device))
         return dqi * dkl.to(dqi.dtype), dki * dkl.to(dki.dtype), dwi * dkl, None, None, None, None
 
 

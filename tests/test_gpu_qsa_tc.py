@@ -2,7 +2,7 @@
 import pytest
 import torch
 
-from test_gpu_qsa_edges import ops, rel, test_block_attention as block_attention  # noqa: F401
+from test_gpu_qsa_edges import ops, test_block_attention as block_attention, test_indexer_backward as indexer_backward  # noqa: F401
 from test_kernel_sources import test_waits_of_whole_warps_are_voted as waits_are_voted
 
 gpu = pytest.mark.gpu
@@ -16,6 +16,13 @@ def test_block_attention_tiles(ops, B, nb, nq, nkv, pick):  # noqa: F811
     block_attention(ops, B, nb, nq, nkv, pick)
 
 
-@pytest.mark.parametrize("name", ["qsa_attn_bwd.cu"])
+# enough query blocks for one CTA each (no slices): a half-empty key tile, one and a half key tiles; heads that do not exist
+@gpu
+@pytest.mark.parametrize("B,nb,NI", [(150, 1, 4), (50, 3, 3)])
+def test_indexer_backward_without_slices(ops, B, nb, NI):  # noqa: F811
+    indexer_backward(ops, NI, B, nb)
+
+
+@pytest.mark.parametrize("name", ["qsa_attn_bwd.cu", "qsa_index_bwd.cu"])
 def test_waits_of_whole_warps(name):
     waits_are_voted(name)
