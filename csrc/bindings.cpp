@@ -7,7 +7,7 @@
 namespace q38 {
 std::atomic<long long> g_launches{0};
 at::Tensor qsa_first_query_lp(const at::Tensor& q_first, const at::Tensor& ki, const at::Tensor& w_first, double scale);   // qsa_first.cu
-bool gemm_bf16_pair(const at::Tensor& a, const at::Tensor& b, at::Tensor& c, double alpha, bool accumulate, at::Tensor& err);   // gemm_pair.cu
+bool gemm_bf16_pair(const Mat& a, const Mat& b, const Mat& c, double alpha, bool accumulate, int* err);   // gemm_pair.cu
 }
 
 TORCH_LIBRARY(q38, m) {
@@ -16,6 +16,7 @@ TORCH_LIBRARY(q38, m) {
   m.def("gemm_bf16_persistent(Tensor a, Tensor b, Tensor(a!) c, bool a_mn_major, bool b_mn_major, float alpha, bool accumulate, Tensor(b!) err, int splits, Tensor? addend=None, float beta=0.0) -> ()",
         [](const at::Tensor& a, const at::Tensor& b, at::Tensor& c, bool amn, bool bmn, double alpha, bool acc, at::Tensor& err, int64_t splits,
            c10::optional<at::Tensor> addend, double beta) {
+          TORCH_CHECK(a.dim() == 3 && b.dim() == 3 && c.dim() == 3, "gemm_bf16_persistent: [batch, rows, cols] tensors required");
           q38::gemm_bf16_persistent(a, b, c, amn, bmn, alpha, acc, err, splits, addend, beta);
         });
   m.def("mxfp8_pick_bn(int N) -> int", &q38::mxfp8_pick_bn);
@@ -45,15 +46,13 @@ TORCH_LIBRARY(q38, m) {
         [](const at::Tensor& a, const at::Tensor& b, bool amn, bool bmn, double alpha, bool fp32, at::Tensor& err) {
           TORCH_CHECK(a.dim() == 2 && b.dim() == 2, "gemm2d: 2-D operands required");
           auto c = at::empty({a.size(amn ? 1 : 0), b.size(bmn ? 1 : 0)}, a.options().dtype(fp32 ? at::kFloat : at::kBFloat16));
-          auto c3 = c.unsqueeze(0);
-          q38::gemm_bf16_persistent(a.unsqueeze(0), b.unsqueeze(0), c3, amn, bmn, alpha, false, err, -1);
+          q38::gemm_bf16_persistent(a, b, c, amn, bmn, alpha, false, err, -1);
           return c;
         });
   m.def("gemm2d_out(Tensor a, Tensor b, Tensor(a!) c, bool a_mn_major, bool b_mn_major, float alpha, bool accumulate, Tensor(b!) err, int splits) -> ()",
         [](const at::Tensor& a, const at::Tensor& b, at::Tensor& c, bool amn, bool bmn, double alpha, bool acc, at::Tensor& err, int64_t splits) {
           TORCH_CHECK(a.dim() == 2 && b.dim() == 2 && c.dim() == 2, "gemm2d_out: 2-D tensors required");
-          auto c3 = c.unsqueeze(0);
-          q38::gemm_bf16_persistent(a.unsqueeze(0), b.unsqueeze(0), c3, amn, bmn, alpha, acc, err, splits);
+          q38::gemm_bf16_persistent(a, b, c, amn, bmn, alpha, acc, err, splits);
         });
   m.def("cast_shadow_except(Tensor params, Tensor(a!) shadow, int skip_start, int skip_count, Tensor? err) -> ()",
         [](const at::Tensor& p, at::Tensor& sh, int64_t s0, int64_t n, c10::optional<at::Tensor> err) { q38::cast_shadow_except(p, sh, s0, n, err); });
@@ -82,7 +81,10 @@ TORCH_LIBRARY(q38, m) {
         [](const at::Tensor& q, const at::Tensor& k, double scale, at::Tensor& err) { return q38::qsa_block_stats_tc(q, k, scale, err); });
   m.def("qsa_indexer_fwd(Tensor qi, Tensor ki, Tensor wi, float scale) -> Tensor");
   m.def("gemm_pair(Tensor a, Tensor b, Tensor(a!) c, float alpha, bool accumulate, Tensor(b!) err) -> bool",
-        [](const at::Tensor& a, const at::Tensor& b, at::Tensor& c, double alpha, bool acc, at::Tensor& err) { return q38::gemm_bf16_pair(a, b, c, alpha, acc, err); });
+        [](const at::Tensor& a, const at::Tensor& b, at::Tensor& c, double alpha, bool acc, at::Tensor& err) { 
+          TORCH_CHECK(a.dim() == 3 && b.dim() == 3 && c.dim() == 3, "gemm_pair: [batch, rows, cols] tensors required");
+          return q38::gemm_bf16_pair(a, b, c, alpha, acc, err.data_ptr<int>());
+        });
   m.def("qsa_first_query_lp(Tensor q_first, Tensor ki, Tensor w_first, float scale) -> Tensor", &q38::qsa_first_query_lp);
   m.def("qsa_kl_combine(Tensor? stats, Tensor blse, int nq) -> Tensor[]");
   m.def("qsa_select(Tensor lp_blk, int budget) -> Tensor[]");

@@ -247,9 +247,9 @@ bool gemm_pair_enabled() {
 
 // C = alpha * A B^T (+ C) for K-major bf16 A [batch, M, K] and B [batch, N, K]; C bf16 or fp32, storable by TMA.  Returns false when
 // the shape is not taken (the caller then runs the one-CTA kernel).
-bool gemm_bf16_pair(const at::Tensor& a, const at::Tensor& b, at::Tensor& c, double alpha, bool accumulate, at::Tensor& err) {
-  const int batch = a.size(0), M = a.size(1), K = a.size(2), N = b.size(1);
-  const bool out_fp32 = c.scalar_type() == at::kFloat;
+bool gemm_bf16_pair(const Mat& a, const Mat& b, const Mat& c, double alpha, bool accumulate, int* err) {
+  const int batch = a.batch, M = a.rows, K = a.cols, N = b.rows;
+  const bool out_fp32 = c.type == at::kFloat;
   const int c_eb = out_fp32 ? 4 : 2;
   if (M < 2 * G2_BM || N < 64 || K % 8 != 0) return false;
   // N tile: a multiple of 32 (store boxes) whose half is a multiple of 8 rows; as in the one-CTA kernel, the most useful columns per tile time
@@ -268,14 +268,14 @@ bool gemm_bf16_pair(const at::Tensor& a, const at::Tensor& b, at::Tensor& c, dou
   p.tiles_m = (M + 2 * G2_BM - 1) / (2 * G2_BM); p.tiles_n = (N + bn - 1) / bn;
   p.total_kb = (K + G2_BK - 1) / G2_BK;
   p.work_items = p.tiles_m * p.tiles_n * batch;
-  p.alpha = (float)alpha; p.err = err.data_ptr<int>();
+  p.alpha = (float)alpha; p.err = err;
   const int stage_bytes = G2_BM * 128 + bn / 2 * 128, fixed = 1024 + 1024 + 8 * 2 * 4096;
   p.stages = std::min(G2_MAX_STAGES, (227 * 1024 - fixed) / stage_bytes);
   if (p.stages < 3) return false;
   const int smem = p.stages * stage_bytes + fixed;
-  CUtensorMap ta = make_tmap_box(a.data_ptr(), 2, K, M, batch, a.stride(1), a.stride(0), G2_BM, 128);
-  CUtensorMap tb = make_tmap_box(b.data_ptr(), 2, K, N, batch, b.stride(1), b.stride(0), bn / 2, 128);
-  CUtensorMap tc = make_tmap_box(c.data_ptr(), c_eb, N, M, batch, c.stride(1), c.stride(0), 32, 32 * c_eb);
+  CUtensorMap ta = make_tmap_box(a.ptr, 2, K, M, batch, a.row_stride, a.batch_stride, G2_BM, 128);
+  CUtensorMap tb = make_tmap_box(b.ptr, 2, K, N, batch, b.row_stride, b.batch_stride, bn / 2, 128);
+  CUtensorMap tc = make_tmap_box(c.ptr, c_eb, N, M, batch, c.row_stride, c.batch_stride, 32, 32 * c_eb);
   const int clusters = std::max(1, std::min(p.work_items, kNumSMs / 2));
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(2 * clusters); cfg.blockDim = dim3(G2_THREADS); cfg.dynamicSmemBytes = smem; cfg.stream = at::cuda::getCurrentCUDAStream();

@@ -337,37 +337,37 @@ static void launch_p(const CUtensorMap& ta, const CUtensorMap& tb, const CUtenso
 }
 
 bool gemm_pair_enabled();                                                                                                         // gemm_pair.cu
-bool gemm_bf16_pair(const at::Tensor& a, const at::Tensor& b, at::Tensor& c, double alpha, bool accumulate, at::Tensor& err);   // gemm_pair.cu
+bool gemm_bf16_pair(const Mat& a, const Mat& b, const Mat& c, double alpha, bool accumulate, int* err);   // gemm_pair.cu
 
 // Same contract as gemm_bf16 (bf16 operands only).
-void gemm_bf16_persistent(const at::Tensor& a, const at::Tensor& b, at::Tensor& c, bool a_mn_major, bool b_mn_major, double alpha,
-                          bool accumulate, at::Tensor& err, int64_t splits, const c10::optional<at::Tensor>& addend, double beta) {
-  const bool tf32 = a.scalar_type() == at::kFloat;
-  TORCH_CHECK(a.is_cuda() && (tf32 || a.scalar_type() == at::kBFloat16) && b.scalar_type() == a.scalar_type() && a.dim() == 3 && b.dim() == 3 && c.dim() == 3,
-              "gemm_bf16_persistent: bf16 (or fp32 for tf32 math) [batch, rows, cols] operands required");
+void gemm_bf16_persistent(const at::Tensor& a_, const at::Tensor& b_, const at::Tensor& c_, bool a_mn_major, bool b_mn_major, double alpha,
+                          bool accumulate, const at::Tensor& err, int64_t splits, const c10::optional<at::Tensor>& addend, double beta) {
+  const Mat a(a_), b(b_), c(c_);
+  const bool tf32 = a.type == at::kFloat;
+  TORCH_CHECK((tf32 || a.type == at::kBFloat16) && b.type == a.type, "gemm_bf16_persistent: bf16 (or fp32 for tf32 math) [batch, rows, cols] operands required");
   TORCH_CHECK(!tf32 || (!a_mn_major && !b_mn_major), "gemm_bf16_persistent: the tf32 path takes K-major operands only");
   const int eb = tf32 ? 4 : 2, bk = 128 / eb;
-  TORCH_CHECK(a.stride(2) == 1 && b.stride(2) == 1 && c.stride(2) == 1, "gemm_bf16_persistent: innermost dimension must be contiguous");
-  const c10::cuda::CUDAGuard guard(a.device());
-  const int batch = a.size(0);
-  const int M = a_mn_major ? a.size(2) : a.size(1), K = a_mn_major ? a.size(1) : a.size(2);
-  const int N = b_mn_major ? b.size(2) : b.size(1), Kb = b_mn_major ? b.size(1) : b.size(2);
-  TORCH_CHECK(K == Kb && b.size(0) == batch && c.size(0) == batch && c.size(1) == M && c.size(2) == N, "gemm_bf16_persistent: shape mismatch");
-  const bool out_fp32 = c.scalar_type() == at::kFloat;
-  TORCH_CHECK(out_fp32 || c.scalar_type() == at::kBFloat16, "gemm_bf16_persistent: output must be bf16 or fp32");
+  TORCH_CHECK(a.col_stride == 1 && b.col_stride == 1 && c.col_stride == 1, "gemm_bf16_persistent: innermost dimension must be contiguous");
+  const c10::cuda::CUDAGuard guard(a_.device());
+  const int batch = a.batch;
+  const int M = a_mn_major ? a.cols : a.rows, K = a_mn_major ? a.rows : a.cols;
+  const int N = b_mn_major ? b.cols : b.rows, Kb = b_mn_major ? b.rows : b.cols;
+  TORCH_CHECK(K == Kb && b.batch == batch && c.batch == batch && c.rows == M && c.cols == N, "gemm_bf16_persistent: shape mismatch");
+  const bool out_fp32 = c.type == at::kFloat;
+  TORCH_CHECK(out_fp32 || c.type == at::kBFloat16, "gemm_bf16_persistent: output must be bf16 or fp32");
   const int c_eb = out_fp32 ? 4 : 2, c_vec = 16 / c_eb;
-  const bool tma_out = c.stride(1) % c_vec == 0 && (reinterpret_cast<uintptr_t>(c.data_ptr()) & 15) == 0 && (batch == 1 || c.stride(0) % c_vec == 0);
+  const bool tma_out = c.row_stride % c_vec == 0 && (reinterpret_cast<uintptr_t>(c.ptr) & 15) == 0 && (batch == 1 || c.batch_stride % c_vec == 0);
   // bf16 outputs accumulate through the TMA unit only (cp.reduce.async.bulk.tensor adds in the tensor's element type)
   TORCH_CHECK(!accumulate || out_fp32 || (tma_out && !tf32 && !addend.has_value()), "accumulating into a bf16 output requires a TMA-storable output and no addend");
   // K-major x K-major products with a TMA-storable output may run on SM pairs (cta_group::2, gemm_pair.cu) when switched on
   if (gemm_pair_enabled() && !tf32 && !a_mn_major && !b_mn_major && tma_out && !addend.has_value() && (!accumulate || !out_fp32) &&
-      gemm_bf16_pair(a, b, c, alpha, accumulate, err))
+      gemm_bf16_pair(a, b, c, alpha, accumulate, err.data_ptr<int>()))
     return;
   int bn = pick_bn(N, tma_out ? 32 : 16);
   if (b_mn_major) bn = (bn + 63) / 64 * 64;                    // MN-major B is loaded in 64-wide boxes
   bn = std::min(bn, 256);
-  Q38_TRACE("[gemm_p] M=%d N=%d K=%d batch=%d a=%p b=%p c=%p strides a(%lld,%lld) b(%lld,%lld) c(%lld,%lld)\n", M, N, K, batch, a.data_ptr(), b.data_ptr(), c.data_ptr(),
-            (long long)a.stride(0), (long long)a.stride(1), (long long)b.stride(0), (long long)b.stride(1), (long long)c.stride(0), (long long)c.stride(1));
+  Q38_TRACE("[gemm_p] M=%d N=%d K=%d batch=%d a=%p b=%p c=%p strides a(%lld,%lld) b(%lld,%lld) c(%lld,%lld)\n", M, N, K, batch, a.ptr, b.ptr, c.ptr,
+            (long long)a.batch_stride, (long long)a.row_stride, (long long)b.batch_stride, (long long)b.row_stride, (long long)c.batch_stride, (long long)c.row_stride);
   PGemmArgs p{};
   p.M = M; p.N = N; p.K = K; p.batch = batch; p.bn = bn;
   p.tiles_m = (M + P_BM - 1) / P_BM; p.tiles_n = (N + bn - 1) / bn;
@@ -383,7 +383,7 @@ void gemm_bf16_persistent(const at::Tensor& a, const at::Tensor& b, at::Tensor& 
   p.kb_per_split = (p.total_kb + nsplit - 1) / nsplit;
   p.splits = (p.total_kb + p.kb_per_split - 1) / p.kb_per_split;
   p.work_items = p.tiles_m * p.tiles_n * batch * p.splits;
-  p.C = c.data_ptr(); p.ldc = c.stride(1); p.c_batch_stride = c.stride(0); p.alpha = (float)alpha; p.err = err.data_ptr<int>();
+  p.C = c.ptr; p.ldc = c.row_stride; p.c_batch_stride = c.batch_stride; p.alpha = (float)alpha; p.err = err.data_ptr<int>();
   p.Cin = nullptr; p.ldcin = 0; p.cin_batch_stride = 0; p.beta = 0.f;
   if (addend.has_value()) {
     TORCH_CHECK(!out_fp32 && addend->scalar_type() == at::kBFloat16 && addend->dim() == 3 && addend->size(0) == batch && addend->size(1) == M &&
@@ -392,11 +392,11 @@ void gemm_bf16_persistent(const at::Tensor& a, const at::Tensor& b, at::Tensor& 
   }
   CUtensorMap ta, tb;
   Q38_TRACE("[gemm_p] args bn=%d tiles=%dx%d splits=%d items=%d\n", bn, p.tiles_m, p.tiles_n, p.splits, p.work_items);
-  ta = make_tmap_box(a.data_ptr(), eb, a.size(2), a.size(1), batch, a.stride(1), a.stride(0), a_mn_major ? 64 : P_BM, 128);
+  ta = make_tmap_box(a.ptr, eb, a.cols, a.rows, batch, a.row_stride, a.batch_stride, a_mn_major ? 64 : P_BM, 128);
   Q38_TRACE("[gemm_p] map A encoded\n");
-  tb = make_tmap_box(b.data_ptr(), eb, b.size(2), b.size(1), batch, b.stride(1), b.stride(0), b_mn_major ? 64 : bn, 128);
+  tb = make_tmap_box(b.ptr, eb, b.cols, b.rows, batch, b.row_stride, b.batch_stride, b_mn_major ? 64 : bn, 128);
   Q38_TRACE("[gemm_p] operand maps encoded\n");
-  CUtensorMap tc = tma_out ? make_tmap_box(c.data_ptr(), c_eb, N, M, batch, c.stride(1), c.stride(0), 32, 32 * c_eb) : ta;
+  CUtensorMap tc = tma_out ? make_tmap_box(c.ptr, c_eb, N, M, batch, c.row_stride, c.batch_stride, 32, 32 * c_eb) : ta;
   cudaStream_t stream = at::cuda::getCurrentCUDAStream();
   if (tf32) {
     launch_p<false, false, true>(ta, tb, tc, tma_out, p, out_fp32, accumulate, stream);

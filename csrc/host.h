@@ -16,12 +16,25 @@ CUtensorMap make_tmap_bf16(const void* base, int64_t inner, int64_t rows, int64_
 CUtensorMap make_tmap_box(const void* base, int elem_bytes, int64_t inner, int64_t rows, int64_t batch, int64_t row_stride_elems,
                           int64_t batch_stride_elems, int box_rows, int box_inner_bytes);
 
+// A GEMM operand or output: [batch, rows, cols] with contiguous columns.  Made from a 3-D tensor or, without the cost of a view, from a 2-D one.
+struct Mat {
+  void* ptr;
+  at::ScalarType type;
+  int64_t batch, rows, cols, batch_stride, row_stride, col_stride;
+  Mat(const at::Tensor& t) : ptr(t.data_ptr()), type(t.scalar_type()) {
+    TORCH_CHECK(t.is_cuda() && (t.dim() == 2 || t.dim() == 3), "GEMM operands: CUDA tensors of two or three dimensions required");
+    const int d = t.dim() - 2;
+    batch = d ? t.size(0) : 1; batch_stride = d ? t.stride(0) : 0;
+    rows = t.size(d); cols = t.size(d + 1); row_stride = t.stride(d); col_stride = t.stride(d + 1);
+  }
+};
+
 // gemm.cu
 void gemm_bf16(const at::Tensor& a, const at::Tensor& b, at::Tensor& c, bool a_mn_major, bool b_mn_major, double alpha,
                bool accumulate, at::Tensor& err, int64_t splits);
 
-void gemm_bf16_persistent(const at::Tensor& a, const at::Tensor& b, at::Tensor& c, bool a_mn_major, bool b_mn_major, double alpha,
-                          bool accumulate, at::Tensor& err, int64_t splits, const c10::optional<at::Tensor>& addend = c10::nullopt, double beta = 0.0);
+void gemm_bf16_persistent(const at::Tensor& a, const at::Tensor& b, const at::Tensor& c, bool a_mn_major, bool b_mn_major, double alpha,
+                          bool accumulate, const at::Tensor& err, int64_t splits, const c10::optional<at::Tensor>& addend = c10::nullopt, double beta = 0.0);
 
 // mxfp8.cu
 int64_t mxfp8_pick_bn(int64_t N);

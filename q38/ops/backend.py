@@ -9,7 +9,7 @@ import os
 
 import torch
 
-from . import error_flag, gemm, load
+from . import PERSISTENT_GEMM, error_flag, gemm, load
 
 
 def _bf16_weight(weight):
@@ -160,6 +160,15 @@ class _SideStream:
         self.pending = True
         return out
 
+    def handle(self):
+        """The stream as the native layer passes take it (empty: run inline); work issued on it is joined like that of `run`."""
+        if not self.enabled:
+            return ()
+        if self.stream is None:
+            self.stream = torch.cuda.Stream()
+        self.pending = True
+        return self.stream.stream_id, self.stream.device_index, self.stream.device_type
+
     def join(self):
         if self.pending:
             torch.cuda.current_stream().wait_stream(self.stream)
@@ -309,6 +318,29 @@ class _MhcPreNorm(torch.autograd.Function):
         take = DEFERRED_GRADS.take
         return (dX.view(B_, S, n, h), dA, take(B_w, dBw), take(b_pre, dbias[0:4]), take(b_post, dbias[4:8]), take(b_res, dbias[8:24]),
                 take(alphas, dbias[24:27]), take(norm_w, dnw), None, None, None, None)
+
+
+class _MhcPreNormLayer(torch.autograd.Function):
+    """`_MhcPreNorm` with the launches of a pass made in one native call (csrc/layers.cpp)."""
+
+    @staticmethod
+    def forward(ctx, X, A_w, B_w, b_pre, b_post, b_res, alphas, norm_w, iters, eps, out_bf16, link, deterministic):
+        xout, coef, X2, *saved = load().mhc_layer_fwd(X, A_w, B_w, b_pre, b_post, b_res, alphas, norm_w, iters, eps, out_bf16, error_flag(X.device))
+        ctx.save_for_backward(A_w, B_w, b_pre, b_post, b_res, alphas, norm_w, coef, X2, *saved)
+        ctx.iters, ctx.link, ctx.shape, ctx.deterministic = iters, link, X.shape, deterministic
+        return xout.view(*X.shape[:2], X.shape[3]), coef
+
+    @staticmethod
+    def backward(ctx, dxout, dcoef):
+        tensors = ctx.saved_tensors                                  # unpacked once: checkpointing recomputes on the first access only
+        params, saved = tensors[:7], tensors[7:]
+        grads, grad_of = _grad_buffers(params[:1], ctx.needs_input_grad[1:2])
+        dXo, ctx.link.dXo = ctx.link.dXo, None
+        dX, dBw, dbias, dnw, dA = load().mhc_layer_bwd(dxout, dcoef, dXo, saved, *params, ctx.iters, error_flag(dxout.device), grads, grad_of, WGRAD_STREAM.handle(),
+                                                       ctx.deterministic)
+        take, (A_w, B_w, b_pre, b_post, b_res, alphas, norm_w) = DEFERRED_GRADS.take, params
+        return (dX.view(ctx.shape), None if dA is None else dA.to(A_w.dtype), take(B_w, dBw), take(b_pre, dbias[0:4]), take(b_post, dbias[4:8]),
+                take(b_res, dbias[8:24]), take(alphas, dbias[24:27]), take(norm_w, dnw), None, None, None, None, None)
 
 
 class _MhcPost(torch.autograd.Function):
@@ -651,6 +683,97 @@ class _Experts(torch.autograd.Function):
         return dx, d_top_w, None, d_gate_up, d_down
 
 
+# ---- whole layers, one native call per pass (csrc/layers.cpp) ----------------------------------------------------------------------
+# The same launches as the op-by-op path below them in each hook, which stays for what a layer call does not cover (debug switches, expert
+# parallelism, MXFP8, shapes that leave the tensor-core GEMM).  The Python cost of an op is 10 to 30 us, several times that of its launch, and a layer has
+# 10 to 45 of them: 256 tokens of q38_c1 were bound by the host in every layer and direction.
+def _grad_buffers(weights, needed):
+    """(gradient buffers, position of each weight's buffer): -1 where a weight has none, -2 where its gradient is not wanted."""
+    grads, grad_of = [], []
+    for w, need in zip(weights, needed):
+        grad = w.grad if need else None
+        grad_of.append(-2 if not need else -1 if grad is None else len(grads))
+        if grad is not None:
+            grads.append(grad)
+    return grads, grad_of
+
+
+def _fresh(delta, weight):
+    return None if delta is None else delta.view(weight.shape).to(weight.dtype)
+
+
+def _will_save(x, *params):
+    return torch.is_grad_enabled() and (x.requires_grad or any(p.requires_grad for p in params))
+
+
+class _GdnLayer(torch.autograd.Function):
+    @staticmethod
+    def forward(ctx, x, w_qkv, w_z, w_b, w_a, w_out, conv_w, A_log, dt_bias, norm_w, Hk, Hv, eps, deterministic, save):
+        params = (w_qkv, w_z, w_b, w_a, w_out, conv_w, A_log, dt_bias, norm_w)
+        y, *saved = load().gdn_layer_fwd(x, [_bf16_weight(w) for w in params[:5]], *params[5:], Hk, Hv, eps, error_flag(x.device), save)
+        ctx.save_for_backward(*params, *saved)
+        ctx.args, ctx.shape, ctx.deterministic = (Hk, Hv, eps), x.shape, deterministic
+        return y
+
+    @staticmethod
+    def backward(ctx, dy):
+        tensors = ctx.saved_tensors
+        params, saved = tensors[:9], tensors[9:]
+        need = ctx.needs_input_grad
+        out = load().gdn_layer_bwd(dy, saved, [_bf16_weight(w) for w in params[:5]], *params[5:], *ctx.args, error_flag(dy.device), need[0],
+                                   *_grad_buffers(params[:5], need[1:6]), WGRAD_STREAM.handle(), ctx.deterministic)
+        small = [DEFERRED_GRADS.take(p, d) for p, d in zip(params[5:], out[1:5])]
+        return (out[0].view(ctx.shape) if need[0] else None, *map(_fresh, out[5:], params[:5]), *small, None, None, None, None, None)
+
+
+class _QsaLayer(torch.autograd.Function):
+    @staticmethod
+    def forward(ctx, x, w_q, w_k, w_v, w_o, wq, wk, ww, q_norm, k_norm, cos, sin, q_eps, k_eps, scale, budget, dense, want_kl, main_tc, deterministic, save):
+        ctx.set_materialize_grads(False)
+        indexer = () if wq is None else (wq, wk, ww)
+        params = (w_q, w_k, w_v, w_o, *indexer)
+        y, kl, *saved = load().qsa_layer_fwd(x, [_bf16_weight(w) for w in params[:4]], [_bf16_weight(w) for w in indexer], q_norm, k_norm, cos, sin, q_eps, k_eps, scale,
+                                             budget, dense, want_kl, main_tc, error_flag(x.device), save)
+        ctx.save_for_backward(*params, q_norm, k_norm, *saved)
+        ctx.n, ctx.scale, ctx.shape, ctx.deterministic = len(params), scale, x.shape, deterministic
+        need = ctx.needs_input_grad                                  # the two outputs depend on disjoint parameters
+        ctx.mark_non_differentiable(*(out for out, parts in ((y, need[:5] + need[8:10]), (kl, need[5:8])) if out is not None and not any(parts)))
+        return y, kl
+
+    @staticmethod
+    def backward(ctx, dy, dkl):
+        n, need = ctx.n, ctx.needs_input_grad
+        tensors = ctx.saved_tensors
+        params, (q_norm, k_norm), saved = tensors[:n], tensors[n:n + 2], tensors[n + 2:]
+        grads, grad_of = _grad_buffers(params, need[1:1 + n])
+        out = load().qsa_layer_bwd(dy, dkl, saved, [_bf16_weight(w) for w in params[:4]], q_norm, k_norm, ctx.scale, error_flag(saved[0].device), need[0] and dy is not None,
+                                   grads, grad_of, WGRAD_STREAM.handle(), ctx.deterministic)
+        norms = [None if d is None else DEFERRED_GRADS.take(p, d) for p, d in zip((q_norm, k_norm), out[1:3])]
+        dw = list(map(_fresh, out[3:], params))
+        return (None if out[0] is None else out[0].view(ctx.shape), *dw, *[None] * (7 - n), *norms, *[None] * 11)
+
+
+class _MoeLayer(torch.autograd.Function):
+    @staticmethod
+    def forward(ctx, x, w_router, w_sg, w_su, w_sl, w_sd, w_gate_up, w_down, topk, deterministic, save):
+        ctx.set_materialize_grads(False)
+        params = (w_router, w_sg, w_su, w_sl, w_sd, w_gate_up, w_down)
+        y, prob_sum, counts, *saved = load().moe_layer_fwd(x, [_bf16_weight(w) for w in params], topk, error_flag(x.device), save)
+        ctx.save_for_backward(*params, *saved)
+        ctx.deterministic = deterministic
+        ctx.mark_non_differentiable(*((counts,) if any(ctx.needs_input_grad[:2]) else (counts, prob_sum)))
+        return y, prob_sum, counts
+
+    @staticmethod
+    def backward(ctx, dy, d_prob_sum, _counts):
+        tensors = ctx.saved_tensors
+        params, saved = tensors[:7], tensors[7:]
+        need = ctx.needs_input_grad
+        out = load().moe_layer_bwd(dy, d_prob_sum, saved, [_bf16_weight(w) for w in params], error_flag(saved[0].device), need[0], *_grad_buffers(params, need[1:8]),
+                                   WGRAD_STREAM.handle(), ctx.deterministic)
+        return (out[0], *map(_fresh, out[1:], params), None, None, None)
+
+
 def _nvtx(name):
     """With Q38_NVTX=1 every call of the decorated hook is an NVTX range (visible in Nsight timelines); otherwise a no-op."""
     def wrap(fn):
@@ -738,6 +861,11 @@ class Backend:
                 print(f"[q38.ops] WARNING: tensor-core GEMM layout '{name}' failed its self-check "
                       f"(rel err {err:.3e}, kernel error {bad}); using the library matmul for it", flush=True)
 
+    def native_layers(self, hidden):
+        """Whether every product of a layer of this width runs on the persistent tensor-core GEMM in the default grouping."""
+        return (PERSISTENT_GEMM and hidden % 8 == 0 and self.layouts["nt"] and self.layouts["nn"] and self.layouts["tn"]
+                and os.environ.get("Q38_MULTI_LINEAR", "2") == "2")
+
     # ---- hooks called by the model -----------------------------------------------------------------------------
     def linear(self, x, weight):
         return _Linear.apply(x, weight, self)
@@ -763,6 +891,12 @@ class Backend:
     @_nvtx("q38.mhc_pre_norm")
     def mhc_pre_norm(self, mhc, norm, X, dtype):
         link = _MhcLink()
+        rank, h = mhc.A.weight.shape[0], X.shape[-1]
+        if (self.native_layers(h) and rank % 8 == 0 and X.dtype == torch.float32 and X.is_contiguous() and X.data_ptr() % 16 == 0 and mhc.A.weight.data_ptr() % 16 == 0
+                and X.numel() and dtype in (torch.bfloat16, torch.float32) and not os.environ.get("Q38_MHC_FP32_GEMM")):
+            x, coef = _MhcPreNormLayer.apply(X, mhc.A.weight, mhc.B.weight, mhc.b_pre, mhc.b_post, mhc.b_res, mhc.alphas, norm.weight,
+                                             mhc.iters, norm.eps, dtype == torch.bfloat16, link, self.deterministic)
+            return x, (X, coef, link)
         x, coef = _MhcPreNorm.apply(X, mhc.A.weight, mhc.B.weight, mhc.b_pre, mhc.b_post, mhc.b_res, mhc.alphas, norm.weight,
                                     mhc.iters, norm.eps, dtype, link)
         return x, (X, coef, link)
@@ -790,6 +924,9 @@ class Backend:
         if x.dtype != torch.bfloat16 or S % 64 or m.head_k_dim != 64 or m.head_v_dim != 64:
             return None
         from ..models import modeling
+        if self.native_layers(x.shape[-1]) and not self.hybrid_delta_rule and x.numel():
+            params = (m.in_proj_qkv.weight, m.in_proj_z.weight, m.in_proj_b.weight, m.in_proj_a.weight, m.out_proj.weight, m.conv1d.weight, m.A_log, m.dt_bias, m.norm.weight)
+            return _GdnLayer.apply(x, *params, m.num_k_heads, m.num_v_heads, float(m.norm.variance_epsilon), self.deterministic, _will_save(x, *params))
         F = torch.nn.functional
         p_qkv, z, p_b, p_a = self.linears(x, m.in_proj_qkv.weight, m.in_proj_z.weight, m.in_proj_b.weight, m.in_proj_a.weight)
         qkv = _ConvSilu.apply(p_qkv, m.conv1d.weight)
@@ -828,6 +965,13 @@ class Backend:
         hd = attn.head_dim
         if x.dtype != torch.bfloat16 or hd != 64 or S % 64 or S > 8192 or (indexer is not None and (indexer.d_ih != 64 or indexer.n_ih > 4)):
             return None
+        want_kl = want_kl and indexer is not None
+        if (self.native_layers(x.shape[-1]) and cos.shape[-1] == 16 and x.numel() and self.selection_override is None and not os.environ.get("Q38_INDEXER_BASELINE")
+                and not (want_kl and modeling.QSA_STAT.get("on"))):
+            index_w = (None, None, None) if indexer is None else (indexer.wq.weight, indexer.wk.weight, indexer.ww.weight)
+            params = (attn.q_proj.weight, attn.k_proj.weight, attn.v_proj.weight, attn.o_proj.weight, *index_w, attn.q_norm.weight, attn.k_norm.weight)
+            return _QsaLayer.apply(x, *params, cos, sin, float(attn.q_norm.eps), float(attn.k_norm.eps), float(attn.scaling), budget, dense or indexer is None, want_kl,
+                                   os.environ.get("Q38_QSA_TC", "1") != "0", self.deterministic, _will_save(x, *(p for p in params if p is not None)))
         p_q, p_k, p_v = self.linears(x, attn.q_proj.weight, attn.k_proj.weight, attn.v_proj.weight)
         qg = p_q.view(B, S, -1, 2 * hd)
         if cos.shape[-1] == 16:
@@ -916,6 +1060,14 @@ class Backend:
         shape = x.shape
         x2 = x.reshape(-1, h)
         shared = block.shared_expert
+        if (self.native_layers(h) and self.ep is None and not self.fp8_ffn and x2.shape[0] and shared.gate_proj.weight.shape[0] % 8 == 0
+                and block.shared_expert_gate.weight.shape[0] == 1):
+            params = (block.gate.weight, shared.gate_proj.weight, shared.up_proj.weight, block.shared_expert_gate.weight, shared.down_proj.weight,
+                      experts.gate_up_proj, experts.down_proj)
+            y, prob_sum, counts = _MoeLayer.apply(x2, *params, block.gate.top_k, self.deterministic, _will_save(x2, *params))
+            if block._recording():
+                block.stats_sink.add(counts, prob_sum, x2.shape[0])
+            return y.reshape(shape)
         logits, sg, su, gate_logit = self.linears(x2, block.gate.weight, shared.gate_proj.weight, shared.up_proj.weight, block.shared_expert_gate.weight)
         top_w, top_idx, prob_sum, counts = _Route.apply(logits, block.gate.top_k)
         if block._recording():
@@ -963,6 +1115,11 @@ class _LinearCE(torch.autograd.Function):
         ops = load()
         h2 = hidden.reshape(-1, hidden.shape[-1]).to(torch.bfloat16).contiguous()
         w = _bf16_weight(weight)
+        ctx.backend, ctx.shape, ctx.dtype, ctx.native = backend, hidden.shape, hidden.dtype, backend.native_layers(h2.shape[1])
+        if ctx.native:
+            total, dlogits = ops.linear_ce_fwd(h2, w, target, rows, error_flag(h2.device))
+            ctx.save_for_backward(h2, weight, dlogits)
+            return total
         total = torch.zeros((), dtype=torch.float32, device=hidden.device)
         # the gradients of all chunks in one buffer: the backward is then two GEMMs over all rows, whose tiles fill the SMs' last wave better
         # than a pair per chunk (d(hidden) of 16384 x 10112 x 576: 384 tiles in three waves of 148, against 192 in two, twice)
@@ -975,7 +1132,6 @@ class _LinearCE(torch.autograd.Function):
                 logits.copy_(backend.mm_nt(h2[o:o + rows], w))
             total = total + ops.ce_inplace(logits, target[o:o + rows].contiguous()).sum()
         ctx.save_for_backward(h2, weight, dlogits)
-        ctx.backend, ctx.shape, ctx.dtype = backend, hidden.shape, hidden.dtype
         return total
 
     @staticmethod
@@ -984,6 +1140,10 @@ class _LinearCE(torch.autograd.Function):
         backend, w, gs = ctx.backend, _bf16_weight(weight), g.to(torch.bfloat16)
         if not h2.shape[0]:
             return torch.empty_like(h2).view(ctx.shape).to(ctx.dtype), None, None, None, None
+        if ctx.native:
+            dh, dw = load().linear_ce_bwd(g, h2, w, dlogits, error_flag(h2.device), *_grad_buffers((weight,), ctx.needs_input_grad[1:2]), WGRAD_STREAM.handle(),
+                                          backend.deterministic)
+            return dh.view(ctx.shape).to(ctx.dtype), _fresh(dw, weight), None, None, None
         dh = scale_bf16(backend.mm_nn(dlogits, w), gs)
         dw = backend.weight_grad(dlogits, scale_bf16(h2, gs), weight) if ctx.needs_input_grad[1] else None
         return dh.view(ctx.shape).to(ctx.dtype), dw, None, None, None
