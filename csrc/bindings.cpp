@@ -89,7 +89,7 @@ TORCH_LIBRARY(q38, m) {
   m.def("qsa_kl_combine(Tensor? stats, Tensor blse, int nq) -> Tensor[]");
   m.def("qsa_select(Tensor lp_blk, int budget) -> Tensor[]");
   m.def("qsa_indexer_bwd(Tensor qi, Tensor ki, Tensor wi, Tensor blse, Tensor dblse, float gscale, float scale, Tensor(a!)? err=None) -> Tensor[]");
-  m.def("qsa_attn_fwd(Tensor q, Tensor k, Tensor v, Tensor? count, Tensor? index, float scale) -> Tensor[]");
+  m.def("qsa_attn_fwd(Tensor q, Tensor k, Tensor v, Tensor? count, Tensor? index, float scale, Tensor(a!)? err=None) -> Tensor[]");
   m.def("qsa_attn_bwd(Tensor q, Tensor k, Tensor v, Tensor o, Tensor dout, Tensor lse, Tensor sel, float scale, Tensor(a!)? err=None) -> Tensor[]");
   m.def("ep_publish_counts(Tensor offsets, int rank, int[] peer_counts) -> ()",
         [](const at::Tensor& o, int64_t rank, std::vector<int64_t> peers) { q38::ep_publish_counts(o, rank, peers); });
@@ -176,8 +176,8 @@ TORCH_LIBRARY_IMPL(q38, CUDA, m) {
   m.impl("qsa_kl_combine", [](c10::optional<at::Tensor> stats, const at::Tensor& blse, int64_t nq) { return q38::qsa_kl_combine(stats, blse, nq); });
   m.impl("qsa_select", &q38::qsa_select);
   m.impl("qsa_indexer_bwd", &q38::qsa_indexer_bwd);
-  m.impl("qsa_attn_fwd", [](const at::Tensor& q, const at::Tensor& k, const at::Tensor& v, c10::optional<at::Tensor> c, c10::optional<at::Tensor> i, double s) {
-    return q38::qsa_attn_fwd(q, k, v, c, i, s);
+  m.impl("qsa_attn_fwd", [](const at::Tensor& q, const at::Tensor& k, const at::Tensor& v, c10::optional<at::Tensor> c, c10::optional<at::Tensor> i, double s, c10::optional<at::Tensor> err) {
+    return q38::qsa_attn_fwd(q, k, v, c, i, s, err);
   });
   m.impl("qsa_attn_bwd", &q38::qsa_attn_bwd);
   m.impl("conv_silu_fwd", &q38::conv_silu_fwd);

@@ -148,7 +148,7 @@ std::vector<at::Tensor> qsa_indexer_bwd(const at::Tensor& qi, const at::Tensor& 
 at::Tensor qsa_block_stats_tc(const at::Tensor& q, const at::Tensor& k, double scale, at::Tensor& err);
 // qsa_attn.cu, qsa_attn_bwd.cu
 std::vector<at::Tensor> qsa_attn_fwd(const at::Tensor& q, const at::Tensor& k, const at::Tensor& v, const c10::optional<at::Tensor>& count,
-                                     const c10::optional<at::Tensor>& index, double scale);
+                                     const c10::optional<at::Tensor>& index, double scale, const c10::optional<at::Tensor>& err);
 std::vector<at::Tensor> qsa_attn_bwd(const at::Tensor& q, const at::Tensor& k, const at::Tensor& v, const at::Tensor& o, const at::Tensor& dout,
                                      const at::Tensor& lse, const at::Tensor& sel, double scale, const c10::optional<at::Tensor>& err);
 // ep.cu

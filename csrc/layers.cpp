@@ -205,7 +205,7 @@ Tensors qsa_layer_fwd(const Tensor& x, at::TensorList w, at::TensorList wi, cons
     count = sel[0];
     index = sel[1];
   }
-  auto a = qsa_attn_fwd(q, k, v, count, index, scale);
+  auto a = qsa_attn_fwd(q, k, v, count, index, scale, err);
   const Tensor o = a[0].view({B, S, -1});
   const Tensor go = sigmoid_mul_fwd(o, gate).view({B * S, -1});
   const Tensor y = mm_nt(go, w[3], err).view({B, S, -1});

@@ -3,19 +3,20 @@
 // Query block i attends to the key blocks listed in index[b, i, :count[b, i]] (all <= i, own block included); inside the
 // own block the mask is causal.  `dense` ignores the lists and uses every block j <= i (the warm-up phase).
 //
-//   qsa_attn_fwd     grid (nq, nb, B): online-softmax over the selected key blocks; writes o token-major [B,S,nq,64]
-//                    and the row log-sum-exp.
+// Online softmax over the selected key blocks; writes o token-major [B,S,nq,64] and the row log-sum-exp.
 // The backward pass is in qsa_attn_bwd.cu; the [B,nb,nb] selection matrix, built on the device, serves both.
 #include <ATen/ATen.h>
 #include <ATen/cuda/CUDAContext.h>
 #include <c10/cuda/CUDAGuard.h>
 
-#include "common.cuh"
+#include "f32x2.cuh"
 #include "host.h"
-#include "mma_tile.cuh"
+#include "ptx.cuh"
 #include "qsa_blocks.cuh"
 
 namespace q38 {
+
+using bf16 = __nv_bfloat16;
 
 // sel[b, i, j] = 1 iff query block i attends key block j
 __global__ void qsa_selection_matrix_kernel(const int* __restrict__ count, const int* __restrict__ index, int kmax, int nb, int dense,
@@ -33,90 +34,199 @@ __global__ void qsa_selection_matrix_kernel(const int* __restrict__ count, const
   }
 }
 
-// The kernel keeps a CTA's queries as A fragments in registers for its whole loop, passes probabilities between products in registers, and
-// fetches the next block's two tiles while the current one is computed: one barrier per block and no probability tile in shared memory.
-// It is bound by the warp MMA rate and the exponentials between (tensor pipe 46-57 % busy, 35 % with a shared-memory probability tile and
-// unbuffered loads).  16384 tokens of four sequences, 22 query heads, eight blocks per query: 242 -> 183 us.
-__global__ void __launch_bounds__(128, 4) qsa_attn_fwd_kernel(const bf16* __restrict__ q, const bf16* __restrict__ k, const bf16* __restrict__ v,
-                                                              const unsigned char* __restrict__ sel, bf16* __restrict__ o, float* __restrict__ lse,
-                                                              int S, int nq, int nkv, float scale) {
-  extern __shared__ __align__(16) uint8_t smem_bytes[];
-  bf16* KV = reinterpret_cast<bf16*>(smem_bytes);          // two buffers of {K, V}
-  unsigned short* list = reinterpret_cast<unsigned short*>(KV + 4 * TILE_ELEMS);
-  __shared__ int count;
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  // late query blocks (longest lists) first, so that the last CTAs to start are short
-  const int nb = S / 64, i = nb - 1 - blockIdx.y, h = blockIdx.x, b = blockIdx.z, kvh = h / (nq / nkv);
-  const bf16* kbase = k + ((long long)b * nkv + kvh) * S * 64;
-  const bf16* vbase = v + ((long long)b * nkv + kvh) * S * 64;
-  load_tile_async(KV + 2 * TILE_ELEMS, q + (((long long)b * nq + h) * S + (long long)i * 64) * 64, 64, tid);
-  cp_async_commit();
-  const int n = list_blocks(sel + ((long long)b * nb + i) * nb, 1, 0, i + 1, list, &count);
-  auto fetch = [&](int t) {
-    const long long off = (long long)list[t] * 4096;
-    load_tile_async(KV + (t & 1) * 2 * TILE_ELEMS, kbase + off, 64, tid);
-    load_tile_async(KV + ((t & 1) * 2 + 1) * TILE_ELEMS, vbase + off, 64, tid);
-  };
-  if (n > 0) fetch(0);
-  cp_async_commit();
-  cp_async_wait<1>();
-  __syncthreads();
-  uint32_t aq[4][4];
-  load_a(KV + 2 * TILE_ELEMS, aq, warp, lane);
-  const int r0 = 16 * warp + (lane >> 2), cq = 2 * (lane & 3);
-  float m[2] = {-INFINITY, -INFINITY}, l[2] = {0.f, 0.f};
-  float out[8][4];
-  zero_acc(out);
-  for (int t = 0; t < n; ++t) {
-    cp_async_wait<0>();
-    __syncthreads();                                       // this block's tiles are visible; the other buffer's readers are done
-    if (t + 1 < n) fetch(t + 1);
-    cp_async_commit();
-    const bf16* Ks = KV + (t & 1) * 2 * TILE_ELEMS;
-    float s[8][4];
-    zero_acc(s);
-    mma_rows<true, 4, 8>(aq, Ks, s, lane);
-    const bool diag = list[t] == i;
-    float tm[2] = {-INFINITY, -INFINITY}, rs[2] = {0.f, 0.f}, corr[2];
-#pragma unroll
-    for (int nt = 0; nt < 8; ++nt)
-#pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        s[nt][e] = diag && 8 * nt + cq + (e & 1) > r0 + 8 * (e >> 1) ? -INFINITY : s[nt][e] * scale;
-        tm[e >> 1] = fmaxf(tm[e >> 1], s[nt][e]);
+// One CTA per (two heads of a KV group, query block, batch): a tile of 128 rows (64 queries of each head, which attend to the same blocks)
+// against one block of 64 keys.  S = Q K^T and O += P V are tcgen05 products with their results in TMEM; one thread owns a row: maximum,
+// exponentials and sum without a shuffle, P packed over the scores it came from (the A operand of the second product), O rescaled in place when the row's maximum moves.
+// Four CTAs per SM (128 TMEM columns, 48 KB each) cover each other's chains: the products of a tile take 300 of its 1700 cycles, the exponentials 512
+// per SM.  Every operation and its order are those of the warp-MMA kernel that stood here (scores, sums of a row in four interleaved parts, four K = 16
+// steps per product), so the results have its bits.  16384 tokens of four sequences, 22 heads, eight blocks per query: 182 -> 118 us; dense, 8192 tokens
+// of two sequences, 16 heads: 260 -> 143; one of 8192, 28 heads: 122 -> 77.  A grid that leaves SMs idle pays the longer chain of a tile (640 tokens, 5 heads: 9.5 -> 14 us).  Every mbarrier wait is bounded and reports through the error word.
+constexpr int AF_THREADS = 192, AF_STAGES = 2;             // TMA warp, MMA warp, four warps of row threads
+constexpr int HALF_BYTES = 64 * 128, TILE_BYTES = 2 * HALF_BYTES;
+constexpr uint32_t COL_S = 0, COL_O = 64;
+
+struct FwdArgs {
+  const unsigned char* sel;
+  bf16* o;
+  float* lse;
+  int S, nq, nkv;
+  float scale;
+  int* err;
+};
+
+__global__ void __launch_bounds__(AF_THREADS, 4) qsa_attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
+                                                                     const __grid_constant__ CUtensorMap tmV, FwdArgs p) {
+  extern __shared__ __align__(1024) uint8_t smem[];
+  if (ptx::smem_u32(smem) & 1023u) { if (threadIdx.x == 0) report_error(p.err, ERR_BOUNDS); return; }
+  uint8_t *q_tile = smem, *ring = smem + TILE_BYTES;                     // a ring stage is {K, V}
+  uint64_t* bars = reinterpret_cast<uint64_t*>(ring + AF_STAGES * TILE_BYTES);
+  uint64_t *q_full = bars, *kv_full = bars + 1, *kv_empty = kv_full + AF_STAGES, *s_full = kv_empty + AF_STAGES, *p_full = s_full + 1, *o_full = p_full + 1;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(o_full + 1);
+  int* count = reinterpret_cast<int*>(tmem_slot + 1);
+  unsigned short* list = reinterpret_cast<unsigned short*>(bars + 16);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  // late query blocks (longest lists) of all sequences first, so that the last CTAs to start are short
+  const int nb = p.S / 64, i = nb - 1 - blockIdx.y, rep = p.nq / p.nkv, pairs = (rep + 1) / 2, b = blockIdx.x / (p.nkv * pairs);
+  const int kvh = blockIdx.x / pairs % p.nkv, first = 2 * (blockIdx.x % pairs), h0 = kvh * rep + first;
+  const bool both = first + 1 < rep;                                     // an odd head has its tile to itself
+  if (threadIdx.x == 0) {
+    ptx::prefetch_tensormap(&tmQ);
+    ptx::prefetch_tensormap(&tmK);
+    ptx::prefetch_tensormap(&tmV);
+    ptx::mbar_init(q_full, 1);
+    for (int s = 0; s < AF_STAGES; ++s) { ptx::mbar_init(&kv_full[s], 1); ptx::mbar_init(&kv_empty[s], 1); }
+    ptx::mbar_init(s_full, 1);
+    ptx::mbar_init(p_full, 4);
+    ptx::mbar_init(o_full, 1);
+    ptx::fence_barrier_init();
+    ptx::mbar_expect_tx(q_full, TILE_BYTES);                             // while the list is made
+    for (int x = 0; x < 2; ++x) ptx::tma_load_3d(q_tile + x * HALF_BYTES, &tmQ, q_full, 0, (b * p.nq + (x && both ? h0 + 1 : h0)) * p.S + i * 64, 0);
+  }
+  if (warp == 1) { ptx::tmem_alloc(tmem_slot, 128); ptx::tmem_relinquish(); }
+  ptx::tc_fence_before();
+  const int n = list_blocks(p.sel + ((long long)b * nb + i) * nb, 1, 0, i + 1, list, count);        // ends with a barrier
+  ptx::tc_fence_after();
+  const uint32_t tmem = *tmem_slot;
+
+  if (warp == 0) {
+    if (ptx::elect_one()) {
+      const int kv_row0 = (b * p.nkv + kvh) * p.S;
+      int t = 0;
+      for (; t < n; ++t) {
+        const int s = t % AF_STAGES;
+        if (!ptx::mbar_wait(&kv_empty[s], ((t / AF_STAGES) & 1) ^ 1, 1u << 20)) { report_error(p.err, ERR_MMA_WAIT); break; }
+        ptx::mbar_expect_tx(&kv_full[s], TILE_BYTES);
+        ptx::tma_load_3d(ring + s * TILE_BYTES, &tmK, &kv_full[s], 0, kv_row0 + list[t] * 64, 0);
+        ptx::tma_load_3d(ring + s * TILE_BYTES + HALF_BYTES, &tmV, &kv_full[s], 0, kv_row0 + list[t] * 64, 0);
       }
-#pragma unroll
-    for (int x = 0; x < 2; ++x) {
-      tm[x] = fmaxf(tm[x], __shfl_xor_sync(0xffffffffu, tm[x], 1));
-      tm[x] = fmaxf(tm[x], __shfl_xor_sync(0xffffffffu, tm[x], 2));
-      const float mn = fmaxf(m[x], tm[x]);
-      corr[x] = __expf(m[x] - mn);
-      m[x] = mn;
-#pragma unroll
-      for (int nt = 0; nt < 8; ++nt) { out[nt][2 * x] *= corr[x]; out[nt][2 * x + 1] *= corr[x]; }
+      // copies in flight land before this thread, and with it the CTA, ends
+      ptx::mbar_wait(q_full, 0, 1u << 20);
+      for (int u = t > AF_STAGES ? t - AF_STAGES : 0; u < t; ++u) ptx::mbar_wait(&kv_full[u % AF_STAGES], (u / AF_STAGES) & 1, 1u << 20);
     }
+  } else if (warp == 1) {
+    if (ptx::elect_one()) {
+      const uint32_t id_s = ptx::umma_idesc_bf16(128, 64, false, false), id_o = ptx::umma_idesc_bf16(128, 64, false, true), qa = ptx::smem_u32(q_tile);
+      bool ok = ptx::mbar_wait(q_full, 0, 1u << 20);
+      if (!ok) report_error(p.err, ERR_TMA_WAIT);
+      for (int t = 0; t < n && ok; ++t) {
+        const uint32_t kb = ptx::smem_u32(ring + (t % AF_STAGES) * TILE_BYTES), vb = kb + HALF_BYTES;
+        if (!ptx::mbar_wait(&kv_full[t % AF_STAGES], (t / AF_STAGES) & 1, 1u << 20)) { report_error(p.err, ERR_TMA_WAIT); break; }
+        ptx::tc_fence_after();
 #pragma unroll
-    for (int nt = 0; nt < 8; ++nt)
+        for (int k = 0; k < 4; ++k)                                      // over P of the block before, which the product issued last has read
+          ptx::umma_f16(tmem + COL_S, ptx::umma_smem_desc_sw128(qa + k * 32, 0, 1024), ptx::umma_smem_desc_sw128(kb + k * 32, 0, 1024), id_s, k != 0);
+        ptx::umma_commit(s_full);
+        if (!ptx::mbar_wait(p_full, t & 1, 1u << 22)) { report_error(p.err, ERR_EPILOGUE_WAIT); break; }
+        ptx::tc_fence_after();
 #pragma unroll
-      for (int e = 0; e < 4; ++e) { s[nt][e] = __expf(s[nt][e] - m[e >> 1]); rs[e >> 1] += s[nt][e]; }
-#pragma unroll
-    for (int x = 0; x < 2; ++x) {
-      rs[x] += __shfl_xor_sync(0xffffffffu, rs[x], 1);
-      rs[x] += __shfl_xor_sync(0xffffffffu, rs[x], 2);
-      l[x] = l[x] * corr[x] + rs[x];
+        for (int k = 0; k < 4; ++k)
+          ptx::umma_f16_ta(tmem + COL_O, tmem + COL_S + 8 * k, ptx::umma_smem_desc_sw128(vb + k * 2048, HALF_BYTES, 1024), id_o, (t | k) != 0);
+        ptx::umma_commit(&kv_empty[t % AF_STAGES]);
+        ptx::umma_commit(o_full);
+      }
     }
-    uint32_t ap[4][4];
-    pack_a<4>(s, ap);
-    mma_rows<false, 4, 8>(ap, Ks + TILE_ELEMS, out, lane);
-  }
-  cp_async_wait<0>();
+  } else {
+    const int quarter = warp & 3, r = 32 * quarter + lane, tin = r & 63, h = h0 + (quarter >> 1);
+    const bool active = quarter < 2 || both;                             // whole warps
+    const uint32_t ts = tmem + COL_S + (uint32_t(32 * quarter) << 16), to = tmem + COL_O + (uint32_t(32 * quarter) << 16);
+    const uint64_t scale = pair2(p.scale, p.scale), log2e = pair2(1.4426950408889634f, 1.4426950408889634f);
+    float m = -INFINITY, l = 0.f, corr = 1.f;
+    // The scores of one block -> P; `diag`: keys after the query's own position are hidden.
+    auto softmax = [&](auto diag) {
+      uint32_t s[32];
+      auto score = [&](int half, int e) {                                // keys 32 half + 2 e and the next one
+        float2 f = unpair(mul2(pair2(__uint_as_float(s[2 * e]), __uint_as_float(s[2 * e + 1])), scale));
+        if (diag.value && 32 * half + 2 * e > tin) f.x = -INFINITY;
+        if (diag.value && 32 * half + 2 * e + 1 > tin) f.y = -INFINITY;
+        return f;
+      };
+      float mx[2] = {-INFINITY, -INFINITY};
 #pragma unroll
-  for (int nt = 0; nt < 8; ++nt) { out[nt][0] /= l[0]; out[nt][1] /= l[0]; out[nt][2] /= l[1]; out[nt][3] /= l[1]; }
-  acc_to_global(out, o + (((long long)b * S + (long long)i * 64) * nq + h) * 64, (long long)nq * 64, warp, lane);
-  if ((lane & 3) == 0) {
+      for (int half = 1; half >= 0; --half) {                            // the first half stays in registers for the second pass
+        ptx::tmem_ld_32x32b_x32(ts + 32 * half, s);
+        ptx::tmem_ld_wait();
 #pragma unroll
-    for (int x = 0; x < 2; ++x) lse[((long long)b * nq + h) * S + (long long)i * 64 + r0 + 8 * x] = m[x] + __logf(l[x]);
+        for (int e = 0; e < 16; ++e) {
+          const float2 f = score(half, e);
+          mx[0] = fmaxf(mx[0], f.x);
+          mx[1] = fmaxf(mx[1], f.y);
+        }
+      }
+      const float mn = fmaxf(m, fmaxf(mx[0], mx[1]));
+      corr = __expf(m - mn);
+      m = mn;
+      const uint64_t minus_m = pair2(-m, -m);
+      float sum[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+      for (int half = 0; half < 2; ++half) {
+        if (half) { ptx::tmem_ld_32x32b_x32(ts + 32, s); ptx::tmem_ld_wait(); }
+        uint32_t pk[16];
+#pragma unroll
+        for (int e = 0; e < 16; ++e) {
+          const float2 f = score(half, e);
+          float2 x = unpair(mul2(add2(pair2(f.x, f.y), minus_m), log2e));
+          x.x = exp2_approx(x.x);
+          x.y = exp2_approx(x.y);
+          sum[e & 3] += x.x;
+          sum[e & 3] += x.y;
+          pk[e] = bf16_pair(x);
+        }
+        ptx::tmem_st_32x32b_x16(ts + 16 * half, pk);
+      }
+      l = fmaf(l, corr, (sum[0] + sum[1]) + (sum[2] + sum[3]));
+    };
+    bool ok = true;
+    for (int t = 0; t < n; ++t) {
+      if (!ptx::mbar_wait_warp(s_full, t & 1, 1u << 22)) { report_error(p.err, ERR_EPILOGUE_WAIT); ok = false; break; }
+      if (active) {
+        ptx::tc_fence_after();
+        if (list[t] == i) softmax(std::true_type());
+        else softmax(std::false_type());
+      }
+      if (t > 0) {
+        if (!ptx::mbar_wait_warp(o_full, (t - 1) & 1, 1u << 22)) { report_error(p.err, ERR_EPILOGUE_WAIT); ok = false; break; }
+        if (__any_sync(0xffffffffu, corr != 1.f)) {                      // also where corr is NaN
+          ptx::tc_fence_after();
+          const uint64_t c2 = pair2(corr, corr);
+#pragma unroll
+          for (int half = 0; half < 2; ++half) {
+            uint32_t x[32];
+            ptx::tmem_ld_32x32b_x32(to + 32 * half, x);
+            ptx::tmem_ld_wait();
+#pragma unroll
+            for (int e = 0; e < 16; ++e) {
+              const float2 f = unpair(mul2(pair2(__uint_as_float(x[2 * e]), __uint_as_float(x[2 * e + 1])), c2));
+              x[2 * e] = __float_as_uint(f.x);
+              x[2 * e + 1] = __float_as_uint(f.y);
+            }
+            ptx::tmem_st_32x32b_x32(to + 32 * half, x);
+          }
+        }
+      }
+      ptx::tmem_st_wait();
+      ptx::tc_fence_before();
+      __syncwarp();
+      if (lane == 0) ptx::mbar_arrive(p_full);
+    }
+    if (ok && n > 0 && !ptx::mbar_wait_warp(o_full, (n - 1) & 1, 1u << 22)) { report_error(p.err, ERR_EPILOGUE_WAIT); ok = false; }
+    if (ok && active) {
+      ptx::tc_fence_after();
+      bf16* dst = p.o + (((long long)b * p.S + (long long)i * 64 + tin) * p.nq + h) * 64;
+#pragma unroll
+      for (int half = 0; half < 2; ++half) {
+        uint32_t x[32];
+        ptx::tmem_ld_32x32b_x32(to + 32 * half, x);
+        ptx::tmem_ld_wait();
+        auto two = [&](int e) { return bf16_pair(make_float2((n ? __uint_as_float(x[e]) : 0.f) / l, (n ? __uint_as_float(x[e + 1]) : 0.f) / l)); };
+#pragma unroll
+        for (int v = 0; v < 4; ++v) *reinterpret_cast<uint4*>(dst + 32 * half + 8 * v) = make_uint4(two(8 * v), two(8 * v + 2), two(8 * v + 4), two(8 * v + 6));
+      }
+      p.lse[((long long)b * p.nq + h) * p.S + (long long)i * 64 + tin] = m + __logf(l);
+    }
   }
+  ptx::tc_fence_before();
+  __syncthreads();
+  if (warp == 1) ptx::tmem_dealloc(tmem, 128);
 }
 
 // ---- host ----------------------------------------------------------------------------------------------------------------------
@@ -133,20 +243,24 @@ static at::Tensor selection_matrix(const c10::optional<at::Tensor>& count, const
 
 // Returns {o [B,S,nq,64] bf16, lse [B,nq,S] fp32, sel [B,nb,nb] uint8}
 std::vector<at::Tensor> qsa_attn_fwd(const at::Tensor& q, const at::Tensor& k, const at::Tensor& v, const c10::optional<at::Tensor>& count,
-                                     const c10::optional<at::Tensor>& index, double scale) {
+                                     const c10::optional<at::Tensor>& index, double scale, const c10::optional<at::Tensor>& err) {
   check_heads(q, "qsa_attn_fwd q"); check_heads(k, "qsa_attn_fwd k"); check_heads(v, "qsa_attn_fwd v");
   const c10::cuda::CUDAGuard guard(q.device());
   const int B = q.size(0), nq = q.size(1), S = q.size(2), nkv = k.size(1), nb = S / 64;
-  TORCH_CHECK(S % 64 == 0 && nq % nkv == 0, "qsa_attn_fwd: bad shapes");
+  TORCH_CHECK(S % 64 == 0 && nkv > 0 && nq % nkv == 0 && k.sizes() == v.sizes() && k.size(0) == B && k.size(2) == S, "qsa_attn_fwd: bad shapes");
   auto stream = at::cuda::getCurrentCUDAStream();
   auto sel = selection_matrix(count, index, B, nb, q.options(), stream);
   auto o = at::empty({B, S, nq, 64}, q.options());
   auto lse = at::empty({B, nq, S}, q.options().dtype(at::kFloat));
-  const int smem = 4 * TILE_ELEMS * 2 + list_bytes(nb);
+  const CUtensorMap tq = make_tmap_box(q.data_ptr(), 2, 64, (int64_t)B * nq * S, 1, 64, 0, 64, 128), tk = make_tmap_box(k.data_ptr(), 2, 64, (int64_t)B * nkv * S, 1, 64, 0, 64, 128),
+                    tv = make_tmap_box(v.data_ptr(), 2, 64, (int64_t)B * nkv * S, 1, 64, 0, 64, 128);
+  FwdArgs p{};
+  p.sel = sel.data_ptr<unsigned char>(); p.o = (bf16*)o.data_ptr(); p.lse = lse.data_ptr<float>();
+  p.S = S; p.nq = nq; p.nkv = nkv; p.scale = (float)scale; p.err = err.has_value() ? err->data_ptr<int>() : nullptr;
+  const int smem = (1 + AF_STAGES) * TILE_BYTES + 128 + list_bytes(nb);
   static bool cfg = false;
   if (!cfg) { allow_smem(qsa_attn_fwd_kernel); cfg = true; }
-  qsa_attn_fwd_kernel<<<dim3(nq, nb, B), 128, smem, stream>>>((const bf16*)q.data_ptr(), (const bf16*)k.data_ptr(), (const bf16*)v.data_ptr(),
-      sel.data_ptr<unsigned char>(), (bf16*)o.data_ptr(), lse.data_ptr<float>(), S, nq, nkv, (float)scale);
+  qsa_attn_fwd_kernel<<<dim3(B * nkv * ((nq / nkv + 1) / 2), nb), AF_THREADS, smem, stream>>>(tq, tk, tv, p);
   C10_CUDA_KERNEL_LAUNCH_CHECK();
   count_launch();
   return {o, lse, sel};

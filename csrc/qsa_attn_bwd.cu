@@ -14,7 +14,7 @@
 // next tile are issued as soon as the threads have read the current ones.  dQ is bound by the exponentials (512 cycles of the special-function
 // units per tile; a tile takes 920 where the lists are long), dK / dV by shared memory: operand reads, TMA writes and the P / dS
 // tile come to 176 KB per tile, 1400 of its 1600 cycles.  Against the warp-MMA kernels in their place (16384 tokens of four sequences, 22 query heads,
-// eight blocks per query): dQ 219 -> 124 us, dK / dV 290 -> 201; dense, 8192 tokens of two sequences, 16 heads: 308 -> 123 and 399 -> 213.
+// eight blocks per query): dQ 219 -> 122 us, dK / dV 290 -> 200; dense, 8192 tokens of two sequences, 16 heads: 308 -> 121 and 399 -> 213.
 // Every mbarrier wait is bounded and reports through the error word.
 #include <ATen/ATen.h>
 #include <ATen/cuda/CUDAContext.h>
@@ -78,9 +78,9 @@ __global__ void __launch_bounds__(AB_THREADS, 2) qsa_attn_bwd_q_kernel(const __g
   float* dsum = reinterpret_cast<float*>(bars + 32);                     // [2][128]
   unsigned short* list = reinterpret_cast<unsigned short*>(dsum + 256);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  // late query blocks (longest lists) first, so that the last CTAs to start are short
-  const int nb = p.S / 64, i = nb - 1 - blockIdx.y, b = blockIdx.z, rep = p.nq / p.nkv, pairs = (rep + 1) / 2;
-  const int kvh = blockIdx.x / pairs, first = 2 * (blockIdx.x % pairs), h0 = kvh * rep + first;
+  // late query blocks (longest lists) of all sequences first, so that the last CTAs to start are short
+  const int nb = p.S / 64, i = nb - 1 - blockIdx.y, rep = p.nq / p.nkv, pairs = (rep + 1) / 2, b = blockIdx.x / (p.nkv * pairs);
+  const int kvh = blockIdx.x / pairs % p.nkv, first = 2 * (blockIdx.x % pairs), h0 = kvh * rep + first;
   const bool both = first + 1 < rep;                                     // an odd head has its tile to itself
   if (threadIdx.x == 0) {
     ptx::prefetch_tensormap(&tmQ);
@@ -94,6 +94,12 @@ __global__ void __launch_bounds__(AB_THREADS, 2) qsa_attn_bwd_q_kernel(const __g
     for (int s = 0; s < 2; ++s) { ptx::mbar_init(&ds_full[s], 8); ptx::mbar_init(&ds_empty[s], 1); }
     ptx::mbar_init(out_full, 1);
     ptx::fence_barrier_init();
+    ptx::mbar_expect_tx(in_full, 2 * TILE_BYTES);                        // while the list is made
+    for (int x = 0; x < 2; ++x) {
+      const int h = x && both ? h0 + 1 : h0;
+      ptx::tma_load_3d(q_tile + x * HALF_BYTES, &tmQ, in_full, 0, (b * p.nq + h) * p.S + i * 64, 0);
+      ptx::tma_load_3d(do_tile + x * HALF_BYTES, &tmDO, in_full, 0, b * p.S + i * 64, h);
+    }
   }
   if (warp == 1) { ptx::tmem_alloc(tmem_slot, 256); ptx::tmem_relinquish(); }
   ptx::tc_fence_before();
@@ -103,13 +109,7 @@ __global__ void __launch_bounds__(AB_THREADS, 2) qsa_attn_bwd_q_kernel(const __g
 
   if (warp == 0) {
     if (ptx::elect_one()) {
-      const int row0 = i * 64, kv_row0 = (b * p.nkv + kvh) * p.S;
-      ptx::mbar_expect_tx(in_full, 2 * TILE_BYTES);
-      for (int x = 0; x < 2; ++x) {
-        const int h = x && both ? h0 + 1 : h0;
-        ptx::tma_load_3d(q_tile + x * HALF_BYTES, &tmQ, in_full, 0, (b * p.nq + h) * p.S + row0, 0);
-        ptx::tma_load_3d(do_tile + x * HALF_BYTES, &tmDO, in_full, 0, b * p.S + row0, h);
-      }
+      const int kv_row0 = (b * p.nkv + kvh) * p.S;
       int t = 0;
       for (; t < n; ++t) {
         const int s = t % Q_STAGES;
@@ -424,7 +424,7 @@ std::vector<at::Tensor> qsa_attn_bwd(const at::Tensor& q, const at::Tensor& k, c
   const int smem_q = (2 + Q_STAGES) * TILE_BYTES + 1024 + 256 + 1024 + list_bytes(nb), smem_kv = (1 + 2 * KV_STAGES + 2) * TILE_BYTES + 256 + list_bytes(nb);
   static bool cfg = false;
   if (!cfg) { allow_smem(qsa_attn_bwd_q_kernel); allow_smem(qsa_attn_bwd_kv_kernel); cfg = true; }
-  qsa_attn_bwd_q_kernel<<<dim3(nkv * ((rep + 1) / 2), nb, B), AB_THREADS, smem_q, stream>>>(tq, tk, tv, tdo, p);
+  qsa_attn_bwd_q_kernel<<<dim3(B * nkv * ((rep + 1) / 2), nb), AB_THREADS, smem_q, stream>>>(tq, tk, tv, tdo, p);
   C10_CUDA_KERNEL_LAUNCH_CHECK();
   qsa_attn_bwd_kv_kernel<<<dim3(p.parts * nkv, nb, B), AB_THREADS, smem_kv, stream>>>(tq, tk, tv, tdo, p);
   C10_CUDA_KERNEL_LAUNCH_CHECK();

@@ -582,7 +582,7 @@ class _BlockAttention(torch.autograd.Function):
     @staticmethod
     def forward(ctx, q, k, v, count, index, scale):
         q, k, v = q.contiguous(), k.contiguous(), v.contiguous()
-        o, lse, sel = load().qsa_attn_fwd(q, k, v, count, index, scale)
+        o, lse, sel = load().qsa_attn_fwd(q, k, v, count, index, scale, error_flag(q.device))
         ctx.save_for_backward(q, k, v, o, lse, sel)
         ctx.scale = scale
         return o

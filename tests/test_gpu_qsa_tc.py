@@ -23,6 +23,6 @@ def test_indexer_backward_without_slices(ops, B, nb, NI):  # noqa: F811
     indexer_backward(ops, NI, B, nb)
 
 
-@pytest.mark.parametrize("name", ["qsa_attn_bwd.cu", "qsa_index_bwd.cu"])
+@pytest.mark.parametrize("name", ["qsa_attn.cu", "qsa_attn_bwd.cu", "qsa_index_bwd.cu"])
 def test_waits_of_whole_warps(name):
     waits_are_voted(name)
