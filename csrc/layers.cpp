@@ -30,7 +30,7 @@ Tensor rows_of(const Tensor& x) { return x.reshape({-1, x.size(-1)}).to(at::kBFl
 // A 2-D tensor whose row stride TMA accepts: narrow matrices (one column per head, say) are copied into rows padded to 16 bytes.
 Tensor tma_rows(const Tensor& t) {
   const int64_t n = t.size(1), per16 = 16 / t.element_size();
-  if (n % per16 == 0 && t.is_contiguous()) return t;
+  if (t.stride(1) == 1 && t.stride(0) >= n && t.stride(0) % per16 == 0 && (reinterpret_cast<uintptr_t>(t.data_ptr()) & 15) == 0) return t;
   auto view = at::empty({t.size(0), (n + per16 - 1) / per16 * per16}, t.options()).narrow(1, 0, n);
   view.copy_(t);
   return view;
