@@ -8,6 +8,7 @@
 
 #include "common.cuh"
 #include "host.h"
+#include "launch.cuh"
 
 namespace q38 {
 
@@ -15,6 +16,7 @@ constexpr int CE_THREADS = 256, CE_MAX_PER_THREAD = 64;          // rows up to 1
 
 __global__ void __launch_bounds__(CE_THREADS) ce_inplace_kernel(__nv_bfloat16* __restrict__ logits, const long long* __restrict__ target,
                                                                 float* __restrict__ loss, int V, long long ld) {
+  grid_wait();
   __shared__ float scratch[32];
   const long long row = blockIdx.x;
   __nv_bfloat162* p = reinterpret_cast<__nv_bfloat162*>(logits + row * ld);
@@ -71,6 +73,7 @@ __global__ void __launch_bounds__(CE_THREADS) ce_inplace_kernel(__nv_bfloat16* _
 template <int NV>
 __global__ void __launch_bounds__(CE_THREADS) ce_inplace_vec_kernel(__nv_bfloat16* __restrict__ logits, const long long* __restrict__ target,
                                                                     float* __restrict__ loss, int V, long long ld) {
+  grid_wait();
   __shared__ float scratch[32];
   const long long row = blockIdx.x;
   uint4* p = reinterpret_cast<uint4*>(logits + row * ld);
@@ -136,7 +139,7 @@ __global__ void __launch_bounds__(CE_THREADS) ce_inplace_vec_kernel(__nv_bfloat1
 
 template <int NV>
 static void launch_ce_vec(at::Tensor& logits, const at::Tensor& target, at::Tensor& loss, int V) {
-  ce_inplace_vec_kernel<NV><<<(unsigned)logits.size(0), CE_THREADS, 0, at::cuda::getCurrentCUDAStream()>>>(
+  launch(ce_inplace_vec_kernel<NV>, (unsigned)logits.size(0), CE_THREADS, 0, at::cuda::getCurrentCUDAStream(), 
       (__nv_bfloat16*)logits.data_ptr(), reinterpret_cast<const long long*>(target.data_ptr<int64_t>()), loss.data_ptr<float>(), V, V);
 }
 
@@ -161,7 +164,7 @@ at::Tensor ce_inplace(at::Tensor& logits, const at::Tensor& target) {
       default: launch_ce_vec<8>(logits, target, loss, V); break;
     }
   } else if (logits.size(0))
-    ce_inplace_kernel<<<(unsigned)logits.size(0), CE_THREADS, 0, at::cuda::getCurrentCUDAStream()>>>((__nv_bfloat16*)logits.data_ptr(), reinterpret_cast<const long long*>(target.data_ptr<int64_t>()),
+    launch(ce_inplace_kernel, (unsigned)logits.size(0), CE_THREADS, 0, at::cuda::getCurrentCUDAStream(), (__nv_bfloat16*)logits.data_ptr(), reinterpret_cast<const long long*>(target.data_ptr<int64_t>()),
                                                                                                     loss.data_ptr<float>(), V, V);
   C10_CUDA_KERNEL_LAUNCH_CHECK();
   count_launch();

@@ -7,6 +7,7 @@
 
 #include "common.cuh"
 #include "host.h"
+#include "launch.cuh"
 
 namespace q38 {
 
@@ -67,6 +68,7 @@ __device__ __forceinline__ void conv_fwd_run(const bf16* __restrict__ xb, const 
   }
 }
 __global__ void __launch_bounds__(128) conv_silu_fwd_kernel(const bf16* __restrict__ x, const float* __restrict__ w, bf16* __restrict__ y, int S, int C) {
+  grid_wait();
   const int c = 2 * (blockIdx.x * 128 + threadIdx.x);
   if (c >= C) return;
   const int t0 = blockIdx.y * RUN, b = blockIdx.z;
@@ -139,6 +141,7 @@ __device__ __forceinline__ void conv_bwd_run(const bf16* __restrict__ xb, const 
 }
 __global__ void __launch_bounds__(128, 8) conv_silu_bwd_kernel(const bf16* __restrict__ x, const float* __restrict__ w, const bf16* __restrict__ dy,
                                                                bf16* __restrict__ dx, float* __restrict__ dw, int S, int C) {
+  grid_wait();
   const int c = 2 * (blockIdx.x * 128 + threadIdx.x);
   if (c >= C) return;
   const int t0 = blockIdx.y * RUN_BWD, b = blockIdx.z;
@@ -163,7 +166,7 @@ at::Tensor conv_silu_fwd(const at::Tensor& x, const at::Tensor& w) {
   const int B = x.size(0), S = x.size(1), C = x.size(2);
   auto y = at::empty_like(x);
   dim3 grid((C / 2 + 127) / 128, (S + RUN - 1) / RUN, B);
-  conv_silu_fwd_kernel<<<grid, 128, 0, at::cuda::getCurrentCUDAStream()>>>((const bf16*)x.data_ptr(), w.data_ptr<float>(), (bf16*)y.data_ptr(), S, C);
+  launch(conv_silu_fwd_kernel, grid, 128, 0, at::cuda::getCurrentCUDAStream(), (const bf16*)x.data_ptr(), w.data_ptr<float>(), (bf16*)y.data_ptr(), S, C);
   C10_CUDA_KERNEL_LAUNCH_CHECK();
   count_launch();
   return y;
@@ -176,7 +179,7 @@ std::vector<at::Tensor> conv_silu_bwd(const at::Tensor& x, const at::Tensor& w, 
   auto dx = at::empty_like(x);
   auto dw = at::zeros({C, KW}, x.options().dtype(at::kFloat));
   dim3 grid((C / 2 + 127) / 128, (S + RUN_BWD - 1) / RUN_BWD, B);
-  conv_silu_bwd_kernel<<<grid, 128, 0, at::cuda::getCurrentCUDAStream()>>>((const bf16*)x.data_ptr(), w.data_ptr<float>(), (const bf16*)dy.data_ptr(),
+  launch(conv_silu_bwd_kernel, grid, 128, 0, at::cuda::getCurrentCUDAStream(), (const bf16*)x.data_ptr(), w.data_ptr<float>(), (const bf16*)dy.data_ptr(),
                                                                            (bf16*)dx.data_ptr(), dw.data_ptr<float>(), S, C);
   C10_CUDA_KERNEL_LAUNCH_CHECK();
   count_launch();

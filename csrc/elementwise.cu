@@ -6,6 +6,7 @@
 
 #include "common.cuh"
 #include "host.h"
+#include "launch.cuh"
 
 namespace q38 {
 
@@ -16,6 +17,7 @@ template <typename InT, typename OutT>
 __global__ void __launch_bounds__(32 * ROWS_PER_CTA) rmsnorm_fwd_kernel(const InT* __restrict__ x, const float* __restrict__ w,
                                                                         OutT* __restrict__ y, float* __restrict__ rstd,
                                                                         int rows, int dim, float eps) {
+  grid_wait();
   const int row = blockIdx.x * ROWS_PER_CTA + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (row >= rows) return;
   const InT* xr = x + (size_t)row * dim;
@@ -34,6 +36,7 @@ __global__ void __launch_bounds__(32 * ROWS_PER_CTA) rmsnorm_bwd_kernel(const Gr
                                                                         const float* __restrict__ w, const float* __restrict__ rstd,
                                                                         InT* __restrict__ dx, float* __restrict__ dw_partial,
                                                                         int rows, int dim) {
+  grid_wait();
   extern __shared__ float dw_acc[];            // [dim], accumulated over this CTA's rows
   for (int i = threadIdx.x; i < dim; i += blockDim.x) dw_acc[i] = 0.f;
   __syncthreads();
@@ -66,7 +69,7 @@ std::vector<at::Tensor> rmsnorm_fwd(const at::Tensor& x, const at::Tensor& w, do
   if (rows == 0) return {y, rstd};
   const int grid = (rows + ROWS_PER_CTA - 1) / ROWS_PER_CTA;
   auto stream = at::cuda::getCurrentCUDAStream();
-#define LAUNCH(InT, OutT) rmsnorm_fwd_kernel<InT, OutT><<<grid, 32 * ROWS_PER_CTA, 0, stream>>>( \
+#define LAUNCH(InT, OutT) launch(rmsnorm_fwd_kernel<InT, OutT>, grid, 32 * ROWS_PER_CTA, 0, stream,  \
       (const InT*)x.data_ptr(), w.data_ptr<float>(), (OutT*)y.data_ptr(), rstd.data_ptr<float>(), rows, dim, (float)eps)
   if (x.scalar_type() == at::kFloat) { if (out_bf16) LAUNCH(float, __nv_bfloat16); else LAUNCH(float, float); }
   else if (x.scalar_type() == at::kBFloat16) { if (out_bf16) LAUNCH(__nv_bfloat16, __nv_bfloat16); else LAUNCH(__nv_bfloat16, float); }
@@ -88,7 +91,7 @@ std::vector<at::Tensor> rmsnorm_bwd(const at::Tensor& dy, const at::Tensor& x, c
   const int grid = std::min((rows + ROWS_PER_CTA - 1) / ROWS_PER_CTA, kNumSMs * 4);
   auto stream = at::cuda::getCurrentCUDAStream();
   const size_t smem = dim * sizeof(float);
-#define LAUNCH(InT, GradT) rmsnorm_bwd_kernel<InT, GradT><<<grid, 32 * ROWS_PER_CTA, smem, stream>>>( \
+#define LAUNCH(InT, GradT) launch(rmsnorm_bwd_kernel<InT, GradT>, grid, 32 * ROWS_PER_CTA, smem, stream,  \
       (const GradT*)dy.data_ptr(), (const InT*)x.data_ptr(), w.data_ptr<float>(), rstd.data_ptr<float>(), (InT*)dx.data_ptr(), \
       dw.data_ptr<float>(), rows, dim)
   const bool xf = x.scalar_type() == at::kFloat, gf = dy.scalar_type() == at::kFloat;
@@ -124,6 +127,7 @@ __device__ __forceinline__ float group8_sum(float v) {
 
 __global__ void __launch_bounds__(256) gated_rmsnorm_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ gate,
                                                                  const float* __restrict__ w, __nv_bfloat16* __restrict__ y, int rows, float eps) {
+  grid_wait();
   const int sub = threadIdx.x & 7;
   const long long row = ((long long)blockIdx.x * 256 + threadIdx.x) >> 3;
   const bool live = row < rows;
@@ -151,6 +155,7 @@ __global__ void __launch_bounds__(256) gated_rmsnorm_bwd_kernel(const __nv_bfloa
                                                                  const __nv_bfloat16* __restrict__ gate, const float* __restrict__ w,
                                                                  __nv_bfloat16* __restrict__ dx, __nv_bfloat16* __restrict__ dgate,
                                                                  float* __restrict__ dw, int rows, float eps) {
+  grid_wait();
   __shared__ float dw_acc[64];
   if (threadIdx.x < 64) dw_acc[threadIdx.x] = 0.f;
   __syncthreads();
@@ -219,6 +224,7 @@ __global__ void __launch_bounds__(256) gated_rmsnorm_bwd_kernel(const __nv_bfloa
 // ---- SwiGLU: y = bf16(silu(g)) * u, elementwise on bf16 (eight elements per thread) --------------------------------------
 __global__ void __launch_bounds__(256) swiglu_fwd_kernel(const __nv_bfloat16* __restrict__ g, const __nv_bfloat16* __restrict__ u,
                                                           __nv_bfloat16* __restrict__ y, long long n8) {
+  grid_wait();
   const long long i = (long long)blockIdx.x * 256 + threadIdx.x;
   if (i >= n8) return;
   float gv[8], uv[8], o[8];
@@ -232,6 +238,7 @@ __global__ void __launch_bounds__(256) swiglu_fwd_kernel(const __nv_bfloat16* __
 __global__ void __launch_bounds__(256) swiglu_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ g,
                                                           const __nv_bfloat16* __restrict__ u, __nv_bfloat16* __restrict__ dg,
                                                           __nv_bfloat16* __restrict__ du, long long n8) {
+  grid_wait();
   const long long i = (long long)blockIdx.x * 256 + threadIdx.x;
   if (i >= n8) return;
   float dv[8], gv[8], uv[8], og[8], ou[8];
@@ -254,7 +261,7 @@ at::Tensor swiglu_fwd(const at::Tensor& g, const at::Tensor& u) {
   const c10::cuda::CUDAGuard guard(g.device());
   auto y = at::empty_like(g);
   const long long n8 = g.numel() / 8;
-  if (n8) swiglu_fwd_kernel<<<(unsigned)((n8 + 255) / 256), 256, 0, at::cuda::getCurrentCUDAStream()>>>(
+  if (n8) launch(swiglu_fwd_kernel, (unsigned)((n8 + 255) / 256), 256, 0, at::cuda::getCurrentCUDAStream(), 
       (const __nv_bfloat16*)g.data_ptr(), (const __nv_bfloat16*)u.data_ptr(), (__nv_bfloat16*)y.data_ptr(), n8);
   C10_CUDA_KERNEL_LAUNCH_CHECK();
   count_launch();
@@ -266,7 +273,7 @@ std::vector<at::Tensor> swiglu_bwd(const at::Tensor& dy, const at::Tensor& g, co
   const c10::cuda::CUDAGuard guard(g.device());
   auto dg = at::empty_like(g), du = at::empty_like(u);
   const long long n8 = g.numel() / 8;
-  if (n8) swiglu_bwd_kernel<<<(unsigned)((n8 + 255) / 256), 256, 0, at::cuda::getCurrentCUDAStream()>>>(
+  if (n8) launch(swiglu_bwd_kernel, (unsigned)((n8 + 255) / 256), 256, 0, at::cuda::getCurrentCUDAStream(), 
       (const __nv_bfloat16*)dy.data_ptr(), (const __nv_bfloat16*)g.data_ptr(), (const __nv_bfloat16*)u.data_ptr(), (__nv_bfloat16*)dg.data_ptr(),
       (__nv_bfloat16*)du.data_ptr(), n8);
   C10_CUDA_KERNEL_LAUNCH_CHECK();
@@ -277,6 +284,7 @@ std::vector<at::Tensor> swiglu_bwd(const at::Tensor& dy, const at::Tensor& g, co
 // ---- y = x * factor[0] on bf16, eight elements per thread (a library product with a one-element device tensor runs element by element: 16 us
 // instead of 6 for 8192 x 576) ---------------------------------------------------------------------------------------------
 __global__ void __launch_bounds__(256) scale_bf16_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ factor, __nv_bfloat16* __restrict__ y, long long n8) {
+  grid_wait();
   const long long i = (long long)blockIdx.x * 256 + threadIdx.x;
   if (i >= n8) return;
   const float f = __bfloat162float(*factor);
@@ -294,7 +302,7 @@ at::Tensor scale_bf16(const at::Tensor& x, const at::Tensor& factor) {
   auto y = at::empty_like(x);
   const long long n8 = x.numel() / 8;
   if (n8) {
-    scale_bf16_kernel<<<(unsigned)((n8 + 255) / 256), 256, 0, at::cuda::getCurrentCUDAStream()>>>((const __nv_bfloat16*)x.data_ptr(), (const __nv_bfloat16*)factor.data_ptr(),
+    launch(scale_bf16_kernel, (unsigned)((n8 + 255) / 256), 256, 0, at::cuda::getCurrentCUDAStream(), (const __nv_bfloat16*)x.data_ptr(), (const __nv_bfloat16*)factor.data_ptr(),
                                                                                                   (__nv_bfloat16*)y.data_ptr(), n8);
     C10_CUDA_KERNEL_LAUNCH_CHECK();
     count_launch();
@@ -305,6 +313,7 @@ at::Tensor scale_bf16(const at::Tensor& x, const at::Tensor& factor) {
 // ---- output gate of the attention layer: y = x * bf16(sigmoid(g)), elementwise on bf16 (eight elements per thread) -------
 __global__ void __launch_bounds__(256) sigmoid_mul_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ g,
                                                                __nv_bfloat16* __restrict__ y, long long n8) {
+  grid_wait();
   const long long i = (long long)blockIdx.x * 256 + threadIdx.x;
   if (i >= n8) return;
   float xv[8], gv[8], o[8];
@@ -318,6 +327,7 @@ __global__ void __launch_bounds__(256) sigmoid_mul_fwd_kernel(const __nv_bfloat1
 __global__ void __launch_bounds__(256) sigmoid_mul_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ x,
                                                                const __nv_bfloat16* __restrict__ g, __nv_bfloat16* __restrict__ dx,
                                                                __nv_bfloat16* __restrict__ dg, long long n8) {
+  grid_wait();
   const long long i = (long long)blockIdx.x * 256 + threadIdx.x;
   if (i >= n8) return;
   float dv[8], xv[8], gv[8], ox[8], og[8];
@@ -340,7 +350,7 @@ at::Tensor sigmoid_mul_fwd(const at::Tensor& x, const at::Tensor& g) {
   const c10::cuda::CUDAGuard guard(x.device());
   auto y = at::empty_like(x);
   const long long n8 = x.numel() / 8;
-  if (n8) sigmoid_mul_fwd_kernel<<<(unsigned)((n8 + 255) / 256), 256, 0, at::cuda::getCurrentCUDAStream()>>>(
+  if (n8) launch(sigmoid_mul_fwd_kernel, (unsigned)((n8 + 255) / 256), 256, 0, at::cuda::getCurrentCUDAStream(), 
       (const __nv_bfloat16*)x.data_ptr(), (const __nv_bfloat16*)g.data_ptr(), (__nv_bfloat16*)y.data_ptr(), n8);
   C10_CUDA_KERNEL_LAUNCH_CHECK();
   count_launch();
@@ -352,7 +362,7 @@ std::vector<at::Tensor> sigmoid_mul_bwd(const at::Tensor& dy, const at::Tensor& 
   const c10::cuda::CUDAGuard guard(x.device());
   auto dx = at::empty_like(x), dg = at::empty_like(g);
   const long long n8 = x.numel() / 8;
-  if (n8) sigmoid_mul_bwd_kernel<<<(unsigned)((n8 + 255) / 256), 256, 0, at::cuda::getCurrentCUDAStream()>>>(
+  if (n8) launch(sigmoid_mul_bwd_kernel, (unsigned)((n8 + 255) / 256), 256, 0, at::cuda::getCurrentCUDAStream(), 
       (const __nv_bfloat16*)dy.data_ptr(), (const __nv_bfloat16*)x.data_ptr(), (const __nv_bfloat16*)g.data_ptr(), (__nv_bfloat16*)dx.data_ptr(),
       (__nv_bfloat16*)dg.data_ptr(), n8);
   C10_CUDA_KERNEL_LAUNCH_CHECK();
@@ -363,6 +373,7 @@ std::vector<at::Tensor> sigmoid_mul_bwd(const at::Tensor& dy, const at::Tensor& 
 // ---- shared-expert merge: out = routed + sigmoid(logit_t) * shared  (one warp per token row, 16-byte accesses) ------------
 __global__ void __launch_bounds__(256) gate_add_fwd_kernel(const __nv_bfloat16* __restrict__ routed, const __nv_bfloat16* __restrict__ shared,
                                                             const __nv_bfloat16* __restrict__ logit, __nv_bfloat16* __restrict__ out, int T, int h) {
+  grid_wait();
   const int lane = threadIdx.x & 31;
   const long long t = (long long)blockIdx.x * 8 + (threadIdx.x >> 5);
   if (t >= T) return;
@@ -381,6 +392,7 @@ __global__ void __launch_bounds__(256) gate_add_fwd_kernel(const __nv_bfloat16* 
 __global__ void __launch_bounds__(256) gate_add_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ shared,
                                                             const __nv_bfloat16* __restrict__ logit, __nv_bfloat16* __restrict__ dshared,
                                                             __nv_bfloat16* __restrict__ dlogit, int T, int h) {
+  grid_wait();
   const int lane = threadIdx.x & 31;
   const long long t = (long long)blockIdx.x * 8 + (threadIdx.x >> 5);
   if (t >= T) return;
@@ -405,7 +417,7 @@ at::Tensor gate_add_fwd(const at::Tensor& routed, const at::Tensor& shared, cons
   const c10::cuda::CUDAGuard guard(routed.device());
   const int T = routed.size(0), h = routed.size(1);
   auto out = at::empty_like(routed);
-  if (T) gate_add_fwd_kernel<<<(T + 7) / 8, 256, 0, at::cuda::getCurrentCUDAStream()>>>(
+  if (T) launch(gate_add_fwd_kernel, (T + 7) / 8, 256, 0, at::cuda::getCurrentCUDAStream(), 
       (const __nv_bfloat16*)routed.data_ptr(), (const __nv_bfloat16*)shared.data_ptr(), (const __nv_bfloat16*)logit.data_ptr(), (__nv_bfloat16*)out.data_ptr(), T, h);
   C10_CUDA_KERNEL_LAUNCH_CHECK();
   count_launch();
@@ -417,7 +429,7 @@ std::vector<at::Tensor> gate_add_bwd(const at::Tensor& dy, const at::Tensor& sha
   const c10::cuda::CUDAGuard guard(dy.device());
   const int T = dy.size(0), h = dy.size(1);
   auto dshared = at::empty_like(shared), dlogit = at::empty_like(logit);
-  if (T) gate_add_bwd_kernel<<<(T + 7) / 8, 256, 0, at::cuda::getCurrentCUDAStream()>>>(
+  if (T) launch(gate_add_bwd_kernel, (T + 7) / 8, 256, 0, at::cuda::getCurrentCUDAStream(), 
       (const __nv_bfloat16*)dy.data_ptr(), (const __nv_bfloat16*)shared.data_ptr(), (const __nv_bfloat16*)logit.data_ptr(), (__nv_bfloat16*)dshared.data_ptr(),
       (__nv_bfloat16*)dlogit.data_ptr(), T, h);
   C10_CUDA_KERNEL_LAUNCH_CHECK();
@@ -429,6 +441,7 @@ std::vector<at::Tensor> gate_add_bwd(const at::Tensor& dy, const at::Tensor& sha
 __global__ void __launch_bounds__(256) gdn_gates_fwd_kernel(const __nv_bfloat16* __restrict__ b_raw, const __nv_bfloat16* __restrict__ a_raw,
                                                              const float* __restrict__ A_log, const float* __restrict__ dt_bias,
                                                              __nv_bfloat16* __restrict__ beta, float* __restrict__ g, long long n, int H) {
+  grid_wait();
   const long long i = (long long)blockIdx.x * 256 + threadIdx.x;
   if (i >= n) return;
   const int h = i % H;
@@ -444,6 +457,7 @@ __global__ void __launch_bounds__(256) gdn_gates_bwd_kernel(const __nv_bfloat16*
                                                              const float* __restrict__ A_log, const float* __restrict__ dt_bias,
                                                              __nv_bfloat16* __restrict__ db_raw, __nv_bfloat16* __restrict__ da_raw,
                                                              float* __restrict__ dA_log, float* __restrict__ ddt_bias, long long rows, int H) {
+  grid_wait();
   extern __shared__ float acc[];                     // [2 * H]
   for (int i = threadIdx.x; i < 2 * H; i += blockDim.x) acc[i] = 0.f;
   __syncthreads();
@@ -483,7 +497,7 @@ std::vector<at::Tensor> gdn_gates_fwd(const at::Tensor& b_raw, const at::Tensor&
   const long long n = b_raw.numel();
   auto beta = at::empty_like(b_raw);
   auto g = at::empty(b_raw.sizes(), b_raw.options().dtype(at::kFloat));
-  if (n) gdn_gates_fwd_kernel<<<(unsigned)((n + 255) / 256), 256, 0, at::cuda::getCurrentCUDAStream()>>>(
+  if (n) launch(gdn_gates_fwd_kernel, (unsigned)((n + 255) / 256), 256, 0, at::cuda::getCurrentCUDAStream(), 
       (const __nv_bfloat16*)b_raw.data_ptr(), (const __nv_bfloat16*)a_raw.data_ptr(), A_log.data_ptr<float>(), dt_bias.data_ptr<float>(),
       (__nv_bfloat16*)beta.data_ptr(), g.data_ptr<float>(), n, H);
   C10_CUDA_KERNEL_LAUNCH_CHECK();
@@ -501,7 +515,7 @@ std::vector<at::Tensor> gdn_gates_bwd(const at::Tensor& dbeta, const at::Tensor&
   const long long rows = b_raw.numel() / H;
   auto db = at::empty_like(b_raw), da = at::empty_like(a_raw);
   auto dA = at::zeros({H}, A_log.options()), dbias = at::zeros({H}, A_log.options());
-  if (rows) gdn_gates_bwd_kernel<<<(unsigned)std::min<long long>((rows + 11) / 12, 4 * kNumSMs), 256, 2 * H * sizeof(float), at::cuda::getCurrentCUDAStream()>>>(
+  if (rows) launch(gdn_gates_bwd_kernel, (unsigned)std::min<long long>((rows + 11) / 12, 4 * kNumSMs), 256, 2 * H * sizeof(float), at::cuda::getCurrentCUDAStream(), 
       (const __nv_bfloat16*)dbeta.data_ptr(), dg.data_ptr<float>(), (const __nv_bfloat16*)b_raw.data_ptr(), (const __nv_bfloat16*)a_raw.data_ptr(),
       A_log.data_ptr<float>(), dt_bias.data_ptr<float>(), (__nv_bfloat16*)db.data_ptr(), (__nv_bfloat16*)da.data_ptr(), dA.data_ptr<float>(),
       dbias.data_ptr<float>(), rows, H);
@@ -516,7 +530,7 @@ at::Tensor gated_rmsnorm_fwd(const at::Tensor& x, const at::Tensor& gate, const 
   const c10::cuda::CUDAGuard guard(x.device());
   const int rows = x.numel() / 64;
   auto y = at::empty_like(x);
-  if (rows) gated_rmsnorm_fwd_kernel<<<(rows + 31) / 32, 256, 0, at::cuda::getCurrentCUDAStream()>>>(
+  if (rows) launch(gated_rmsnorm_fwd_kernel, (rows + 31) / 32, 256, 0, at::cuda::getCurrentCUDAStream(), 
       (const __nv_bfloat16*)x.data_ptr(), (const __nv_bfloat16*)gate.data_ptr(), w.data_ptr<float>(), (__nv_bfloat16*)y.data_ptr(), rows, (float)eps);
   C10_CUDA_KERNEL_LAUNCH_CHECK();
   count_launch();
@@ -529,7 +543,7 @@ std::vector<at::Tensor> gated_rmsnorm_bwd(const at::Tensor& dy, const at::Tensor
   const int rows = x.numel() / 64;
   auto dx = at::empty_like(x), dgate = at::empty_like(gate);
   auto dw = at::zeros({64}, x.options().dtype(at::kFloat));
-  if (rows) gated_rmsnorm_bwd_kernel<<<std::min((rows + 31) / 32, kNumSMs * 8), 256, 0, at::cuda::getCurrentCUDAStream()>>>(
+  if (rows) launch(gated_rmsnorm_bwd_kernel, std::min((rows + 31) / 32, kNumSMs * 8), 256, 0, at::cuda::getCurrentCUDAStream(), 
       (const __nv_bfloat16*)dy.data_ptr(), (const __nv_bfloat16*)x.data_ptr(), (const __nv_bfloat16*)gate.data_ptr(), w.data_ptr<float>(),
       (__nv_bfloat16*)dx.data_ptr(), (__nv_bfloat16*)dgate.data_ptr(), dw.data_ptr<float>(), rows, (float)eps);
   C10_CUDA_KERNEL_LAUNCH_CHECK();
@@ -543,6 +557,7 @@ __global__ void __launch_bounds__(256) adamw_flat_kernel(float* __restrict__ p, 
                                                           const float* __restrict__ grad_scale, size_t n, float lr, float wd, float b1,
                                                           float b2, float eps, float inv_bc1, float inv_sqrt_bc2,
                                                           const float* __restrict__ hyper, const int* __restrict__ err) {
+  grid_wait();
   if (err != nullptr && *reinterpret_cast<const volatile int*>(err) != 0) return;   // a peer missed a barrier: leave parameters and moments untouched
   const float gs = grad_scale ? *grad_scale : 1.f;
   if (hyper) { lr = hyper[0]; inv_bc1 = hyper[1]; inv_sqrt_bc2 = hyper[2]; }   // step-dependent scalars from device memory (CUDA-graph replay)
@@ -569,7 +584,7 @@ void adamw_flat(at::Tensor& p, const at::Tensor& g, at::Tensor& m, at::Tensor& v
   if (!n) return;
   const double bc1 = 1.0 - std::pow(beta1, (double)step), bc2 = 1.0 - std::pow(beta2, (double)step);
   const int grid = (int)std::min<size_t>((n + 255) / 256, (size_t)kNumSMs * 16);
-  adamw_flat_kernel<<<grid, 256, 0, at::cuda::getCurrentCUDAStream()>>>(
+  launch(adamw_flat_kernel, grid, 256, 0, at::cuda::getCurrentCUDAStream(), 
       p.data_ptr<float>(), g.data_ptr<float>(), m.data_ptr<float>(), v.data_ptr<float>(),
       shadow.has_value() ? (__nv_bfloat16*)shadow->data_ptr() : nullptr, grad_scale.has_value() ? grad_scale->data_ptr<float>() : nullptr,
       n, (float)lr, (float)wd, (float)beta1, (float)beta2, (float)eps, (float)(1.0 / bc1), (float)(1.0 / std::sqrt(bc2)),
@@ -580,6 +595,7 @@ void adamw_flat(at::Tensor& p, const at::Tensor& g, at::Tensor& m, at::Tensor& v
 
 // ---- sum of squares of a flat fp32 tensor -> one fp32 scalar (double accumulation across CTAs) ------------------------
 __global__ void __launch_bounds__(256) sum_squares_kernel(const float* __restrict__ x, size_t n, double* __restrict__ out) {
+  grid_wait();
   __shared__ float scratch[32];
   float acc = 0.f;
   for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) acc += x[i] * x[i];
@@ -594,7 +610,7 @@ at::Tensor sum_squares(const at::Tensor& x) {
   const size_t n = x.numel();
   if (n) {
     const int grid = (int)std::min<size_t>((n + 255) / 256, (size_t)kNumSMs * 8);
-    sum_squares_kernel<<<grid, 256, 0, at::cuda::getCurrentCUDAStream()>>>(x.data_ptr<float>(), n, out.data_ptr<double>());
+    launch(sum_squares_kernel, grid, 256, 0, at::cuda::getCurrentCUDAStream(), x.data_ptr<float>(), n, out.data_ptr<double>());
     C10_CUDA_KERNEL_LAUNCH_CHECK();
   count_launch();
   }

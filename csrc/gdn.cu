@@ -25,6 +25,7 @@
 
 #include "common.cuh"
 #include "host.h"
+#include "launch.cuh"
 #include "gdn_tile.cuh"
 #include "mma_tile.cuh"
 
@@ -55,6 +56,7 @@ template <int W>
 __global__ void __launch_bounds__(64 * W + 64) gdn_scan_fwd_kernel(const __grid_constant__ gdn::Maps4 maps, const bf16* __restrict__ u, const float* __restrict__ dch,
                                                                    bf16* __restrict__ o, bf16* __restrict__ vnew, bf16* __restrict__ states, int NT, int H,
                                                                    int* __restrict__ err) {
+  grid_wait();
   using namespace gdn;
   using L = ScanSmem<W>;
   extern __shared__ __align__(1024) uint8_t scan_smem[];
@@ -164,6 +166,7 @@ __global__ void __launch_bounds__(256) gdn_scan_bwd_kernel(const bf16* __restric
                                                            const bf16* __restrict__ states, const bf16* __restrict__ dout, bf16* __restrict__ dw,
                                                            bf16* __restrict__ du, bf16* __restrict__ dP, bf16* __restrict__ dqg, bf16* __restrict__ dkg,
                                                            float* __restrict__ dd, int NT, int H) {
+  grid_wait();
   extern __shared__ __align__(16) uint8_t smem_bytes[];
   bf16* sm = reinterpret_cast<bf16*>(smem_bytes);
   // two buffers of seven tiles: w, P, qg, kg, vnew, state, do ; then dS (bf16) and dv_new (bf16)
@@ -286,7 +289,7 @@ std::vector<at::Tensor> gdn_scan_fwd(const at::Tensor& w, const at::Tensor& u, c
     constexpr int smem = ScanSmem<W>::BYTES;
     static bool configured = false;
     if (!configured) { C10_CUDA_CHECK(cudaFuncSetAttribute(gdn_scan_fwd_kernel<W>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem)); configured = true; }
-    gdn_scan_fwd_kernel<W><<<dim3((int)BH, 4 / W), 64 * W + 64, smem, at::cuda::getCurrentCUDAStream()>>>(
+    q38::launch(gdn_scan_fwd_kernel<W>, dim3((int)BH, 4 / W), 64 * W + 64, smem, at::cuda::getCurrentCUDAStream(), 
         maps, (const bf16*)u.data_ptr(), dch.data_ptr<float>(), (bf16*)o.data_ptr(), save ? (bf16*)vnew.data_ptr() : nullptr,
         save ? (bf16*)states.data_ptr() : nullptr, (int)NT, (int)H, err.has_value() ? err->data_ptr<int>() : nullptr);
   };
@@ -315,7 +318,7 @@ std::vector<at::Tensor> gdn_scan_bwd(const at::Tensor& w, const at::Tensor& P, c
   const int smem = 16 * TILE_ELEMS * 2;
   static bool configured = false;
   if (!configured) { C10_CUDA_CHECK(cudaFuncSetAttribute(gdn_scan_bwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem)); configured = true; }
-  gdn_scan_bwd_kernel<<<(int)BH, 256, smem, at::cuda::getCurrentCUDAStream()>>>(
+  launch(gdn_scan_bwd_kernel, (int)BH, 256, smem, at::cuda::getCurrentCUDAStream(), 
       (const bf16*)w.data_ptr(), (const bf16*)P.data_ptr(), (const bf16*)qg.data_ptr(), (const bf16*)kg.data_ptr(), dch.data_ptr<float>(),
       (const bf16*)vnew.data_ptr(), (const bf16*)states.data_ptr(), (const bf16*)dout.data_ptr(), (bf16*)dw.data_ptr(), (bf16*)du.data_ptr(),
       (bf16*)dP.data_ptr(), (bf16*)dqg.data_ptr(), (bf16*)dkg.data_ptr(), dd.data_ptr<float>(), (int)NT, (int)H);
@@ -343,6 +346,7 @@ __global__ void __launch_bounds__(128, 4) gdn_prep_fwd_kernel(const bf16* __rest
                                                               bf16* __restrict__ u_out, bf16* __restrict__ P_out, bf16* __restrict__ qg_out,
                                                               bf16* __restrict__ kg_out, bf16* __restrict__ Tm_out, float* __restrict__ carry,
                                                               float* __restrict__ gc_out, int S, int Hk, int Hv, long long qk_ld, long long v_ld) {
+  grid_wait();
   extern __shared__ __align__(16) uint8_t smem_bytes[];
   bf16* sm = reinterpret_cast<bf16*>(smem_bytes);
   bf16 *Qn = sm, *Kn = sm + TILE_ELEMS, *KBG = sm + 2 * TILE_ELEMS, *VB = sm + 3 * TILE_ELEMS, *Tm = sm + 4 * TILE_ELEMS;
@@ -571,6 +575,7 @@ __global__ void __launch_bounds__(256, 2) gdn_prep_bwd_kernel(const bf16* __rest
                                                               bf16* __restrict__ dq, bf16* __restrict__ dk, bf16* __restrict__ dv,
                                                               float* __restrict__ dg, float* __restrict__ dbeta, int S, int Hk, int Hv,
                                                               long long qk_ld, long long v_ld, long long dqk_ld, long long dv_ld) {
+  grid_wait();
   extern __shared__ __align__(16) uint8_t smem_bytes[];
   bf16* sm = reinterpret_cast<bf16*>(smem_bytes);
   bf16 *Qn = sm, *Kn = sm + TILE_ELEMS, *St = sm + 2 * TILE_ELEMS, *Do = sm + 3 * TILE_ELEMS, *Vn = sm + 4 * TILE_ELEMS, *Ds = sm + 5 * TILE_ELEMS;
@@ -883,7 +888,7 @@ std::vector<at::Tensor> gdn_prep_fwd(const at::Tensor& q, const at::Tensor& k, c
   constexpr int smem = 5 * TILE_ELEMS * 2 + 256 * 4;
   static bool configured = false;
   if (!configured) { C10_CUDA_CHECK(cudaFuncSetAttribute(gdn_prep_fwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem)); configured = true; }
-  gdn_prep_fwd_kernel<<<dim3((int)NT, (int)BH), 128, smem, at::cuda::getCurrentCUDAStream()>>>(
+  launch(gdn_prep_fwd_kernel, dim3((int)NT, (int)BH), 128, smem, at::cuda::getCurrentCUDAStream(), 
       (const bf16*)q.data_ptr(), (const bf16*)k.data_ptr(), (const bf16*)v.data_ptr(), g.data_ptr<float>(), (const bf16*)beta.data_ptr(),
       (bf16*)out[0].data_ptr(), (bf16*)out[1].data_ptr(), (bf16*)out[2].data_ptr(), (bf16*)out[3].data_ptr(), (bf16*)out[4].data_ptr(),
       save ? (bf16*)out[5].data_ptr() : nullptr, out[6].data_ptr<float>(), out[7].data_ptr<float>(), (int)S, (int)Hk, (int)Hv, (long long)q.stride(1), (long long)v.stride(1));
@@ -911,7 +916,7 @@ std::vector<at::Tensor> gdn_prep_bwd(const at::Tensor& q, const at::Tensor& k, c
   constexpr int smem = 12 * TILE_ELEMS * 2 + 648 * 4;
   static bool configured = false;
   if (!configured) { C10_CUDA_CHECK(cudaFuncSetAttribute(gdn_prep_bwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem)); configured = true; }
-  gdn_prep_bwd_kernel<<<dim3((int)NT, (int)(B * Hk)), 256, smem, at::cuda::getCurrentCUDAStream()>>>(
+  launch(gdn_prep_bwd_kernel, dim3((int)NT, (int)(B * Hk)), 256, smem, at::cuda::getCurrentCUDAStream(), 
       (const bf16*)q.data_ptr(), (const bf16*)k.data_ptr(), (const bf16*)v.data_ptr(), g.data_ptr<float>(), (const bf16*)beta.data_ptr(),
       (const bf16*)Tm.data_ptr(), (const bf16*)w.data_ptr(), (const bf16*)u.data_ptr(), (const bf16*)vnew.data_ptr(), (const bf16*)states.data_ptr(),
       (const bf16*)dout.data_ptr(), (const bf16*)du.data_ptr(), (const bf16*)dstate.data_ptr(), dd.data_ptr<float>(), dq_ptr, dk_ptr, dv_ptr,

@@ -14,6 +14,7 @@
 #include "common.cuh"
 #include "gdn_tile.cuh"
 #include "host.h"
+#include "launch.cuh"
 
 namespace q38 {
 
@@ -21,6 +22,7 @@ template <int W>
 __global__ void __launch_bounds__(32 * W) gdn_chain_bwd_kernel(const __grid_constant__ gdn::Maps4 maps, const bf16* __restrict__ dout, const bf16* __restrict__ states,
                                                                const float* __restrict__ dch, bf16* __restrict__ du, bf16* __restrict__ dstate,
                                                                float* __restrict__ dd, int NT, int H, int* __restrict__ err) {
+  grid_wait();
   using namespace gdn;
   extern __shared__ __align__(1024) uint8_t scan_smem[];
   // STAGES x {w, P, qg, kg}, then per warp two pairs of slices {do, S} (a pair that has been read takes the outputs), then the barriers
@@ -143,7 +145,7 @@ std::vector<at::Tensor> gdn_chain_bwd(const at::Tensor& w, const at::Tensor& P, 
     constexpr int smem = gdn::STAGES * 4 * gdn::TILE_BYTES + W * 4 * gdn::SLICE_BYTES + 64;
     static bool configured = false;
     if (!configured) { C10_CUDA_CHECK(cudaFuncSetAttribute(gdn_chain_bwd_kernel<W>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem)); configured = true; }
-    gdn_chain_bwd_kernel<W><<<dim3((int)BH, 4 / W), 32 * W, smem, at::cuda::getCurrentCUDAStream()>>>(
+    q38::launch(gdn_chain_bwd_kernel<W>, dim3((int)BH, 4 / W), 32 * W, smem, at::cuda::getCurrentCUDAStream(), 
         maps, (const bf16*)dout.data_ptr(), (const bf16*)states.data_ptr(), dch.data_ptr<float>(), (bf16*)du.data_ptr(), (bf16*)dstate.data_ptr(),
         dd.data_ptr<float>(), (int)NT, (int)H, err.has_value() ? err->data_ptr<int>() : nullptr);
   };

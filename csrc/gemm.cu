@@ -21,6 +21,7 @@
 
 #include "ptx.cuh"
 #include "host.h"
+#include "launch.cuh"
 
 namespace q38 {
 
@@ -43,6 +44,7 @@ constexpr int gemm_smem_bytes() { return STAGES * (BM * 128 + BN * 128) + 1024 /
 template <int EB, int BN, bool A_MN, bool B_MN, typename OutT, bool ACCUM>
 __global__ void __launch_bounds__(GEMM_THREADS) gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA,
                                                                   const __grid_constant__ CUtensorMap tmB, GemmArgs p) {
+  grid_wait();
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw = ptx::smem_u32(smem_raw);
   uint8_t* smem = smem_raw + ((1024u - (raw & 1023u)) & 1023u);
@@ -266,7 +268,7 @@ static void launch(const CUtensorMap& ta, const CUtensorMap& tb, const GemmArgs&
     configured = true;
   }
   dim3 grid((p.N + BN - 1) / BN, (p.M + BM - 1) / BM, p.batch * p.splits);
-  kernel<<<grid, GEMM_THREADS, smem, stream>>>(ta, tb, p);
+  launch(kernel, grid, GEMM_THREADS, smem, stream, ta, tb, p);
   C10_CUDA_KERNEL_LAUNCH_CHECK();
   count_launch();
 }

@@ -20,6 +20,7 @@
 
 #include "ptx.cuh"
 #include "host.h"
+#include "launch.cuh"
 
 namespace q38 {
 
@@ -111,6 +112,7 @@ __global__ void __launch_bounds__(G2_THREADS) gemm_pair_kernel(const __grid_cons
   ptx2::cluster_sync();                              // the peer's barriers are initialised before anything of ours can reach them
   ptx::tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  grid_wait();
 
   auto decode = [&](int w, int& bz, int& m0, int& n0) {
     const int tn = w % p.tiles_n; w /= p.tiles_n;
@@ -279,15 +281,17 @@ bool gemm_bf16_pair(const Mat& a, const Mat& b, const Mat& c, double alpha, bool
   const int clusters = std::max(1, std::min(p.work_items, kNumSMs / 2));
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(2 * clusters); cfg.blockDim = dim3(G2_THREADS); cfg.dynamicSmemBytes = smem; cfg.stream = at::cuda::getCurrentCUDAStream();
-  cudaLaunchAttribute attr[1];
+  cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeClusterDimension;
   attr[0].val.clusterDim.x = 2; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
-  cfg.attrs = attr; cfg.numAttrs = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr; cfg.numAttrs = 2;
   // The number of clusters that can be resident at once (pairs must sit in one TPC) bounds the grid: with a static walk over the
   // tiles, clusters beyond it would run as a second wave.
 #define Q38_PAIR(OutT, ACC) { auto k = gemm_pair_kernel<OutT, ACC>; static int resident = 0; \
     if (!resident) { C10_CUDA_CHECK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024)); \
-      cudaLaunchConfig_t probe = cfg; probe.gridDim = dim3(kNumSMs); probe.dynamicSmemBytes = 227 * 1024 - 1024; int n = 0; \
+      cudaLaunchConfig_t probe = cfg; probe.numAttrs = 1; probe.gridDim = dim3(kNumSMs); probe.dynamicSmemBytes = 227 * 1024 - 1024; int n = 0; \
       if (cudaOccupancyMaxActiveClusters(&n, k, &probe) != cudaSuccess || n < 1) { (void)cudaGetLastError(); n = kNumSMs / 2; } \
       resident = n; if (std::getenv("Q38_GEMM_TRACE")) std::fprintf(stderr, "[gemm_pair] resident clusters %d\n", n); } \
     cfg.gridDim = dim3(2 * std::max(1, std::min(p.work_items, resident))); \

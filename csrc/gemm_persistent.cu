@@ -16,6 +16,7 @@
 
 #include "ptx.cuh"
 #include "host.h"
+#include "launch.cuh"
 
 namespace q38 {
 
@@ -67,6 +68,7 @@ __global__ void __launch_bounds__(P_THREADS) gemm_persistent_kernel(const __grid
   __syncthreads();
   ptx::tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  grid_wait();
 
   // work item -> (batch, m tile, n tile, split); n fastest so consecutive items reuse the A tile from L2
   auto decode = [&](int w, int& bz, int& m0, int& n0, int& kb_begin, int& num_kb) {
@@ -313,7 +315,7 @@ static void launch_p(const CUtensorMap& ta, const CUtensorMap& tb, const CUtenso
             p.total_kb, (int)tma_out, (int)out_fp32, (int)accum, (int)A_MN, (int)B_MN);
 #define Q38_LAUNCH(OutT, ACC, TMAO) { auto k = gemm_persistent_kernel<A_MN, B_MN, OutT, ACC, TMAO, TF32>; static bool cfg = false; \
     if (!cfg) { C10_CUDA_CHECK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024)); cfg = true; } \
-    k<<<grid, P_THREADS, smem, stream>>>(ta, tb, tc, p); }
+    launch(k, grid, P_THREADS, smem, stream, ta, tb, tc, p); }
   if constexpr (TF32) {
     if (!out_fp32) { if (tma_out) Q38_LAUNCH(__nv_bfloat16, false, true) else Q38_LAUNCH(__nv_bfloat16, false, false) }
     else if (tma_out) { if (accum) Q38_LAUNCH(float, true, true) else Q38_LAUNCH(float, false, true) }

@@ -17,6 +17,7 @@
 
 #include "common.cuh"
 #include "host.h"
+#include "launch.cuh"
 
 namespace q38 {
 
@@ -77,6 +78,7 @@ template <int GS, int KS, typename F> __device__ __forceinline__ void sinkhorn_h
 
 // coef[t, 8..24): logits in, doubly normalised residual mix out.
 __global__ void __launch_bounds__(SK) mhc_sinkhorn_fwd_kernel(float* __restrict__ coef, int T, int iters) {
+  grid_wait();
   const int t = blockIdx.x * SK + threadIdx.x;
   if (t >= T) return;
   float4* row = reinterpret_cast<float4*>(coef + (size_t)t * NCOEF + 8);
@@ -96,6 +98,7 @@ __global__ void __launch_bounds__(SK) mhc_sinkhorn_fwd_kernel(float* __restrict_
 // every y is the one of the forward.  Going back by p *= s from the divisors alone takes 20 KB instead of 40 and rounds p forty times more: the
 // gradient of a token was then 25 to 35 % further from the 64-bit one (2.2e-7 instead of 1.8e-7 for logits of unit spread).
 __global__ void __launch_bounds__(SK) mhc_sinkhorn_bwd_kernel(const float* __restrict__ zsave, MhcParams P, float* __restrict__ dcoef, int T, int iters) {
+  grid_wait();
   extern __shared__ float iterates[];        // [iters][16][SK]
   const int t = blockIdx.x * SK + threadIdx.x;
   if (t >= T) return;
@@ -169,6 +172,7 @@ __global__ void __launch_bounds__(32 * WARPS) mhc_coef_fwd_kernel(const float* _
                                                                   float* __restrict__ coef, float* __restrict__ zsave,
                                                                   float* __restrict__ inv_save, float* __restrict__ rstd_save, int T, int h,
                                                                   int r, int iters, float norm_eps) {
+  grid_wait();
   extern __shared__ float sm[];
   float* Bs = sm;                               // [24 * r]
   float* xin_s = sm + NCOEF * r;                // [WARPS * h]
@@ -228,6 +232,7 @@ __global__ void __launch_bounds__(32 * WARPS) mhc_coef_fwd_kernel(const float* _
 template <typename YT>
 __global__ void __launch_bounds__(256) mhc_post_fwd_kernel(const float* __restrict__ X, const YT* __restrict__ y,
                                                            const float* __restrict__ coef, float* __restrict__ Xout, int T, int h) {
+  grid_wait();
   const int h4 = h >> 2;
   const size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= (size_t)T * h4) return;
@@ -261,6 +266,7 @@ template <typename YT>
 __global__ void __launch_bounds__(32 * WARPS) mhc_post_bwd_kernel(const float* __restrict__ dXo, const float* __restrict__ X,
                                                                   const YT* __restrict__ y, const float* __restrict__ coef,
                                                                   YT* __restrict__ dy, float* __restrict__ dcoef, int T, int h) {
+  grid_wait();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int t = blockIdx.x * WARPS + warp;
   if (t >= T) return;
@@ -306,6 +312,7 @@ __global__ void __launch_bounds__(32 * WARPS) mhc_pre_bwd_a_kernel(const GT* __r
                                                                    float* __restrict__ dcoef, float* __restrict__ dLraw, float* __restrict__ c1_out,
                                                                    float* __restrict__ dxin_out, float* __restrict__ dBw, float* __restrict__ dbias,
                                                                    float* __restrict__ dnorm_w, int T, int h, int r, int iters) {
+  grid_wait();
   extern __shared__ float sm[];
   float* Bs = sm;                      // [24 * r]
   float* dB_s = Bs + NCOEF * r;        // [24 * r]   CTA-level accumulation of dB
@@ -409,6 +416,7 @@ template <typename GT>
 __global__ void __launch_bounds__(256) mhc_pre_bwd_c_kernel(float* __restrict__ dX, const GT* __restrict__ G, const float* __restrict__ dXo,
                                                             const float* __restrict__ X, const float* __restrict__ dxin, const float* __restrict__ coef,
                                                             const float* __restrict__ c1, int T, int h) {
+  grid_wait();
   const int h4 = h >> 2;
   const size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= (size_t)T * h4) return;
@@ -484,6 +492,7 @@ __global__ void __launch_bounds__(32 * RW, 4) mhc_coef_fwd_rows_kernel(const flo
                                                                        float* __restrict__ coef, float* __restrict__ zsave,
                                                                        float* __restrict__ inv_save, float* __restrict__ rstd_save, int T, int h,
                                                                        int r, float norm_eps) {
+  grid_wait();
   extern __shared__ float sm[];
   const int RP = r + 1;
   float* Bs = sm;                               // [24][r + 1]
@@ -558,6 +567,7 @@ __global__ void __launch_bounds__(32 * RW, 3) mhc_pre_bwd_rows_kernel(const GT* 
                                                                       const float* __restrict__ rstd_save, float* __restrict__ dcoef,
                                                                       float* __restrict__ dxin_out, float* __restrict__ dnorm_w,
                                                                       __nv_bfloat16* __restrict__ xbf, int T, int h) {
+  grid_wait();
   extern __shared__ float sm[];
   float* dnw_s = sm;                   // [h]
   for (int i = threadIdx.x; i < h; i += blockDim.x) dnw_s[i] = 0.f;
@@ -636,6 +646,7 @@ __global__ void __launch_bounds__(32 * CW) mhc_coef_bwd_kernel(const float* __re
                                                                const float* __restrict__ zsave, const float* __restrict__ inv_save,
                                                                const float* __restrict__ dcoef, float* __restrict__ dLraw, float* __restrict__ c1_out,
                                                                float* __restrict__ dlin_out, float* __restrict__ dbias, int T, int h, int r) {
+  grid_wait();
   extern __shared__ float sm[];
   const int RP = r + 1;
   float* Bs = sm;                      // [24][r + 1]
@@ -688,6 +699,7 @@ __global__ void __launch_bounds__(32 * CW) mhc_coef_bwd_kernel(const float* __re
 constexpr int DB_TOK = 64;
 __global__ void __launch_bounds__(256) mhc_dB_kernel(const float* __restrict__ dlin, const float* __restrict__ Lraw, const float* __restrict__ inv,
                                                      float* __restrict__ dBw, int T, int r) {
+  grid_wait();
   extern __shared__ float sm[];
   float* dl_s = sm;                    // [DB_TOK][24]
   float* l_s = sm + DB_TOK * NCOEF;    // [DB_TOK][r]
@@ -725,14 +737,14 @@ std::vector<at::Tensor> mhc_coef_fwd(const at::Tensor& X, const at::Tensor& Lraw
   if (r <= 96 && nq <= 8) {
     const size_t smem = NCOEF * (r + 1) * sizeof(float);
     const int grid = std::min((T + RW - 1) / RW, 4 * kNumSMs);
-#define Q38_ROWS(OutT, NQ) mhc_coef_fwd_rows_kernel<OutT, NQ><<<grid, 32 * RW, smem, stream>>>(X.data_ptr<float>(), Lraw.data_ptr<float>(), P, norm_w.data_ptr<float>(), \
+#define Q38_ROWS(OutT, NQ) launch(mhc_coef_fwd_rows_kernel<OutT, NQ>, grid, 32 * RW, smem, stream, X.data_ptr<float>(), Lraw.data_ptr<float>(), P, norm_w.data_ptr<float>(), \
       (OutT*)xout.data_ptr(), coef.data_ptr<float>(), z.data_ptr<float>(), inv.data_ptr<float>(), rstd.data_ptr<float>(), T, h, r, (float)norm_eps)
 #define Q38_ROWS_NQ(OutT) switch (nq) { case 1: Q38_ROWS(OutT, 1); break; case 2: Q38_ROWS(OutT, 2); break; case 3: Q38_ROWS(OutT, 3); break; case 4: Q38_ROWS(OutT, 4); break; \
       case 5: Q38_ROWS(OutT, 5); break; case 6: Q38_ROWS(OutT, 6); break; default: Q38_ROWS(OutT, 8); break; }
     if (out_bf16) Q38_ROWS_NQ(__nv_bfloat16) else Q38_ROWS_NQ(float)
 #undef Q38_ROWS_NQ
 #undef Q38_ROWS
-    mhc_sinkhorn_fwd_kernel<<<(T + SK - 1) / SK, SK, 0, stream>>>(coef.data_ptr<float>(), T, (int)iters);
+    launch(mhc_sinkhorn_fwd_kernel, (T + SK - 1) / SK, SK, 0, stream, coef.data_ptr<float>(), T, (int)iters);
     C10_CUDA_KERNEL_LAUNCH_CHECK();
     count_launch(2);
     return {xout, coef, z, inv, rstd};
@@ -742,12 +754,12 @@ std::vector<at::Tensor> mhc_coef_fwd(const at::Tensor& X, const at::Tensor& Lraw
   if (out_bf16) {
     auto k = mhc_coef_fwd_kernel<__nv_bfloat16>;
     C10_CUDA_CHECK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024));
-    k<<<grid, 32 * WARPS, smem, stream>>>(X.data_ptr<float>(), Lraw.data_ptr<float>(), P, norm_w.data_ptr<float>(), (__nv_bfloat16*)xout.data_ptr(),
+    launch(k, grid, 32 * WARPS, smem, stream, X.data_ptr<float>(), Lraw.data_ptr<float>(), P, norm_w.data_ptr<float>(), (__nv_bfloat16*)xout.data_ptr(),
                                           coef.data_ptr<float>(), z.data_ptr<float>(), inv.data_ptr<float>(), rstd.data_ptr<float>(), T, h, r, (int)iters, (float)norm_eps);
   } else {
     auto k = mhc_coef_fwd_kernel<float>;
     C10_CUDA_CHECK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024));
-    k<<<grid, 32 * WARPS, smem, stream>>>(X.data_ptr<float>(), Lraw.data_ptr<float>(), P, norm_w.data_ptr<float>(), xout.data_ptr<float>(),
+    launch(k, grid, 32 * WARPS, smem, stream, X.data_ptr<float>(), Lraw.data_ptr<float>(), P, norm_w.data_ptr<float>(), xout.data_ptr<float>(),
                                           coef.data_ptr<float>(), z.data_ptr<float>(), inv.data_ptr<float>(), rstd.data_ptr<float>(), T, h, r, (int)iters, (float)norm_eps);
   }
   C10_CUDA_KERNEL_LAUNCH_CHECK();
@@ -764,9 +776,9 @@ at::Tensor mhc_post_fwd(const at::Tensor& X, const at::Tensor& y, const at::Tens
   const size_t n = (size_t)T * (h / 4);
   auto stream = at::cuda::getCurrentCUDAStream();
   if (y.scalar_type() == at::kBFloat16)
-    mhc_post_fwd_kernel<__nv_bfloat16><<<(n + 255) / 256, 256, 0, stream>>>(X.data_ptr<float>(), (const __nv_bfloat16*)y.data_ptr(), coef.data_ptr<float>(), out.data_ptr<float>(), T, h);
+    launch(mhc_post_fwd_kernel<__nv_bfloat16>, (n + 255) / 256, 256, 0, stream, X.data_ptr<float>(), (const __nv_bfloat16*)y.data_ptr(), coef.data_ptr<float>(), out.data_ptr<float>(), T, h);
   else
-    mhc_post_fwd_kernel<float><<<(n + 255) / 256, 256, 0, stream>>>(X.data_ptr<float>(), y.data_ptr<float>(), coef.data_ptr<float>(), out.data_ptr<float>(), T, h);
+    launch(mhc_post_fwd_kernel<float>, (n + 255) / 256, 256, 0, stream, X.data_ptr<float>(), y.data_ptr<float>(), coef.data_ptr<float>(), out.data_ptr<float>(), T, h);
   C10_CUDA_KERNEL_LAUNCH_CHECK();
   count_launch();
   return out;
@@ -781,10 +793,10 @@ std::vector<at::Tensor> mhc_post_bwd(const at::Tensor& dXo, const at::Tensor& X,
   auto stream = at::cuda::getCurrentCUDAStream();
   const int grid = (T + WARPS - 1) / WARPS;
   if (y.scalar_type() == at::kBFloat16)
-    mhc_post_bwd_kernel<__nv_bfloat16><<<grid, 32 * WARPS, 0, stream>>>(dXo.data_ptr<float>(), X.data_ptr<float>(), (const __nv_bfloat16*)y.data_ptr(),
+    launch(mhc_post_bwd_kernel<__nv_bfloat16>, grid, 32 * WARPS, 0, stream, dXo.data_ptr<float>(), X.data_ptr<float>(), (const __nv_bfloat16*)y.data_ptr(),
                                                                         coef.data_ptr<float>(), (__nv_bfloat16*)dy.data_ptr(), dcoef.data_ptr<float>(), T, h);
   else
-    mhc_post_bwd_kernel<float><<<grid, 32 * WARPS, 0, stream>>>(dXo.data_ptr<float>(), X.data_ptr<float>(), y.data_ptr<float>(), coef.data_ptr<float>(),
+    launch(mhc_post_bwd_kernel<float>, grid, 32 * WARPS, 0, stream, dXo.data_ptr<float>(), X.data_ptr<float>(), y.data_ptr<float>(), coef.data_ptr<float>(),
                                                                 dy.data_ptr<float>(), dcoef.data_ptr<float>(), T, h);
   C10_CUDA_KERNEL_LAUNCH_CHECK();
   count_launch();
@@ -812,7 +824,7 @@ std::vector<at::Tensor> mhc_pre_bwd_a(const at::Tensor& dxout, const at::Tensor&
     auto dlin = at::empty({T, NCOEF}, f32);
     auto xbf = at::empty({T, NB * h}, f32.dtype(at::kBFloat16));
     const int grid_r = std::min((T + RW - 1) / RW, 3 * kNumSMs);
-#define Q38_ROWS(GT, NQ) mhc_pre_bwd_rows_kernel<GT, NQ><<<grid_r, 32 * RW, h * sizeof(float), stream>>>((const GT*)dxout.data_ptr(), X.data_ptr<float>(), \
+#define Q38_ROWS(GT, NQ) launch(mhc_pre_bwd_rows_kernel<GT, NQ>, grid_r, 32 * RW, h * sizeof(float), stream, (const GT*)dxout.data_ptr(), X.data_ptr<float>(), \
       norm_w.data_ptr<float>(), coef.data_ptr<float>(), rstd.data_ptr<float>(), dcoef.data_ptr<float>(), dxin.data_ptr<float>(), dnw.data_ptr<float>(), \
       (__nv_bfloat16*)xbf.data_ptr(), T, h)
 #define Q38_ROWS_NQ(GT) switch (nq) { case 1: Q38_ROWS(GT, 1); break; case 2: Q38_ROWS(GT, 2); break; case 3: Q38_ROWS(GT, 3); break; case 4: Q38_ROWS(GT, 4); break; \
@@ -827,15 +839,15 @@ std::vector<at::Tensor> mhc_pre_bwd_a(const at::Tensor& dxout, const at::Tensor&
       C10_CUDA_CHECK(cudaFuncSetAttribute(mhc_sinkhorn_bwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 16 * SK * MAX_SINKHORN * (int)sizeof(float)));
       configured = true;
     }
-    mhc_sinkhorn_bwd_kernel<<<(T + SK - 1) / SK, SK, 16 * SK * iters * sizeof(float), stream>>>(z.data_ptr<float>(), P, dcoef.data_ptr<float>(), T, (int)iters);
+    launch(mhc_sinkhorn_bwd_kernel, (T + SK - 1) / SK, SK, 16 * SK * iters * sizeof(float), stream, z.data_ptr<float>(), P, dcoef.data_ptr<float>(), T, (int)iters);
     C10_CUDA_KERNEL_LAUNCH_CHECK();
     count_launch();
-    mhc_coef_bwd_kernel<<<std::min((T + CW - 1) / CW, 8 * kNumSMs), 32 * CW, (NCOEF * (r + 1) + 32) * sizeof(float), stream>>>(
+    launch(mhc_coef_bwd_kernel, std::min((T + CW - 1) / CW, 8 * kNumSMs), 32 * CW, (NCOEF * (r + 1) + 32) * sizeof(float), stream, 
         Lraw.data_ptr<float>(), P, coef.data_ptr<float>(), z.data_ptr<float>(), inv.data_ptr<float>(), dcoef.data_ptr<float>(), dLraw.data_ptr<float>(),
         c1.data_ptr<float>(), dlin.data_ptr<float>(), dbias.data_ptr<float>(), T, h, r);
     C10_CUDA_KERNEL_LAUNCH_CHECK();
     count_launch();
-    mhc_dB_kernel<<<(T + DB_TOK - 1) / DB_TOK, 256, DB_TOK * (NCOEF + r) * sizeof(float), stream>>>(dlin.data_ptr<float>(), Lraw.data_ptr<float>(), inv.data_ptr<float>(),
+    launch(mhc_dB_kernel, (T + DB_TOK - 1) / DB_TOK, 256, DB_TOK * (NCOEF + r) * sizeof(float), stream, dlin.data_ptr<float>(), Lraw.data_ptr<float>(), inv.data_ptr<float>(),
                                                                                                   dBw.data_ptr<float>(), T, r);
     C10_CUDA_KERNEL_LAUNCH_CHECK();
     count_launch();
@@ -845,7 +857,7 @@ std::vector<at::Tensor> mhc_pre_bwd_a(const at::Tensor& dxout, const at::Tensor&
   const int grid = (T + WARPS - 1) / WARPS;
 #define LAUNCH(GT) { auto k = mhc_pre_bwd_a_kernel<GT>; \
     C10_CUDA_CHECK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024)); \
-    k<<<grid, 32 * WARPS, smem, stream>>>((const GT*)dxout.data_ptr(), X.data_ptr<float>(), Lraw.data_ptr<float>(), P, norm_w.data_ptr<float>(), \
+    launch(k, grid, 32 * WARPS, smem, stream, (const GT*)dxout.data_ptr(), X.data_ptr<float>(), Lraw.data_ptr<float>(), P, norm_w.data_ptr<float>(), \
       coef.data_ptr<float>(), z.data_ptr<float>(), inv.data_ptr<float>(), rstd.data_ptr<float>(), dcoef.data_ptr<float>(), dLraw.data_ptr<float>(), \
       c1.data_ptr<float>(), dxin.data_ptr<float>(), dBw.data_ptr<float>(), dbias.data_ptr<float>(), dnw.data_ptr<float>(), T, h, r, (int)iters); }
   if (dxout.scalar_type() == at::kBFloat16) LAUNCH(__nv_bfloat16) else LAUNCH(float)
@@ -866,10 +878,10 @@ at::Tensor mhc_pre_bwd_c(const at::Tensor& G, const at::Tensor& dXo, const at::T
   const size_t n = (size_t)T * (h / 4);
   auto stream = at::cuda::getCurrentCUDAStream();
   if (G.scalar_type() == at::kFloat)
-    mhc_pre_bwd_c_kernel<float><<<(n + 255) / 256, 256, 0, stream>>>(dX.data_ptr<float>(), G.data_ptr<float>(), dXo.data_ptr<float>(), X.data_ptr<float>(),
+    launch(mhc_pre_bwd_c_kernel<float>, (n + 255) / 256, 256, 0, stream, dX.data_ptr<float>(), G.data_ptr<float>(), dXo.data_ptr<float>(), X.data_ptr<float>(),
                                                                      dxin.data_ptr<float>(), coef.data_ptr<float>(), c1.data_ptr<float>(), T, h);
   else
-    mhc_pre_bwd_c_kernel<__nv_bfloat16><<<(n + 255) / 256, 256, 0, stream>>>(dX.data_ptr<float>(), (const __nv_bfloat16*)G.data_ptr(), dXo.data_ptr<float>(),
+    launch(mhc_pre_bwd_c_kernel<__nv_bfloat16>, (n + 255) / 256, 256, 0, stream, dX.data_ptr<float>(), (const __nv_bfloat16*)G.data_ptr(), dXo.data_ptr<float>(),
                                                                              X.data_ptr<float>(), dxin.data_ptr<float>(), coef.data_ptr<float>(), c1.data_ptr<float>(), T, h);
   C10_CUDA_KERNEL_LAUNCH_CHECK();
   count_launch();

@@ -17,6 +17,7 @@
 
 #include "ptx.cuh"
 #include "host.h"
+#include "launch.cuh"
 #include "q38_noalloc.h"
 
 namespace q38 {
@@ -38,6 +39,7 @@ __global__ void __launch_bounds__(256) moe_route_fwd_kernel(const __nv_bfloat16*
                                                             float* __restrict__ top_w, int* __restrict__ top_idx,
                                                             float* __restrict__ probs_out, float* __restrict__ counts,
                                                             RouteSums* __restrict__ sums, float* __restrict__ prob_sum) {
+  grid_wait();
   __shared__ float s_ps[8][64];
   __shared__ unsigned int s_cnt[64];
   __shared__ bool last;
@@ -109,6 +111,7 @@ __global__ void __launch_bounds__(256) moe_route_bwd_kernel(const float* __restr
                                                             const float* __restrict__ top_w, const float* __restrict__ d_top_w,
                                                             const float* __restrict__ d_prob_sum, int T, int E, int K,
                                                             __nv_bfloat16* __restrict__ dlogits) {
+  grid_wait();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int t = blockIdx.x * 8 + warp;
   if (t >= T) return;
@@ -149,6 +152,7 @@ constexpr int SORT_THREADS = 256, SORT_ITERS = 4, SORT_CHUNK = SORT_THREADS * SO
 // inv_perm entry becomes -1 and the tail of perm stays unwritten) and ERR_BOUNDS is recorded when an error word is given.
 __global__ void __launch_bounds__(SORT_THREADS) moe_hist_kernel(const int* __restrict__ expert_of_pair, int P, int E, int* __restrict__ block_counts,
                                                                 int* __restrict__ err) {
+  grid_wait();
   __shared__ int cnt[64];
   if (threadIdx.x < 64) cnt[threadIdx.x] = 0;
   __syncthreads();
@@ -170,6 +174,7 @@ __global__ void __launch_bounds__(SORT_THREADS) moe_hist_kernel(const int* __res
 constexpr int SCAN_SEGS = 16;
 __global__ void __launch_bounds__(64 * SCAN_SEGS) moe_scan_kernel(int* __restrict__ block_counts, int nblocks, int E, int* __restrict__ offsets,
                                                                   int* __restrict__ sched, int max_tiles, int tile_rows) {
+  grid_wait();
   __shared__ int part[SCAN_SEGS][64], tot[64], off[65], tstart[65];
   const int e = threadIdx.x & 63, seg = threadIdx.x >> 6, lane = threadIdx.x & 31;
   const int per = (nblocks + SCAN_SEGS - 1) / SCAN_SEGS, b0 = min(seg * per, nblocks), b1 = min(b0 + per, nblocks);
@@ -219,6 +224,7 @@ __global__ void __launch_bounds__(64 * SCAN_SEGS) moe_scan_kernel(int* __restric
 
 __global__ void __launch_bounds__(SORT_THREADS) moe_scatter_kernel(const int* __restrict__ expert_of_pair, int P, int E,
                                                                    const int* __restrict__ block_base, int* __restrict__ perm, int* __restrict__ inv_perm) {
+  grid_wait();
   __shared__ int cursor[64];
   __shared__ int warp_cnt[SORT_THREADS / 32][64];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -257,6 +263,7 @@ __global__ void __launch_bounds__(SORT_THREADS) moe_scatter_kernel(const int* __
 // x_sorted[pos, :] = x[perm[pos] / k, :]   (one warp per sorted row, 16-byte copies; h % 8 == 0)
 __global__ void __launch_bounds__(256) moe_gather_kernel(const __nv_bfloat16* __restrict__ x, const int* __restrict__ perm, int P, int K, int h,
                                                          __nv_bfloat16* __restrict__ out) {
+  grid_wait();
   const int row = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (row >= P) return;
   const uint4* src = reinterpret_cast<const uint4*>(x + (size_t)(perm[row] / K) * h);
@@ -270,6 +277,7 @@ __global__ void __launch_bounds__(256) moe_gather_kernel(const __nv_bfloat16* __
 template <bool WEIGHTED>
 __global__ void __launch_bounds__(256) moe_slot_sum_kernel(const __nv_bfloat16* __restrict__ rows, const int* __restrict__ inv_perm, const float* __restrict__ top_w, int T, int K,
                                                            int pieces, __nv_bfloat16* __restrict__ out) {
+  grid_wait();
   const long long id = (long long)blockIdx.x * 256 + threadIdx.x;
   if (id >= (long long)T * pieces) return;
   const int t = (int)(id / pieces), i = (int)(id - (long long)t * pieces);
@@ -306,6 +314,7 @@ __global__ void __launch_bounds__(256) moe_slot_sum_kernel(const __nv_bfloat16* 
 __global__ void __launch_bounds__(256) moe_combine_fwd_kernel(const __nv_bfloat16* __restrict__ y_sorted, const int* __restrict__ inv_perm,
                                                               const float* __restrict__ top_w, int T, int K, int h,
                                                               __nv_bfloat16* __restrict__ out) {
+  grid_wait();
   const int t = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (t >= T) return;
   for (int i = lane; i < h / 2; i += 32) {
@@ -325,6 +334,7 @@ __global__ void __launch_bounds__(256) moe_combine_fwd_kernel(const __nv_bfloat1
 __global__ void __launch_bounds__(256) moe_combine_bwd_kernel(const __nv_bfloat16* __restrict__ dout, const __nv_bfloat16* __restrict__ y_sorted,
                                                               const int* __restrict__ inv_perm, const float* __restrict__ top_w, int T, int K, int h,
                                                               __nv_bfloat16* __restrict__ dy_sorted, float* __restrict__ d_top_w) {
+  grid_wait();
   const int pair = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (pair >= T * K) return;
   const int t = pair / K, pos = inv_perm[pair];
@@ -343,6 +353,7 @@ __global__ void __launch_bounds__(256) moe_combine_bwd_kernel(const __nv_bfloat1
 // dx[t,:] = sum_j dx_sorted[inv_perm[t*k+j], :]
 __global__ void __launch_bounds__(256) moe_unpermute_sum_kernel(const __nv_bfloat16* __restrict__ dx_sorted, const int* __restrict__ inv_perm,
                                                                 int T, int K, int h, __nv_bfloat16* __restrict__ dx) {
+  grid_wait();
   const int t = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (t >= T) return;
   for (int i = lane; i < h / 2; i += 32) {
@@ -395,6 +406,7 @@ struct GroupedArgs {
 template <int EPI, bool A_MN, bool B_MN>
 __global__ void __launch_bounds__(G_THREADS) grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                                                                  GroupedArgs p) {
+  grid_wait();
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw = ptx::smem_u32(smem_raw);
   uint8_t* smem = smem_raw + ((1024u - (raw & 1023u)) & 1023u);
@@ -657,7 +669,7 @@ static void launch_grouped(const CUtensorMap& ta, const CUtensorMap& tb, Grouped
   const int smem = p.stages * (G_BM * G_BK * 2 + nacc * p.bn_alloc * G_BK * 2) + 1024 + 256;
   static int configured = 0;
   if (configured < smem) { C10_CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024)); configured = 227 * 1024; }
-  kernel<<<grid, G_THREADS, smem, stream>>>(ta, tb, p);
+  launch(kernel, grid, G_THREADS, smem, stream, ta, tb, p);
   C10_CUDA_KERNEL_LAUNCH_CHECK();
   count_launch();
 }
@@ -771,7 +783,7 @@ std::vector<at::Tensor> moe_route_fwd(const at::Tensor& logits, int64_t k) {
   auto sums = at::zeros({(int64_t)sizeof(RouteSums)}, logits.options().dtype(at::kByte));
   auto counts = T ? at::empty({E}, f32) : at::zeros({E}, f32), psum = T ? at::empty({E}, f32) : at::zeros({E}, f32);
   auto top_idx = at::empty({T, k}, logits.options().dtype(at::kInt));
-  if (T) moe_route_fwd_kernel<<<(T + 7) / 8, 256, 0, at::cuda::getCurrentCUDAStream()>>>((const __nv_bfloat16*)logits.data_ptr(), T, E, (int)k, top_w.data_ptr<float>(),
+  if (T) launch(moe_route_fwd_kernel, (T + 7) / 8, 256, 0, at::cuda::getCurrentCUDAStream(), (const __nv_bfloat16*)logits.data_ptr(), T, E, (int)k, top_w.data_ptr<float>(),
       top_idx.data_ptr<int>(), probs.data_ptr<float>(), counts.data_ptr<float>(), reinterpret_cast<RouteSums*>(sums.data_ptr()), psum.data_ptr<float>());
   C10_CUDA_KERNEL_LAUNCH_CHECK();
   count_launch();
@@ -783,7 +795,7 @@ at::Tensor moe_route_bwd(const at::Tensor& probs, const at::Tensor& top_idx, con
   const c10::cuda::CUDAGuard guard(probs.device());
   const int T = probs.size(0), E = probs.size(1), k = top_idx.size(1);
   auto dlogits = at::empty({T, E}, probs.options().dtype(at::kBFloat16));
-  if (T) moe_route_bwd_kernel<<<(T + 7) / 8, 256, 0, at::cuda::getCurrentCUDAStream()>>>(probs.data_ptr<float>(), top_idx.data_ptr<int>(), top_w.data_ptr<float>(),
+  if (T) launch(moe_route_bwd_kernel, (T + 7) / 8, 256, 0, at::cuda::getCurrentCUDAStream(), probs.data_ptr<float>(), top_idx.data_ptr<int>(), top_w.data_ptr<float>(),
       d_top_w.data_ptr<float>(), d_prob_sum.has_value() ? d_prob_sum->data_ptr<float>() : nullptr, T, E, k, (__nv_bfloat16*)dlogits.data_ptr());
   C10_CUDA_KERNEL_LAUNCH_CHECK();
   count_launch();
@@ -801,10 +813,10 @@ std::vector<at::Tensor> moe_sort(const at::Tensor& top_idx, int64_t E, const c10
   auto block_counts = at::empty({std::max(nblocks, 1) * (int)E}, i32), perm = at::empty({P}, i32), inv = at::empty({P}, i32);
   auto offsets = at::empty({(int)E + 1}, i32), sched = at::empty({1 + 3 * max_tiles}, i32);
   auto stream = at::cuda::getCurrentCUDAStream();
-  if (nblocks) moe_hist_kernel<<<nblocks, SORT_THREADS, 0, stream>>>(top_idx.data_ptr<int>(), P, (int)E, block_counts.data_ptr<int>(),
+  if (nblocks) launch(moe_hist_kernel, nblocks, SORT_THREADS, 0, stream, top_idx.data_ptr<int>(), P, (int)E, block_counts.data_ptr<int>(),
                                                                      err.has_value() ? err->data_ptr<int>() : nullptr);
-  moe_scan_kernel<<<1, 64 * SCAN_SEGS, 0, stream>>>(block_counts.data_ptr<int>(), nblocks, (int)E, offsets.data_ptr<int>(), sched.data_ptr<int>(), max_tiles, G_BM);
-  if (nblocks) moe_scatter_kernel<<<nblocks, SORT_THREADS, 0, stream>>>(top_idx.data_ptr<int>(), P, (int)E, block_counts.data_ptr<int>(), perm.data_ptr<int>(), inv.data_ptr<int>());
+  launch(moe_scan_kernel, 1, 64 * SCAN_SEGS, 0, stream, block_counts.data_ptr<int>(), nblocks, (int)E, offsets.data_ptr<int>(), sched.data_ptr<int>(), max_tiles, G_BM);
+  if (nblocks) launch(moe_scatter_kernel, nblocks, SORT_THREADS, 0, stream, top_idx.data_ptr<int>(), P, (int)E, block_counts.data_ptr<int>(), perm.data_ptr<int>(), inv.data_ptr<int>());
   C10_CUDA_KERNEL_LAUNCH_CHECK();
   count_launch(3);
   return {perm, inv, offsets, sched};
@@ -816,7 +828,7 @@ at::Tensor moe_gather(const at::Tensor& x, const at::Tensor& perm, int64_t k) {
   const int P = perm.numel(), h = x.size(1);
   TORCH_CHECK(h % 8 == 0, "moe_gather: hidden size must be a multiple of 8");
   auto out = at::empty({P, h}, x.options());
-  if (P) moe_gather_kernel<<<(P + 7) / 8, 256, 0, at::cuda::getCurrentCUDAStream()>>>((const __nv_bfloat16*)x.data_ptr(), perm.data_ptr<int>(), P, (int)k, h, (__nv_bfloat16*)out.data_ptr());
+  if (P) launch(moe_gather_kernel, (P + 7) / 8, 256, 0, at::cuda::getCurrentCUDAStream(), (const __nv_bfloat16*)x.data_ptr(), perm.data_ptr<int>(), P, (int)k, h, (__nv_bfloat16*)out.data_ptr());
   C10_CUDA_KERNEL_LAUNCH_CHECK();
   count_launch();
   return out;
@@ -834,9 +846,9 @@ at::Tensor moe_combine_fwd(const at::Tensor& y_sorted, const at::Tensor& inv_per
   const int T = top_w.size(0), k = top_w.size(1), h = y_sorted.size(1);
   auto out = at::empty({T, h}, y_sorted.options());
   if (T && row_pieces(h, k, {y_sorted.data_ptr(), out.data_ptr()}))
-    moe_slot_sum_kernel<true><<<(unsigned)(((long long)T * (h / 8) + 255) / 256), 256, 0, at::cuda::getCurrentCUDAStream()>>>((const __nv_bfloat16*)y_sorted.data_ptr(),
+    launch(moe_slot_sum_kernel<true>, (unsigned)(((long long)T * (h / 8) + 255) / 256), 256, 0, at::cuda::getCurrentCUDAStream(), (const __nv_bfloat16*)y_sorted.data_ptr(),
         inv_perm.data_ptr<int>(), top_w.data_ptr<float>(), T, k, h / 8, (__nv_bfloat16*)out.data_ptr());
-  else if (T) moe_combine_fwd_kernel<<<(T + 7) / 8, 256, 0, at::cuda::getCurrentCUDAStream()>>>((const __nv_bfloat16*)y_sorted.data_ptr(), inv_perm.data_ptr<int>(),
+  else if (T) launch(moe_combine_fwd_kernel, (T + 7) / 8, 256, 0, at::cuda::getCurrentCUDAStream(), (const __nv_bfloat16*)y_sorted.data_ptr(), inv_perm.data_ptr<int>(),
       top_w.data_ptr<float>(), T, k, h, (__nv_bfloat16*)out.data_ptr());
   C10_CUDA_KERNEL_LAUNCH_CHECK();
   count_launch();
@@ -849,7 +861,7 @@ std::vector<at::Tensor> moe_combine_bwd(const at::Tensor& dout, const at::Tensor
   const int T = top_w.size(0), k = top_w.size(1), h = y_sorted.size(1);
   auto dy = at::empty_like(y_sorted);
   auto dw = at::empty({T, k}, top_w.options());
-  if (T) moe_combine_bwd_kernel<<<(T * k + 7) / 8, 256, 0, at::cuda::getCurrentCUDAStream()>>>((const __nv_bfloat16*)dout.data_ptr(), (const __nv_bfloat16*)y_sorted.data_ptr(),
+  if (T) launch(moe_combine_bwd_kernel, (T * k + 7) / 8, 256, 0, at::cuda::getCurrentCUDAStream(), (const __nv_bfloat16*)dout.data_ptr(), (const __nv_bfloat16*)y_sorted.data_ptr(),
       inv_perm.data_ptr<int>(), top_w.data_ptr<float>(), T, k, h, (__nv_bfloat16*)dy.data_ptr(), dw.data_ptr<float>());
   C10_CUDA_KERNEL_LAUNCH_CHECK();
   count_launch();
@@ -862,9 +874,9 @@ at::Tensor moe_unpermute_sum(const at::Tensor& dx_sorted, const at::Tensor& inv_
   const int h = dx_sorted.size(1);
   auto dx = at::empty({T, h}, dx_sorted.options());
   if (T && row_pieces(h, k, {dx_sorted.data_ptr(), dx.data_ptr()}))
-    moe_slot_sum_kernel<false><<<(unsigned)((T * (h / 8) + 255) / 256), 256, 0, at::cuda::getCurrentCUDAStream()>>>((const __nv_bfloat16*)dx_sorted.data_ptr(), inv_perm.data_ptr<int>(),
+    launch(moe_slot_sum_kernel<false>, (unsigned)((T * (h / 8) + 255) / 256), 256, 0, at::cuda::getCurrentCUDAStream(), (const __nv_bfloat16*)dx_sorted.data_ptr(), inv_perm.data_ptr<int>(),
         nullptr, (int)T, (int)k, h / 8, (__nv_bfloat16*)dx.data_ptr());
-  else if (T) moe_unpermute_sum_kernel<<<((int)T + 7) / 8, 256, 0, at::cuda::getCurrentCUDAStream()>>>((const __nv_bfloat16*)dx_sorted.data_ptr(), inv_perm.data_ptr<int>(), (int)T, (int)k, h,
+  else if (T) launch(moe_unpermute_sum_kernel, ((int)T + 7) / 8, 256, 0, at::cuda::getCurrentCUDAStream(), (const __nv_bfloat16*)dx_sorted.data_ptr(), inv_perm.data_ptr<int>(), (int)T, (int)k, h,
       (__nv_bfloat16*)dx.data_ptr());
   C10_CUDA_KERNEL_LAUNCH_CHECK();
   count_launch();
@@ -906,9 +918,9 @@ extern "C" int q38_moe_sort_static(const int* expert_of_pair, int P, int experts
   int* scratch = sort_static_scratch_for_current_device();
   if (scratch == nullptr) return Q38_NOALLOC_CUDA_ERROR;
   // Every word of the scratch that the scan and scatter kernels read is written by the histogram kernel first.
-  moe_hist_kernel<<<nblocks, SORT_THREADS, 0, stream>>>(expert_of_pair, P, experts, scratch, nullptr);
-  moe_scan_kernel<<<1, 64 * SCAN_SEGS, 0, stream>>>(scratch, nblocks, experts, offsets, sched, max_tiles, G_BM);
-  moe_scatter_kernel<<<nblocks, SORT_THREADS, 0, stream>>>(expert_of_pair, P, experts, scratch, perm, inv_perm);
+  launch(moe_hist_kernel, nblocks, SORT_THREADS, 0, stream, expert_of_pair, P, experts, scratch, nullptr);
+  launch(moe_scan_kernel, 1, 64 * SCAN_SEGS, 0, stream, scratch, nblocks, experts, offsets, sched, max_tiles, G_BM);
+  launch(moe_scatter_kernel, nblocks, SORT_THREADS, 0, stream, expert_of_pair, P, experts, scratch, perm, inv_perm);
   if (cudaGetLastError() != cudaSuccess) return Q38_NOALLOC_CUDA_ERROR;
   count_launch(3);
   return Q38_NOALLOC_OK;

@@ -23,6 +23,7 @@
 
 #include "ptx.cuh"
 #include "host.h"
+#include "launch.cuh"
 
 namespace q38 {
 
@@ -55,6 +56,7 @@ __device__ __forceinline__ void pg_store16(__nv_bfloat16* dst, const float (&v)[
 template <int EPI, bool B_MN, bool A_MN = false>
 __global__ void __launch_bounds__(PG_THREADS) grouped_persistent_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                                                                         PGroupedArgs p) {
+  grid_wait();
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw = ptx::smem_u32(smem_raw);
   uint8_t* smem = smem_raw + ((1024u - (raw & 1023u)) & 1023u);
@@ -379,7 +381,7 @@ static void pg_launch(const CUtensorMap& ta, const CUtensorMap& tb, PGroupedArgs
   static bool configured = false;
   if (!configured) { C10_CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024)); configured = true; }
   const int grid = std::max(1, std::min(max_tiles * p.tiles_n, kNumSMs));
-  kernel<<<grid, PG_THREADS, smem, stream>>>(ta, tb, p);
+  launch(kernel, grid, PG_THREADS, smem, stream, ta, tb, p);
   C10_CUDA_KERNEL_LAUNCH_CHECK();
   count_launch();
 }

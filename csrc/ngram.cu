@@ -15,6 +15,7 @@
 
 #include "common.cuh"
 #include "host.h"
+#include "launch.cuh"
 
 namespace q38 {
 
@@ -34,6 +35,7 @@ __global__ void __launch_bounds__(32 * NG_WARPS) ngram_fwd_kernel(const long lon
                                                                   const float* __restrict__ emb3, const float* __restrict__ norm_w,
                                                                   __nv_bfloat16* __restrict__ e, float* __restrict__ rstd_out, int* __restrict__ rows_out,
                                                                   int B, int T, int h, long long vocab, long long eos, long long rows, float eps) {
+  grid_wait();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const long long tok = (long long)blockIdx.x * NG_WARPS + warp;
   if (tok >= (long long)B * T) return;
@@ -71,6 +73,7 @@ __global__ void __launch_bounds__(32 * NG_WARPS) ngram_bwd_kernel(const __nv_bfl
                                                                   const float* __restrict__ norm_w, const float* __restrict__ rstd_in,
                                                                   float* __restrict__ g2, float* __restrict__ g3, float* __restrict__ dnorm_w,
                                                                   long long tokens, int h) {
+  grid_wait();
   extern __shared__ float dw_s[];                   // [h]
   for (int i = threadIdx.x; i < h; i += blockDim.x) dw_s[i] = 0.f;
   __syncthreads();
@@ -102,6 +105,7 @@ __global__ void __launch_bounds__(32 * NG_WARPS) ngram_bwd_kernel(const __nv_bfl
 // Token-embedding backward: grad[ids[t], :] += dout[t, :] with fp32 atomics, one warp per token.
 __global__ void __launch_bounds__(32 * NG_WARPS) embed_bwd_kernel(const long long* __restrict__ ids, const float* __restrict__ dout, float* __restrict__ grad,
                                                                   long long tokens, int h, long long vocab) {
+  grid_wait();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const long long tok = (long long)blockIdx.x * NG_WARPS + warp;
   if (tok >= tokens) return;
@@ -118,7 +122,7 @@ void embed_bwd(const at::Tensor& ids, const at::Tensor& dout, at::Tensor& grad) 
               "embed_bwd: int64 ids, fp32 gradient rows and an fp32 [vocab,h] gradient table required");
   const c10::cuda::CUDAGuard guard(ids.device());
   const long long tokens = ids.numel();
-  if (tokens) embed_bwd_kernel<<<(unsigned)((tokens + NG_WARPS - 1) / NG_WARPS), 32 * NG_WARPS, 0, at::cuda::getCurrentCUDAStream()>>>(
+  if (tokens) launch(embed_bwd_kernel, (unsigned)((tokens + NG_WARPS - 1) / NG_WARPS), 32 * NG_WARPS, 0, at::cuda::getCurrentCUDAStream(), 
       (const long long*)ids.data_ptr<int64_t>(), dout.data_ptr<float>(), grad.data_ptr<float>(), tokens, (int)grad.size(1), (long long)grad.size(0));
   C10_CUDA_KERNEL_LAUNCH_CHECK();
   count_launch();
@@ -137,7 +141,7 @@ std::vector<at::Tensor> ngram_fwd(const at::Tensor& ids, const at::Tensor& emb2,
   auto rstd = at::empty({B, T}, emb2.options());
   auto rows = at::empty({B, T, 2}, emb2.options().dtype(at::kInt));
   const long long tokens = (long long)B * T;
-  ngram_fwd_kernel<<<(unsigned)((tokens + NG_WARPS - 1) / NG_WARPS), 32 * NG_WARPS, 0, at::cuda::getCurrentCUDAStream()>>>(
+  launch(ngram_fwd_kernel, (unsigned)((tokens + NG_WARPS - 1) / NG_WARPS), 32 * NG_WARPS, 0, at::cuda::getCurrentCUDAStream(), 
       (const long long*)ids.data_ptr<int64_t>(), emb2.data_ptr<float>(), emb3.data_ptr<float>(), norm_w.data_ptr<float>(), (__nv_bfloat16*)e.data_ptr(),
       rstd.data_ptr<float>(), rows.data_ptr<int>(), B, T, h, (long long)vocab, (long long)eos, (long long)emb2.size(0), (float)eps);
   C10_CUDA_KERNEL_LAUNCH_CHECK();
@@ -155,7 +159,7 @@ at::Tensor ngram_bwd(const at::Tensor& de, const at::Tensor& rows, const at::Ten
   const int h = emb2.size(1);
   const long long tokens = de.numel() / h;
   auto dw = at::zeros({h}, emb2.options());
-  ngram_bwd_kernel<<<(unsigned)((tokens + NG_WARPS - 1) / NG_WARPS), 32 * NG_WARPS, h * sizeof(float), at::cuda::getCurrentCUDAStream()>>>(
+  launch(ngram_bwd_kernel, (unsigned)((tokens + NG_WARPS - 1) / NG_WARPS), 32 * NG_WARPS, h * sizeof(float), at::cuda::getCurrentCUDAStream(), 
       (const __nv_bfloat16*)de.data_ptr(), rows.data_ptr<int>(), emb2.data_ptr<float>(), emb3.data_ptr<float>(), norm_w.data_ptr<float>(), rstd.data_ptr<float>(),
       g2.data_ptr<float>(), g3.data_ptr<float>(), dw.data_ptr<float>(), tokens, h);
   C10_CUDA_KERNEL_LAUNCH_CHECK();

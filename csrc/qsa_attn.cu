@@ -11,6 +11,7 @@
 
 #include "f32x2.cuh"
 #include "host.h"
+#include "launch.cuh"
 #include "ptx.cuh"
 #include "qsa_blocks.cuh"
 
@@ -21,6 +22,7 @@ using bf16 = __nv_bfloat16;
 // sel[b, i, j] = 1 iff query block i attends key block j
 __global__ void qsa_selection_matrix_kernel(const int* __restrict__ count, const int* __restrict__ index, int kmax, int nb, int dense,
                                             unsigned char* __restrict__ sel) {
+  grid_wait();
   const int b = blockIdx.y, i = blockIdx.x;
   unsigned char* row = sel + ((long long)b * nb + i) * nb;
   for (int j = threadIdx.x; j < nb; j += blockDim.x) row[j] = dense ? (j <= i) : 0;
@@ -56,6 +58,7 @@ struct FwdArgs {
 
 __global__ void __launch_bounds__(AF_THREADS, 4) qsa_attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                                                                      const __grid_constant__ CUtensorMap tmV, FwdArgs p) {
+  grid_wait();
   extern __shared__ __align__(1024) uint8_t smem[];
   if (ptx::smem_u32(smem) & 1023u) { if (threadIdx.x == 0) report_error(p.err, ERR_BOUNDS); return; }
   uint8_t *q_tile = smem, *ring = smem + TILE_BYTES;                     // a ring stage is {K, V}
@@ -235,7 +238,7 @@ static at::Tensor selection_matrix(const c10::optional<at::Tensor>& count, const
   auto sel = at::empty({B, nb, nb}, opts.dtype(at::kByte));
   const bool dense = !count.has_value();
   if (!dense) TORCH_CHECK(count->scalar_type() == at::kInt && index->scalar_type() == at::kInt && count->is_contiguous() && index->is_contiguous(), "qsa: int32 block lists required");
-  qsa_selection_matrix_kernel<<<dim3(nb, B), 64, 0, stream>>>(dense ? nullptr : count->data_ptr<int>(), dense ? nullptr : index->data_ptr<int>(),
+  launch(qsa_selection_matrix_kernel, dim3(nb, B), 64, 0, stream, dense ? nullptr : count->data_ptr<int>(), dense ? nullptr : index->data_ptr<int>(),
                                                               dense ? 0 : (int)index->size(2), nb, dense ? 1 : 0, sel.data_ptr<unsigned char>());
   count_launch();
   return sel;
@@ -260,7 +263,7 @@ std::vector<at::Tensor> qsa_attn_fwd(const at::Tensor& q, const at::Tensor& k, c
   const int smem = (1 + AF_STAGES) * TILE_BYTES + 128 + list_bytes(nb);
   static bool cfg = false;
   if (!cfg) { allow_smem(qsa_attn_fwd_kernel); cfg = true; }
-  qsa_attn_fwd_kernel<<<dim3(B * nkv * ((nq / nkv + 1) / 2), nb), AF_THREADS, smem, stream>>>(tq, tk, tv, p);
+  launch(qsa_attn_fwd_kernel, dim3(B * nkv * ((nq / nkv + 1) / 2), nb), AF_THREADS, smem, stream, tq, tk, tv, p);
   C10_CUDA_KERNEL_LAUNCH_CHECK();
   count_launch();
   return {o, lse, sel};

@@ -22,6 +22,7 @@
 
 #include "f32x2.cuh"
 #include "host.h"
+#include "launch.cuh"
 #include "ptx.cuh"
 #include "qsa_blocks.cuh"
 
@@ -67,6 +68,7 @@ __device__ __forceinline__ void row_grads(const uint32_t (&s)[32], const uint32_
 
 __global__ void __launch_bounds__(AB_THREADS, 2) qsa_attn_bwd_q_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                                                                        const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmDO, BwdArgs p) {
+  grid_wait();
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = smem_raw + ((1024u - (ptx::smem_u32(smem_raw) & 1023u)) & 1023u);
   uint8_t *q_tile = smem, *do_tile = smem + TILE_BYTES, *ring = smem + 2 * TILE_BYTES;              // a ring stage is {K, V}
@@ -233,6 +235,7 @@ __global__ void __launch_bounds__(AB_THREADS, 2) qsa_attn_bwd_q_kernel(const __g
 
 __global__ void __launch_bounds__(AB_THREADS, 2) qsa_attn_bwd_kv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                                                                         const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmDO, BwdArgs p) {
+  grid_wait();
   extern __shared__ __align__(1024) uint8_t smem[];                     // without slack for the alignment two CTAs fit an SM
   if (ptx::smem_u32(smem) & 1023u) { if (threadIdx.x == 0) report_error(p.err, ERR_BOUNDS); return; }
   uint8_t *kv = smem, *ring = smem + TILE_BYTES, *pds = ring + KV_STAGES * 2 * TILE_BYTES;          // {K, V}; stages of {dO, Q}; {P, dS}
@@ -424,9 +427,9 @@ std::vector<at::Tensor> qsa_attn_bwd(const at::Tensor& q, const at::Tensor& k, c
   const int smem_q = (2 + Q_STAGES) * TILE_BYTES + 1024 + 256 + 1024 + list_bytes(nb), smem_kv = (1 + 2 * KV_STAGES + 2) * TILE_BYTES + 256 + list_bytes(nb);
   static bool cfg = false;
   if (!cfg) { allow_smem(qsa_attn_bwd_q_kernel); allow_smem(qsa_attn_bwd_kv_kernel); cfg = true; }
-  qsa_attn_bwd_q_kernel<<<dim3(B * nkv * ((rep + 1) / 2), nb), AB_THREADS, smem_q, stream>>>(tq, tk, tv, tdo, p);
+  launch(qsa_attn_bwd_q_kernel, dim3(B * nkv * ((rep + 1) / 2), nb), AB_THREADS, smem_q, stream, tq, tk, tv, tdo, p);
   C10_CUDA_KERNEL_LAUNCH_CHECK();
-  qsa_attn_bwd_kv_kernel<<<dim3(p.parts * nkv, nb, B), AB_THREADS, smem_kv, stream>>>(tq, tk, tv, tdo, p);
+  launch(qsa_attn_bwd_kv_kernel, dim3(p.parts * nkv, nb, B), AB_THREADS, smem_kv, stream, tq, tk, tv, tdo, p);
   C10_CUDA_KERNEL_LAUNCH_CHECK();
   count_launch(2);
   return {dq, dk32.to(at::kBFloat16), dv32.to(at::kBFloat16)};

@@ -11,6 +11,7 @@
 
 #include "common.cuh"
 #include "host.h"
+#include "launch.cuh"
 
 namespace q38 {
 
@@ -22,6 +23,7 @@ constexpr float QF_MASKED = -1e9f;
 __global__ void __launch_bounds__(QF_THREADS) qsa_first_query_lp_kernel(const __nv_bfloat16* __restrict__ q_first, const __nv_bfloat16* __restrict__ ki,
                                                                         const float* __restrict__ w_first, float* __restrict__ lp_blk, int S, int NI,
                                                                         float scale) {
+  grid_wait();
   extern __shared__ __align__(16) float qf_smem[];
   float* qs = qf_smem;                       // [NI][64]
   float* ws = qs + QF_HEADS_MAX * 64;        // [NI]
@@ -94,7 +96,7 @@ at::Tensor qsa_first_query_lp(const at::Tensor& q_first, const at::Tensor& ki, c
   const c10::cuda::CUDAGuard guard(q_first.device());
   auto lp = at::empty({B, nb, nb}, q_first.options().dtype(at::kFloat));
   const int smem = (QF_HEADS_MAX * 64 + 4 + 36 + S) * 4;
-  qsa_first_query_lp_kernel<<<dim3(nb, B), QF_THREADS, smem, at::cuda::getCurrentCUDAStream()>>>(
+  launch(qsa_first_query_lp_kernel, dim3(nb, B), QF_THREADS, smem, at::cuda::getCurrentCUDAStream(), 
       (const __nv_bfloat16*)q_first.data_ptr(), (const __nv_bfloat16*)ki.data_ptr(), w_first.data_ptr<float>(), lp.data_ptr<float>(), S, NI, (float)scale);
   C10_CUDA_KERNEL_LAUNCH_CHECK();
   count_launch();

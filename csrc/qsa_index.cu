@@ -16,6 +16,7 @@
 
 #include "common.cuh"
 #include "host.h"
+#include "launch.cuh"
 #include "mma_tile.cuh"
 
 namespace q38 {
@@ -57,6 +58,7 @@ __device__ __forceinline__ void frag_row_max_sum(const float (&acc)[8][4], bool 
 // grid (nb, nq, B).  stats[b, h, t, j] = (max, sumexp) of scale * q_h(t).k(s) over s in block j, s <= t.
 __global__ void __launch_bounds__(128) qsa_main_block_stats_kernel(const bf16* __restrict__ q, const bf16* __restrict__ k, float2* __restrict__ stats,
                                                                    int S, int nq, int nkv, float scale) {
+  grid_wait();
   extern __shared__ __align__(16) uint8_t smem_bytes[];
   bf16* Qs = reinterpret_cast<bf16*>(smem_bytes);
   bf16* Ks = Qs + TILE_ELEMS;                      // two buffers
@@ -96,6 +98,7 @@ __global__ void __launch_bounds__(128) qsa_main_block_stats_kernel(const bf16* _
 // The query fragments of all heads stay in registers, the next key block is fetched while the current one is scored, one barrier per block.
 __global__ void __launch_bounds__(128, 3) qsa_indexer_fwd_kernel(const bf16* __restrict__ qi, const bf16* __restrict__ ki, const float* __restrict__ wi,
                                                                  float* __restrict__ blse, int S, int NI, float scale) {
+  grid_wait();
   extern __shared__ __align__(16) uint8_t smem_bytes[];
   bf16* Qs = reinterpret_cast<bf16*>(smem_bytes);          // NI tiles
   bf16* Ks = Qs + NI_MAX * TILE_ELEMS;                     // two buffers
@@ -161,6 +164,7 @@ __global__ void __launch_bounds__(128, 3) qsa_indexer_fwd_kernel(const bf16* __r
 __global__ void __launch_bounds__(256) qsa_kl_combine_kernel(const float2* __restrict__ stats, const float* __restrict__ blse, float* __restrict__ P,
                                                              float* __restrict__ lp_blk, float* __restrict__ kl_tok, float* __restrict__ dblse,
                                                              int B, int S, int nq, int want_target) {
+  grid_wait();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const long long tok = (long long)blockIdx.x * 8 + warp;
   if (tok >= (long long)B * S) return;
@@ -220,6 +224,7 @@ __global__ void __launch_bounds__(256) qsa_kl_combine_kernel(const float2* __res
 // One warp per (batch, query block).  count[b, j] = min(j + 1, k); index[b, j, :k] sorted by decreasing score.
 __global__ void __launch_bounds__(256) qsa_select_kernel(const float* __restrict__ lp_blk, long long row_stride, int B, int nb, int K,
                                                          int* __restrict__ count, int* __restrict__ index) {
+  grid_wait();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int id = blockIdx.x * 8 + warp;
   if (id >= B * nb) return;
@@ -264,7 +269,7 @@ at::Tensor qsa_main_block_stats(const at::Tensor& q, const at::Tensor& k, double
   const int smem = 3 * TILE_ELEMS * 2;
   static bool cfg = false;
   if (!cfg) { C10_CUDA_CHECK(cudaFuncSetAttribute(qsa_main_block_stats_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem)); cfg = true; }
-  qsa_main_block_stats_kernel<<<dim3(nb, nq, B), 128, smem, at::cuda::getCurrentCUDAStream()>>>((const bf16*)q.data_ptr(), (const bf16*)k.data_ptr(),
+  launch(qsa_main_block_stats_kernel, dim3(nb, nq, B), 128, smem, at::cuda::getCurrentCUDAStream(), (const bf16*)q.data_ptr(), (const bf16*)k.data_ptr(),
       reinterpret_cast<float2*>(stats.data_ptr<float>()), S, nq, nkv, (float)scale);
   C10_CUDA_KERNEL_LAUNCH_CHECK();
   count_launch();
@@ -281,7 +286,7 @@ at::Tensor qsa_indexer_fwd(const at::Tensor& qi, const at::Tensor& ki, const at:
   const int smem = (NI_MAX + 2) * TILE_ELEMS * 2;
   static bool cfg = false;
   if (!cfg) { C10_CUDA_CHECK(cudaFuncSetAttribute(qsa_indexer_fwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem)); cfg = true; }
-  qsa_indexer_fwd_kernel<<<dim3(nb, B, std::min(nb, 4)), 128, smem, at::cuda::getCurrentCUDAStream()>>>((const bf16*)qi.data_ptr(), (const bf16*)ki.data_ptr(), wi.data_ptr<float>(),
+  launch(qsa_indexer_fwd_kernel, dim3(nb, B, std::min(nb, 4)), 128, smem, at::cuda::getCurrentCUDAStream(), (const bf16*)qi.data_ptr(), (const bf16*)ki.data_ptr(), wi.data_ptr<float>(),
       blse.data_ptr<float>(), S, NI, (float)scale);
   C10_CUDA_KERNEL_LAUNCH_CHECK();
   count_launch(2);
@@ -297,7 +302,7 @@ std::vector<at::Tensor> qsa_kl_combine(const c10::optional<at::Tensor>& stats, c
   auto opts = blse.options();
   auto P = at::empty({want ? B : 0, S, nb}, opts), lp = at::empty({B, S, nb}, opts), kl = at::empty({want ? B : 0, S}, opts), dbl = at::empty({want ? B : 0, S, nb}, opts);
   const long long tokens = (long long)B * S;
-  qsa_kl_combine_kernel<<<(unsigned)((tokens + 7) / 8), 256, 0, at::cuda::getCurrentCUDAStream()>>>(
+  launch(qsa_kl_combine_kernel, (unsigned)((tokens + 7) / 8), 256, 0, at::cuda::getCurrentCUDAStream(), 
       want ? reinterpret_cast<const float2*>(stats->data_ptr<float>()) : nullptr, blse.data_ptr<float>(), want ? P.data_ptr<float>() : nullptr,
       lp.data_ptr<float>(), want ? kl.data_ptr<float>() : nullptr, want ? dbl.data_ptr<float>() : nullptr, B, S, (int)nq, want ? 1 : 0);
   C10_CUDA_KERNEL_LAUNCH_CHECK();
@@ -315,7 +320,7 @@ std::vector<at::Tensor> qsa_select(const at::Tensor& lp_blk, int64_t budget) {
   auto i32 = lp_blk.options().dtype(at::kInt);
   auto count = at::empty({B, nb}, i32), index = at::empty({B, nb, k}, i32);
   const long long row_stride = (Q == nb) ? nb : (long long)64 * nb;
-  qsa_select_kernel<<<(B * nb + 7) / 8, 256, 0, at::cuda::getCurrentCUDAStream()>>>(lp_blk.data_ptr<float>(), row_stride, B, nb, (int)budget, count.data_ptr<int>(), index.data_ptr<int>());
+  launch(qsa_select_kernel, (B * nb + 7) / 8, 256, 0, at::cuda::getCurrentCUDAStream(), lp_blk.data_ptr<float>(), row_stride, B, nb, (int)budget, count.data_ptr<int>(), index.data_ptr<int>());
   C10_CUDA_KERNEL_LAUNCH_CHECK();
   count_launch();
   return {count, index};

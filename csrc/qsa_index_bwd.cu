@@ -28,6 +28,7 @@
 
 #include "f32x2.cuh"
 #include "host.h"
+#include "launch.cuh"
 #include "ptx.cuh"
 
 namespace q38 {
@@ -50,6 +51,7 @@ struct IndexBwdArgs {
 
 __global__ void __launch_bounds__(IB_THREADS, 1) qsa_indexer_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                                                                         const __grid_constant__ CUtensorMap tmDK, IndexBwdArgs p) {
+  grid_wait();
   extern __shared__ __align__(1024) uint8_t smem[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int nb = p.S / 64, i = nb - 1 - blockIdx.y, b = blockIdx.x / p.Z, z = blockIdx.x % p.Z;       // late query blocks (longest loops) of all sequences first
@@ -344,6 +346,7 @@ __global__ void __launch_bounds__(IB_THREADS, 1) qsa_indexer_bwd_kernel(const __
 // first of a row's eight threads also takes its head weight.
 __global__ void __launch_bounds__(256) qsa_indexer_sum_q_kernel(const float* __restrict__ part, const float* __restrict__ dw_part, __nv_bfloat16* __restrict__ dqi,
                                                                 float* __restrict__ dwi, int B, int NI, int S, int Z) {
+  grid_wait();
   const long long id = (long long)blockIdx.x * 256 + threadIdx.x, rows = (long long)B * NI * S, row = id >> 3;
   if (row >= rows) return;
   const int s = (int)(row % S), n = min((s / 64 + 2) / 2, Z);
@@ -396,11 +399,11 @@ std::vector<at::Tensor> qsa_indexer_bwd(const at::Tensor& qi, const at::Tensor& 
   static bool cfg = false;
   if (!cfg) { C10_CUDA_CHECK(cudaFuncSetAttribute(qsa_indexer_bwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, IB_SMEM)); cfg = true; }
   auto stream = at::cuda::getCurrentCUDAStream();
-  qsa_indexer_bwd_kernel<<<dim3(B * Z, nb), IB_THREADS, IB_SMEM, stream>>>(tq, tk, tdk, p);
+  launch(qsa_indexer_bwd_kernel, dim3(B * Z, nb), IB_THREADS, IB_SMEM, stream, tq, tk, tdk, p);
   C10_CUDA_KERNEL_LAUNCH_CHECK();
   count_launch();
   if (Z > 1) {
-    qsa_indexer_sum_q_kernel<<<(unsigned)(((long long)B * NI * S * 8 + 255) / 256), 256, 0, stream>>>(part.data_ptr<float>(), dw_part.data_ptr<float>(), (__nv_bfloat16*)dqi.data_ptr(),
+    launch(qsa_indexer_sum_q_kernel, (unsigned)(((long long)B * NI * S * 8 + 255) / 256), 256, 0, stream, part.data_ptr<float>(), dw_part.data_ptr<float>(), (__nv_bfloat16*)dqi.data_ptr(),
         dwi.data_ptr<float>(), B, NI, S, Z);
     C10_CUDA_KERNEL_LAUNCH_CHECK();
     count_launch();

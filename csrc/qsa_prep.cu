@@ -15,6 +15,7 @@
 
 #include "common.cuh"
 #include "host.h"
+#include "launch.cuh"
 
 namespace q38 {
 
@@ -50,6 +51,7 @@ __global__ void __launch_bounds__(32 * HP_WARPS) qsa_headprep_fwd_kernel(const b
                                                                          const float* __restrict__ cosv, const float* __restrict__ sinv, int Bc,
                                                                          bf16* __restrict__ out, bf16* __restrict__ gate, float* __restrict__ rstd_out,
                                                                          int S, int H, unsigned rows, float eps, bool round_products) {
+  grid_wait();
   const int lane = threadIdx.x & 31, m = lane & 7;
   float wv[8];
 #pragma unroll
@@ -103,6 +105,7 @@ __global__ void __launch_bounds__(32 * HP_WARPS) qsa_headprep_bwd_kernel(const b
                                                                          const float* __restrict__ cosv, const float* __restrict__ sinv, int Bc,
                                                                          const float* __restrict__ rstd_in, bf16* __restrict__ dsrc, float* __restrict__ dw,
                                                                          int S, int H, unsigned rows) {
+  grid_wait();
   __shared__ float dw_s[64];
   if (threadIdx.x < 64) dw_s[threadIdx.x] = 0.f;
   __syncthreads();
@@ -188,7 +191,7 @@ std::vector<at::Tensor> qsa_headprep_fwd(const at::Tensor& src_in, const c10::op
   auto rstd = at::empty({w.has_value() ? B : 0, S, H}, src.options().dtype(at::kFloat));
   const long long rows = (long long)B * S * H;
   TORCH_CHECK(rows < (1ll << 31), "qsa_headprep_fwd: too many rows");
-  qsa_headprep_fwd_kernel<<<headprep_grid(rows), 32 * HP_WARPS, 0, at::cuda::getCurrentCUDAStream()>>>(
+  launch(qsa_headprep_fwd_kernel, headprep_grid(rows), 32 * HP_WARPS, 0, at::cuda::getCurrentCUDAStream(), 
       (const bf16*)src.data_ptr(), (int)src.size(3), w.has_value() ? w->data_ptr<float>() : nullptr, cosv.data_ptr<float>(), sinv.data_ptr<float>(), (int)cosv.size(0),
       (bf16*)out.data_ptr(), split_gate ? (bf16*)gate.data_ptr() : nullptr, w.has_value() ? rstd.data_ptr<float>() : nullptr, S, H, (unsigned)rows, (float)eps, round_products);
   C10_CUDA_KERNEL_LAUNCH_CHECK();
@@ -213,7 +216,7 @@ std::vector<at::Tensor> qsa_headprep_bwd(const at::Tensor& dout_in, const c10::o
   auto dw = at::zeros({64}, src.options().dtype(at::kFloat));
   const long long rows = (long long)B * S * H;
   TORCH_CHECK(rows < (1ll << 31), "qsa_headprep_bwd: too many rows");
-  qsa_headprep_bwd_kernel<<<headprep_grid(rows), 32 * HP_WARPS, 0, at::cuda::getCurrentCUDAStream()>>>(
+  launch(qsa_headprep_bwd_kernel, headprep_grid(rows), 32 * HP_WARPS, 0, at::cuda::getCurrentCUDAStream(), 
       (const bf16*)dout.data_ptr(), split ? (const bf16*)dgate->data_ptr() : nullptr, (const bf16*)src.data_ptr(), (int)src.size(3),
       w.has_value() ? w->data_ptr<float>() : nullptr, cosv.data_ptr<float>(), sinv.data_ptr<float>(), (int)cosv.size(0),
       w.has_value() ? rstd.data_ptr<float>() : nullptr, (bf16*)dsrc.data_ptr(), dw.data_ptr<float>(), S, H, (unsigned)rows);

@@ -18,6 +18,7 @@
 
 #include "ptx.cuh"
 #include "host.h"
+#include "launch.cuh"
 
 namespace q38 {
 
@@ -37,6 +38,7 @@ __device__ __forceinline__ float fast_exp2(float x) {
 }
 
 __global__ void __launch_bounds__(QT_THREADS, 2) qsa_block_stats_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK, QsaTcArgs p) {
+  grid_wait();
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw = ptx::smem_u32(smem_raw);
   uint8_t* smem = smem_raw + ((1024u - (raw & 1023u)) & 1023u);
@@ -173,7 +175,7 @@ at::Tensor qsa_block_stats_tc(const at::Tensor& q, const at::Tensor& k, double s
   const int smem = QT_ROWS * 128 + QT_STAGES * QT_KEYS * 128 + 1024 + 256;
   static bool configured = false;
   if (!configured) { C10_CUDA_CHECK(cudaFuncSetAttribute(qsa_block_stats_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem)); configured = true; }
-  qsa_block_stats_tc_kernel<<<dim3(S / QT_ROWS, nq, B), QT_THREADS, smem, at::cuda::getCurrentCUDAStream()>>>(tq, tk, p);
+  launch(qsa_block_stats_tc_kernel, dim3(S / QT_ROWS, nq, B), QT_THREADS, smem, at::cuda::getCurrentCUDAStream(), tq, tk, p);
   C10_CUDA_KERNEL_LAUNCH_CHECK();
   count_launch();
   return stats;

@@ -59,3 +59,20 @@ def test_error_word_is_declared_as_written(op):
     """These kernels store into the device's error word when a wait runs out, so their schemas say that the argument is mutated."""
     schema = re.search(r'm\.def\("' + op + r"\(([^\"]*)\) ->", code_of("bindings.cpp")).group(1)
     assert re.search(r"Tensor\([a-z]!\)\??\s+err\b", schema), schema
+
+
+def test_kernels_wait_for_the_kernels_before_them():
+    """A kernel started by `launch` (programmatic dependent launch) may begin before its predecessor's writes are visible: each waits, and none
+    releases its successor early, whose blocks could hold tensor memory that the running kernel's blocks have yet to allocate."""
+    for path in sorted(CSRC.glob("*.cu")):
+        code = code_of(path.name)
+        assert "launch_dependents" not in code, path.name
+        if '#include "launch.cuh"' not in code:
+            continue
+        bodies = re.split(r"\n(?:template[^\n]*\n)?(?:static )?__global__", code)[1:]
+        assert bodies, path.name
+        for body in bodies:
+            name = re.search(r"(\w+)\s*\((?!\d)", re.sub(r"__launch_bounds__\([^)]*(?:\([^)]*\))?[^)]*\)", "", body)).group(1)
+            end = body.find("\n}")
+            assert "grid_wait();" in body[:end], (path.name, name)
+        assert "<<<" not in code, path.name
