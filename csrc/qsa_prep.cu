@@ -7,7 +7,8 @@
 // Eight lanes per (b, s, h) row, 16 bytes (eight dims) each, so the rotary partner of a row's lanes 0 and 1 is the other one; a warp holds
 // four rows at a time and strides over the rows with the whole grid.  Bound by memory.  With one warp and 4-byte accesses per row, 64-bit
 // divisions for its position and, in the backward, 64 global atomics per eight rows, the kernels ran at a fifth of the copy bandwidth
-// (projections of 16384 tokens, 22 + 2 + 4 + 1 heads: forward 124 -> 57 us, backward 250 -> 80 us).
+// (projections of 16384 tokens, 22 + 2 + 4 + 1 heads: forward 124 -> 57 us, backward 250 -> 80 us; with registers for five and four CTAs
+// per SM and grids of just those, 54 and 65: with 76 registers the backward ran eight CTAs per SM as three waves of three).
 // cos/sin: fp32 [Bc, S, 16] with Bc in {1, B}; they are rounded to bf16 as the PyTorch path does before use.
 #include <ATen/ATen.h>
 #include <ATen/cuda/CUDAContext.h>
@@ -47,7 +48,7 @@ __device__ __forceinline__ float row_sum(float (&p)[4]) {
 }
 
 // `round_products` (PyTorch's bf16 rotary arithmetic): both products are rounded to bf16 before they are added.
-__global__ void __launch_bounds__(32 * HP_WARPS) qsa_headprep_fwd_kernel(const bf16* __restrict__ src, int src_row, const float* __restrict__ w,
+__global__ void __launch_bounds__(32 * HP_WARPS, 5) qsa_headprep_fwd_kernel(const bf16* __restrict__ src, int src_row, const float* __restrict__ w,
                                                                          const float* __restrict__ cosv, const float* __restrict__ sinv, int Bc,
                                                                          bf16* __restrict__ out, bf16* __restrict__ gate, float* __restrict__ rstd_out,
                                                                          int S, int H, unsigned rows, float eps, bool round_products) {
@@ -100,7 +101,7 @@ __global__ void __launch_bounds__(32 * HP_WARPS) qsa_headprep_fwd_kernel(const b
   }
 }
 
-__global__ void __launch_bounds__(32 * HP_WARPS) qsa_headprep_bwd_kernel(const bf16* __restrict__ dout, const bf16* __restrict__ dgate,
+__global__ void __launch_bounds__(32 * HP_WARPS, 4) qsa_headprep_bwd_kernel(const bf16* __restrict__ dout, const bf16* __restrict__ dgate,
                                                                          const bf16* __restrict__ src, int src_row, const float* __restrict__ w,
                                                                          const float* __restrict__ cosv, const float* __restrict__ sinv, int Bc,
                                                                          const float* __restrict__ rstd_in, bf16* __restrict__ dsrc, float* __restrict__ dw,
@@ -164,7 +165,7 @@ __global__ void __launch_bounds__(32 * HP_WARPS) qsa_headprep_bwd_kernel(const b
 }
 
 // Enough CTAs to fill the chip several times over, few enough that a warp handles many rows (the backward adds one weight gradient per CTA).
-static unsigned headprep_grid(long long rows) { return (unsigned)std::max<long long>(1, std::min<long long>((rows + 4 * HP_WARPS - 1) / (4 * HP_WARPS), kNumSMs * 8)); }
+static unsigned headprep_grid(long long rows, int resident) { return (unsigned)std::max<long long>(1, std::min<long long>((rows + 4 * HP_WARPS - 1) / (4 * HP_WARPS), kNumSMs * resident)); }
 
 // The kernels read 16-byte pieces; a contiguous view that starts elsewhere is copied first.  Other strides go on to the checks as they are (a copy
 // would make them contiguous).
@@ -191,7 +192,7 @@ std::vector<at::Tensor> qsa_headprep_fwd(const at::Tensor& src_in, const c10::op
   auto rstd = at::empty({w.has_value() ? B : 0, S, H}, src.options().dtype(at::kFloat));
   const long long rows = (long long)B * S * H;
   TORCH_CHECK(rows < (1ll << 31), "qsa_headprep_fwd: too many rows");
-  launch(qsa_headprep_fwd_kernel, headprep_grid(rows), 32 * HP_WARPS, 0, at::cuda::getCurrentCUDAStream(), 
+  launch(qsa_headprep_fwd_kernel, headprep_grid(rows, 5), 32 * HP_WARPS, 0, at::cuda::getCurrentCUDAStream(), 
       (const bf16*)src.data_ptr(), (int)src.size(3), w.has_value() ? w->data_ptr<float>() : nullptr, cosv.data_ptr<float>(), sinv.data_ptr<float>(), (int)cosv.size(0),
       (bf16*)out.data_ptr(), split_gate ? (bf16*)gate.data_ptr() : nullptr, w.has_value() ? rstd.data_ptr<float>() : nullptr, S, H, (unsigned)rows, (float)eps, round_products);
   C10_CUDA_KERNEL_LAUNCH_CHECK();
@@ -216,7 +217,7 @@ std::vector<at::Tensor> qsa_headprep_bwd(const at::Tensor& dout_in, const c10::o
   auto dw = at::zeros({64}, src.options().dtype(at::kFloat));
   const long long rows = (long long)B * S * H;
   TORCH_CHECK(rows < (1ll << 31), "qsa_headprep_bwd: too many rows");
-  launch(qsa_headprep_bwd_kernel, headprep_grid(rows), 32 * HP_WARPS, 0, at::cuda::getCurrentCUDAStream(), 
+  launch(qsa_headprep_bwd_kernel, headprep_grid(rows, 4), 32 * HP_WARPS, 0, at::cuda::getCurrentCUDAStream(), 
       (const bf16*)dout.data_ptr(), split ? (const bf16*)dgate->data_ptr() : nullptr, (const bf16*)src.data_ptr(), (int)src.size(3),
       w.has_value() ? w->data_ptr<float>() : nullptr, cosv.data_ptr<float>(), sinv.data_ptr<float>(), (int)cosv.size(0),
       w.has_value() ? rstd.data_ptr<float>() : nullptr, (bf16*)dsrc.data_ptr(), dw.data_ptr<float>(), S, H, (unsigned)rows);
