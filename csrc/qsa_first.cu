@@ -1,5 +1,5 @@
 // Indexer block log-probabilities for block selection only (evaluation, and training steps that take no KL term): selection
-// looks at the first query of every 64-token block, so only those S/64 queries are scored.  One CTA per (query block, batch):
+// looks at the first query of every 64-token block, so only those S/64 queries are scored:
 //     I[s]      = sum_h w_h relu(bf16(q_h . k_s)) * scale          for the keys s <= 64 i  (causal for the query at 64 i)
 //     lp_blk[j] = logsumexp_{s in block j} I[s] - logsumexp_s I[s]  for j <= i, a large negative number for j > i
 // The same rounding points as the full indexer kernel (qsa_index.cu) and the PyTorch specification: q.k is rounded to bf16 before
@@ -15,49 +15,63 @@
 
 namespace q38 {
 
-// 512 threads score the keys (with 128 the last query blocks, up to 64 keys per thread, took 147 us of a one-sequence prefill of 8192
-// tokens, now 59); the sum over all keys keeps the order that 128 threads give it.
-constexpr int QF_THREADS = 512, QF_SUM = 128, QF_HEADS_MAX = 4;
+// Two kernels: scores of 256 keys against four queries per CTA, a key per thread (qsa_first_scores), then one CTA per query for the sums and the blocks.  With all keys
+// of a query in one CTA the last of them had 16 rows of 128 bytes per thread to fetch one after the other: 59 us for one sequence of 8192 tokens, now
+// 30 (23 and 7; 29 and 7 with one query per CTA).  The sum over all keys keeps the order that 128 threads give it.
+constexpr int QF_THREADS = 512, QF_SUM = 128, QF_HEADS_MAX = 4, QF_KEYS = 256, QF_QUERIES = 4;
 constexpr float QF_MASKED = -1e9f;
 
-__global__ void __launch_bounds__(QF_THREADS) qsa_first_query_lp_kernel(const __nv_bfloat16* __restrict__ q_first, const __nv_bfloat16* __restrict__ ki,
-                                                                        const float* __restrict__ w_first, float* __restrict__ lp_blk, int S, int NI,
-                                                                        float scale) {
+__global__ void __launch_bounds__(QF_KEYS) qsa_first_scores_kernel(const __nv_bfloat16* __restrict__ q_first, const __nv_bfloat16* __restrict__ ki,
+                                                                   const float* __restrict__ w_first, float* __restrict__ scores, int S, int NI, float scale) {
   grid_wait();
-  extern __shared__ __align__(16) float qf_smem[];
-  float* qs = qf_smem;                       // [NI][64]
-  float* ws = qs + QF_HEADS_MAX * 64;        // [NI]
-  float* red = ws + 4;                       // [36]
-  float* scores = red + 36;                  // [S]
-  const int i = blockIdx.x, b = blockIdx.y, nb = S / 64, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int nkeys = 64 * i + 1;
-  for (int e = tid; e < NI * 64; e += QF_THREADS) {
-    const int h = e >> 6, d = e & 63;
-    qs[e] = __bfloat162float(q_first[(((long long)b * NI + h) * nb + i) * 64 + d]);
+  const int nb = S / 64, i0 = (gridDim.y - 1 - blockIdx.y) * QF_QUERIES, b = blockIdx.z, n = min(QF_QUERIES, nb - i0), tid = threadIdx.x, s = blockIdx.x * QF_KEYS + tid;
+  if ((int)blockIdx.x * QF_KEYS > 64 * (i0 + n - 1)) return;     // no causal key here
+  __shared__ __align__(16) float qs[QF_QUERIES][QF_HEADS_MAX * 64];
+  __shared__ float ws[QF_QUERIES][QF_HEADS_MAX];
+  for (int e = tid; e < n * NI * 64; e += QF_KEYS) {
+    const int x = e / (NI * 64), r = e % (NI * 64);
+    qs[x][r] = __bfloat162float(q_first[(((long long)b * NI + (r >> 6)) * nb + i0 + x) * 64 + (r & 63)]);
   }
-  if (tid < NI) ws[tid] = w_first[((long long)b * nb + i) * NI + tid];
+  if (tid < n * NI) ws[tid / NI][tid % NI] = w_first[((long long)b * nb + i0 + tid / NI) * NI + tid % NI];
   __syncthreads();
-  float m = -INFINITY;
-  for (int s = tid; s < nkeys; s += QF_THREADS) {
-    const uint4* krow = reinterpret_cast<const uint4*>(ki + ((long long)b * S + s) * 64);
+  if (s > 64 * (i0 + n - 1)) return;
+  const uint4* krow = reinterpret_cast<const uint4*>(ki + ((long long)b * S + s) * 64);
+  uint4 key[8];
+#pragma unroll
+  for (int c = 0; c < 8; ++c) key[c] = krow[c];
+  for (int x = 0; x < n; ++x) {
+    if (s > 64 * (i0 + x)) continue;
     float dot[QF_HEADS_MAX] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
     for (int c = 0; c < 8; ++c) {
-      const uint4 raw = krow[c];
-      const __nv_bfloat162* h2 = reinterpret_cast<const __nv_bfloat162*>(&raw);
+      const __nv_bfloat162* h2 = reinterpret_cast<const __nv_bfloat162*>(&key[c]);
       float kv[8];
 #pragma unroll
       for (int e = 0; e < 4; ++e) { kv[2 * e] = __low2float(h2[e]); kv[2 * e + 1] = __high2float(h2[e]); }
 #pragma unroll
       for (int h = 0; h < QF_HEADS_MAX; ++h) {
         if (h >= NI) break;
-        const float4 qa = *reinterpret_cast<const float4*>(qs + h * 64 + 8 * c), qb = *reinterpret_cast<const float4*>(qs + h * 64 + 8 * c + 4);
+        const float4 qa = *reinterpret_cast<const float4*>(&qs[x][h * 64 + 8 * c]), qb = *reinterpret_cast<const float4*>(&qs[x][h * 64 + 8 * c + 4]);
         dot[h] += qa.x * kv[0] + qa.y * kv[1] + qa.z * kv[2] + qa.w * kv[3] + qb.x * kv[4] + qb.y * kv[5] + qb.z * kv[6] + qb.w * kv[7];
       }
     }
     float score = 0.f;
 #pragma unroll
-    for (int h = 0; h < QF_HEADS_MAX; ++h) if (h < NI) score += ws[h] * (fmaxf(bf16_round(dot[h]), 0.f) * scale);
+    for (int h = 0; h < QF_HEADS_MAX; ++h) if (h < NI) score += ws[x][h] * (fmaxf(bf16_round(dot[h]), 0.f) * scale);
+    scores[((long long)b * nb + i0 + x) * S + s] = score;
+  }
+}
+
+__global__ void __launch_bounds__(QF_THREADS) qsa_first_query_lp_kernel(const float* __restrict__ scored, float* __restrict__ lp_blk, int S) {
+  grid_wait();
+  extern __shared__ __align__(16) float qf_smem[];
+  float* red = qf_smem;                      // [36]
+  float* scores = red + 36;                  // [S]
+  const int i = gridDim.x - 1 - blockIdx.x, b = blockIdx.y, nb = S / 64, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int nkeys = 64 * i + 1;
+  float m = -INFINITY;
+  for (int s = tid; s < nkeys; s += QF_THREADS) {
+    const float score = scored[((long long)b * nb + i) * S + s];
     scores[s] = score;
     m = fmaxf(m, score);
   }
@@ -95,11 +109,13 @@ at::Tensor qsa_first_query_lp(const at::Tensor& q_first, const at::Tensor& ki, c
               "qsa_first_query_lp: at most 4 heads, S = 64 nb <= 8192, fp32 weights [B,nb,NI]");
   const c10::cuda::CUDAGuard guard(q_first.device());
   auto lp = at::empty({B, nb, nb}, q_first.options().dtype(at::kFloat));
-  const int smem = (QF_HEADS_MAX * 64 + 4 + 36 + S) * 4;
-  launch(qsa_first_query_lp_kernel, dim3(nb, B), QF_THREADS, smem, at::cuda::getCurrentCUDAStream(), 
-      (const __nv_bfloat16*)q_first.data_ptr(), (const __nv_bfloat16*)ki.data_ptr(), w_first.data_ptr<float>(), lp.data_ptr<float>(), S, NI, (float)scale);
+  auto scores = at::empty({B, nb, S}, q_first.options().dtype(at::kFloat));       // causal entries are written and read
+  auto stream = at::cuda::getCurrentCUDAStream();
+  launch(qsa_first_scores_kernel, dim3((S + QF_KEYS - 1) / QF_KEYS, (nb + QF_QUERIES - 1) / QF_QUERIES, B), QF_KEYS, 0, stream, (const __nv_bfloat16*)q_first.data_ptr(), (const __nv_bfloat16*)ki.data_ptr(),
+         w_first.data_ptr<float>(), scores.data_ptr<float>(), S, NI, (float)scale);
+  launch(qsa_first_query_lp_kernel, dim3(nb, B), QF_THREADS, (36 + S) * 4, stream, scores.data_ptr<float>(), lp.data_ptr<float>(), S);
   C10_CUDA_KERNEL_LAUNCH_CHECK();
-  count_launch();
+  count_launch(2);
   return lp;
 }
 
