@@ -151,7 +151,7 @@ __global__ void __launch_bounds__(256) gated_rmsnorm_fwd_kernel(const __nv_bfloa
   if (live) reinterpret_cast<uint4*>(y + row * 64)[sub] = pack8(out);
 }
 
-__global__ void __launch_bounds__(256) gated_rmsnorm_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ x,
+__global__ void __launch_bounds__(256, 3) gated_rmsnorm_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ x,
                                                                  const __nv_bfloat16* __restrict__ gate, const float* __restrict__ w,
                                                                  __nv_bfloat16* __restrict__ dx, __nv_bfloat16* __restrict__ dgate,
                                                                  float* __restrict__ dw, int rows, float eps) {
@@ -167,7 +167,8 @@ __global__ void __launch_bounds__(256) gated_rmsnorm_bwd_kernel(const __nv_bfloa
   const long long first = ((long long)blockIdx.x * 256 + threadIdx.x) >> 3;
   // every 8-lane group walks rows first, first + stride, ...; the loop bound is uniform per warp up to the last iteration,
   // where finished groups keep shuffling on zeros
-  // the next row's three pieces are in flight while the current one is evaluated (344064 rows: 55 -> 44 us; the bytes need 34)
+  // the next row's three pieces are in flight while the current one is evaluated (344064 rows: 55 -> 44 us; with 80
+  // instead of 96 registers, so three CTAs per SM, and a grid of those 37; the bytes need 34)
   uint4 nx, ng, nd;
   auto fetch = [&](long long row) {
     nx = ng = nd = make_uint4(0, 0, 0, 0);
@@ -543,7 +544,7 @@ std::vector<at::Tensor> gated_rmsnorm_bwd(const at::Tensor& dy, const at::Tensor
   const int rows = x.numel() / 64;
   auto dx = at::empty_like(x), dgate = at::empty_like(gate);
   auto dw = at::zeros({64}, x.options().dtype(at::kFloat));
-  if (rows) launch(gated_rmsnorm_bwd_kernel, std::min((rows + 31) / 32, kNumSMs * 8), 256, 0, at::cuda::getCurrentCUDAStream(), 
+  if (rows) launch(gated_rmsnorm_bwd_kernel, std::min((rows + 31) / 32, kNumSMs * 3), 256, 0, at::cuda::getCurrentCUDAStream(), 
       (const __nv_bfloat16*)dy.data_ptr(), (const __nv_bfloat16*)x.data_ptr(), (const __nv_bfloat16*)gate.data_ptr(), w.data_ptr<float>(),
       (__nv_bfloat16*)dx.data_ptr(), (__nv_bfloat16*)dgate.data_ptr(), dw.data_ptr<float>(), rows, (float)eps);
   C10_CUDA_KERNEL_LAUNCH_CHECK();
