@@ -88,7 +88,7 @@ TORCH_LIBRARY(q38, m) {
   m.def("qsa_first_query_lp(Tensor q_first, Tensor ki, Tensor w_first, float scale) -> Tensor", &q38::qsa_first_query_lp);
   m.def("qsa_kl_combine(Tensor? stats, Tensor blse, int nq) -> Tensor[]");
   m.def("qsa_select(Tensor lp_blk, int budget) -> Tensor[]");
-  m.def("qsa_indexer_bwd(Tensor qi, Tensor ki, Tensor wi, Tensor blse, Tensor dblse, float gscale, float scale, Tensor(a!)? err=None) -> Tensor[]");
+  m.def("qsa_indexer_bwd(Tensor qi, Tensor ki, Tensor wi, Tensor blse, Tensor dblse, float gscale, float scale, Tensor(a!)? err=None, Tensor? upstream=None) -> Tensor[]");
   m.def("qsa_attn_fwd(Tensor q, Tensor k, Tensor v, Tensor? count, Tensor? index, float scale, Tensor(a!)? err=None) -> Tensor[]");
   m.def("qsa_attn_bwd(Tensor q, Tensor k, Tensor v, Tensor o, Tensor dout, Tensor lse, Tensor sel, float scale, Tensor(a!)? err=None) -> Tensor[]");
   m.def("ep_publish_counts(Tensor offsets, int rank, int[] peer_counts) -> ()",

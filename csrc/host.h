@@ -143,7 +143,7 @@ at::Tensor qsa_indexer_fwd(const at::Tensor& qi, const at::Tensor& ki, const at:
 std::vector<at::Tensor> qsa_kl_combine(const c10::optional<at::Tensor>& stats, const at::Tensor& blse, int64_t nq);
 std::vector<at::Tensor> qsa_select(const at::Tensor& lp_blk, int64_t budget);
 std::vector<at::Tensor> qsa_indexer_bwd(const at::Tensor& qi, const at::Tensor& ki, const at::Tensor& wi, const at::Tensor& blse, const at::Tensor& dblse,
-                                        double gscale, double scale, const c10::optional<at::Tensor>& err);
+                                        double gscale, double scale, const c10::optional<at::Tensor>& err, const c10::optional<at::Tensor>& upstream);
 // qsa_tc.cu
 at::Tensor qsa_block_stats_tc(const at::Tensor& q, const at::Tensor& k, double scale, at::Tensor& err);
 // qsa_attn.cu, qsa_attn_bwd.cu

@@ -198,7 +198,7 @@ Tensors qsa_layer_fwd(const Tensor& x, at::TensorList w, at::TensorList wi, cons
       lp = qsa_first_query_lp(qi, ki, wt, i_scale);
     }
   }
-  const Tensor v = p_v.transpose(1, 2).contiguous();
+  const Tensor v = p_v.transpose(1, 2);                                  // the kernels read it token by token
   OptTensor count, index;
   if (!dense && !wi.empty()) {
     auto sel = qsa_select(lp, budget);
@@ -228,11 +228,10 @@ Tensors qsa_layer_bwd(const OptTensor& dy, const OptTensor& dkl, at::TensorList 
     const Tensor &p_qi = saved[15], &p_ki = saved[16], &qi = saved[17], &ki = saved[18], &wt = saved[19], &blse = saved[20], &dblse = saved[21];
     const int64_t NI = qi.size(1);
     const double w_scale = std::pow((double)NI, -0.5);
-    auto d = qsa_indexer_bwd(qi, ki, wt, blse, dblse, 1.0 / (double)T, std::pow(64.0, -0.5), err);
-    const Tensor k16 = dkl->to(at::kBFloat16);
-    const Tensor dqi = qsa_headprep_bwd(d[0] * k16, c10::nullopt, p_qi, c10::nullopt, c, s, saved[22])[0];
-    const Tensor dki = qsa_headprep_bwd((d[1] * k16).unsqueeze(1), c10::nullopt, p_ki, c10::nullopt, c, s, saved[23])[0];
-    const Tensor dwi = ((d[2] * *dkl) * w_scale).to(at::kBFloat16);
+    auto d = qsa_indexer_bwd(qi, ki, wt, blse, dblse, 1.0 / (double)T, std::pow(64.0, -0.5), err, f32(*dkl));
+    const Tensor dqi = qsa_headprep_bwd(d[0], c10::nullopt, p_qi, c10::nullopt, c, s, saved[22])[0];
+    const Tensor dki = qsa_headprep_bwd(d[1].unsqueeze(1), c10::nullopt, p_ki, c10::nullopt, c, s, saved[23])[0];
+    const Tensor dwi = (d[2] * w_scale).to(at::kBFloat16);
     out[7] = wg.linear(4, dqi.view({T, -1}), x2);
     out[8] = wg.linear(5, dki.view({T, -1}), x2);
     out[9] = wg.linear(6, dwi.view({T, -1}), x2);

@@ -51,7 +51,7 @@ struct FwdArgs {
   const unsigned char* sel;
   bf16* o;
   float* lse;
-  int S, nq, nkv;
+  int S, nq, nkv, v_tokens;
   float scale;
   int* err;
 };
@@ -100,7 +100,7 @@ __global__ void __launch_bounds__(AF_THREADS, 4) qsa_attn_fwd_kernel(const __gri
         if (!ptx::mbar_wait(&kv_empty[s], ((t / AF_STAGES) & 1) ^ 1, 1u << 20)) { report_error(p.err, ERR_MMA_WAIT); break; }
         ptx::mbar_expect_tx(&kv_full[s], TILE_BYTES);
         ptx::tma_load_3d(ring + s * TILE_BYTES, &tmK, &kv_full[s], 0, kv_row0 + list[t] * 64, 0);
-        ptx::tma_load_3d(ring + s * TILE_BYTES + HALF_BYTES, &tmV, &kv_full[s], 0, kv_row0 + list[t] * 64, 0);
+        ptx::tma_load_3d(ring + s * TILE_BYTES + HALF_BYTES, &tmV, &kv_full[s], 0, (p.v_tokens ? b * p.S : kv_row0) + list[t] * 64, p.v_tokens ? kvh : 0);
       }
       // copies in flight land before this thread, and with it the CTA, ends
       ptx::mbar_wait(q_full, 0, 1u << 20);
@@ -247,7 +247,8 @@ static at::Tensor selection_matrix(const c10::optional<at::Tensor>& count, const
 // Returns {o [B,S,nq,64] bf16, lse [B,nq,S] fp32, sel [B,nb,nb] uint8}
 std::vector<at::Tensor> qsa_attn_fwd(const at::Tensor& q, const at::Tensor& k, const at::Tensor& v, const c10::optional<at::Tensor>& count,
                                      const c10::optional<at::Tensor>& index, double scale, const c10::optional<at::Tensor>& err) {
-  check_heads(q, "qsa_attn_fwd q"); check_heads(k, "qsa_attn_fwd k"); check_heads(v, "qsa_attn_fwd v");
+  check_heads(q, "qsa_attn_fwd q"); check_heads(k, "qsa_attn_fwd k"); 
+  const bool v_tokens = check_values(v, "qsa_attn_fwd v");
   const c10::cuda::CUDAGuard guard(q.device());
   const int B = q.size(0), nq = q.size(1), S = q.size(2), nkv = k.size(1), nb = S / 64;
   TORCH_CHECK(S % 64 == 0 && nkv > 0 && nq % nkv == 0 && k.sizes() == v.sizes() && k.size(0) == B && k.size(2) == S, "qsa_attn_fwd: bad shapes");
@@ -256,10 +257,10 @@ std::vector<at::Tensor> qsa_attn_fwd(const at::Tensor& q, const at::Tensor& k, c
   auto o = at::empty({B, S, nq, 64}, q.options());
   auto lse = at::empty({B, nq, S}, q.options().dtype(at::kFloat));
   const CUtensorMap tq = make_tmap_box(q.data_ptr(), 2, 64, (int64_t)B * nq * S, 1, 64, 0, 64, 128), tk = make_tmap_box(k.data_ptr(), 2, 64, (int64_t)B * nkv * S, 1, 64, 0, 64, 128),
-                    tv = make_tmap_box(v.data_ptr(), 2, 64, (int64_t)B * nkv * S, 1, 64, 0, 64, 128);
+                    tv = value_map(v, v_tokens);
   FwdArgs p{};
   p.sel = sel.data_ptr<unsigned char>(); p.o = (bf16*)o.data_ptr(); p.lse = lse.data_ptr<float>();
-  p.S = S; p.nq = nq; p.nkv = nkv; p.scale = (float)scale; p.err = err.has_value() ? err->data_ptr<int>() : nullptr;
+  p.S = S; p.nq = nq; p.nkv = nkv; p.v_tokens = v_tokens; p.scale = (float)scale; p.err = err.has_value() ? err->data_ptr<int>() : nullptr;
   const int smem = (1 + AF_STAGES) * TILE_BYTES + 128 + list_bytes(nb);
   static bool cfg = false;
   if (!cfg) { allow_smem(qsa_attn_fwd_kernel); cfg = true; }

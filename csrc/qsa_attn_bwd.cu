@@ -42,7 +42,7 @@ struct BwdArgs {
   const unsigned char* sel;
   __nv_bfloat16* dq;
   float *dk, *dv;
-  int S, nq, nkv, parts;
+  int S, nq, nkv, parts, v_tokens;
   float scale;
   int* err;
 };
@@ -118,7 +118,7 @@ __global__ void __launch_bounds__(AB_THREADS, 2) qsa_attn_bwd_q_kernel(const __g
         if (!ptx::mbar_wait(&kv_empty[s], ((t / Q_STAGES) & 1) ^ 1, 1u << 20)) { report_error(p.err, ERR_MMA_WAIT); break; }
         ptx::mbar_expect_tx(&kv_full[s], TILE_BYTES);
         ptx::tma_load_3d(ring + s * TILE_BYTES, &tmK, &kv_full[s], 0, kv_row0 + list[t] * 64, 0);
-        ptx::tma_load_3d(ring + s * TILE_BYTES + HALF_BYTES, &tmV, &kv_full[s], 0, kv_row0 + list[t] * 64, 0);
+        ptx::tma_load_3d(ring + s * TILE_BYTES + HALF_BYTES, &tmV, &kv_full[s], 0, (p.v_tokens ? b * p.S : kv_row0) + list[t] * 64, p.v_tokens ? kvh : 0);
       }
       // copies in flight land before this thread, and with it the CTA, ends
       ptx::mbar_wait(in_full, 0, 1u << 20);
@@ -278,7 +278,7 @@ __global__ void __launch_bounds__(AB_THREADS, 2) qsa_attn_bwd_kv_kernel(const __
       const int kv_row = (b * p.nkv + kvh) * p.S + j * 64;
       ptx::mbar_expect_tx(kv_full, TILE_BYTES);
       ptx::tma_load_3d(kv, &tmK, kv_full, 0, kv_row, 0);
-      ptx::tma_load_3d(kv + HALF_BYTES, &tmV, kv_full, 0, kv_row, 0);
+      ptx::tma_load_3d(kv + HALF_BYTES, &tmV, kv_full, 0, p.v_tokens ? b * p.S + j * 64 : kv_row, p.v_tokens ? kvh : 0);
       int t = 0, at = 2 * t0 / rep, head = 2 * t0 % rep;
       for (; t < n; ++t) {
         const int s = t % KV_STAGES;
@@ -388,9 +388,12 @@ __global__ void __launch_bounds__(AB_THREADS, 2) qsa_attn_bwd_kv_kernel(const __
       ptx::tc_fence_after();
       ptx::tmem_ld_32x32b_x32(tmem + COL_OUT + (quarter < 2 ? 0 : 64) + 32 * half + lanes, x);
       ptx::tmem_ld_wait();
-      float* out = (quarter < 2 ? p.dv : p.dk) + (((long long)b * p.nkv + kvh) * p.S + (long long)j * 64 + 32 * half) * 64 + tin;
+      const int key = j * 64 + 32 * half;
+      const bool tokens = quarter < 2 && p.v_tokens;                     // dV is laid out like V
+      const long long step = tokens ? p.nkv * 64 : 64;
+      float* out = (quarter < 2 ? p.dv : p.dk) + (tokens ? (((long long)b * p.S + key) * p.nkv + kvh) * 64 : (((long long)b * p.nkv + kvh) * p.S + key) * 64) + tin;
 #pragma unroll
-      for (int e = 0; e < 32; ++e) atomicAdd(out + e * 64, __uint_as_float(x[e]));
+      for (int e = 0; e < 32; ++e) atomicAdd(out + e * step, __uint_as_float(x[e]));
     }
   }
   ptx::tc_fence_before();
@@ -403,7 +406,8 @@ __global__ void __launch_bounds__(AB_THREADS, 2) qsa_attn_bwd_kv_kernel(const __
 // Returns {dq [B,nq,S,64], dk, dv [B,nkv,S,64]}
 std::vector<at::Tensor> qsa_attn_bwd(const at::Tensor& q, const at::Tensor& k, const at::Tensor& v, const at::Tensor& o, const at::Tensor& dout,
                                      const at::Tensor& lse, const at::Tensor& sel, double scale, const c10::optional<at::Tensor>& err) {
-  check_heads(q, "qsa_attn_bwd q"); check_heads(k, "qsa_attn_bwd k"); check_heads(v, "qsa_attn_bwd v");
+  check_heads(q, "qsa_attn_bwd q"); check_heads(k, "qsa_attn_bwd k"); 
+  const bool v_tokens = check_values(v, "qsa_attn_bwd v");
   const c10::cuda::CUDAGuard guard(q.device());
   const int B = q.size(0), nq = q.size(1), S = q.size(2), nkv = k.size(1), nb = S / 64;
   TORCH_CHECK(S % 64 == 0 && nkv > 0 && nq % nkv == 0 && k.sizes() == v.sizes() && k.size(0) == B && k.size(2) == S, "qsa_attn_bwd: bad shapes");
@@ -413,15 +417,15 @@ std::vector<at::Tensor> qsa_attn_bwd(const at::Tensor& q, const at::Tensor& k, c
   TORCH_CHECK(lse.scalar_type() == at::kFloat && lse.is_contiguous() && lse.numel() == (int64_t)B * nq * S && sel.scalar_type() == at::kByte && sel.is_contiguous() &&
               sel.numel() == (int64_t)B * nb * nb, "qsa_attn_bwd: lse [B,nq,S] and sel [B,nb,nb] of the forward required");
   auto dq = at::empty_like(q);
-  auto dk32 = at::zeros(k.sizes(), k.options().dtype(at::kFloat)), dv32 = at::zeros(v.sizes(), v.options().dtype(at::kFloat));
+  auto dkv32 = at::zeros({2, k.numel()}, k.options().dtype(at::kFloat));
   auto D = at::empty({B, nq, S}, q.options().dtype(at::kFloat));
   auto stream = at::cuda::getCurrentCUDAStream();
   const CUtensorMap tq = make_tmap_box(q.data_ptr(), 2, 64, (int64_t)B * nq * S, 1, 64, 0, 64, 128), tk = make_tmap_box(k.data_ptr(), 2, 64, (int64_t)B * nkv * S, 1, 64, 0, 64, 128),
-                    tv = make_tmap_box(v.data_ptr(), 2, 64, (int64_t)B * nkv * S, 1, 64, 0, 64, 128), tdo = make_tmap_box(dout.data_ptr(), 2, 64, (int64_t)B * S, nq, nq * 64, 64, 64, 128);
+                    tv = value_map(v, v_tokens), tdo = make_tmap_box(dout.data_ptr(), 2, 64, (int64_t)B * S, nq, nq * 64, 64, 64, 128);
   const int rep = nq / nkv;
   BwdArgs p{};
   p.o = (const __nv_bfloat16*)o.data_ptr(); p.dout = (const __nv_bfloat16*)dout.data_ptr(); p.lse = lse.data_ptr<float>(); p.D = D.data_ptr<float>();
-  p.sel = sel.data_ptr<unsigned char>(); p.dq = (__nv_bfloat16*)dq.data_ptr(); p.dk = dk32.data_ptr<float>(); p.dv = dv32.data_ptr<float>();
+  p.sel = sel.data_ptr<unsigned char>(); p.dq = (__nv_bfloat16*)dq.data_ptr(); p.dk = dkv32.data_ptr<float>(); p.dv = p.dk + k.numel(); p.v_tokens = v_tokens;
   p.S = S; p.nq = nq; p.nkv = nkv; p.scale = (float)scale; p.err = err.has_value() ? err->data_ptr<int>() : nullptr;
   p.parts = std::min(8, (nb * rep + 31) / 32);
   const int smem_q = (2 + Q_STAGES) * TILE_BYTES + 1024 + 256 + 1024 + list_bytes(nb), smem_kv = (1 + 2 * KV_STAGES + 2) * TILE_BYTES + 256 + list_bytes(nb);
@@ -432,7 +436,9 @@ std::vector<at::Tensor> qsa_attn_bwd(const at::Tensor& q, const at::Tensor& k, c
   launch(qsa_attn_bwd_kv_kernel, dim3(p.parts * nkv, nb, B), AB_THREADS, smem_kv, stream, tq, tk, tv, tdo, p);
   C10_CUDA_KERNEL_LAUNCH_CHECK();
   count_launch(2);
-  return {dq, dk32.to(at::kBFloat16), dv32.to(at::kBFloat16)};
+  const auto dkv = dkv32.to(at::kBFloat16);
+  const auto dv = dkv.select(0, 1);
+  return {dq, dkv.select(0, 0).view(k.sizes()), v_tokens ? dv.view({B, S, nkv, 64}).transpose(1, 2) : dv.view(v.sizes())};
 }
 
 }  // namespace q38

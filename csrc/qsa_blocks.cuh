@@ -4,6 +4,7 @@
 #include <c10/cuda/CUDAException.h>
 
 #include "common.cuh"
+#include "host.h"
 
 namespace q38 {
 
@@ -32,6 +33,18 @@ template <typename K> void allow_smem(K kernel) { C10_CUDA_CHECK(cudaFuncSetAttr
 
 inline void check_heads(const at::Tensor& t, const char* name) {
   TORCH_CHECK(t.is_cuda() && t.scalar_type() == at::kBFloat16 && t.is_contiguous() && t.dim() == 4 && t.size(3) == 64, name, ": contiguous bf16 [B,H,S,64] required");
+}
+
+// Values [B,H,S,64]: contiguous, or the transposed view of a projection's output [B,S,H,64].  Returns whether it is the latter.
+inline bool check_values(const at::Tensor& v, const char* name) {
+  const bool tokens = v.dim() == 4 && v.size(3) == 64 && v.stride(3) == 1 && v.stride(1) == 64 && v.stride(2) == v.size(1) * 64 && v.stride(0) == v.size(2) * v.size(1) * 64;
+  if (!tokens || !v.is_cuda() || v.scalar_type() != at::kBFloat16) check_heads(v, name);
+  return tokens;
+}
+// Its tensor map: a box of 64 rows starts at {0, b S + row, head} in the transposed view, at {0, (b H + head) S + row, 0} otherwise.
+inline CUtensorMap value_map(const at::Tensor& v, bool tokens) {
+  const int64_t B = v.size(0), H = v.size(1), S = v.size(2);
+  return tokens ? make_tmap_box(v.data_ptr(), 2, 64, B * S, H, H * 64, 64, 64, 128) : make_tmap_box(v.data_ptr(), 2, 64, B * H * S, 1, 64, 0, 64, 128);
 }
 
 }  // namespace q38

@@ -41,7 +41,7 @@ constexpr int IB_SMEM = (2 + IB_STAGES + 4 + 2) * IB_TILE + 2 * 256 * 4 + IB_HEA
 
 struct IndexBwdArgs {
   const __nv_bfloat16* qi;
-  const float *wi, *blse, *dblse;
+  const float *wi, *blse, *dblse, *upstream;
   __nv_bfloat16* dqi;                                                   // without slices
   float *dwi, *part, *dw_part;                                          // with slices: [Z,B,NI,S,64], [Z,B,S,NI]
   int B, S, NI, Z;
@@ -102,13 +102,14 @@ __global__ void __launch_bounds__(IB_THREADS, 1) qsa_indexer_bwd_kernel(const __
         ptx::tma_load_3d(q_tile + x * 2048, &tmQ, q_full, 0, i * 64 + 32 * u + 16 * half, h < p.NI ? b * p.NI + h : p.B * p.NI);
       }
     }
+    const float gscale = p.upstream != nullptr ? p.gscale * *p.upstream : p.gscale;
     float v[8];
     auto fetch = [&](int m) {
 #pragma unroll
       for (int x = 0; x < 8; ++x) {                                      // key block x >> 2, blse or dblse, queries lane and lane + 32
         const int blk = 2 * (z + m * p.Z) + (x >> 2);
         const float* src = (x & 2) ? p.dblse : p.blse;
-        v[x] = blk < nb ? src[((long long)b * p.S + i * 64 + lane + 32 * (x & 1)) * nb + blk] * ((x & 2) ? p.gscale : 1.f) : 0.f;
+        v[x] = blk < nb ? src[((long long)b * p.S + i * 64 + lane + 32 * (x & 1)) * nb + blk] * ((x & 2) ? gscale : 1.f) : 0.f;
       }
     };
     fetch(0);
@@ -373,9 +374,9 @@ void check_rows(const at::Tensor& t, const char* name) {
 
 }  // namespace
 
-// Returns {dqi [B,NI,S,64] bf16, dki [B,S,64] bf16, dwi [B,S,NI] fp32}; gscale multiplies dblse (upstream grad / token count).
+// Returns {dqi [B,NI,S,64] bf16, dki [B,S,64] bf16, dwi [B,S,NI] fp32}; gscale (one over the token count) and, where given, the one-element upstream gradient multiply dblse.
 std::vector<at::Tensor> qsa_indexer_bwd(const at::Tensor& qi, const at::Tensor& ki, const at::Tensor& wi, const at::Tensor& blse, const at::Tensor& dblse,
-                                        double gscale, double scale, const c10::optional<at::Tensor>& err) {
+                                        double gscale, double scale, const c10::optional<at::Tensor>& err, const c10::optional<at::Tensor>& upstream) {
   check_rows(qi, "qsa_indexer_bwd q"); check_rows(ki, "qsa_indexer_bwd k");
   const c10::cuda::CUDAGuard guard(qi.device());
   TORCH_CHECK(qi.dim() == 4 && qi.size(1) <= IB_HEADS && qi.size(2) % 64 == 0, "qsa_indexer_bwd: at most 4 indexer heads and whole blocks of 64 tokens");
@@ -383,6 +384,7 @@ std::vector<at::Tensor> qsa_indexer_bwd(const at::Tensor& qi, const at::Tensor& 
   TORCH_CHECK(ki.numel() == (int64_t)B * S * 64, "qsa_indexer_bwd: k must be [B,S,64]");
   auto rows = [&](const at::Tensor& t, int64_t n) { return t.is_cuda() && t.scalar_type() == at::kFloat && t.is_contiguous() && t.numel() == (int64_t)B * S * n; };
   TORCH_CHECK(rows(wi, NI) && rows(blse, nb) && rows(dblse, nb), "qsa_indexer_bwd: contiguous fp32 w [B,S,heads], blse and dblse [B,S,blocks] required");
+  TORCH_CHECK(!upstream.has_value() || (upstream->is_cuda() && upstream->scalar_type() == at::kFloat && upstream->numel() == 1), "qsa_indexer_bwd: upstream gradient of one fp32 element required");
   // One CTA per query block while these fill the SMs; otherwise its key tiles are shared by up to four.
   const int Z = std::min(std::min((nb + 1) / 2, 4), std::max(1, kNumSMs / std::max(1, B * nb)));
   auto f32 = qi.options().dtype(at::kFloat);
@@ -393,6 +395,7 @@ std::vector<at::Tensor> qsa_indexer_bwd(const at::Tensor& qi, const at::Tensor& 
   p.qi = (const __nv_bfloat16*)qi.data_ptr(); p.wi = wi.data_ptr<float>(); p.blse = blse.data_ptr<float>(); p.dblse = dblse.data_ptr<float>();
   p.dqi = (__nv_bfloat16*)dqi.data_ptr(); p.dwi = dwi.data_ptr<float>();
   if (Z > 1) { p.part = part.data_ptr<float>(); p.dw_part = dw_part.data_ptr<float>(); }
+  p.upstream = upstream.has_value() ? upstream->data_ptr<float>() : nullptr;
   p.B = B; p.S = S; p.NI = NI; p.Z = Z; p.gscale = (float)gscale; p.scale = (float)scale; p.err = err.has_value() ? err->data_ptr<int>() : nullptr;
   const CUtensorMap tq = make_tmap_box(qi.data_ptr(), 2, 64, S, (int64_t)B * NI, 64, (int64_t)S * 64, 16, 128), tk = make_tmap_box(ki.data_ptr(), 2, 64, S, B, 64, (int64_t)S * 64, 128, 128),
                     tdk = make_tmap_box(dki32.data_ptr(), 4, 64, S, B, 64, (int64_t)S * 64, 32, 128);

@@ -200,7 +200,7 @@ std::vector<at::Tensor> qsa_headprep_fwd(const at::Tensor& src_in, const c10::op
   return {out, gate, rstd};
 }
 
-// dout [B,H,S,64], dgate [B,S,H*64] (with split_gate) -> {dsrc like src, dw [64] (zeros without a norm)}
+// dout [B,H,S,64], dgate [B,S,H*64] (with split_gate) -> {dsrc like src, dw [64] (empty without a norm)}
 std::vector<at::Tensor> qsa_headprep_bwd(const at::Tensor& dout_in, const c10::optional<at::Tensor>& dgate_in, const at::Tensor& src_in, const c10::optional<at::Tensor>& w,
                                          const at::Tensor& cos_in, const at::Tensor& sin_in, const at::Tensor& rstd) {
   const at::Tensor dout = aligned16(dout_in), src = aligned16(src_in), cosv = aligned16(cos_in), sinv = aligned16(sin_in);
@@ -214,7 +214,7 @@ std::vector<at::Tensor> qsa_headprep_bwd(const at::Tensor& dout_in, const c10::o
   TORCH_CHECK(!split || (dgate->scalar_type() == at::kBFloat16 && dgate->is_contiguous() && dgate->numel() == (long long)B * S * H * 64), "qsa_headprep_bwd: bad gate gradient");
   check_tables(cosv, sinv, B, S);
   auto dsrc = at::empty_like(src);
-  auto dw = at::zeros({64}, src.options().dtype(at::kFloat));
+  auto dw = w.has_value() ? at::zeros({64}, src.options().dtype(at::kFloat)) : at::empty({0}, src.options().dtype(at::kFloat));
   const long long rows = (long long)B * S * H;
   TORCH_CHECK(rows < (1ll << 31), "qsa_headprep_bwd: too many rows");
   launch(qsa_headprep_bwd_kernel, headprep_grid(rows, 4), 32 * HP_WARPS, 0, at::cuda::getCurrentCUDAStream(), 

@@ -26,3 +26,24 @@ def test_indexer_backward_without_slices(ops, B, nb, NI):  # noqa: F811
 @pytest.mark.parametrize("name", ["qsa_attn.cu", "qsa_attn_bwd.cu", "qsa_index_bwd.cu"])
 def test_waits_of_whole_warps(name):
     waits_are_voted(name)
+
+
+@gpu
+@pytest.mark.parametrize("nkv", [1, 2])
+def test_values_as_a_transposed_view(ops, nkv):  # noqa: F811
+    """Values may be the transposed view of a projection's output: the same results, and their gradient in that layout."""
+    B, nq, S = 2, 4, 192
+    gen = torch.Generator(device="cuda").manual_seed(nkv)
+    q, k, do = (torch.randn(s, device="cuda", generator=gen).to(torch.bfloat16) for s in ((B, nq, S, 64), (B, nkv, S, 64), (B, S, nq, 64)))
+    v = torch.randn(B, S, nkv, 64, device="cuda", generator=gen).to(torch.bfloat16).transpose(1, 2)
+    lib = ops.load()
+    results = []
+    for values in (v, v.contiguous()):
+        o, lse, sel = lib.qsa_attn_fwd(q, k, values, None, None, 0.125)
+        results.append((o, lse, *lib.qsa_attn_bwd(q, k, values, o, do, lse, sel, 0.125)))
+    assert results[0][4].stride() == v.stride()
+    for i, (a, b) in enumerate(zip(*results)):
+        # key and value gradients: fp32 sums whose order varies, rounded to bf16 once
+        assert torch.equal(a, b) if i < 3 else ((a.float() - b.float()).norm() <= 4e-3 * b.float().norm())
+    with pytest.raises(RuntimeError, match="contiguous bf16"):
+        lib.qsa_attn_fwd(q, k, v.expand(B, nkv, S, 64)[..., ::1].transpose(2, 3).contiguous().transpose(2, 3), None, None, 0.125)
