@@ -79,7 +79,7 @@ TORCH_LIBRARY(q38, m) {
   m.def("qsa_main_block_stats(Tensor q, Tensor k, float scale) -> Tensor");
   m.def("qsa_block_stats_tc(Tensor q, Tensor k, float scale, Tensor(a!) err) -> Tensor",
         [](const at::Tensor& q, const at::Tensor& k, double scale, at::Tensor& err) { return q38::qsa_block_stats_tc(q, k, scale, err); });
-  m.def("qsa_indexer_fwd(Tensor qi, Tensor ki, Tensor wi, float scale) -> Tensor");
+  m.def("qsa_indexer_fwd(Tensor qi, Tensor ki, Tensor wi, float scale, Tensor(a!)? err=None) -> Tensor");
   m.def("gemm_pair(Tensor a, Tensor b, Tensor(a!) c, float alpha, bool accumulate, Tensor(b!) err) -> bool",
         [](const at::Tensor& a, const at::Tensor& b, at::Tensor& c, double alpha, bool acc, at::Tensor& err) { 
           TORCH_CHECK(a.dim() == 3 && b.dim() == 3 && c.dim() == 3, "gemm_pair: [batch, rows, cols] tensors required");

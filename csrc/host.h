@@ -137,9 +137,9 @@ std::vector<at::Tensor> gdn_rule_bwd(const at::Tensor& qkv, const at::Tensor& g,
 // gdn_chain.cu
 std::vector<at::Tensor> gdn_chain_bwd(const at::Tensor& w, const at::Tensor& P, const at::Tensor& qg, const at::Tensor& kg, const at::Tensor& dch,
                                       const at::Tensor& states, const at::Tensor& dout, int64_t B, int64_t H, const c10::optional<at::Tensor>& err);
-// qsa_index.cu, qsa_index_bwd.cu
+// qsa_index.cu, qsa_index_fwd.cu, qsa_index_bwd.cu
 at::Tensor qsa_main_block_stats(const at::Tensor& q, const at::Tensor& k, double scale);
-at::Tensor qsa_indexer_fwd(const at::Tensor& qi, const at::Tensor& ki, const at::Tensor& wi, double scale);
+at::Tensor qsa_indexer_fwd(const at::Tensor& qi, const at::Tensor& ki, const at::Tensor& wi, double scale, const c10::optional<at::Tensor>& err);
 std::vector<at::Tensor> qsa_kl_combine(const c10::optional<at::Tensor>& stats, const at::Tensor& blse, int64_t nq);
 std::vector<at::Tensor> qsa_select(const at::Tensor& lp_blk, int64_t budget);
 std::vector<at::Tensor> qsa_indexer_bwd(const at::Tensor& qi, const at::Tensor& ki, const at::Tensor& wi, const at::Tensor& blse, const at::Tensor& dblse,

@@ -183,7 +183,7 @@ Tensors qsa_layer_fwd(const Tensor& x, at::TensorList w, at::TensorList wi, cons
       const Tensor ki = hki[0].select(1, 0), wt = (mm_nt(x2, wi[2], err).view({B, S, NI}).to(at::kFloat) * w_scale).contiguous();
       Tensor e = err;
       const Tensor stats = S % 128 == 0 && main_tc ? qsa_block_stats_tc(q, k, scale, e) : qsa_main_block_stats(q, k, scale);
-      const Tensor blse = qsa_indexer_fwd(hqi[0], ki, wt, i_scale);
+      const Tensor blse = qsa_indexer_fwd(hqi[0], ki, wt, i_scale, err);
       auto comb = qsa_kl_combine(stats, blse, q.size(1));
       lp = comb[1];
       kl = comb[2].mean();

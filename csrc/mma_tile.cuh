@@ -1,6 +1,6 @@
 // 64x64x64 bf16 tile products on the warp-level tensor-core path (mma.sync m16n8k16, fp32 accumulation) for kernels
-// whose chains of small dependent products are latency bound: the delta-rule scan, the QSA indexer and the block-sparse
-// attention.  Four warps cooperate on one 64x64 output; warp w owns rows 16w..16w+15 and keeps them in registers.
+// whose chains of small dependent products are latency bound (the delta rule), and for block masses of sequence lengths that the
+// tcgen05 kernel does not take.  Four warps cooperate on one 64x64 output; warp w owns rows 16w..16w+15 and keeps them in registers.
 #pragma once
 #include "common.cuh"
 
@@ -68,16 +68,6 @@ __device__ __forceinline__ void acc_to_smem(const float (&acc)[8][4], bf16* __re
   for (int nt = 0; nt < 8; ++nt) {
     *reinterpret_cast<__nv_bfloat162*>(dst + r * LDS + 8 * nt + cq) = __floats2bfloat162_rn(acc[nt][0], acc[nt][1]);
     *reinterpret_cast<__nv_bfloat162*>(dst + (r + 8) * LDS + 8 * nt + cq) = __floats2bfloat162_rn(acc[nt][2], acc[nt][3]);
-  }
-}
-
-// Accumulator fragment -> dense [64,64] bf16 tile in global memory with row stride `ld` elements.
-__device__ __forceinline__ void acc_to_global(const float (&acc)[8][4], bf16* __restrict__ dst, long long ld, int warp, int lane, float scale = 1.f) {
-  const int r = 16 * warp + (lane >> 2), cq = 2 * (lane & 3);
-#pragma unroll
-  for (int nt = 0; nt < 8; ++nt) {
-    *reinterpret_cast<__nv_bfloat162*>(dst + (long long)r * ld + 8 * nt + cq) = __floats2bfloat162_rn(acc[nt][0] * scale, acc[nt][1] * scale);
-    *reinterpret_cast<__nv_bfloat162*>(dst + (long long)(r + 8) * ld + 8 * nt + cq) = __floats2bfloat162_rn(acc[nt][2] * scale, acc[nt][3] * scale);
   }
 }
 
@@ -157,7 +147,7 @@ __device__ __forceinline__ void load_tile_async_256(bf16* __restrict__ dst, cons
 
 // ---- products whose A operand stays in registers -----------------------------------------------------------------------
 // A warp's accumulator fragment of one product, packed to bf16, is the A fragment of the next product (the layouts of m16n8k16
-// agree), so probabilities and score gradients go from one product to the next without shared memory or a barrier.
+// agree), so results go from one product to the next without shared memory or a barrier.
 
 // A fragments of rows 16 wr .. + 15 of a padded tile, all four 16-deep k steps.
 __device__ __forceinline__ void load_a(const bf16* __restrict__ As, uint32_t (&a)[4][4], int wr, int lane) {

@@ -2,12 +2,10 @@
 //
 //   qsa_main_block_stats  dense causal scores of the main attention (all heads), reduced on the fly to a per
 //                         (head, query, key block) pair (max, sum exp): the raw material of the distillation target.
-//   qsa_indexer_fwd       indexer scores I[t,s] = sum_j w_j(t) relu(q_j(t).k(s)) / 8, reduced to the block log-sum-exp
-//                         bLSE[t,b] = log sum_{s in b, s<=t} exp I[t,s].  The [S,S] score matrix never exists in memory.
 //   qsa_kl_combine        per token: target P[t,b] (head-averaged block mass), lp_blk[t,b] = bLSE - logsumexp_b bLSE,
 //                         KL_t = sum_b P (log P - lp_blk) and the gradient seed (exp(lp_blk) - P).
 //   qsa_select            per query block: top-k key blocks from the first query's lp_blk (own block forced, future excluded).
-// The backward pass of the scores is in qsa_index_bwd.cu.
+// The scores themselves are formed in qsa_index_fwd.cu, their gradients in qsa_index_bwd.cu.
 //
 // Layouts: main q [B,nq,S,64], main k [B,nkv,S,64], indexer q [B,NI,S,64], indexer k [B,S,64] (bf16); w [B,S,NI] fp32.
 #include <ATen/ATen.h>
@@ -21,7 +19,6 @@
 
 namespace q38 {
 
-constexpr int NI_MAX = 4;
 constexpr float MASKED = -1e9f;
 
 // Row-wise (max, sum exp(x - max)) of a fragment tile; entries with col > row + diag_shift are excluded when `diag`.
@@ -91,72 +88,6 @@ __global__ void __launch_bounds__(128) qsa_main_block_stats_kernel(const bf16* _
     }
     __syncthreads();
   }
-}
-
-// ---- indexer forward ---------------------------------------------------------------------------------------------------
-// grid (nb, B).  blse[b, t, j] for j <= block(t); entries j > block(t) are left untouched (the caller pre-fills them).
-// The query fragments of all heads stay in registers, the next key block is fetched while the current one is scored, one barrier per block.
-__global__ void __launch_bounds__(128, 3) qsa_indexer_fwd_kernel(const bf16* __restrict__ qi, const bf16* __restrict__ ki, const float* __restrict__ wi,
-                                                                 float* __restrict__ blse, int S, int NI, float scale) {
-  grid_wait();
-  extern __shared__ __align__(16) uint8_t smem_bytes[];
-  bf16* Qs = reinterpret_cast<bf16*>(smem_bytes);          // NI tiles
-  bf16* Ks = Qs + NI_MAX * TILE_ELEMS;                     // two buffers
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  // Query block i scores key blocks j <= i; late query blocks (most work) are issued first and the key loop of a query block is
-  // shared by gridDim.z CTAs (j = z, z + gridDim.z, ...), each writing its own columns of blse.
-  const int nb = S / 64, i = nb - 1 - blockIdx.x, b = blockIdx.y, jstep = gridDim.z;
-  if ((int)blockIdx.z > i) return;
-  for (int hh = 0; hh < NI; ++hh) load_tile_async(Qs + hh * TILE_ELEMS, qi + (((long long)b * NI + hh) * S + (long long)i * 64) * 64, 64, tid);
-  const bf16* kbase = ki + (long long)b * S * 64;
-  load_tile_async(Ks, kbase + (long long)blockIdx.z * 4096, 64, tid);
-  cp_async_commit();
-  const int r0 = 16 * warp + (lane >> 2);
-  float wrow[2][NI_MAX];
-#pragma unroll
-  for (int hrow = 0; hrow < 2; ++hrow)
-#pragma unroll
-    for (int hh = 0; hh < NI_MAX; ++hh) wrow[hrow][hh] = hh < NI ? wi[((long long)b * S + (long long)i * 64 + r0 + 8 * hrow) * NI + hh] * scale : 0.f;
-  cp_async_wait<0>();
-  __syncthreads();
-  uint32_t aq[NI_MAX][4][4];
-#pragma unroll
-  for (int hh = 0; hh < NI_MAX; ++hh) if (hh < NI) load_a(Qs + hh * TILE_ELEMS, aq[hh], warp, lane);
-  int buf = 0;
-  for (int j = blockIdx.z; j <= i; j += jstep, buf ^= 1) {
-    cp_async_wait<0>();
-    __syncthreads();                                       // this key block is visible; the other buffer's readers are done
-    if (j + jstep <= i) load_tile_async(Ks + (buf ^ 1) * TILE_ELEMS, kbase + (long long)(j + jstep) * 4096, 64, tid);
-    cp_async_commit();
-    float score[8][4];
-    zero_acc(score);
-#pragma unroll
-    for (int hh = 0; hh < NI_MAX; ++hh) {
-      if (hh < NI) {
-#pragma unroll
-        for (int half = 0; half < 2; ++half) {
-          float acc[4][4];
-          zero_acc(acc);
-          mma_rows<true, 4, 4>(aq[hh], Ks + buf * TILE_ELEMS + 32 * half * LDS, acc, lane);
-#pragma unroll
-          for (int nt = 0; nt < 4; ++nt)
-#pragma unroll
-            for (int e = 0; e < 4; ++e)                    // the reference rounds q.k to bf16 before the relu (its matmul output dtype)
-              score[4 * half + nt][e] += wrow[e >> 1][hh] * fmaxf(bf16_round(acc[nt][e]), 0.f);
-        }
-      }
-    }
-    float mx[2], sm[2];
-    frag_row_max_sum(score, j == i, warp, lane, mx, sm);
-    if ((lane & 3) == 0) {
-#pragma unroll
-      for (int hrow = 0; hrow < 2; ++hrow) {
-        const long long t = (long long)i * 64 + r0 + 8 * hrow;
-        blse[((long long)b * S + t) * nb + j] = mx[hrow] + __logf(sm[hrow]);
-      }
-    }
-  }
-  cp_async_wait<0>();
 }
 
 // ---- combine: target mass, lp_blk, KL --------------------------------------------------------------------------------
@@ -274,23 +205,6 @@ at::Tensor qsa_main_block_stats(const at::Tensor& q, const at::Tensor& k, double
   C10_CUDA_KERNEL_LAUNCH_CHECK();
   count_launch();
   return stats;
-}
-
-// qi [B,NI,S,64], ki [B,S,64], wi [B,S,NI] fp32 -> blse [B,S,nb] fp32 (non-causal entries = -1e9)
-at::Tensor qsa_indexer_fwd(const at::Tensor& qi, const at::Tensor& ki, const at::Tensor& wi, double scale) {
-  check4(qi, "qsa_indexer_fwd q"); check4(ki, "qsa_indexer_fwd k");
-  const c10::cuda::CUDAGuard guard(qi.device());
-  const int B = qi.size(0), NI = qi.size(1), S = qi.size(2), nb = S / 64;
-  TORCH_CHECK(NI <= NI_MAX && S % 64 == 0 && wi.scalar_type() == at::kFloat && wi.is_contiguous(), "qsa_indexer_fwd: at most 4 indexer heads");
-  auto blse = at::full({B, S, nb}, (double)MASKED, qi.options().dtype(at::kFloat));
-  const int smem = (NI_MAX + 2) * TILE_ELEMS * 2;
-  static bool cfg = false;
-  if (!cfg) { C10_CUDA_CHECK(cudaFuncSetAttribute(qsa_indexer_fwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem)); cfg = true; }
-  launch(qsa_indexer_fwd_kernel, dim3(nb, B, std::min(nb, 4)), 128, smem, at::cuda::getCurrentCUDAStream(), (const bf16*)qi.data_ptr(), (const bf16*)ki.data_ptr(), wi.data_ptr<float>(),
-      blse.data_ptr<float>(), S, NI, (float)scale);
-  C10_CUDA_KERNEL_LAUNCH_CHECK();
-  count_launch(2);
-  return blse;
 }
 
 // Returns {P [B,S,nb], lp_blk [B,S,nb], kl_tok [B,S], dblse [B,S,nb]}; stats may be undefined when no target is wanted.

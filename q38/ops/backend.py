@@ -436,7 +436,7 @@ class _IndexerKL(torch.autograd.Function):
             stats = ops.qsa_block_stats_tc(q_main, k_main, main_scale, error_flag(q_main.device))      # tcgen05 kernel (csrc/qsa_tc.cu)
         else:
             stats = ops.qsa_main_block_stats(q_main, k_main, main_scale)
-        blse = ops.qsa_indexer_fwd(qi, ki, wi, idx_scale)
+        blse = ops.qsa_indexer_fwd(qi, ki, wi, idx_scale, error_flag(qi.device))
         P, lp_blk, kl_tok, dblse = ops.qsa_kl_combine(stats, blse, q_main.shape[1])
         ctx.save_for_backward(qi, ki, wi, blse, dblse)
         ctx.idx_scale = idx_scale
@@ -954,7 +954,7 @@ class Backend:
         if q_main is not None:
             return _IndexerKL.apply(qi, ki, wi, q_main, k_main, main_scale, D ** -0.5)
         ops = load()
-        blse = ops.qsa_indexer_fwd(qi.detach(), ki.detach(), wi.detach(), D ** -0.5)
+        blse = ops.qsa_indexer_fwd(qi.detach(), ki.detach(), wi.detach(), D ** -0.5, error_flag(qi.device))
         return None, ops.qsa_kl_combine(None, blse, 1)[1]
 
     @_nvtx("q38.qsa_attention")

@@ -176,7 +176,7 @@ def bench_qsa(rows, shape, T, iters, pk, seq=4096):
     blse = lib.qsa_indexer_fwd(qi, ki, wi, 0.125)
     dblse = torch.randn_like(blse) * 1e-3
     t = timeit(lambda: lib.qsa_indexer_bwd(qi, ki, wi, blse, dblse, 1.0 / (B * seq), 0.125), iters)
-    report(rows, f"qsa_indexer_bwd (q and k kernels) B={B}", t, flops=3 * 4 * causal_tiles * 2.0 * 64 ** 3, pk=pk)
+    report(rows, f"qsa_indexer_bwd B={B}", t, flops=3 * 4 * causal_tiles * 2.0 * 64 ** 3, pk=pk)
     lp = torch.randn(B, seq // 64, seq // 64, device="cuda")
     count, index = lib.qsa_select(lp, shape["qsa_blocks"])
     t = timeit(lambda: lib.qsa_attn_fwd(q, k, v, count, index, 0.125), iters)

@@ -23,7 +23,28 @@ def test_indexer_backward_without_slices(ops, B, nb, NI):  # noqa: F811
     indexer_backward(ops, NI, B, nb)
 
 
-@pytest.mark.parametrize("name", ["qsa_attn.cu", "qsa_attn_bwd.cu", "qsa_index_bwd.cu"])
+# half a query tile, an odd last one, key blocks shared by several CTAs; fewer heads than the kernel holds
+@gpu
+@pytest.mark.parametrize("B,nb,NI", [(1, 1, 4), (2, 3, 1), (1, 21, 3)])
+def test_indexer_forward(ops, B, nb, NI):  # noqa: F811
+    S = 64 * nb
+    gen = torch.Generator(device="cuda").manual_seed(nb)
+    qi = torch.randn(B, NI, S, 64, device="cuda", generator=gen).to(torch.bfloat16)
+    ki = torch.randn(B, S, 64, device="cuda", generator=gen).to(torch.bfloat16)
+    wi = torch.randn(B, S, NI, device="cuda", generator=gen) / 2
+    blse = ops.load().qsa_indexer_fwd(qi, ki, wi, 0.125).double()
+    causal = torch.ones(S, S, dtype=torch.bool, device="cuda").tril()
+    dots = (qi.double() @ ki.double()[:, None].transpose(-1, -2)).to(torch.bfloat16).double()
+    score = (torch.relu(dots) * 0.125 * wi.double().transpose(1, 2)[..., None]).sum(1).masked_fill(~causal, float("-inf"))
+    want = score.unflatten(-1, (nb, 64)).logsumexp(-1)
+    own = (torch.arange(S, device="cuda")[:, None] // 64 >= torch.arange(nb, device="cuda")[None]).expand_as(want)
+    assert (blse[~own] == -1e9).all()
+    # fp32 sums; a product that lies on a rounding boundary of bf16 may fall to the other side: 2^-8 of |q.k| <= 40, times scale and |w| <= 2
+    assert (blse - want)[own].abs().max() < 2 ** -8 * 40 * 0.125 * 2
+    assert (blse - want)[own].pow(2).mean().sqrt() < 1e-3
+
+
+@pytest.mark.parametrize("name", ["qsa_attn.cu", "qsa_attn_bwd.cu", "qsa_index_fwd.cu", "qsa_index_bwd.cu"])
 def test_waits_of_whole_warps(name):
     waits_are_voted(name)
 
