@@ -120,16 +120,18 @@ __global__ void __launch_bounds__(G2_THREADS) gemm_pair_kernel(const __grid_cons
     m0 = tm * 2 * G2_BM; n0 = tn * p.bn;
   };
 
+  auto advance = [&](int& s, uint32_t& odd) { if (++s == p.stages) { s = 0; odd ^= 1; } };        // a division by the number of stages would cost each K block
+
   if (warp == 0) {
     if (ptx::elect_one()) {
-      uint32_t it = 0;
+      int s = 0;                                             // stage of the K block; its ring has gone round an odd number of times
+      uint32_t odd = 0;
       bool ok = true;
       for (int w = cluster_id; w < p.work_items && ok; w += num_clusters) {
         int bz, m0, n0;
         decode(w, bz, m0, n0);
-        for (int kb = 0; kb < p.total_kb; ++kb, ++it) {
-          const int s = it % p.stages;
-          if (!ptx::mbar_wait(&empty[s], ((it / p.stages) & 1) ^ 1, 1u << 20)) { report_error(p.err, ERR_MMA_WAIT); ok = false; break; }
+        for (int kb = 0; kb < p.total_kb; ++kb, advance(s, odd)) {
+          if (!ptx::mbar_wait(&empty[s], odd ^ 1, 1u << 20)) { report_error(p.err, ERR_MMA_WAIT); ok = false; break; }
           uint8_t* a_dst = smem + s * STAGE_BYTES;
           uint8_t* b_dst = a_dst + A_BYTES;
           const uint32_t leader_full = ptx2::map_to_rank(&full[s], 0);
@@ -144,16 +146,16 @@ __global__ void __launch_bounds__(G2_THREADS) gemm_pair_kernel(const __grid_cons
   } else if (warp == 1) {
     if (rank == 0 && ptx::elect_one()) {
       const uint32_t idesc = ptx::umma_idesc_bf16(2 * G2_BM, p.bn, false, false);
-      uint32_t it = 0, tile = 0;
+      int s = 0;
+      uint32_t odd = 0, tile = 0;
       bool ok = true;
       for (int w = cluster_id; w < p.work_items && ok; w += num_clusters, ++tile) {
         const int acc = tile & 1;
         if (!ptx::mbar_wait(&acc_empty[acc], ((tile >> 1) & 1) ^ 1, 1u << 22)) { report_error(p.err, ERR_EPILOGUE_WAIT); ok = false; break; }
         ptx::tc_fence_after();
         const uint32_t d_tmem = tmem_base + acc * G2_ACC_COLS;
-        for (int kb = 0; kb < p.total_kb; ++kb, ++it) {
-          const int s = it % p.stages;
-          if (!ptx::mbar_wait(&full[s], (it / p.stages) & 1, 1u << 20)) { report_error(p.err, ERR_TMA_WAIT); ok = false; break; }
+        for (int kb = 0; kb < p.total_kb; ++kb, advance(s, odd)) {
+          if (!ptx::mbar_wait(&full[s], odd, 1u << 20)) { report_error(p.err, ERR_TMA_WAIT); ok = false; break; }
           ptx::tc_fence_after();
           const uint32_t a_base = ptx::smem_u32(smem + s * STAGE_BYTES), b_base = a_base + A_BYTES;
 #pragma unroll

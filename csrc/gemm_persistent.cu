@@ -1,7 +1,7 @@
 // Persistent bf16 GEMM: one CTA per SM walks a list of (tile, K-split) work items.  Three roles run concurrently and are
 // decoupled by mbarrier rings, so the accumulator read-out of one tile overlaps the MMAs of the next:
 //
-//   warp 0   TMA producer: fills a 4-stage ring of {A 128 x 64, B bn x 64} bf16 tiles across tile boundaries
+//   warp 0   TMA producer: fills a ring of four to eight stages of {A 128 x 64, B bn x 64} bf16 tiles across tile boundaries
 //   warp 1   MMA issuer (one elected lane): tcgen05.mma into one of two TMEM accumulators (256 columns each)
 //   warps 2-5 epilogue: tcgen05.ld of the finished accumulator, conversion, global stores (or fp32 accumulation)
 //
@@ -20,11 +20,11 @@
 
 namespace q38 {
 
-constexpr int P_BM = 128, P_BK = 64, P_STAGES = 4, P_THREADS = 192, P_ACC_COLS = 256;
+constexpr int P_BM = 128, P_BK = 64, P_MAX_STAGES = 8, P_THREADS = 192, P_ACC_COLS = 256;
 
 struct PGemmArgs {
   int M, N, K, batch, bn;
-  int tiles_m, tiles_n, splits, kb_per_split, total_kb, work_items;
+  int tiles_m, tiles_n, splits, kb_per_split, total_kb, work_items, stages;
   void* C;
   long long ldc, c_batch_stride;
   float alpha;
@@ -47,19 +47,19 @@ __global__ void __launch_bounds__(P_THREADS) gemm_persistent_kernel(const __grid
   const uint32_t raw = ptx::smem_u32(smem_raw);
   uint8_t* smem = smem_raw + ((1024u - (raw & 1023u)) & 1023u);
   const int A_BYTES = P_BM * 128, B_BYTES = p.bn * 128, STAGE_BYTES = A_BYTES + B_BYTES;
-  uint64_t* full = reinterpret_cast<uint64_t*>(smem + P_STAGES * STAGE_BYTES);
-  uint64_t* empty = full + P_STAGES;
-  uint64_t* acc_full = empty + P_STAGES;        // [2]
+  uint64_t* full = reinterpret_cast<uint64_t*>(smem + p.stages * STAGE_BYTES);
+  uint64_t* empty = full + P_MAX_STAGES;
+  uint64_t* acc_full = empty + P_MAX_STAGES;        // [2]
   uint64_t* acc_empty = acc_full + 2;           // [2]
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + 2);
-  uint8_t* stage_out = smem + P_STAGES * STAGE_BYTES + 1024;     // [4 warps][2 buffers][32 rows x 128 bytes], 1024-byte aligned
+  uint8_t* stage_out = smem + p.stages * STAGE_BYTES + 1024;     // [4 warps][2 buffers][32 rows x 128 bytes], 1024-byte aligned
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
   if (threadIdx.x == 0) {
     ptx::prefetch_tensormap(&tmA);
     ptx::prefetch_tensormap(&tmB);
     if (TMA_OUT) ptx::prefetch_tensormap(&tmC);
-    for (int s = 0; s < P_STAGES; ++s) { ptx::mbar_init(&full[s], 1); ptx::mbar_init(&empty[s], 1); }
+    for (int s = 0; s < p.stages; ++s) { ptx::mbar_init(&full[s], 1); ptx::mbar_init(&empty[s], 1); }
     for (int a = 0; a < 2; ++a) { ptx::mbar_init(&acc_full[a], 1); ptx::mbar_init(&acc_empty[a], 4); }   // four epilogue warps release an accumulator
     ptx::fence_barrier_init();
   }
@@ -80,16 +80,18 @@ __global__ void __launch_bounds__(P_THREADS) gemm_persistent_kernel(const __grid
     num_kb = min(p.kb_per_split, p.total_kb - kb_begin);
   };
 
+  auto advance = [&](int& s, uint32_t& odd) { if (++s == p.stages) { s = 0; odd ^= 1; } };        // a division by the number of stages would cost each K block
+
   if (warp == 0) {
     if (ptx::elect_one()) {
-      uint32_t it = 0;                                       // global K-block counter: stage = it % STAGES, round = it / STAGES
+      int s = 0;                                             // stage of the K block; its ring has gone round an odd number of times
+      uint32_t odd = 0;
       bool ok = true;
       for (int w = blockIdx.x; w < p.work_items && ok; w += gridDim.x) {
         int bz, m0, n0, kb_begin, num_kb;
         decode(w, bz, m0, n0, kb_begin, num_kb);
-        for (int kb = 0; kb < num_kb; ++kb, ++it) {
-          const int s = it % P_STAGES;
-          if (!ptx::mbar_wait(&empty[s], ((it / P_STAGES) & 1) ^ 1, 1u << 20)) { report_error(p.err, ERR_MMA_WAIT); ok = false; break; }
+        for (int kb = 0; kb < num_kb; ++kb, advance(s, odd)) {
+          if (!ptx::mbar_wait(&empty[s], odd ^ 1, 1u << 20)) { report_error(p.err, ERR_MMA_WAIT); ok = false; break; }
           uint8_t* a_dst = smem + s * STAGE_BYTES;
           uint8_t* b_dst = a_dst + A_BYTES;
           ptx::mbar_expect_tx(&full[s], STAGE_BYTES);
@@ -111,7 +113,8 @@ __global__ void __launch_bounds__(P_THREADS) gemm_persistent_kernel(const __grid
   } else if (warp == 1) {
     if (ptx::elect_one()) {
       const uint32_t idesc = TF32 ? ptx::umma_idesc_tf32(P_BM, p.bn, false, false) : ptx::umma_idesc_bf16(P_BM, p.bn, A_MN, B_MN);
-      uint32_t it = 0, tile = 0;
+      int s = 0;
+      uint32_t odd = 0, tile = 0;
       bool ok = true;
       for (int w = blockIdx.x; w < p.work_items && ok; w += gridDim.x, ++tile) {
         int bz, m0, n0, kb_begin, num_kb;
@@ -121,9 +124,8 @@ __global__ void __launch_bounds__(P_THREADS) gemm_persistent_kernel(const __grid
         if (!ptx::mbar_wait(&acc_empty[acc], ((tile >> 1) & 1) ^ 1, 1u << 22)) { report_error(p.err, ERR_EPILOGUE_WAIT); ok = false; break; }
         ptx::tc_fence_after();
         const uint32_t d_tmem = tmem_base + acc * P_ACC_COLS;
-        for (int kb = 0; kb < num_kb; ++kb, ++it) {
-          const int s = it % P_STAGES;
-          if (!ptx::mbar_wait(&full[s], (it / P_STAGES) & 1, 1u << 20)) { report_error(p.err, ERR_TMA_WAIT); ok = false; break; }
+        for (int kb = 0; kb < num_kb; ++kb, advance(s, odd)) {
+          if (!ptx::mbar_wait(&full[s], odd, 1u << 20)) { report_error(p.err, ERR_TMA_WAIT); ok = false; break; }
           ptx::tc_fence_after();
           const uint32_t a_base = ptx::smem_u32(smem + s * STAGE_BYTES), b_base = a_base + A_BYTES;
 #pragma unroll
@@ -309,7 +311,7 @@ static int pick_splits(int tiles, int total_kb) {
 template <bool A_MN, bool B_MN, bool TF32 = false>
 static void launch_p(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& tc, bool tma_out, const PGemmArgs& p, bool out_fp32, bool accum,
                      cudaStream_t stream) {
-  const int smem = P_STAGES * (P_BM * 128 + p.bn * 128) + 1024 /* alignment */ + 1024 /* barriers */ + 4 * 2 * 4096 /* output staging */;
+  const int smem = p.stages * (P_BM * 128 + p.bn * 128) + 1024 /* alignment */ + 1024 /* barriers */ + 4 * 2 * 4096 /* output staging */;
   const int grid = std::min(p.work_items, kNumSMs);
   Q38_TRACE("[gemm_p] launch grid=%d smem=%d bn=%d items=%d splits=%d kb=%d tma_out=%d fp32=%d acc=%d amn=%d bmn=%d\n", grid, smem, p.bn, p.work_items, p.splits,
             p.total_kb, (int)tma_out, (int)out_fp32, (int)accum, (int)A_MN, (int)B_MN);
@@ -374,6 +376,9 @@ void gemm_bf16_persistent(const at::Tensor& a_, const at::Tensor& b_, const at::
   p.M = M; p.N = N; p.K = K; p.batch = batch; p.bn = bn;
   p.tiles_m = (M + P_BM - 1) / P_BM; p.tiles_n = (N + bn - 1) / bn;
   p.total_kb = (K + bk - 1) / bk;
+  // As many stages as fit beside the output staging: a narrow tile (the stream projections, N = 56 .. 128) loads little per stage, and four of them
+  // keep 64 KB of A per SM in flight, less than the latency of memory asks for (18 projections of a nine-layer prefill, 16384 x 56 x 1792 tf32: 510 -> 428 us).
+  p.stages = std::min(P_MAX_STAGES, (227 * 1024 - 2048 - 4 * 2 * 4096) / (P_BM * 128 + bn * 128));
   int nsplit = 1;
   if (accumulate && out_fp32) {
     if (splits > 0) nsplit = (int)splits;
