@@ -964,10 +964,10 @@ extern "C" int q38_moe_sort_static(const int* expert_of_pair, int P, int experts
   int* scratch = sort_static_scratch_for_current_device();
   if (scratch == nullptr) return Q38_NOALLOC_CUDA_ERROR;
   // Every word of the scratch that the scan and scatter kernels read is written by the histogram kernel first.
-  launch(moe_hist_kernel, nblocks, SORT_THREADS, 0, stream, expert_of_pair, P, experts, scratch, nullptr);
-  launch(moe_scan_kernel, 1, 64 * SCAN_SEGS, 0, stream, scratch, nblocks, experts, offsets, sched, max_tiles, G_BM);
-  launch(moe_scatter_kernel, nblocks, SORT_THREADS, 0, stream, expert_of_pair, P, experts, scratch, perm, inv_perm);
-  if (cudaGetLastError() != cudaSuccess) return Q38_NOALLOC_CUDA_ERROR;
+  // A launch that fails returns its error, which also stays for the caller's cudaGetLastError; nothing is launched after it.
+  if (try_launch(moe_hist_kernel, nblocks, SORT_THREADS, 0, stream, expert_of_pair, P, experts, scratch, nullptr) != cudaSuccess) return Q38_NOALLOC_CUDA_ERROR;
+  if (try_launch(moe_scan_kernel, 1, 64 * SCAN_SEGS, 0, stream, scratch, nblocks, experts, offsets, sched, max_tiles, G_BM) != cudaSuccess) return Q38_NOALLOC_CUDA_ERROR;
+  if (try_launch(moe_scatter_kernel, nblocks, SORT_THREADS, 0, stream, expert_of_pair, P, experts, scratch, perm, inv_perm) != cudaSuccess) return Q38_NOALLOC_CUDA_ERROR;
   count_launch(3);
   return Q38_NOALLOC_OK;
 }

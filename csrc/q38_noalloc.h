@@ -36,7 +36,7 @@ enum {
   Q38_NOALLOC_OK = 0,
   Q38_NOALLOC_TOO_LARGE = 1,      // P > Q38_SORT_STATIC_MAX_PAIRS or experts > 64
   Q38_NOALLOC_BAD_ARGUMENT = 2,   // null pointer, non-positive size, or a schedule buffer that is too small
-  Q38_NOALLOC_CUDA_ERROR = 3,     // a CUDA runtime call failed (set-up or launch); see cudaGetLastError
+  Q38_NOALLOC_CUDA_ERROR = 3,     // a CUDA runtime call failed (set-up or launch); its error is left for cudaGetLastError
 };
 
 #ifdef __cplusplus

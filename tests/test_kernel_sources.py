@@ -76,3 +76,16 @@ def test_kernels_wait_for_the_kernels_before_them():
             end = body.find("\n}")
             assert "grid_wait();" in body[:end], (path.name, name)
         assert "<<<" not in code, path.name
+
+
+def test_c_entry_points_report_launch_errors():
+    """`launch` throws; an exception that crosses a C boundary ends the caller's process.  Functions with C linkage use `try_launch`, and nothing
+    else that throws."""
+    found = 0
+    for path in sorted(CSRC.glob("*.cu")) + sorted(CSRC.glob("*.cpp")):
+        code = code_of(path.name)
+        for m in re.finditer(r'extern "C"[^{;]*\)\s*(?:noexcept\s*)?\{', code):
+            body = code[m.start():code.find("\n}", m.start())]
+            found += 1
+            assert not re.search(r"\blaunch\(|C10_CUDA_|TORCH_CHECK|\bat::", body), path.name
+    assert found

@@ -7,6 +7,9 @@ via ctypes with raw device pointers, twice in a row (the second call reuses the 
 different problem), and compares each result with the regular `moe_sort` operator.  The file name makes pytest collect
 it last."""
 import ctypes
+import subprocess
+import sys
+from pathlib import Path
 
 import pytest
 import torch
@@ -67,3 +70,38 @@ def test_static_scratch_sort_matches_operator():
     assert fn(idx.data_ptr(), 100, 65, perm.data_ptr(), inv.data_ptr(), offsets.data_ptr(), sched.data_ptr(), 200, ctypes.c_void_p(stream.cuda_stream)) == 1
     assert fn(None, 100, 8, perm.data_ptr(), inv.data_ptr(), offsets.data_ptr(), sched.data_ptr(), 200, ctypes.c_void_p(stream.cuda_stream)) == 2
     ops.check_errors()
+
+
+FAILED_LAUNCH = """
+import ctypes, torch
+from q38 import ops
+ops.load()
+fn = ctypes.CDLL(ops.loaded_library()).q38_moe_sort_static
+fn.argtypes = [ctypes.c_void_p, ctypes.c_int, ctypes.c_int] + [ctypes.c_void_p] * 4 + [ctypes.c_int, ctypes.c_void_p]
+words = torch.zeros(7, 4096, dtype=torch.int32, device="cuda")
+args = [words[0].data_ptr(), 1024, 8] + [words[i].data_ptr() for i in range(1, 5)] + [16]
+assert fn(*args, torch.cuda.current_stream().cuda_stream) == 0          # resolves the scratch outside of the capture
+torch.cuda.synchronize()
+runtime = ctypes.CDLL(next(line.split()[-1] for line in open("/proc/self/maps") if "libcudart" in line))
+runtime.cudaGetErrorName.restype = ctypes.c_char_p
+stream, graph = torch.cuda.Stream(), ctypes.c_void_p()
+handle = ctypes.c_void_p(stream.cuda_stream)
+assert runtime.cudaStreamBeginCapture(handle, 2) == 0
+assert runtime.cudaStreamSynchronize(handle) != 0                       # not allowed in a capture: the runtime refuses it and invalidates the capture
+runtime.cudaGetLastError()
+code = fn(*args, handle)
+last = runtime.cudaGetErrorName(runtime.cudaGetLastError()).decode()
+runtime.cudaStreamEndCapture(handle, ctypes.byref(graph))
+runtime.cudaGetLastError()
+print("code", code, last)
+assert fn(*args, torch.cuda.current_stream().cuda_stream) == 0          # the context is as it was
+torch.cuda.synchronize()
+"""
+
+
+def test_failed_launch_is_a_status():
+    """A launch that the runtime refuses (a stream whose capture has become invalid) comes back as a status with the error left for
+    cudaGetLastError.  In a child process: an exception through the C boundary would end it."""
+    child = subprocess.run([sys.executable, "-c", FAILED_LAUNCH], cwd=Path(__file__).resolve().parents[1], capture_output=True, text=True, timeout=300)
+    assert child.returncode == 0, child.stderr[-2000:]
+    assert child.stdout.split()[:2] == ["code", "3"] and "CaptureInvalidated" in child.stdout, child.stdout
