@@ -301,6 +301,7 @@ __global__ void __launch_bounds__(PG_THREADS) grouped_persistent_kernel(const __
         }
       } else
       for (int c0 = 16 * group; c0 < p.bn; c0 += 32) {
+        __syncwarp();                                       // the read takes whole warps; rows past the expert's last store nothing
         uint32_t r[16];
         ptx::tmem_ld_32x32b_x16(lane_addr + c0, r);
         const int c = n0 + c0;

@@ -263,6 +263,7 @@ __global__ void __launch_bounds__(MX_THREADS) mxfp8_grouped_gemm_kernel(const __
       const bool live = r_local < rows_valid;
       __nv_bfloat16* o_row = p.out + (long long)(a_row0 + r_local) * p.ldo;
       for (int c0 = 0; c0 < p.bn; c0 += 16) {
+        __syncwarp();                                    // the read takes whole warps; rows past the expert's last store nothing
         uint32_t r[16];
         ptx::tmem_ld_32x32b_x16(lane_addr + c0, r);
         ptx::tmem_ld_wait();

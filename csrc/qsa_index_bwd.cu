@@ -303,11 +303,11 @@ __global__ void __launch_bounds__(IB_THREADS, 1) qsa_indexer_bwd_kernel(const __
       const float wv = w_s[64 * h + tin];
       float dw = 0.f;
       for (int x = half; x < 2; ++x) {
+        __syncwarp();                                                    // the read takes whole warps; with 1 or 3 heads only half of the lanes store
         uint32_t e[32];
         ptx::tmem_ld_32x32b_x32(tmem + COL_E + 64 * u + 32 * x + (uint32_t(32 * quarter) << 16), e);
         ptx::tmem_ld_wait();
-        if (h >= p.NI) continue;
-        if (half == 0) {
+        if (half == 0 && h < p.NI) {
           const uint4* q = reinterpret_cast<const uint4*>(p.qi + row * 64 + 32 * x);
 #pragma unroll
           for (int v = 0; v < 4; ++v) {
@@ -318,13 +318,13 @@ __global__ void __launch_bounds__(IB_THREADS, 1) qsa_indexer_bwd_kernel(const __
               dw += __uint_as_float(ys[k] << 16) * __uint_as_float(e[8 * v + 2 * k]) + __uint_as_float(ys[k] & 0xffff0000u) * __uint_as_float(e[8 * v + 2 * k + 1]);
           }
         }
-        if (x != half) continue;
-        if (p.part != nullptr) {
+        const bool store = x == half && h < p.NI;
+        if (store && p.part != nullptr) {
           float4* dst = reinterpret_cast<float4*>(p.part + ((long long)z * p.B * p.NI * p.S + row) * 64 + 32 * x);
 #pragma unroll
           for (int v = 0; v < 8; ++v)
             dst[v] = make_float4(__uint_as_float(e[4 * v]) * wv, __uint_as_float(e[4 * v + 1]) * wv, __uint_as_float(e[4 * v + 2]) * wv, __uint_as_float(e[4 * v + 3]) * wv);
-        } else {
+        } else if (store) {
           uint4* dst = reinterpret_cast<uint4*>(p.dqi + row * 64 + 32 * x);
           auto pk = [&](int k) { return bf16_pair(make_float2(__uint_as_float(e[k]) * wv, __uint_as_float(e[k + 1]) * wv)); };
 #pragma unroll

@@ -89,3 +89,32 @@ def test_c_entry_points_report_launch_errors():
             found += 1
             assert not re.search(r"\blaunch\(|C10_CUDA_|TORCH_CHECK|\bat::", body), path.name
     assert found
+
+
+# conditions of a `continue` that whole warps agree on
+WARP_UNIFORM = r"k\.num_kb == 0|EPI == \w+|TMA_OUT|jb > row0 / 64 \+ \(quarter >> 1\)"
+
+
+@pytest.mark.parametrize("name", sorted(p.name for p in CSRC.glob("*.cu") if "tmem_ld" in p.read_text()))
+def test_no_lane_skips_ahead_of_a_tensor_memory_read(name):
+    """tcgen05.ld and tcgen05.st need all lanes of a warp.  Lanes that leave a round of a loop early (`continue` under a condition of their own) meet
+    the others at a __syncwarp() before the next round's read."""
+    code = code_of(name)
+    for m in re.finditer(r"\bcontinue;", code):
+        heads, opened = [], []
+        for i, ch in enumerate(code[:m.start()]):
+            if ch == "{":
+                heads.append(code[code.rfind("\n", 0, i) + 1:i])
+                opened.append(i)
+            elif ch == "}":
+                heads.pop()
+                opened.pop()
+        loop = max(k for k, head in enumerate(heads) if re.search(r"\b(for|while) \(", head))
+        depth, end = 1, opened[loop] + 1
+        while depth:
+            depth += {"{": 1, "}": -1}.get(code[end], 0)
+            end += 1
+        body = code[opened[loop] + 1:end]
+        condition = code[code.rfind("\n", 0, m.start()) + 1:m.start()] + " ".join(heads[loop + 1:])
+        if re.search(r"tmem_(ld|st)_32", body) and not re.search(WARP_UNIFORM, condition):
+            assert body.lstrip().startswith("__syncwarp();"), (name, condition)
