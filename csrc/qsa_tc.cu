@@ -35,10 +35,13 @@ struct QsaTcArgs {
 };
 
 constexpr float EXP2_C0 = 1.f, EXP2_C1 = 0.693147004f, EXP2_C2 = 0.240222424f, EXP2_C3 = 0.0555073358f, EXP2_C4 = 0.00967151299f, EXP2_C5 = 0.00132647273f;
-// 2^x for two x <= 0 on the FMA pipe: x = i + f with i the nearest whole number, a polynomial for 2^f on [-1/2, 1/2] (degree 5, fitted for the smallest
-// largest relative error: 2e-7 in fp32, as ex2.approx), i added to the exponent.  Below 2^-126 the result is that.
+// 2^x for two x <= 0 on the FMA pipe.  Range reduction as in Cody and Waite, Software Manual for the Elementary Functions: x = i + f with i the nearest
+// whole number, found by adding 1.5 * 2^23 (whole numbers end up in the low bits), a polynomial for 2^f on [-1/2, 1/2] (degree 5, fitted with
+// Remez' exchange for the smallest largest relative error: 2e-7 in fp32, as ex2.approx), times 2^i.  Below 2^-126 the result is that.  A NaN stays one,
+// as in ex2.approx: the clamp keeps it and the product carries it (adding i to the exponent bits would turn it into a number).
+__device__ __forceinline__ float max_or_nan(float a, float b) { float y; asm("max.NaN.f32 %0, %1, %2;" : "=f"(y) : "f"(a), "f"(b)); return y; }
 __device__ __forceinline__ float2 poly_exp2(float2 x) {
-  const uint64_t magic = pair2(12582912.f, 12582912.f), v = pair2(fmaxf(x.x, -126.f), fmaxf(x.y, -126.f));        // 1.5 * 2^23: whole numbers end up in the low bits
+  const uint64_t magic = pair2(12582912.f, 12582912.f), v = pair2(max_or_nan(x.x, -126.f), max_or_nan(x.y, -126.f));
   const uint64_t t = add2(v, magic), f = add2(v, mul2(add2(t, pair2(-12582912.f, -12582912.f)), pair2(-1.f, -1.f)));
   uint64_t p = pair2(EXP2_C5, EXP2_C5);
   p = fma2(p, f, pair2(EXP2_C4, EXP2_C4));
@@ -46,8 +49,8 @@ __device__ __forceinline__ float2 poly_exp2(float2 x) {
   p = fma2(p, f, pair2(EXP2_C2, EXP2_C2));
   p = fma2(p, f, pair2(EXP2_C1, EXP2_C1));
   p = fma2(p, f, pair2(EXP2_C0, EXP2_C0));
-  const float2 i = unpair(t), r = unpair(p);
-  return make_float2(__int_as_float(__float_as_int(r.x) + (__float_as_int(i.x) << 23)), __int_as_float(__float_as_int(r.y) + (__float_as_int(i.y) << 23)));
+  const float2 i = unpair(t);
+  return unpair(mul2(p, pair2(__int_as_float((__float_as_int(i.x) << 23) + 0x3f800000), __int_as_float((__float_as_int(i.y) << 23) + 0x3f800000))));
 }
 
 __global__ void __launch_bounds__(QT_THREADS, 2) qsa_block_stats_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK, QsaTcArgs p) {

@@ -68,3 +68,38 @@ def test_values_as_a_transposed_view(ops, nkv):  # noqa: F811
         assert torch.equal(a, b) if i < 3 else ((a.float() - b.float()).norm() <= 4e-3 * b.float().norm())
     with pytest.raises(RuntimeError, match="contiguous bf16"):
         lib.qsa_attn_fwd(q, k, v.expand(B, nkv, S, 64)[..., ::1].transpose(2, 3).contiguous().transpose(2, 3), None, None, 0.125)
+
+
+def block_stats(ops, q, k):  # noqa: F811
+    stats = ops.load().qsa_block_stats_tc(q, k, 0.125, ops.error_flag()).double()
+    return stats[..., 0], stats[..., 1]
+
+
+@gpu
+@pytest.mark.parametrize("at", range(8))
+@pytest.mark.parametrize("bad", [float("nan"), float("inf")])
+def test_block_statistics_show_a_bad_key(ops, at, bad):  # noqa: F811
+    """Full blocks take two of every eight exponentials through a polynomial: a key whose scores are NaN or infinite shows in the sum wherever it stands."""
+    gen = torch.Generator(device="cuda").manual_seed(at)
+    q, k = (torch.randn(1, h, 256, 64, device="cuda", generator=gen).to(torch.bfloat16) for h in (2, 1))
+    k[0, 0, 8 * at + at] = bad
+    m, total = block_stats(ops, q, k)
+    assert not total[0, :, 64:, 0].isfinite().any() and not total[0, :, 8 * at + at:64, 0].isfinite().any()
+    assert total[0, :, 192:, 1:3].isfinite().all()
+
+
+@gpu
+@pytest.mark.parametrize("alone", [False, True])
+def test_block_statistics_accuracy(ops, alone):  # noqa: F811
+    """Against 64 bits, with all keys and with the sums left to the keys that go through the polynomial (`alone`: the others score 60 lower)."""
+    gen = torch.Generator(device="cuda").manual_seed(7)
+    q, k = (torch.randn(1, h, 1024, 64, device="cuda", generator=gen).to(torch.bfloat16) for h in (4, 1))
+    if alone:
+        q[..., 0], k[..., 0] = 8, 0
+        k.view(1, 1, 128, 8, 64)[:, :, :, :6, 0] = -60
+    m, total = block_stats(ops, q, k)
+    score = (q.double() @ k.double().transpose(-1, -2) / 8).unflatten(-1, (16, 64))
+    full = torch.arange(1024, device="cuda")[:, None] // 64 > torch.arange(16, device="cuda")[None]
+    err = ((m + total.log()) - score.logsumexp(-1))[:, :, full].abs()
+    # fp32 throughout: 64 products of at most 500 in all (2^-24 each), an argument of the exponential of at most 200 (2^-24), an exponential of 2^-21
+    assert err.max() < 500 / 8 * 2 ** -23 + 200 * 2 ** -24 + 2 ** -21
