@@ -161,10 +161,13 @@ __global__ void __launch_bounds__(IB_THREADS, 1) qsa_indexer_bwd_kernel(const __
                            (u | k) != 0);
         if (u == 1) ptx::umma_commit(&dk_full[m & 1]);
         if (m + 1 < n) ok = scores(m + 1, u);
+        // an even query block reaches the first half of its last tile only: zeros times a later block's keys would be NaN where those are not finite
+        const int steps = z + m * p.Z == KT - 1 && (i & 1) == 0 ? 4 : 8;
 #pragma unroll
         for (int k = 0; k < 8; ++k)
-          ptx::umma_f16(tmem + COL_E + 64 * u, ptx::umma_smem_desc_sw128(eb + k * 2048, IB_TILE, 1024), ptx::umma_smem_desc_sw128(kb + k * 2048, IB_TILE, 1024), id_e,
-                        (m | k) != 0);
+          if (k < steps)
+            ptx::umma_f16(tmem + COL_E + 64 * u, ptx::umma_smem_desc_sw128(eb + k * 2048, IB_TILE, 1024), ptx::umma_smem_desc_sw128(kb + k * 2048, IB_TILE, 1024), id_e,
+                          (m | k) != 0);
         ptx::umma_commit(&e_free[u]);
         if (u == 1) ptx::umma_commit(&k_empty[m % IB_STAGES]);
       }
@@ -194,7 +197,7 @@ __global__ void __launch_bounds__(IB_THREADS, 1) qsa_indexer_bwd_kernel(const __
       __syncwarp();
       if (lane == 0) {
         const int row = (z + m * p.Z) * 128 + 32 * quarter;
-        if (row < p.S) {
+        if (row < (i + 1) * 64) {                                        // later keys get nothing from this block (nor NaN from its queries)
           ptx::tma_reduce_add_3d(&tmDK, out, 0, row, b);
           ptx::tma_reduce_add_3d(&tmDK, out + 4096, 32, row, b);
         }

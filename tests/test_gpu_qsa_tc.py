@@ -103,3 +103,24 @@ def test_block_statistics_accuracy(ops, alone):  # noqa: F811
     err = ((m + total.log()) - score.logsumexp(-1))[:, :, full].abs()
     # fp32 throughout: 64 products of at most 500 in all (2^-24 each), an argument of the exponential of at most 200 (2^-24), an exponential of 2^-21
     assert err.max() < 500 / 8 * 2 ** -23 + 200 * 2 ** -24 + 2 ** -21
+
+
+@gpu
+@pytest.mark.parametrize("block", [0, 1, 2, 3])
+def test_indexer_backward_keeps_a_nan_in_its_blocks(ops, block):  # noqa: F811
+    """Key tiles hold two blocks.  A key that is not finite reaches the gradients of no earlier query block, a query none of later keys."""
+    gen = torch.Generator(device="cuda").manual_seed(block)
+    qi, ki = (torch.randn(s, device="cuda", generator=gen).to(torch.bfloat16) for s in ((1, 4, 320, 64), (1, 320, 64)))
+    wi, dblse = torch.randn(1, 320, 4, device="cuda", generator=gen), torch.randn(1, 320, 5, device="cuda", generator=gen)
+    lib, later = ops.load(), slice(64 * block + 64, None)
+    clean = lib.qsa_indexer_bwd(qi, ki, wi, lib.qsa_indexer_fwd(qi, ki, wi, 0.125), dblse, 1.0, 0.125)
+    for bad in (float("nan"), float("inf")):
+        k = ki.clone()
+        k[:, later] = bad
+        dq, _, dw = lib.qsa_indexer_bwd(qi, k, wi, lib.qsa_indexer_fwd(qi, k, wi, 0.125), dblse, 1.0, 0.125)
+        assert torch.equal(dq[:, :, :64 * block + 64], clean[0][:, :, :64 * block + 64]) and torch.equal(dw[:, :64 * block + 64], clean[2][:, :64 * block + 64])
+        q = qi.clone()
+        q[:, :, :64 * block + 64] = bad
+        dk = lib.qsa_indexer_bwd(q, ki, wi, lib.qsa_indexer_fwd(q, ki, wi, 0.125), dblse, 1.0, 0.125)[1]
+        # fp32 sums whose order varies, rounded to bf16 once
+        assert (dk[:, later].float() - clean[1][:, later].float()).norm() <= 4e-3 * clean[1][:, later].float().norm()
