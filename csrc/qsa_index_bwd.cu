@@ -7,18 +7,21 @@
 // One CTA per (64 queries, batch, z) walks key tiles of 128 keys (z, z + Z, ...).  The 64 queries are two units of 32 queries x 4 heads = 128
 // columns; a unit's scores S^T = K Q^T (128 keys x 128 columns) come into TMEM with a key per lane, so that one thread sees all heads of its
 // (query, key) pairs: it rounds q.k to bf16, forms the score, one exponential, and hands on
-//     dI [S_h > 0]       to shared memory, the A operand (transposed) of E += (..)^T K        (accumulated over the loop, two units)
+//     dI [S_h > 0]       to shared memory, the A operand (transposed) of E += (..)^T K        (accumulated over the loop, two units), as two bf16:
+//                        upper bits and what they leave, so that E, and with it dq and dw, sees dI in sixteen bits
 //     dI w_h [S_h > 0]   to TMEM over its own scores, the A operand of dk += (..) Q           (over the two units, then added to memory)
 // Columns are ordered (16-query half, head, query), so that each of a lane's two threads overwrites only scores it has read itself.
 // E needs no weights: dq and dw are both read off it at the end, dw without a sum over lanes.  Key gradients leave through the TMA unit
 // (fp32 adds of 32 x 32 boxes); query gradients are stored, or left in one slice per z that a small kernel adds in ascending order, so they have the same
 // bits in every run.
 //
-// Bound by the instructions per element (16 compute warps issue 0.6 per cycle and scheduler; rounding, masks and packing run at half rate), not by
-// the products (a quarter of the tensor pipe).  An SM takes 2.9 us per key tile.  Two warp-MMA passes with the scores formed twice stood here: four
-// sequences of 4096 with four heads 405 -> 101 us, one 149 -> 60, one of 1024 tokens 33 -> 19.  dk goes before the unit's next scores in the queue and E
-// after them, so that compute warps wait for two products instead of four (152 -> 141), and all sequences' longest query blocks start first (137 -> 101).
-// Against 64 bits dq and dk err as before, dw 20 % less.
+// Bound by the instructions per element (16 compute warps; rounding, masks and packing run at half rate), not by
+// the products.  Two warp-MMA passes with the scores formed twice stood here: four
+// sequences of 4096 with four heads 405 -> 120 us, one 149 -> 70, one of 1024 tokens 33 -> 22.  dk goes before the unit's next scores in the queue and E
+// after them, so that compute warps wait for two products instead of four, and all sequences' longest query blocks start first.
+// With dI in one bf16 it took 98, 59 and 20 us (13 us of the difference are the second operand's stores, 7 its products, 2 the ring of two stages and the single key-gradient
+// boxes that make room for it), but the head weights' gradient, which the passes before summed from fp32 dI, then saw eight bits of it.  Against 64 bits (four sequences of 4096,
+// 2-norm of the error over that of the gradient): dw 6.9e-4 (9.0e-4 with one bf16, 11.2e-4 in the passes before, which rounded q.k there), dq 3.17e-3 (3.49e-3, 3.49e-3), dk 3.90e-3 in all three.
 //
 // Roles: a warp for TMA, blse and dblse, an MMA warp, four warps for the key gradients, eight compute warps per unit.  Every mbarrier
 // wait is bounded and reports through the error word.
@@ -34,10 +37,10 @@
 namespace q38 {
 namespace {
 
-constexpr int IB_HEADS = 4, IB_STAGES = 3, IB_WARPS = 22, IB_THREADS = 32 * IB_WARPS;
+constexpr int IB_HEADS = 4, IB_STAGES = 2, IB_WARPS = 22, IB_THREADS = 32 * IB_WARPS;
 constexpr int IB_TILE = 128 * 128;                                      // bytes: 128 rows of 64 bf16
 constexpr uint32_t COL_S = 0, COL_E = 256, COL_DK = 384;                // two of each: 128, 64 and 64 columns
-constexpr int IB_SMEM = (2 + IB_STAGES + 4 + 2) * IB_TILE + 2 * 256 * 4 + IB_HEADS * 64 * 4 + 256;
+constexpr int IB_SMEM = (2 + IB_STAGES + 8 + 1) * IB_TILE + 2 * 256 * 4 + IB_HEADS * 64 * 4 + 256;
 
 struct IndexBwdArgs {
   const __nv_bfloat16* qi;
@@ -58,8 +61,8 @@ __global__ void __launch_bounds__(IB_THREADS, 1) qsa_indexer_bwd_kernel(const __
   const int KT = (i + 2) / 2, n = z < KT ? (KT - z + p.Z - 1) / p.Z : 0;
   if (n == 0) return;
   if (ptx::smem_u32(smem) & 1023u) { if (threadIdx.x == 0) report_error(p.err, ERR_BOUNDS); return; }
-  uint8_t *q_tile = smem, *k_ring = q_tile + 2 * IB_TILE, *e_tile = k_ring + IB_STAGES * IB_TILE, *dk_out = e_tile + 4 * IB_TILE;
-  float* par = reinterpret_cast<float*>(dk_out + 2 * IB_TILE);           // [2 buffers][2 key blocks][blse, dblse gscale][64 queries]
+  uint8_t *q_tile = smem, *k_ring = q_tile + 2 * IB_TILE, *e_tile = k_ring + IB_STAGES * IB_TILE, *dk_out = e_tile + 8 * IB_TILE;            // e_tile: [upper, lower bits][unit][16-query half]
+  float* par = reinterpret_cast<float*>(dk_out + IB_TILE);           // [2 buffers][2 key blocks][blse, dblse gscale][64 queries]
   float* w_s = par + 2 * 256;                                            // [head][64 queries], times scale
   uint64_t* bars = reinterpret_cast<uint64_t*>(w_s + IB_HEADS * 64);
   uint64_t *q_full = bars, *k_full = bars + 1, *k_empty = k_full + IB_STAGES, *s_full = k_empty + IB_STAGES, *e_free = s_full + 2, *e_full = e_free + 2,
@@ -163,11 +166,14 @@ __global__ void __launch_bounds__(IB_THREADS, 1) qsa_indexer_bwd_kernel(const __
         if (m + 1 < n) ok = scores(m + 1, u);
         // an even query block reaches the first half of its last tile only: zeros times a later block's keys would be NaN where those are not finite
         const int steps = z + m * p.Z == KT - 1 && (i & 1) == 0 ? 4 : 8;
+        for (int low = 0; low < 2; ++low) {
+          const uint32_t ab = eb + low * 4 * IB_TILE;
 #pragma unroll
-        for (int k = 0; k < 8; ++k)
-          if (k < steps)
-            ptx::umma_f16(tmem + COL_E + 64 * u, ptx::umma_smem_desc_sw128(eb + k * 2048, IB_TILE, 1024), ptx::umma_smem_desc_sw128(kb + k * 2048, IB_TILE, 1024), id_e,
-                          (m | k) != 0);
+          for (int k = 0; k < 8; ++k)
+            if (k < steps)
+              ptx::umma_f16(tmem + COL_E + 64 * u, ptx::umma_smem_desc_sw128(ab + k * 2048, IB_TILE, 1024), ptx::umma_smem_desc_sw128(kb + k * 2048, IB_TILE, 1024), id_e,
+                            (m | low | k) != 0);
+        }
         ptx::umma_commit(&e_free[u]);
         if (u == 1) ptx::umma_commit(&k_empty[m % IB_STAGES]);
       }
@@ -175,33 +181,31 @@ __global__ void __launch_bounds__(IB_THREADS, 1) qsa_indexer_bwd_kernel(const __
     }
   } else if (warp < 6) {
     const int quarter = warp & 3;
-    uint8_t* out = dk_out + (warp - 2) * 8192;                           // two boxes of 32 rows x 32 dims
+    uint8_t* out = dk_out + (warp - 2) * 4096;                           // a box of 32 rows x 32 dims
     for (int m = 0; m < n; ++m) {
       if (!ptx::mbar_wait_warp(&dk_full[m & 1], (m >> 1) & 1, 1u << 22)) { report_error(p.err, ERR_EPILOGUE_WAIT); break; }
       ptx::tc_fence_after();
-      uint32_t x[32], y[32];
-      ptx::tmem_ld_32x32b_x32(tmem + COL_DK + 64 * (m & 1) + (uint32_t(32 * quarter) << 16), x);
-      ptx::tmem_ld_32x32b_x32(tmem + COL_DK + 64 * (m & 1) + 32 + (uint32_t(32 * quarter) << 16), y);
+      uint32_t x[2][32];
+      ptx::tmem_ld_32x32b_x32(tmem + COL_DK + 64 * (m & 1) + (uint32_t(32 * quarter) << 16), x[0]);
+      ptx::tmem_ld_32x32b_x32(tmem + COL_DK + 64 * (m & 1) + 32 + (uint32_t(32 * quarter) << 16), x[1]);
       ptx::tmem_ld_wait();
       ptx::tc_fence_before();
-      if (lane == 0) ptx::bulk_wait_read<0>();                           // the boxes of the tile before have been read
       __syncwarp();
       if (lane == 0) ptx::mbar_arrive(&dk_empty[m & 1]);
+      const int row = (z + m * p.Z) * 128 + 32 * quarter;
 #pragma unroll
-      for (int v = 0; v < 8; ++v) {
-        const int at = lane * 128 + ((v ^ (lane & 7)) << 4);
-        *reinterpret_cast<uint4*>(out + at) = make_uint4(x[4 * v], x[4 * v + 1], x[4 * v + 2], x[4 * v + 3]);
-        *reinterpret_cast<uint4*>(out + 4096 + at) = make_uint4(y[4 * v], y[4 * v + 1], y[4 * v + 2], y[4 * v + 3]);
-      }
-      ptx::fence_proxy_async();
-      __syncwarp();
-      if (lane == 0) {
-        const int row = (z + m * p.Z) * 128 + 32 * quarter;
-        if (row < (i + 1) * 64) {                                        // later keys get nothing from this block (nor NaN from its queries)
-          ptx::tma_reduce_add_3d(&tmDK, out, 0, row, b);
-          ptx::tma_reduce_add_3d(&tmDK, out + 4096, 32, row, b);
+      for (int half = 0; half < 2; ++half) {
+        if (lane == 0) ptx::bulk_wait_read<0>();                         // the box before has been read
+        __syncwarp();
+#pragma unroll
+        for (int v = 0; v < 8; ++v)
+          *reinterpret_cast<uint4*>(out + lane * 128 + ((v ^ (lane & 7)) << 4)) = make_uint4(x[half][4 * v], x[half][4 * v + 1], x[half][4 * v + 2], x[half][4 * v + 3]);
+        ptx::fence_proxy_async();
+        __syncwarp();
+        if (lane == 0) {
+          if (row < (i + 1) * 64) ptx::tma_reduce_add_3d(&tmDK, out, 32 * half, row, b);       // later keys get nothing from this block (nor NaN from its queries)
+          ptx::bulk_commit();
         }
-        ptx::bulk_commit();
       }
     }
     if (lane == 0) ptx::bulk_wait<0>();
@@ -273,6 +277,10 @@ __global__ void __launch_bounds__(IB_THREADS, 1) qsa_indexer_bwd_kernel(const __
       if (!ptx::mbar_wait_warp(&e_free[u], (m & 1) ^ 1, 1u << 22)) { report_error(p.err, ERR_EPILOGUE_WAIT); ok = false; break; }
       // [S > 0] as a bit mask per bf16 (the values are not negative)
       auto mask = [&](int at) { return __hgt2_mask(*reinterpret_cast<const __nv_bfloat162*>(&rl[at]), __float2bfloat162_rn(0.f)); };
+      auto store = [&](int low, int h, int c) {
+        *reinterpret_cast<uint4*>(e_row + low * 4 * IB_TILE + (((2 * h + c) ^ (r & 7)) << 4)) =
+            make_uint4(dI[4 * c] & rl[8 * h + 4 * c], dI[4 * c + 1] & rl[8 * h + 4 * c + 1], dI[4 * c + 2] & rl[8 * h + 4 * c + 2], dI[4 * c + 3] & rl[8 * h + 4 * c + 3]);
+      };
 #pragma unroll
       for (int h = 0; h < IB_HEADS; ++h) {
         uint32_t ds[8];
@@ -287,10 +295,14 @@ __global__ void __launch_bounds__(IB_THREADS, 1) qsa_indexer_bwd_kernel(const __
         }
         ptx::tmem_st_32x32b_x8(own + 8 * h, ds);
 #pragma unroll
-        for (int c = 0; c < 2; ++c)
-          *reinterpret_cast<uint4*>(e_row + (((2 * h + c) ^ (r & 7)) << 4)) =
-              make_uint4(dI[4 * c] & rl[8 * h + 4 * c], dI[4 * c + 1] & rl[8 * h + 4 * c + 1], dI[4 * c + 2] & rl[8 * h + 4 * c + 2], dI[4 * c + 3] & rl[8 * h + 4 * c + 3]);
+        for (int c = 0; c < 2; ++c) store(0, h, c);
       }
+#pragma unroll
+      for (int e = 0; e < 8; ++e) dI[e] = bf16_pair(unpair(fma2(widen_pair(dI[e]), minus, d[e])));      // what the upper bits leave
+#pragma unroll
+      for (int h = 0; h < IB_HEADS; ++h)
+#pragma unroll
+        for (int c = 0; c < 2; ++c) store(1, h, c);
       ptx::tmem_st_wait();
       ptx::tc_fence_before();
       ptx::fence_proxy_async();

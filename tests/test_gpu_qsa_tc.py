@@ -124,3 +124,28 @@ def test_indexer_backward_keeps_a_nan_in_its_blocks(ops, block):  # noqa: F811
         dk = lib.qsa_indexer_bwd(q, ki, wi, lib.qsa_indexer_fwd(q, ki, wi, 0.125), dblse, 1.0, 0.125)[1]
         # fp32 sums whose order varies, rounded to bf16 once
         assert (dk[:, later].float() - clean[1][:, later].float()).norm() <= 4e-3 * clean[1][:, later].float().norm()
+
+
+@gpu
+@pytest.mark.parametrize("B,nb", [(1, 1), (1, 21), (4, 64)])
+def test_indexer_weight_gradient_sees_more_than_bf16(ops, B, nb):  # noqa: F811
+    """dw = scale sum_s dI relu(q.k) against 64 bits, with the scores inside dI rounded to bf16 as the kernels do.  dI enters with sixteen bits: 2^-17 per term,
+    2^-20 from the exponential's argument, and where a score falls to the other side of a rounding boundary 2^-8 of it, once in ten thousand: 2^-13 in
+    all.  (dI in one bf16: 5e-4.)"""
+    S = 64 * nb
+    gen = torch.Generator(device="cuda").manual_seed(nb)
+    qi, ki = (torch.randn(s, device="cuda", generator=gen).to(torch.bfloat16) for s in ((B, 4, S, 64), (B, S, 64)))
+    wi, dblse = torch.randn(B, S, 4, device="cuda", generator=gen) / 2, torch.randn(B, S, nb, device="cuda", generator=gen)
+    lib = ops.load()
+    dw = lib.qsa_indexer_bwd(qi, ki, wi, lib.qsa_indexer_fwd(qi, ki, wi, 0.125), dblse, 1.0, 0.125)[2].double()
+    want = torch.zeros_like(dw)
+    for b in range(B):
+        for t0 in range(0, S, 512):
+            t1 = min(S, t0 + 512)
+            dots = torch.relu(qi[b, :, t0:t1].double() @ ki[b, :t1].double().t())
+            hide = torch.arange(t1, device="cuda")[None] > torch.arange(t0, t1, device="cuda")[:, None]
+            score = (dots.to(torch.bfloat16).double() * 0.125 * wi[b, t0:t1].double().t()[..., None]).sum(0).masked_fill(hide, float("-inf"))
+            spread = lambda t: t.repeat_interleave(64, -1)
+            dI = torch.where(hide, 0.0, torch.exp(score - spread(score.unflatten(-1, (-1, 64)).logsumexp(-1))) * spread(dblse[b, t0:t1, :(t1 + 63) // 64].double()))
+            want[b, t0:t1] = (dI * dots).sum(-1).t() * 0.125
+    assert (dw - want).norm() <= 2 ** -13 * want.norm()
