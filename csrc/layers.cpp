@@ -5,7 +5,8 @@
 //
 // Everything that a backward pass needs is returned and saved by the caller's autograd node; nothing is kept here.  Weight gradients go to the
 // parameters' fp32 gradient buffers (`grads`, `grad_of[i]` = position of weight i's buffer, -1: return a fresh fp32 gradient, -2: not wanted),
-// on a second stream when one is given: it waits for the work issued so far, and the tensors it reads are recorded on it.
+// on a second stream when one is given: it waits for the work issued so far, and the tensors it reads are recorded on it.  A pass says whether it
+// put anything there: the caller joins the stream only then.
 #include <ATen/ATen.h>
 #include <ATen/cuda/CUDAContext.h>
 #include <ATen/cuda/CUDAEvent.h>
@@ -23,6 +24,7 @@ namespace {
 using at::Tensor;
 using OptTensor = c10::optional<Tensor>;
 using Tensors = std::vector<Tensor>;
+using BwdResult = std::tuple<Tensors, bool>;                             // gradients; whether work went to the second stream
 
 Tensor f32(const Tensor& t) { return t.to(at::kFloat).contiguous(); }
 Tensor rows_of(const Tensor& x) { return x.reshape({-1, x.size(-1)}).to(at::kBFloat16).contiguous(); }
@@ -54,6 +56,7 @@ struct WeightGrads {
   c10::optional<c10::cuda::CUDAStream> side;
   bool deterministic;
   const Tensor& err;
+  mutable bool on_side = false;
 
   WeightGrads(at::TensorList g, at::IntArrayRef of, at::IntArrayRef stream, bool det, const Tensor& e) : grads(g), grad_of(of), deterministic(det), err(e) {
     if (!stream.empty()) {
@@ -79,6 +82,7 @@ struct WeightGrads {
       launch();
     }
     for (const Tensor& t : used) t.record_stream(*side);
+    on_side = true;
   }
   // dW_i = dy^T x.  Returns an undefined tensor when it went into the buffer or is not wanted.
   Tensor linear(size_t i, const Tensor& dy, const Tensor& x) const {
@@ -131,7 +135,7 @@ Tensors gdn_layer_fwd(const Tensor& x, at::TensorList w, const Tensor& conv_w, c
 }
 
 // `saved` is what the forward returned after y.  Returns {dx, d conv, dA_log, d dt_bias, d norm, dW of qkv, z, b, a, out}.
-Tensors gdn_layer_bwd(const Tensor& dy, at::TensorList saved, at::TensorList w, const Tensor& conv_w, const Tensor& A_log, const Tensor& dt_bias, const Tensor& norm_w,
+BwdResult gdn_layer_bwd(const Tensor& dy, at::TensorList saved, at::TensorList w, const Tensor& conv_w, const Tensor& A_log, const Tensor& dt_bias, const Tensor& norm_w,
                       int64_t Hk, int64_t Hv, double eps, const Tensor& err, bool want_dx, at::TensorList grads, at::IntArrayRef grad_of, at::IntArrayRef stream,
                       bool deterministic) {
   const c10::cuda::CUDAGuard guard(dy.device());
@@ -154,7 +158,7 @@ Tensors gdn_layer_bwd(const Tensor& dy, at::TensorList saved, at::TensorList w, 
     if (want_dx) in.add(d, w[i]);
     dw[i] = wg.linear(i, d, x2);
   }
-  return {in.dx, conv[1], gate[2], gate[3], n[2], dw[0], dw[1], dw[2], dw[3], dw_out};
+  return {Tensors{in.dx, conv[1], gate[2], gate[3], n[2], dw[0], dw[1], dw[2], dw[3], dw_out}, wg.on_side};
 }
 
 // ---- attention with indexer ------------------------------------------------------------------------------------------------------
@@ -216,7 +220,7 @@ Tensors qsa_layer_fwd(const Tensor& x, at::TensorList w, at::TensorList wi, cons
 }
 
 // dy or dkl may be absent.  `saved` is what the forward returned after {y, kl}.  Returns {dx, d q_norm, d k_norm, dW of q, k, v, o, wq, wk, ww}.
-Tensors qsa_layer_bwd(const OptTensor& dy, const OptTensor& dkl, at::TensorList saved, at::TensorList w, const Tensor& q_norm, const Tensor& k_norm, double scale, const Tensor& err,
+BwdResult qsa_layer_bwd(const OptTensor& dy, const OptTensor& dkl, at::TensorList saved, at::TensorList w, const Tensor& q_norm, const Tensor& k_norm, double scale, const Tensor& err,
                       bool want_dx, at::TensorList grads, at::IntArrayRef grad_of, at::IntArrayRef stream, bool deterministic) {
   const Tensor &x2 = saved[0], &p_q = saved[1], &p_k = saved[2], &q = saved[3], &k = saved[4], &v = saved[5], &gate = saved[6], &c = saved[9], &s = saved[10], &o = saved[11],
                &go = saved[14];
@@ -253,7 +257,7 @@ Tensors qsa_layer_bwd(const OptTensor& dy, const OptTensor& dkl, at::TensorList 
     out[1] = hq[1];
     out[2] = hk[1];
   }
-  return out;
+  return {out, wg.on_side};
 }
 
 // ---- experts with the shared expert -----------------------------------------------------------------------------------------------
@@ -286,7 +290,7 @@ Tensors moe_layer_fwd(const Tensor& x, at::TensorList w, int64_t topk, const Ten
 }
 
 // dy or d_prob_sum may be absent.  `saved` is what the forward returned after {y, prob_sum, counts}.  Returns {dx, dW of w[0] .. w[6]}.
-Tensors moe_layer_bwd(const OptTensor& dy, const OptTensor& d_prob_sum, at::TensorList saved, at::TensorList w, const Tensor& err_, bool want_dx, at::TensorList grads,
+BwdResult moe_layer_bwd(const OptTensor& dy, const OptTensor& d_prob_sum, at::TensorList saved, at::TensorList w, const Tensor& err_, bool want_dx, at::TensorList grads,
                       at::IntArrayRef grad_of, at::IntArrayRef stream, bool deterministic) {
   const Tensor &x = saved[0], &sg = saved[1], &su = saved[2], &gl = saved[3], &probs = saved[4], &top_idx = saved[5], &top_w = saved[6], &xs = saved[7], &gu = saved[8],
                &hmid = saved[9], &ys = saved[10], &inv = saved[11], &offsets = saved[12], &sched = saved[13], &mid = saved[14], &shared = saved[15];
@@ -340,7 +344,7 @@ Tensors moe_layer_bwd(const OptTensor& dy, const OptTensor& d_prob_sum, at::Tens
     out[1 + i] = wg.linear(i, d, x);
   }
   if (want_dx) out[0] = dx_experts.defined() ? in.dx.add_(dx_experts) : in.dx;
-  return out;
+  return {out, wg.on_side};
 }
 
 // ---- residual streams ---------------------------------------------------------------------------------------------------------------
@@ -357,7 +361,7 @@ Tensors mhc_layer_fwd(const Tensor& X, const Tensor& A, const Tensor& Bw, const 
 }
 
 // saved = {coef, X2, Lraw, z, inv, rstd}; dXo is the gradient of the sub-layer's output stream (absent: zero).  Returns {dX [T,n,h], dBw, dbias [27], d norm, dA}.
-Tensors mhc_layer_bwd(const Tensor& dxout, const OptTensor& dcoef, const OptTensor& dXo, at::TensorList saved, const Tensor& A, const Tensor& Bw, const Tensor& b_pre,
+BwdResult mhc_layer_bwd(const Tensor& dxout, const OptTensor& dcoef, const OptTensor& dXo, at::TensorList saved, const Tensor& A, const Tensor& Bw, const Tensor& b_pre,
                       const Tensor& b_post, const Tensor& b_res, const Tensor& alphas, const Tensor& norm_w, int64_t iters, const Tensor& err, at::TensorList grads,
                       at::IntArrayRef grad_of, at::IntArrayRef stream, bool deterministic) {
   const Tensor &coef = saved[0], &X2 = saved[1], &Lraw = saved[2], &z = saved[3], &inv = saved[4], &rstd = saved[5];
@@ -383,7 +387,7 @@ Tensors mhc_layer_bwd(const Tensor& dxout, const OptTensor& dcoef, const OptTens
   auto G = at::empty({T, n * h}, dL.options().dtype(at::kBFloat16));
   gemm_bf16_persistent(dL, Ac.t().contiguous(), G, false, false, 1.0, false, err, -1);
   const Tensor up = dXo.has_value() ? dXo->contiguous().view({T, n, h}) : at::zeros_like(X3);
-  return {mhc_pre_bwd_c(G.view({T, n, h}), up, X3, dxin, coef, c1), a[3], a[4], a[5], dA};
+  return {Tensors{mhc_pre_bwd_c(G.view({T, n, h}), up, X3, dxin, coef, c1), a[3], a[4], a[5], dA}, wg.on_side};
 }
 
 // ---- vocabulary loss -----------------------------------------------------------------------------------------------------------------
@@ -402,7 +406,7 @@ Tensors linear_ce_fwd(const Tensor& h2, const Tensor& w, const Tensor& target, i
 }
 
 // Returns {d hidden [T,hidden] bf16, dW}; `g` is the upstream gradient (one element).
-Tensors linear_ce_bwd(const Tensor& g, const Tensor& h2, const Tensor& w, const Tensor& dlogits, const Tensor& err, at::TensorList grads, at::IntArrayRef grad_of,
+BwdResult linear_ce_bwd(const Tensor& g, const Tensor& h2, const Tensor& w, const Tensor& dlogits, const Tensor& err, at::TensorList grads, at::IntArrayRef grad_of,
                       at::IntArrayRef stream, bool deterministic) {
   const c10::cuda::CUDAGuard guard(h2.device());
   const WeightGrads wg(grads, grad_of, stream, deterministic, err);
@@ -411,7 +415,8 @@ Tensors linear_ce_bwd(const Tensor& g, const Tensor& h2, const Tensor& w, const 
     return t.numel() % 8 == 0 && t.is_contiguous() && (reinterpret_cast<uintptr_t>(t.data_ptr()) & 15) == 0 ? scale_bf16(t, gs) : t * gs;
   };
   const Tensor dh = scaled(mm_nn(dlogits, w, err));
-  return {dh, wg.wanted(0) ? wg.linear(0, dlogits, scaled(h2)) : Tensor()};
+  const Tensor dw = wg.wanted(0) ? wg.linear(0, dlogits, scaled(h2)) : Tensor();
+  return {Tensors{dh, dw}, wg.on_side};
 }
 
 }  // namespace q38
@@ -420,19 +425,19 @@ TORCH_LIBRARY_FRAGMENT(q38, m) {
   m.def("gdn_layer_fwd(Tensor x, Tensor[] w, Tensor conv_w, Tensor A_log, Tensor dt_bias, Tensor norm_w, int Hk, int Hv, float eps, Tensor(a!) err, bool save) -> Tensor[]",
         &q38::gdn_layer_fwd);
   m.def("gdn_layer_bwd(Tensor dy, Tensor[] saved, Tensor[] w, Tensor conv_w, Tensor A_log, Tensor dt_bias, Tensor norm_w, int Hk, int Hv, float eps, Tensor(a!) err, bool want_dx, "
-        "Tensor(b!)[] grads, int[] grad_of, int[] stream, bool deterministic) -> Tensor[]", &q38::gdn_layer_bwd);
+        "Tensor(b!)[] grads, int[] grad_of, int[] stream, bool deterministic) -> (Tensor[], bool)", &q38::gdn_layer_bwd);
   m.def("qsa_layer_fwd(Tensor x, Tensor[] w, Tensor[] wi, Tensor q_norm, Tensor k_norm, Tensor cos, Tensor sin, float q_eps, float k_eps, float scale, int budget, bool dense, "
         "bool want_kl, bool main_tc, Tensor(a!) err, bool save) -> Tensor[]", &q38::qsa_layer_fwd);
   m.def("qsa_layer_bwd(Tensor? dy, Tensor? dkl, Tensor[] saved, Tensor[] w, Tensor q_norm, Tensor k_norm, float scale, Tensor(a!) err, bool want_dx, Tensor(b!)[] grads, int[] grad_of, "
-        "int[] stream, bool deterministic) -> Tensor[]", &q38::qsa_layer_bwd);
+        "int[] stream, bool deterministic) -> (Tensor[], bool)", &q38::qsa_layer_bwd);
   m.def("moe_layer_fwd(Tensor x, Tensor[] w, int topk, Tensor(a!) err, bool save) -> Tensor[]", &q38::moe_layer_fwd);
   m.def("moe_layer_bwd(Tensor? dy, Tensor? d_prob_sum, Tensor[] saved, Tensor[] w, Tensor(a!) err, bool want_dx, Tensor(b!)[] grads, int[] grad_of, int[] stream, bool deterministic) "
-        "-> Tensor[]", &q38::moe_layer_bwd);
+        "-> (Tensor[], bool)", &q38::moe_layer_bwd);
   m.def("mhc_layer_fwd(Tensor X, Tensor A, Tensor Bw, Tensor b_pre, Tensor b_post, Tensor b_res, Tensor alphas, Tensor norm_w, int iters, float eps, bool out_bf16, Tensor(a!) err) "
         "-> Tensor[]", &q38::mhc_layer_fwd);
   m.def("mhc_layer_bwd(Tensor dxout, Tensor? dcoef, Tensor? dXo, Tensor[] saved, Tensor A, Tensor Bw, Tensor b_pre, Tensor b_post, Tensor b_res, Tensor alphas, Tensor norm_w, int iters, "
-        "Tensor(a!) err, Tensor(b!)[] grads, int[] grad_of, int[] stream, bool deterministic) -> Tensor[]", &q38::mhc_layer_bwd);
+        "Tensor(a!) err, Tensor(b!)[] grads, int[] grad_of, int[] stream, bool deterministic) -> (Tensor[], bool)", &q38::mhc_layer_bwd);
   m.def("linear_ce_fwd(Tensor h2, Tensor w, Tensor target, int rows, Tensor(a!) err) -> Tensor[]", &q38::linear_ce_fwd);
-  m.def("linear_ce_bwd(Tensor g, Tensor h2, Tensor w, Tensor dlogits, Tensor(a!) err, Tensor(b!)[] grads, int[] grad_of, int[] stream, bool deterministic) -> Tensor[]",
+  m.def("linear_ce_bwd(Tensor g, Tensor h2, Tensor w, Tensor dlogits, Tensor(a!) err, Tensor(b!)[] grads, int[] grad_of, int[] stream, bool deterministic) -> (Tensor[], bool)",
         &q38::linear_ce_bwd);
 }

@@ -161,13 +161,18 @@ class _SideStream:
         return out
 
     def handle(self):
-        """The stream as the native layer passes take it (empty: run inline); work issued on it is joined like that of `run`."""
+        """The stream as the native layer passes take it (empty: run inline).  They say whether they used it, see `done`."""
         if not self.enabled:
             return ()
         if self.stream is None:
             self.stream = torch.cuda.Stream()
-        self.pending = True
         return self.stream.stream_id, self.stream.device_index, self.stream.device_type
+
+    def done(self, result):
+        """The gradients of a native pass; what it issued on the stream is joined like that of `run`."""
+        gradients, used = result
+        self.pending = self.pending or used
+        return gradients
 
     def join(self):
         if self.pending:
@@ -336,8 +341,8 @@ class _MhcPreNormLayer(torch.autograd.Function):
         params, saved = tensors[:7], tensors[7:]
         grads, grad_of = _grad_buffers(params[:1], ctx.needs_input_grad[1:2])
         dXo, ctx.link.dXo = ctx.link.dXo, None
-        dX, dBw, dbias, dnw, dA = load().mhc_layer_bwd(dxout, dcoef, dXo, saved, *params, ctx.iters, error_flag(dxout.device), grads, grad_of, WGRAD_STREAM.handle(),
-                                                       ctx.deterministic)
+        dX, dBw, dbias, dnw, dA = WGRAD_STREAM.done(load().mhc_layer_bwd(dxout, dcoef, dXo, saved, *params, ctx.iters, error_flag(dxout.device), grads, grad_of,
+                                                                         WGRAD_STREAM.handle(), ctx.deterministic))
         take, (A_w, B_w, b_pre, b_post, b_res, alphas, norm_w) = DEFERRED_GRADS.take, params
         return (dX.view(ctx.shape), None if dA is None else dA.to(A_w.dtype), take(B_w, dBw), take(b_pre, dbias[0:4]), take(b_post, dbias[4:8]),
                 take(b_res, dbias[8:24]), take(alphas, dbias[24:27]), take(norm_w, dnw), None, None, None, None, None)
@@ -720,8 +725,8 @@ class _GdnLayer(torch.autograd.Function):
         tensors = ctx.saved_tensors
         params, saved = tensors[:9], tensors[9:]
         need = ctx.needs_input_grad
-        out = load().gdn_layer_bwd(dy, saved, [_bf16_weight(w) for w in params[:5]], *params[5:], *ctx.args, error_flag(dy.device), need[0],
-                                   *_grad_buffers(params[:5], need[1:6]), WGRAD_STREAM.handle(), ctx.deterministic)
+        out = WGRAD_STREAM.done(load().gdn_layer_bwd(dy, saved, [_bf16_weight(w) for w in params[:5]], *params[5:], *ctx.args, error_flag(dy.device), need[0],
+                                                     *_grad_buffers(params[:5], need[1:6]), WGRAD_STREAM.handle(), ctx.deterministic))
         small = [DEFERRED_GRADS.take(p, d) for p, d in zip(params[5:], out[1:5])]
         return (out[0].view(ctx.shape) if need[0] else None, *map(_fresh, out[5:], params[:5]), *small, None, None, None, None, None)
 
@@ -746,8 +751,8 @@ class _QsaLayer(torch.autograd.Function):
         tensors = ctx.saved_tensors
         params, (q_norm, k_norm), saved = tensors[:n], tensors[n:n + 2], tensors[n + 2:]
         grads, grad_of = _grad_buffers(params, need[1:1 + n])
-        out = load().qsa_layer_bwd(dy, dkl, saved, [_bf16_weight(w) for w in params[:4]], q_norm, k_norm, ctx.scale, error_flag(saved[0].device), need[0] and dy is not None,
-                                   grads, grad_of, WGRAD_STREAM.handle(), ctx.deterministic)
+        out = WGRAD_STREAM.done(load().qsa_layer_bwd(dy, dkl, saved, [_bf16_weight(w) for w in params[:4]], q_norm, k_norm, ctx.scale, error_flag(saved[0].device),
+                                                     need[0] and dy is not None, grads, grad_of, WGRAD_STREAM.handle(), ctx.deterministic))
         norms = [None if d is None else DEFERRED_GRADS.take(p, d) for p, d in zip((q_norm, k_norm), out[1:3])]
         dw = list(map(_fresh, out[3:], params))
         return (None if out[0] is None else out[0].view(ctx.shape), *dw, *[None] * (7 - n), *norms, *[None] * 11)
@@ -769,8 +774,8 @@ class _MoeLayer(torch.autograd.Function):
         tensors = ctx.saved_tensors
         params, saved = tensors[:7], tensors[7:]
         need = ctx.needs_input_grad
-        out = load().moe_layer_bwd(dy, d_prob_sum, saved, [_bf16_weight(w) for w in params], error_flag(saved[0].device), need[0], *_grad_buffers(params, need[1:8]),
-                                   WGRAD_STREAM.handle(), ctx.deterministic)
+        out = WGRAD_STREAM.done(load().moe_layer_bwd(dy, d_prob_sum, saved, [_bf16_weight(w) for w in params], error_flag(saved[0].device), need[0],
+                                                     *_grad_buffers(params, need[1:8]), WGRAD_STREAM.handle(), ctx.deterministic))
         return (out[0], *map(_fresh, out[1:], params), None, None, None)
 
 
@@ -1141,8 +1146,8 @@ class _LinearCE(torch.autograd.Function):
         if not h2.shape[0]:
             return torch.empty_like(h2).view(ctx.shape).to(ctx.dtype), None, None, None, None
         if ctx.native:
-            dh, dw = load().linear_ce_bwd(g, h2, w, dlogits, error_flag(h2.device), *_grad_buffers((weight,), ctx.needs_input_grad[1:2]), WGRAD_STREAM.handle(),
-                                          backend.deterministic)
+            dh, dw = WGRAD_STREAM.done(load().linear_ce_bwd(g, h2, w, dlogits, error_flag(h2.device), *_grad_buffers((weight,), ctx.needs_input_grad[1:2]),
+                                                            WGRAD_STREAM.handle(), backend.deterministic))
             return dh.view(ctx.shape).to(ctx.dtype), _fresh(dw, weight), None, None, None
         dh = scale_bf16(backend.mm_nn(dlogits, w), gs)
         dw = backend.weight_grad(dlogits, scale_bf16(h2, gs), weight) if ctx.needs_input_grad[1] else None

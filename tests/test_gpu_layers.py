@@ -121,3 +121,25 @@ def test_layer_call_refuses_forward_mode(modeling):
     with torch.autograd.forward_ad.dual_level():
         with pytest.raises(RuntimeError):
             module(torch.autograd.forward_ad.make_dual(x, torch.ones_like(x)))
+
+
+@pytest.mark.parametrize("kind", ["gdn", "moe", "mhc", "head", "qsa kl"])
+@pytest.mark.parametrize("mode", ["frozen", "fresh", "buffers"])
+def test_side_stream_is_joined_where_it_was_used(modeling, kind, mode):
+    """A pass whose weight gradients are not wanted, or are returned, puts nothing on the second stream; a join there would make a capture wait for a
+    stream that never entered it."""
+    from q38.ops.backend import WGRAD_STREAM
+    module = build(modeling, kind).requires_grad_(mode != "frozen")
+    for p in module.parameters():
+        p.grad = torch.zeros_like(p) if mode == "buffers" else None
+    x = torch.randn((1, S, 4, HIDDEN) if kind == "mhc" else (1, S, HIDDEN), device="cuda").to(torch.float32 if kind == "mhc" else torch.bfloat16).requires_grad_()
+    target = torch.randint(0, 512, (S,), device="cuda")
+    WGRAD_STREAM.enabled = True
+    try:
+        assert not WGRAD_STREAM.pending
+        outs = run(modeling, module, kind, x, target, ("y",) if mode == "frozen" else ("y", "kl"))
+        torch.autograd.backward(outs, [torch.ones_like(o) for o in outs])
+        assert WGRAD_STREAM.pending == (mode == "buffers")
+    finally:
+        WGRAD_STREAM.join()
+        WGRAD_STREAM.enabled = False
