@@ -3,7 +3,8 @@
 // have the same bits.  At a few hundred tokens a pass is bound by the host: each op from Python costs 10 to 30 us (argument
 // parsing, an autograd node, views, small allocations), a launch from here about 4.
 //
-// Everything that a backward pass needs is returned and saved by the caller's autograd node; nothing is kept here.  Weight gradients go to the
+// Everything that a backward pass needs is returned and saved by the caller's autograd node; nothing is kept here.  Inputs are not returned (a result
+// that shares memory with an argument would need a schema that says so): the caller saves them itself, `saved` begins with them.  Weight gradients go to the
 // parameters' fp32 gradient buffers (`grads`, `grad_of[i]` = position of weight i's buffer, -1: return a fresh fp32 gradient, -2: not wanted),
 // on a second stream when one is given: it waits for the work issued so far, and the tensors it reads are recorded on it.  A pass says whether it
 // put anything there: the caller joins the stream only then.
@@ -111,7 +112,7 @@ struct InputGrad {
 }  // namespace
 
 // ---- Gated DeltaNet -----------------------------------------------------------------------------------------------------------
-// w = {qkv, z, b, a, out} (bf16).  Returns {y} or, with `save`, {y, x2, p_qkv, z, p_b, p_a, qkv, beta, g, o, on, (the delta rule's nine)}.
+// w = {qkv, z, b, a, out} (bf16).  Returns {y} or, with `save`, {y, p_qkv, z, p_b, p_a, qkv, beta, g, o, on, (the delta rule's nine)}.
 Tensors gdn_layer_fwd(const Tensor& x, at::TensorList w, const Tensor& conv_w, const Tensor& A_log, const Tensor& dt_bias, const Tensor& norm_w, int64_t Hk, int64_t Hv,
                       double eps, const Tensor& err, bool save) {
   const c10::cuda::CUDAGuard guard(x.device());
@@ -129,18 +130,19 @@ Tensors gdn_layer_fwd(const Tensor& x, at::TensorList w, const Tensor& conv_w, c
   const Tensor on = gated_rmsnorm_fwd(o, p[1].view({-1, 64}), f32(norm_w), eps).view({B * S, -1});
   const Tensor y = mm_nt(on, w[4], err).view({B, S, w[4].size(0)});
   if (!save) return {y};
-  Tensors out = {y, x2, p[0], p[1], p[2], p[3], qkv, gates[0], gates[1], o, on};
+  Tensors out = {y, p[0], p[1], p[2], p[3], qkv, gates[0], gates[1], o, on};
   out.insert(out.end(), rule.begin() + 1, rule.end());
   return out;
 }
 
-// `saved` is what the forward returned after y.  Returns {dx, d conv, dA_log, d dt_bias, d norm, dW of qkv, z, b, a, out}.
+// `saved` is {x, what the forward returned after y}.  Returns {dx, d conv, dA_log, d dt_bias, d norm, dW of qkv, z, b, a, out}.
 BwdResult gdn_layer_bwd(const Tensor& dy, at::TensorList saved, at::TensorList w, const Tensor& conv_w, const Tensor& A_log, const Tensor& dt_bias, const Tensor& norm_w,
                       int64_t Hk, int64_t Hv, double eps, const Tensor& err, bool want_dx, at::TensorList grads, at::IntArrayRef grad_of, at::IntArrayRef stream,
                       bool deterministic) {
   const c10::cuda::CUDAGuard guard(dy.device());
   const WeightGrads wg(grads, grad_of, stream, deterministic, err);
-  const Tensor &x2 = saved[0], &qkv = saved[5], &beta = saved[6], &g = saved[7], &o = saved[8], &on = saved[9];
+  const Tensor x2 = rows_of(saved[0]);
+  const Tensor &qkv = saved[5], &beta = saved[6], &g = saved[7], &o = saved[8], &on = saved[9];
   const at::TensorList p = saved.slice(1, 4);
   const int64_t B = qkv.size(0), S = qkv.size(1);
   const Tensor dy2 = rows_of(dy);
@@ -163,8 +165,8 @@ BwdResult gdn_layer_bwd(const Tensor& dy, at::TensorList saved, at::TensorList w
 
 // ---- attention with indexer ------------------------------------------------------------------------------------------------------
 // w = {q, k, v, o} (bf16), wi = {wq, wk, ww} of the indexer (bf16; empty without one).  The indexer runs with its KL (want_kl), or, for block
-// selection alone (not dense), on the first query of every block.  Returns {y, kl} or, with `save`, {y, kl, x2, p_q, p_k, q, k, v, gate, rstd_q, rstd_k,
-// cos, sin, o, lse, sel, go} and with the KL also {p_qi, p_ki, qi, ki, wi, blse, dblse, rstd_qi, rstd_ki}.
+// selection alone (not dense), on the first query of every block.  Returns {y, kl} or, with `save`, {y, kl, p_q, p_k, q, k, v, gate, rstd_q, rstd_k,
+// o, lse, sel, go} and with the KL also {p_qi, p_ki, qi, ki, wi, blse, dblse, rstd_qi, rstd_ki}.
 Tensors qsa_layer_fwd(const Tensor& x, at::TensorList w, at::TensorList wi, const Tensor& q_norm, const Tensor& k_norm, const Tensor& cos, const Tensor& sin, double q_eps,
                       double k_eps, double scale, int64_t budget, bool dense, bool want_kl, bool main_tc, const Tensor& err, bool save) {
   const c10::cuda::CUDAGuard guard(x.device());
@@ -214,17 +216,17 @@ Tensors qsa_layer_fwd(const Tensor& x, at::TensorList w, at::TensorList wi, cons
   const Tensor go = sigmoid_mul_fwd(o, gate).view({B * S, -1});
   const Tensor y = mm_nt(go, w[3], err).view({B, S, -1});
   if (!save) return {y, kl};
-  Tensors out = {y, kl, x2, p_q, p_k, q, k, v, gate, hq[2], hk[2], c, s, a[0], a[1], a[2], go};
+  Tensors out = {y, kl, p_q, p_k, q, k, v, gate, hq[2], hk[2], a[0], a[1], a[2], go};
   out.insert(out.end(), idx.begin(), idx.end());
   return out;
 }
 
-// dy or dkl may be absent.  `saved` is what the forward returned after {y, kl}.  Returns {dx, d q_norm, d k_norm, dW of q, k, v, o, wq, wk, ww}.
+// dy or dkl may be absent.  `saved` is {x, cos, sin, what the forward returned after {y, kl}}.  Returns {dx, d q_norm, d k_norm, dW of q, k, v, o, wq, wk, ww}.
 BwdResult qsa_layer_bwd(const OptTensor& dy, const OptTensor& dkl, at::TensorList saved, at::TensorList w, const Tensor& q_norm, const Tensor& k_norm, double scale, const Tensor& err,
                       bool want_dx, at::TensorList grads, at::IntArrayRef grad_of, at::IntArrayRef stream, bool deterministic) {
-  const Tensor &x2 = saved[0], &p_q = saved[1], &p_k = saved[2], &q = saved[3], &k = saved[4], &v = saved[5], &gate = saved[6], &c = saved[9], &s = saved[10], &o = saved[11],
-               &go = saved[14];
-  const c10::cuda::CUDAGuard guard(x2.device());
+  const c10::cuda::CUDAGuard guard(saved[0].device());
+  const Tensor x2 = rows_of(saved[0]), c = f32(saved[1]), s = f32(saved[2]);
+  const Tensor &p_q = saved[3], &p_k = saved[4], &q = saved[5], &k = saved[6], &v = saved[7], &gate = saved[8], &o = saved[11], &go = saved[14];
   const WeightGrads wg(grads, grad_of, stream, deterministic, err);
   const int64_t B = q.size(0), S = q.size(2), T = B * S;
   Tensors out(10);
@@ -246,7 +248,7 @@ BwdResult qsa_layer_bwd(const OptTensor& dy, const OptTensor& dkl, at::TensorLis
     out[6] = wg.linear(3, dy2, go);
     auto sg = sigmoid_mul_bwd(dgo, o.view({B, S, -1}), gate);
     auto a = qsa_attn_bwd(q, k, v, o, sg[0].view(o.sizes()), saved[12], saved[13], scale, err);
-    auto hq = qsa_headprep_bwd(a[0], sg[1], p_q, f32(q_norm), c, s, saved[7]), hk = qsa_headprep_bwd(a[1], c10::nullopt, p_k, f32(k_norm), c, s, saved[8]);
+    auto hq = qsa_headprep_bwd(a[0], sg[1], p_q, f32(q_norm), c, s, saved[9]), hk = qsa_headprep_bwd(a[1], c10::nullopt, p_k, f32(k_norm), c, s, saved[10]);
     const Tensor dp[3] = {hq[0].view({T, -1}), hk[0].view({T, -1}), a[2].transpose(1, 2).reshape({T, -1})};
     InputGrad in{err, {}};
     for (int i = 0; i < 3; ++i) {
@@ -286,15 +288,16 @@ Tensors moe_layer_fwd(const Tensor& x, at::TensorList w, int64_t topk, const Ten
   const Tensor shared = mm_nt(mid, w[4], err);
   const Tensor y = gate_add_fwd(routed, shared, p[3]);
   if (!save) return {y, route[4], route[3]};
-  return {y, route[4], route[3], xc, p[1], p[2], p[3], route[2], route[1], route[0], xs, gu, hmid, ys, sort[1], sort[2], sort[3], mid, shared};
+  return {y, route[4], route[3], p[1], p[2], p[3], route[2], route[1], route[0], xs, gu, hmid, ys, sort[1], sort[2], sort[3], mid, shared};
 }
 
-// dy or d_prob_sum may be absent.  `saved` is what the forward returned after {y, prob_sum, counts}.  Returns {dx, dW of w[0] .. w[6]}.
+// dy or d_prob_sum may be absent.  `saved` is {x, what the forward returned after {y, prob_sum, counts}}.  Returns {dx, dW of w[0] .. w[6]}.
 BwdResult moe_layer_bwd(const OptTensor& dy, const OptTensor& d_prob_sum, at::TensorList saved, at::TensorList w, const Tensor& err_, bool want_dx, at::TensorList grads,
                       at::IntArrayRef grad_of, at::IntArrayRef stream, bool deterministic) {
-  const Tensor &x = saved[0], &sg = saved[1], &su = saved[2], &gl = saved[3], &probs = saved[4], &top_idx = saved[5], &top_w = saved[6], &xs = saved[7], &gu = saved[8],
+  const c10::cuda::CUDAGuard guard(saved[0].device());
+  const Tensor x = saved[0].contiguous();
+  const Tensor &sg = saved[1], &su = saved[2], &gl = saved[3], &probs = saved[4], &top_idx = saved[5], &top_w = saved[6], &xs = saved[7], &gu = saved[8],
                &hmid = saved[9], &ys = saved[10], &inv = saved[11], &offsets = saved[12], &sched = saved[13], &mid = saved[14], &shared = saved[15];
-  const c10::cuda::CUDAGuard guard(x.device());
   Tensor err = err_;
   const WeightGrads wg(grads, grad_of, stream, deterministic, err);
   const int64_t T = x.size(0), topk = top_idx.size(1);
@@ -348,7 +351,7 @@ BwdResult moe_layer_bwd(const OptTensor& dy, const OptTensor& d_prob_sum, at::Te
 }
 
 // ---- residual streams ---------------------------------------------------------------------------------------------------------------
-// X [B,S,n,h] fp32.  Returns {normalised input [T,h], coef, X2 [T,n h], Lraw, z, inv, rstd}.
+// X [B,S,n,h] fp32.  Returns {normalised input [T,h], coef, Lraw, z, inv, rstd}.
 Tensors mhc_layer_fwd(const Tensor& X, const Tensor& A, const Tensor& Bw, const Tensor& b_pre, const Tensor& b_post, const Tensor& b_res, const Tensor& alphas,
                       const Tensor& norm_w, int64_t iters, double eps, bool out_bf16, const Tensor& err) {
   const c10::cuda::CUDAGuard guard(X.device());
@@ -357,18 +360,19 @@ Tensors mhc_layer_fwd(const Tensor& X, const Tensor& A, const Tensor& Bw, const 
   auto Lraw = at::empty({X2.size(0), Ac.size(0)}, X2.options());
   gemm_bf16_persistent(X2, Ac, Lraw, false, false, 1.0, false, err, -1);
   auto out = mhc_coef_fwd(X2.view({-1, n, h}), Lraw, f32(Bw), f32(b_pre), f32(b_post), f32(b_res), f32(alphas), f32(norm_w), iters, eps, out_bf16);
-  return {out[0], out[1], X2, Lraw, out[2], out[3], out[4]};
+  return {out[0], out[1], Lraw, out[2], out[3], out[4]};
 }
 
-// saved = {coef, X2, Lraw, z, inv, rstd}; dXo is the gradient of the sub-layer's output stream (absent: zero).  Returns {dX [T,n,h], dBw, dbias [27], d norm, dA}.
+// saved = {X, coef, Lraw, z, inv, rstd}; dXo is the gradient of the sub-layer's output stream (absent: zero).  Returns {dX [T,n,h], dBw, dbias [27], d norm, dA}.
 BwdResult mhc_layer_bwd(const Tensor& dxout, const OptTensor& dcoef, const OptTensor& dXo, at::TensorList saved, const Tensor& A, const Tensor& Bw, const Tensor& b_pre,
                       const Tensor& b_post, const Tensor& b_res, const Tensor& alphas, const Tensor& norm_w, int64_t iters, const Tensor& err, at::TensorList grads,
                       at::IntArrayRef grad_of, at::IntArrayRef stream, bool deterministic) {
-  const Tensor &coef = saved[0], &X2 = saved[1], &Lraw = saved[2], &z = saved[3], &inv = saved[4], &rstd = saved[5];
-  const c10::cuda::CUDAGuard guard(X2.device());
+  const c10::cuda::CUDAGuard guard(saved[0].device());
+  const Tensor X = saved[0].contiguous();
+  const Tensor &coef = saved[1], &Lraw = saved[2], &z = saved[3], &inv = saved[4], &rstd = saved[5];
   const WeightGrads wg(grads, grad_of, stream, deterministic, err);
-  const int64_t T = X2.size(0), h = norm_w.numel(), n = X2.size(1) / h;
-  const Tensor X3 = X2.view({T, n, h}), Ac = f32(A);
+  const int64_t n = X.size(2), h = X.size(3), T = X.size(0) * X.size(1);
+  const Tensor X3 = X.view({T, n, h}), Ac = f32(A);
   Tensor dc = dcoef.has_value() ? dcoef->contiguous() : at::zeros_like(coef);
   auto a = mhc_pre_bwd_a(dxout.reshape({T, h}).contiguous(), X3, Lraw, f32(Bw), f32(b_pre), f32(b_post), f32(b_res), f32(alphas), f32(norm_w), coef, z, inv, rstd, dc, iters);
   const Tensor &dL = a[0], &c1 = a[1], &dxin = a[2], &Xbf = a[6];

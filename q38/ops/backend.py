@@ -330,8 +330,8 @@ class _MhcPreNormLayer(torch.autograd.Function):
 
     @staticmethod
     def forward(ctx, X, A_w, B_w, b_pre, b_post, b_res, alphas, norm_w, iters, eps, out_bf16, link, deterministic):
-        xout, coef, X2, *saved = load().mhc_layer_fwd(X, A_w, B_w, b_pre, b_post, b_res, alphas, norm_w, iters, eps, out_bf16, error_flag(X.device))
-        ctx.save_for_backward(A_w, B_w, b_pre, b_post, b_res, alphas, norm_w, coef, X2, *saved)
+        xout, coef, *saved = load().mhc_layer_fwd(X, A_w, B_w, b_pre, b_post, b_res, alphas, norm_w, iters, eps, out_bf16, error_flag(X.device))
+        ctx.save_for_backward(A_w, B_w, b_pre, b_post, b_res, alphas, norm_w, X, coef, *saved)
         ctx.iters, ctx.link, ctx.shape, ctx.deterministic = iters, link, X.shape, deterministic
         return xout.view(*X.shape[:2], X.shape[3]), coef
 
@@ -716,7 +716,7 @@ class _GdnLayer(torch.autograd.Function):
     def forward(ctx, x, w_qkv, w_z, w_b, w_a, w_out, conv_w, A_log, dt_bias, norm_w, Hk, Hv, eps, deterministic, save):
         params = (w_qkv, w_z, w_b, w_a, w_out, conv_w, A_log, dt_bias, norm_w)
         y, *saved = load().gdn_layer_fwd(x, [_bf16_weight(w) for w in params[:5]], *params[5:], Hk, Hv, eps, error_flag(x.device), save)
-        ctx.save_for_backward(*params, *saved)
+        ctx.save_for_backward(*params, x, *saved)
         ctx.args, ctx.shape, ctx.deterministic = (Hk, Hv, eps), x.shape, deterministic
         return y
 
@@ -739,7 +739,7 @@ class _QsaLayer(torch.autograd.Function):
         params = (w_q, w_k, w_v, w_o, *indexer)
         y, kl, *saved = load().qsa_layer_fwd(x, [_bf16_weight(w) for w in params[:4]], [_bf16_weight(w) for w in indexer], q_norm, k_norm, cos, sin, q_eps, k_eps, scale,
                                              budget, dense, want_kl, main_tc, error_flag(x.device), save)
-        ctx.save_for_backward(*params, q_norm, k_norm, *saved)
+        ctx.save_for_backward(*params, q_norm, k_norm, x, cos, sin, *saved)
         ctx.n, ctx.scale, ctx.shape, ctx.deterministic = len(params), scale, x.shape, deterministic
         need = ctx.needs_input_grad                                  # the two outputs depend on disjoint parameters
         ctx.mark_non_differentiable(*(out for out, parts in ((y, need[:5] + need[8:10]), (kl, need[5:8])) if out is not None and not any(parts)))
@@ -764,7 +764,7 @@ class _MoeLayer(torch.autograd.Function):
         ctx.set_materialize_grads(False)
         params = (w_router, w_sg, w_su, w_sl, w_sd, w_gate_up, w_down)
         y, prob_sum, counts, *saved = load().moe_layer_fwd(x, [_bf16_weight(w) for w in params], topk, error_flag(x.device), save)
-        ctx.save_for_backward(*params, *saved)
+        ctx.save_for_backward(*params, x, *saved)
         ctx.deterministic = deterministic
         ctx.mark_non_differentiable(*((counts,) if any(ctx.needs_input_grad[:2]) else (counts, prob_sum)))
         return y, prob_sum, counts

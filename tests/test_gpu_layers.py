@@ -143,3 +143,32 @@ def test_side_stream_is_joined_where_it_was_used(modeling, kind, mode):
     finally:
         WGRAD_STREAM.join()
         WGRAD_STREAM.enabled = False
+
+
+@pytest.mark.parametrize("kind", ["gdn", "moe", "mhc", "qsa kl", "qsa"])
+def test_layer_results_are_memory_of_their_own(modeling, kind, monkeypatch):
+    """The operators' schemas declare no result that shares memory with an argument, or with another result."""
+    from q38.ops import backend as ops_backend
+    lib, checked = ops_backend.load(), []
+
+    def own(call):
+        def wrapped(*args):
+            results = call(*args)
+            flat = [t for a in args for t in (a if isinstance(a, (list, tuple)) else [a]) if isinstance(t, torch.Tensor) and t.numel()]
+            seen = {t.untyped_storage().data_ptr() for t in flat}
+            for t in results:
+                if t is not None and t.numel():
+                    assert t.untyped_storage().data_ptr() not in seen, t.shape
+                    seen.add(t.untyped_storage().data_ptr())
+            checked.append(1)
+            return results
+        return wrapped
+
+    class Library:
+        def __getattr__(self, name):
+            return own(getattr(lib, name)) if name.endswith("_layer_fwd") else getattr(lib, name)
+
+    monkeypatch.setattr(ops_backend, "load", lambda: Library())
+    x = torch.randn((1, S, 4, HIDDEN) if kind == "mhc" else (1, S, HIDDEN), device="cuda").to(torch.float32 if kind == "mhc" else torch.bfloat16).requires_grad_()
+    run(modeling, build(modeling, kind), kind, x, None, ("y", "kl"))
+    assert checked
