@@ -57,7 +57,13 @@ TORCH_LIBRARY(q38, m) {
   m.def("cast_shadow_except(Tensor params, Tensor(a!) shadow, int skip_start, int skip_count, Tensor? err) -> ()",
         [](const at::Tensor& p, at::Tensor& sh, int64_t s0, int64_t n, c10::optional<at::Tensor> err) { q38::cast_shadow_except(p, sh, s0, n, err); });
   m.def("qsa_headprep_fwd(Tensor src, Tensor? w, Tensor cos, Tensor sin, float eps, bool split_gate, bool round_products=False) -> Tensor[]", &q38::qsa_headprep_fwd);
-  m.def("qsa_headprep_bwd(Tensor dout, Tensor? dgate, Tensor src, Tensor? w, Tensor cos, Tensor sin, Tensor rstd) -> Tensor[]", &q38::qsa_headprep_bwd);
+  m.def("qsa_headprep_bwd(Tensor dout, Tensor? dgate, Tensor src, Tensor? w, Tensor cos, Tensor sin, Tensor rstd) -> Tensor[]",
+        [](const at::Tensor& dout, const c10::optional<at::Tensor>& dgate, const at::Tensor& src, const c10::optional<at::Tensor>& w, const at::Tensor& cos, const at::Tensor& sin,
+           const at::Tensor& rstd) {
+          auto out = q38::qsa_headprep_bwd(dout, dgate, src, w, cos, sin, rstd);
+          if (!w.has_value()) out[1] = at::zeros({64}, src.options().dtype(at::kFloat));      // without a norm: 64 zeros (the layer pass does without them)
+          return out;
+        });
   m.def("gate_add_fwd(Tensor routed, Tensor shared, Tensor logit) -> Tensor", &q38::gate_add_fwd);
   m.def("gate_add_bwd(Tensor dy, Tensor shared, Tensor logit) -> Tensor[]", &q38::gate_add_bwd);
   m.def("gdn_gates_fwd(Tensor b_raw, Tensor a_raw, Tensor A_log, Tensor dt_bias) -> Tensor[]", &q38::gdn_gates_fwd);

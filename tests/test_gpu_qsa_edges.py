@@ -142,3 +142,15 @@ def test_head_preparation_of_views(ops):
             lib.qsa_headprep_fwd(wide[..., first:first + 64], None, cos, sin, 0.0, False)
         with pytest.raises(RuntimeError, match="bad inputs"):
             lib.qsa_headprep_bwd(torch.zeros(B, H, S, 64, device="cuda", dtype=torch.bfloat16), None, wide[..., first:first + 64], None, cos, sin, torch.zeros(0, S, H, device="cuda"))
+
+
+@pytest.mark.parametrize("norm", [False, True])
+def test_head_preparation_weight_gradient_has_the_norm_s_shape(ops, norm):
+    """64 values, zeros without a norm."""
+    B, S, H = 1, 64, 3
+    src, dout = torch.randn(B, S, H, 64, device="cuda").to(torch.bfloat16), torch.randn(B, H, S, 64, device="cuda").to(torch.bfloat16)
+    cos, sin = (torch.rand(1, S, 16, device="cuda") for _ in range(2))
+    w = torch.randn(64, device="cuda") if norm else None
+    rstd = ops.load().qsa_headprep_fwd(src, w, cos, sin, 1e-6, False)[2]
+    dw = ops.load().qsa_headprep_bwd(dout, None, src, w, cos, sin, rstd)[1]
+    assert dw.shape == (64,) and dw.dtype == torch.float32 and bool(dw.any()) == norm
