@@ -70,11 +70,12 @@ __global__ void __launch_bounds__(256) moe_route_fwd_kernel(const __nv_bfloat16*
       float total = 0.f;
       for (int j = 0; j < K; ++j) {
         // arg-max over 64 candidates; ties resolve to the lowest expert index.  Probabilities are not negative and -1 marks what is taken, so the
-        // bit patterns order like the values and one warp reduction finds the largest.
+        // bit patterns order like the values and one warp reduction finds the largest.  A row with a NaN or an infinity among its logits has no
+        // probabilities (all NaN): every slot names expert 0, with weight NaN.
         const int i0 = __float_as_int(a0), i1 = __float_as_int(a1), top = __reduce_max_sync(0xffffffffu, max(i0, i1));
         const unsigned m0 = __ballot_sync(0xffffffffu, i0 == top), m1 = __ballot_sync(0xffffffffu, i1 == top);
         const float best = __int_as_float(top);
-        const int be = m0 != 0 ? __ffs(m0) - 1 : 31 + __ffs(m1);
+        const int be = denom != denom ? 0 : m0 != 0 ? __ffs(m0) - 1 : 31 + __ffs(m1);
         sel_p[j] = best; sel_e[j] = be; total += best;
         if (be == e0) a0 = -1.f;
         if (be == e1) a1 = -1.f;

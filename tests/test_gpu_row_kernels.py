@@ -103,3 +103,19 @@ def test_loss_over_chunk_edges(lib, rows):
         # logits of rms 2 rounded to bf16 (3e-3, so the probabilities move by 0.3 %), then their bf16 gradients and the bf16 outputs (2e-3 rms each)
         rel = lambda a, b: ((a.double() - b).norm() / b.norm()).item()
         assert abs(loss.item() - ref.item()) < 5e-3 * abs(ref.item()) + 5e-2 and rel(hid.grad, hr.grad) < 2e-2 and rel(w.grad, wr.grad) < 2e-2
+
+
+@pytest.mark.parametrize("E,k", [(8, 2), (32, 5), (64, 5)])
+def test_routing_of_rows_without_probabilities(lib, E, k):
+    """A NaN or +infinity among a row's logits, or nothing above -infinity: all slots name expert 0 with weight NaN, and other rows are as they were."""
+    gen = torch.Generator(device="cuda").manual_seed(E)
+    logits = torch.randn(77, E, device="cuda", generator=gen).to(torch.bfloat16)
+    want = lib.moe_route_fwd(logits, k)
+    bad = torch.tensor([0, 9, 40, 76], device="cuda")
+    logits[0, E - 1], logits[9], logits[40, 3], logits[76] = float("nan"), float("nan"), float("inf"), float("-inf")
+    top_w, top_idx, probs, counts, prob_sum = lib.moe_route_fwd(logits, k)
+    good = torch.ones(77, dtype=torch.bool, device="cuda")
+    good[bad] = False
+    assert (top_idx[bad] == 0).all() and top_w[bad].isnan().all() and probs[bad].isnan().all() and prob_sum.isnan().all()
+    assert torch.equal(top_idx[good], want[1][good]) and torch.equal(top_w[good], want[0][good])
+    assert torch.equal(counts, torch.bincount(top_idx.flatten(), minlength=E).float())
