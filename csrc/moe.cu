@@ -30,10 +30,10 @@ constexpr int MAX_TOPK = 8;
 // One warp per token, E <= 64 (two logits per lane).  probs = softmax(logits) in fp32, top-k, renormalise, round the
 // weights to bf16 (the logits' dtype).  Also accumulates assignment counts and probability sums for the balancing loss.
 // Both are the same bits in every run: they are added as whole numbers, the CTAs' probability sums as multiples of 2^-36 (64 bits hold 2^27
-// tokens), and the CTA that finishes last turns them into floats with one rounding.  One warp reduction per slot and 32 tokens
-// per CTA: 16384 tokens 25.6 -> 14.2 us (25.4 with eight tokens per CTA: the atomics of 2048 CTAs on 130 words bound it; a butterfly of
-// value and index for each slot did not matter then).
-constexpr int ROUTE_GROUPS = 4;
+// tokens), and the CTA that finishes last turns them into floats with one rounding.  One warp reduction per slot.  A CTA takes eight tokens at
+// a time, up to four times: the atomics of many CTAs on 130 words bound it (16384 tokens with one round per CTA 27.1 us, with four 15.2), but only where that leaves a CTA
+// for every SM (256 tokens: 8.2 us with four rounds, 5.8 with one; 4096: 10.3 and 9.6 with three).
+constexpr int ROUTE_GROUPS_MAX = 4;
 struct RouteSums {
   unsigned long long prob[64], not_finite;             // multiples of 2^-36; experts with a sum that has no such form, one bit each
   unsigned int count[64], done;                        // assignments; CTAs that have added theirs
@@ -41,7 +41,7 @@ struct RouteSums {
 __global__ void __launch_bounds__(256) moe_route_fwd_kernel(const __nv_bfloat16* __restrict__ logits, int T, int E, int K,
                                                             float* __restrict__ top_w, int* __restrict__ top_idx,
                                                             float* __restrict__ probs_out, float* __restrict__ counts,
-                                                            RouteSums* __restrict__ sums, float* __restrict__ prob_sum) {
+                                                            RouteSums* __restrict__ sums, float* __restrict__ prob_sum, int groups) {
   grid_wait();
   __shared__ float s_ps[8][64];
   __shared__ unsigned int s_cnt[64];
@@ -50,8 +50,8 @@ __global__ void __launch_bounds__(256) moe_route_fwd_kernel(const __nv_bfloat16*
   if (threadIdx.x < 64) s_cnt[threadIdx.x] = 0;
   unsigned long long prob = 0;                         // of expert threadIdx.x
   bool finite = true;
-  for (int g = 0; g < ROUTE_GROUPS; ++g) {             // eight tokens at a time, one per warp
-    const int first = (blockIdx.x * ROUTE_GROUPS + g) * 8, t = first + warp;
+  for (int g = 0; g < groups; ++g) {                   // eight tokens at a time, one per warp
+    const int first = (blockIdx.x * groups + g) * 8, t = first + warp;
     if (first >= T) break;
     s_ps[warp][lane] = s_ps[warp][lane + 32] = 0.f;
     __syncthreads();
@@ -826,8 +826,9 @@ std::vector<at::Tensor> moe_route_fwd(const at::Tensor& logits, int64_t k) {
   auto sums = at::zeros({(int64_t)sizeof(RouteSums)}, logits.options().dtype(at::kByte));
   auto counts = T ? at::empty({E}, f32) : at::zeros({E}, f32), psum = T ? at::empty({E}, f32) : at::zeros({E}, f32);
   auto top_idx = at::empty({T, k}, logits.options().dtype(at::kInt));
-  if (T) launch(moe_route_fwd_kernel, (T + 8 * ROUTE_GROUPS - 1) / (8 * ROUTE_GROUPS), 256, 0, at::cuda::getCurrentCUDAStream(), (const __nv_bfloat16*)logits.data_ptr(), T, E, (int)k, top_w.data_ptr<float>(),
-      top_idx.data_ptr<int>(), probs.data_ptr<float>(), counts.data_ptr<float>(), reinterpret_cast<RouteSums*>(sums.data_ptr()), psum.data_ptr<float>());
+  const int eights = (T + 7) / 8, groups = std::max(1, std::min(ROUTE_GROUPS_MAX, eights / kNumSMs));
+  if (T) launch(moe_route_fwd_kernel, (eights + groups - 1) / groups, 256, 0, at::cuda::getCurrentCUDAStream(), (const __nv_bfloat16*)logits.data_ptr(), T, E, (int)k,
+                top_w.data_ptr<float>(), top_idx.data_ptr<int>(), probs.data_ptr<float>(), counts.data_ptr<float>(), reinterpret_cast<RouteSums*>(sums.data_ptr()), psum.data_ptr<float>(), groups);
   C10_CUDA_KERNEL_LAUNCH_CHECK();
   count_launch();
   return {top_w, top_idx, probs, counts, psum};

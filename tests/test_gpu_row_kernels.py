@@ -119,3 +119,19 @@ def test_routing_of_rows_without_probabilities(lib, E, k):
     assert (top_idx[bad] == 0).all() and top_w[bad].isnan().all() and probs[bad].isnan().all() and prob_sum.isnan().all()
     assert torch.equal(top_idx[good], want[1][good]) and torch.equal(top_w[good], want[0][good])
     assert torch.equal(counts, torch.bincount(top_idx.flatten(), minlength=E).float())
+
+
+# CTAs of one, two, three and four rounds of eight tokens, with a last round that is not full
+@pytest.mark.parametrize("T", [1, 9, 2360, 2361, 3546, 4733])
+def test_routing_over_its_grids(lib, T):
+    gen = torch.Generator(device="cuda").manual_seed(T)
+    logits = torch.randn(T, 64, device="cuda", generator=gen).to(torch.bfloat16)
+    top_w, top_idx, probs, counts, prob_sum = lib.moe_route_fwd(logits, 5)
+    want = logits.double().softmax(-1)
+    # fp32: an exponential of 2^-21, a sum and a division
+    assert ((probs - want).abs() <= 2 ** -19 * want).all()
+    best = probs.topk(5, -1).values
+    assert torch.equal(probs.gather(1, top_idx.long()), best) and (top_idx.sort(-1).values.diff(dim=-1) > 0).all()
+    assert torch.equal(counts, torch.bincount(top_idx.flatten(), minlength=64).float())
+    # sums of eight tokens in fp32, rounded to multiples of 2^-36, and one rounding at the end
+    assert ((prob_sum - probs.double().sum(0)).abs() <= 2 ** -21 * probs.double().sum(0)).all()
