@@ -361,12 +361,15 @@ __global__ void __launch_bounds__(256) moe_combine_bwd_kernel(const __nv_bfloat1
   if (lane == 0) d_top_w[pair] = dot;
 }
 
-// The same on 16-byte pieces (h % 8 == 0): eight lanes per pair, four pairs per warp.  Bound by memory: 81920 pairs of 576, 46 -> 43 us (the bytes need 32).
+// The same on 16-byte pieces (h % 8 == 0), LANES lanes per pair.  Bound by memory where there are many pairs, by the chain of a pair's loads where there are
+// few.  Against one warp and 4-byte pieces per pair: 81920 pairs of 448, 576 and 1024: 43, 44, 65 -> 33, 40, 62 us (half a warp, half a warp, a warp; with eight lanes 33,
+// 42, 73); 320 pairs: 2.4, 2.3, 2.4 -> 1.8, 2.5, 2.4 (eight lanes 3.0, 3.3, 5.1).  A warp for rows of 576, 72 pieces, leaves a quarter of its lanes idle: 53.
+template <int LANES>
 __global__ void __launch_bounds__(256) moe_combine_bwd_vec_kernel(const uint4* __restrict__ dout, const uint4* __restrict__ y_sorted, const int* __restrict__ inv_perm,
                                                                   const float* __restrict__ top_w, int T, int K, int pieces, uint4* __restrict__ dy_sorted,
                                                                   float* __restrict__ d_top_w) {
   grid_wait();
-  const int pair = (int)((blockIdx.x * 256 + threadIdx.x) >> 3), lane = threadIdx.x & 7;
+  const int pair = (int)((blockIdx.x * 256 + threadIdx.x) / LANES), lane = threadIdx.x & (LANES - 1);
   const bool live = pair < T * K;
   float dot = 0.f;
   if (live) {
@@ -374,7 +377,7 @@ __global__ void __launch_bounds__(256) moe_combine_bwd_vec_kernel(const uint4* _
     const uint4 *d = dout + (size_t)(pair / K) * pieces, *y = y_sorted + (size_t)inv_perm[pair] * pieces;
     uint4* dy = dy_sorted + (size_t)inv_perm[pair] * pieces;
 #pragma unroll 3
-    for (int i = lane; i < pieces; i += 8) {
+    for (int i = lane; i < pieces; i += LANES) {
       const uint4 a = d[i], c = y[i];
       const uint32_t as[4] = {a.x, a.y, a.z, a.w}, cs[4] = {c.x, c.y, c.z, c.w};
       uint32_t out[4];
@@ -389,7 +392,7 @@ __global__ void __launch_bounds__(256) moe_combine_bwd_vec_kernel(const uint4* _
     }
   }
 #pragma unroll
-  for (int o = 4; o > 0; o >>= 1) dot += __shfl_xor_sync(0xffffffffu, dot, o);
+  for (int o = LANES / 2; o > 0; o >>= 1) dot += __shfl_xor_sync(0xffffffffu, dot, o);
   if (live && lane == 0) d_top_w[pair] = dot;
 }
 
@@ -906,11 +909,16 @@ std::vector<at::Tensor> moe_combine_bwd(const at::Tensor& dout, const at::Tensor
   auto dy = at::empty_like(y_sorted);
   auto dw = at::empty({T, k}, top_w.options());
   auto wide = [](const at::Tensor& x) { return (reinterpret_cast<uintptr_t>(x.data_ptr()) & 15) == 0; };
-  if (T && h > 0 && h % 8 == 0 && wide(dout) && wide(y_sorted) && wide(dy))
-    launch(moe_combine_bwd_vec_kernel, (unsigned)(((long long)T * k * 8 + 255) / 256), 256, 0, at::cuda::getCurrentCUDAStream(), (const uint4*)dout.data_ptr(),
-           (const uint4*)y_sorted.data_ptr(), inv_perm.data_ptr<int>(), top_w.data_ptr<float>(), T, k, h / 8, (uint4*)dy.data_ptr(), dw.data_ptr<float>());
-  else if (T) launch(moe_combine_bwd_kernel, (T * k + 7) / 8, 256, 0, at::cuda::getCurrentCUDAStream(), (const __nv_bfloat16*)dout.data_ptr(), (const __nv_bfloat16*)y_sorted.data_ptr(),
+  if (T && h > 0 && h % 8 == 0 && wide(dout) && wide(y_sorted) && wide(dy)) {
+    // a warp per pair where its lanes are all busy (h a multiple of 256) or the pairs are few, else half a warp: see the kernel
+    const bool whole = h % 256 == 0 || (long long)T * k * 32 <= 2ll * kNumSMs * 256;
+    launch(whole ? moe_combine_bwd_vec_kernel<32> : moe_combine_bwd_vec_kernel<16>, (unsigned)(((long long)T * k * (whole ? 32 : 16) + 255) / 256), 256, 0,
+           at::cuda::getCurrentCUDAStream(), (const uint4*)dout.data_ptr(), (const uint4*)y_sorted.data_ptr(), inv_perm.data_ptr<int>(), top_w.data_ptr<float>(), T, k, h / 8,
+           (uint4*)dy.data_ptr(), dw.data_ptr<float>());
+  } else if (T) {
+    launch(moe_combine_bwd_kernel, (T * k + 7) / 8, 256, 0, at::cuda::getCurrentCUDAStream(), (const __nv_bfloat16*)dout.data_ptr(), (const __nv_bfloat16*)y_sorted.data_ptr(),
       inv_perm.data_ptr<int>(), top_w.data_ptr<float>(), T, k, h, (__nv_bfloat16*)dy.data_ptr(), dw.data_ptr<float>());
+  }
   C10_CUDA_KERNEL_LAUNCH_CHECK();
   count_launch();
   return {dy, dw};

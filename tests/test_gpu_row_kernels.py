@@ -135,3 +135,19 @@ def test_routing_over_its_grids(lib, T):
     assert torch.equal(counts, torch.bincount(top_idx.flatten(), minlength=64).float())
     # sums of eight tokens in fp32, rounded to multiples of 2^-36, and one rounding at the end
     assert ((prob_sum - probs.double().sum(0)).abs() <= 2 ** -21 * probs.double().sum(0)).all()
+
+
+# whole and half warps per pair (few pairs, the last and the first count on either side; rows that fill a warp), one piece, no whole pieces
+@pytest.mark.parametrize("T,k", [(1, 1), (473, 5), (474, 5), (2000, 2)])
+@pytest.mark.parametrize("h", [8, 36, 264, 448, 512])
+def test_combine_backward(lib, T, k, h):
+    gen = torch.Generator(device="cuda").manual_seed(T + h)
+    inv = torch.randperm(T * k, device="cuda", generator=gen).to(torch.int32)
+    y, dout = (torch.randn(n, h, device="cuda", generator=gen).to(torch.bfloat16) for n in (T * k, T))
+    w = torch.rand(T, k, device="cuda", generator=gen)
+    dy, dw = lib.moe_combine_bwd(dout, y, inv, w)
+    spread = dout.float().repeat_interleave(k, 0)
+    assert torch.equal(dy[inv.long()], (spread * w.view(-1, 1)).to(torch.bfloat16))
+    want = (spread.double() * y[inv.long()].double())
+    # fp32 sums of h products in some order
+    assert ((dw.flatten() - want.sum(-1)).abs() <= h * 2 ** -24 * want.abs().sum(-1) + 1e-30).all()
