@@ -42,7 +42,7 @@ struct BwdArgs {
   const unsigned char* sel;
   __nv_bfloat16* dq;
   float *dk, *dv;
-  int S, nq, nkv, parts, v_tokens;
+  int S, nq, nkv, parts, part_tiles, v_tokens;
   float scale;
   int* err;
 };
@@ -248,9 +248,9 @@ __global__ void __launch_bounds__(AB_THREADS, 2) qsa_attn_bwd_kv_kernel(const __
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int nb = p.S / 64, j = blockIdx.y, b = blockIdx.z, kvh = blockIdx.x / p.parts, part = blockIdx.x % p.parts, rep = p.nq / p.nkv;      // first key blocks (longest lists) first
   const int items = rep * list_blocks(p.sel + (long long)b * nb * nb + j, nb, j, nb, list, count);
-  // The tiles of a key block are split over as many CTAs as give each sixteen, at most `parts`; partial sums are added in fp32.  (Sixteen and
-  // eight CTAs: 201 us; 32 and 8: 227, one wave less even; 8 and 16: 248, because CTAs without work still walk the list.)
-  const int tiles = (items + 1) / 2, parts = min(p.parts, (tiles + 15) / 16);
+  // The tiles of a key block are split over as many CTAs as give each `part_tiles`, at most `parts`; partial sums are added in fp32.  (Sixteen and
+  // eight CTAs: 201 us; 32 and 8: 227, one wave less even; 8 and 16: 248, because CTAs without work still walk the list.  Few key blocks: see the launch.)
+  const int tiles = (items + 1) / 2, parts = min(p.parts, (tiles + p.part_tiles - 1) / p.part_tiles);
   if (part >= parts) return;
   const int t0 = (int)((long long)tiles * part / parts), n = (int)((long long)tiles * (part + 1) / parts) - t0;
   if (threadIdx.x == 0) {
@@ -427,7 +427,11 @@ std::vector<at::Tensor> qsa_attn_bwd(const at::Tensor& q, const at::Tensor& k, c
   p.o = (const __nv_bfloat16*)o.data_ptr(); p.dout = (const __nv_bfloat16*)dout.data_ptr(); p.lse = lse.data_ptr<float>(); p.D = D.data_ptr<float>();
   p.sel = sel.data_ptr<unsigned char>(); p.dq = (__nv_bfloat16*)dq.data_ptr(); p.dk = dkv32.data_ptr<float>(); p.dv = p.dk + k.numel(); p.v_tokens = v_tokens;
   p.S = S; p.nq = nq; p.nkv = nkv; p.scale = (float)scale; p.err = err.has_value() ? err->data_ptr<int>() : nullptr;
-  p.parts = std::min(8, (nb * rep + 31) / 32);
+  // Sixteen tiles a part where that makes about two CTAs per SM (as many as are resident); with fewer key blocks a part gets fewer tiles, down to one: 256 tokens, 16 heads
+  // 32.7 -> 15.5 us for both kernels (19.5 before tensor memory), 1024 tokens, 22 heads 37.5 -> 33.2.  One or four CTAs per SM: 34.2 and 31.8 against 28.6 for 1024 tokens, 16 heads.
+  const int most = (nb * rep + 1) / 2;                                   // tiles of the first key block when every block attends to it
+  p.part_tiles = (int)std::max<int64_t>(1, std::min<int64_t>(16, ((int64_t)B * nkv * nb * most + 2 * kNumSMs - 1) / (2 * kNumSMs)));
+  p.parts = p.part_tiles == 16 ? std::min(8, (most + 15) / 16) : (most + p.part_tiles - 1) / p.part_tiles;
   const int smem_q = (2 + Q_STAGES) * TILE_BYTES + 1024 + 256 + 1024 + list_bytes(nb), smem_kv = (1 + 2 * KV_STAGES + 2) * TILE_BYTES + 256 + list_bytes(nb);
   static bool cfg = false;
   if (!cfg) { allow_smem(qsa_attn_bwd_q_kernel); allow_smem(qsa_attn_bwd_kv_kernel); cfg = true; }

@@ -16,6 +16,13 @@ def test_block_attention_tiles(ops, B, nb, nq, nkv, pick):  # noqa: F811
     block_attention(ops, B, nb, nq, nkv, pick)
 
 
+# one, three, fifteen and sixteen tiles per part, the latter in as many parts as allowed and in fewer
+@gpu
+@pytest.mark.parametrize("B,nb,nq,nkv", [(1, 4, 16, 2), (1, 8, 22, 2), (1, 19, 24, 2), (1, 20, 24, 2), (4, 20, 20, 2)])
+def test_block_attention_parts(ops, B, nb, nq, nkv):  # noqa: F811
+    block_attention(ops, B, nb, nq, nkv, "dense")
+
+
 # enough query blocks for one CTA each (no slices): a half-empty key tile, one and a half key tiles; heads that do not exist
 @gpu
 @pytest.mark.parametrize("B,nb,NI", [(150, 1, 4), (50, 3, 3)])
