@@ -176,8 +176,9 @@ at::Tensor qsa_indexer_fwd(const at::Tensor& qi, const at::Tensor& ki, const at:
   const int B = qi.size(0), NI = qi.size(1), S = qi.size(2), nb = S / 64, tiles = (nb + 1) / 2;
   TORCH_CHECK(ki.numel() == (int64_t)B * S * 64 && wi.numel() == (int64_t)B * S * NI, "qsa_indexer_fwd: k must be [B,S,64] and w [B,S,heads]");
   auto blse = at::full({B, S, nb}, -1e9, qi.options().dtype(at::kFloat));
-  // key blocks of a query tile are shared by as many CTAs as it takes to have about four per SM, at least eight blocks each
-  const int Z = std::max(1, std::min((nb + 7) / 8, 4 * kNumSMs / std::max(1, B * tiles)));
+  // key blocks of a query tile are shared by as many CTAs as it takes to have about four per SM, at least eight blocks each, or one per SM, with fewer
+  // blocks down to one (1024 tokens 12.3 -> 6.2 us, 256 tokens 8.4 -> 5.9)
+  const int rows = std::max(1, B * tiles), Z = std::max({1, std::min((nb + 7) / 8, 4 * kNumSMs / rows), std::min(nb, kNumSMs / rows)});
   const CUtensorMap tq = make_tmap_box(qi.data_ptr(), 2, 64, S, (int64_t)B * NI, 64, (int64_t)S * 64, 128, 128), tk = make_tmap_box(ki.data_ptr(), 2, 64, S, B, 64, (int64_t)S * 64, 64, 128);
   IndexFwdArgs p{};
   p.wi = wi.data_ptr<float>(); p.blse = blse.data_ptr<float>(); p.S = S; p.NI = NI; p.Z = Z; p.scale = (float)scale; p.err = err.has_value() ? err->data_ptr<int>() : nullptr;

@@ -30,9 +30,9 @@ def test_indexer_backward_without_slices(ops, B, nb, NI):  # noqa: F811
     indexer_backward(ops, NI, B, nb)
 
 
-# half a query tile, an odd last one, key blocks shared by several CTAs; fewer heads than the kernel holds
+# half a query tile, an odd last one, a CTA for every key block and for two; several blocks per CTA; fewer heads than the kernel holds
 @gpu
-@pytest.mark.parametrize("B,nb,NI", [(1, 1, 4), (2, 3, 1), (1, 21, 3)])
+@pytest.mark.parametrize("B,nb,NI", [(1, 1, 4), (2, 3, 1), (1, 16, 4), (1, 21, 3), (12, 21, 4)])
 def test_indexer_forward(ops, B, nb, NI):  # noqa: F811
     S = 64 * nb
     gen = torch.Generator(device="cuda").manual_seed(nb)
