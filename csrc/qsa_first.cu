@@ -2,7 +2,7 @@
 // looks at the first query of every 64-token block, so only those S/64 queries are scored:
 //     I[s]      = sum_h w_h relu(bf16(q_h . k_s)) * scale          for the keys s <= 64 i  (causal for the query at 64 i)
 //     lp_blk[j] = logsumexp_{s in block j} I[s] - logsumexp_s I[s]  for j <= i, a large negative number for j > i
-// The same rounding points as the full indexer kernel (qsa_index.cu) and the PyTorch specification: q.k is rounded to bf16 before
+// The same rounding points as the full indexer kernel (qsa_index_fwd.cu) and the PyTorch specification: q.k is rounded to bf16 before
 // the relu.  (Reference: modeling_qwen3_8_moe.py:1126-1131 scores these queries with eager matmul / einsum / log_softmax /
 // logsumexp calls.)
 #include <ATen/ATen.h>
@@ -15,12 +15,14 @@
 
 namespace q38 {
 
-// Two kernels: scores of 256 keys against four queries per CTA, a key per thread (qsa_first_scores), then one CTA per query for the sums and the blocks.  With all keys
+// Two kernels: scores of 256 keys against one, two or four queries per CTA, a key per thread (qsa_first_scores), then one CTA per query for the sums and the blocks.  With all keys
 // of a query in one CTA the last of them had 16 rows of 128 bytes per thread to fetch one after the other: 59 us for one sequence of 8192 tokens, now
-// 30 (23 and 7; 29 and 7 with one query per CTA).  The sum over all keys keeps the order that 128 threads give it.
-constexpr int QF_THREADS = 512, QF_SUM = 128, QF_HEADS_MAX = 4, QF_KEYS = 256, QF_QUERIES = 4;
+// 28 (31 with two queries per CTA, 38 with one).  Short sequences take fewer queries per CTA, which come one after the other: 256 tokens 5.7, 7.1 and 9.5 us with one, two
+// and four (4.8 in one kernel), 1024 tokens 6.4, 7.9 and 10.3 (9.5), two sequences of 2048 12.2, 10.8 and 11.3.  The sum over all keys keeps the order that 128 threads give it.
+constexpr int QF_THREADS = 512, QF_SUM = 128, QF_HEADS_MAX = 4, QF_KEYS = 256;
 constexpr float QF_MASKED = -1e9f;
 
+template <int QF_QUERIES>
 __global__ void __launch_bounds__(QF_KEYS) qsa_first_scores_kernel(const __nv_bfloat16* __restrict__ q_first, const __nv_bfloat16* __restrict__ ki,
                                                                    const float* __restrict__ w_first, float* __restrict__ scores, int S, int NI, float scale) {
   grid_wait();
@@ -111,8 +113,16 @@ at::Tensor qsa_first_query_lp(const at::Tensor& q_first, const at::Tensor& ki, c
   auto lp = at::empty({B, nb, nb}, q_first.options().dtype(at::kFloat));
   auto scores = at::empty({B, nb, S}, q_first.options().dtype(at::kFloat));       // causal entries are written and read
   auto stream = at::cuda::getCurrentCUDAStream();
-  launch(qsa_first_scores_kernel, dim3((S + QF_KEYS - 1) / QF_KEYS, (nb + QF_QUERIES - 1) / QF_QUERIES, B), QF_KEYS, 0, stream, (const __nv_bfloat16*)q_first.data_ptr(), (const __nv_bfloat16*)ki.data_ptr(),
-         w_first.data_ptr<float>(), scores.data_ptr<float>(), S, NI, (float)scale);
+  const int key_tiles = (S + QF_KEYS - 1) / QF_KEYS;
+  auto score = [&](auto kernel, int queries) {
+    launch(kernel, dim3(key_tiles, (nb + queries - 1) / queries, B), QF_KEYS, 0, stream, (const __nv_bfloat16*)q_first.data_ptr(), (const __nv_bfloat16*)ki.data_ptr(),
+           w_first.data_ptr<float>(), scores.data_ptr<float>(), S, NI, (float)scale);
+  };
+  // one query per CTA up to two CTAs per SM, two up to seven (half of the pairs are not causal and end at once): see above
+  const int64_t pairs = (int64_t)key_tiles * nb * B;
+  if (pairs <= 2 * kNumSMs) score(qsa_first_scores_kernel<1>, 1);
+  else if (pairs <= 7 * kNumSMs) score(qsa_first_scores_kernel<2>, 2);
+  else score(qsa_first_scores_kernel<4>, 4);
   launch(qsa_first_query_lp_kernel, dim3(nb, B), QF_THREADS, (36 + S) * 4, stream, scores.data_ptr<float>(), lp.data_ptr<float>(), S);
   C10_CUDA_KERNEL_LAUNCH_CHECK();
   count_launch(2);

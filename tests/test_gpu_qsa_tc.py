@@ -2,6 +2,7 @@
 import pytest
 import torch
 
+from test_gpu_kernels import test_first_query_indexer_log_probabilities as first_query
 from test_gpu_qsa_edges import ops, test_block_attention as block_attention, test_indexer_backward as indexer_backward  # noqa: F401
 from test_kernel_sources import test_waits_of_whole_warps_are_voted as waits_are_voted
 
@@ -156,3 +157,10 @@ def test_indexer_weight_gradient_sees_more_than_bf16(ops, B, nb):  # noqa: F811
             dI = torch.where(hide, 0.0, torch.exp(score - spread(score.unflatten(-1, (-1, 64)).logsumexp(-1))) * spread(dblse[b, t0:t1, :(t1 + 63) // 64].double()))
             want[b, t0:t1] = (dI * dots).sum(-1).t() * 0.125
     assert (dw - want).norm() <= 2 ** -13 * want.norm()
+
+
+# one, two and four queries per CTA, the last CTA of the latter two with one query
+@gpu
+@pytest.mark.parametrize("B,nb,NI", [(1, 1, 4), (1, 17, 3), (1, 37, 4), (3, 41, 2)])
+def test_first_query_grids(ops, B, nb, NI):  # noqa: F811
+    first_query(ops, B, 64 * nb, NI)
