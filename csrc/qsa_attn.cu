@@ -17,6 +17,9 @@
 
 namespace q38 {
 
+void qsa_attn_fwd_small(const at::Tensor& q, const at::Tensor& k, const at::Tensor& v, bool v_tokens, const at::Tensor& sel, const at::Tensor& o, const at::Tensor& lse,
+                        double scale);   // qsa_attn_small.cu
+
 using bf16 = __nv_bfloat16;
 
 // sel[b, i, j] = 1 iff query block i attends key block j
@@ -42,7 +45,8 @@ __global__ void qsa_selection_matrix_kernel(const int* __restrict__ count, const
 // Four CTAs per SM (128 TMEM columns, 48 KB each) cover each other's chains: the products of a tile take 300 of its 1700 cycles, the exponentials 512
 // per SM.  Every operation and its order are those of the warp-MMA kernel that stood here (scores, sums of a row in four interleaved parts, four K = 16
 // steps per product), so the results have its bits.  16384 tokens of four sequences, 22 heads, eight blocks per query: 182 -> 118 us; dense, 8192 tokens
-// of two sequences, 16 heads: 260 -> 143; one of 8192, 28 heads: 122 -> 77.  A grid that leaves SMs idle pays the longer chain of a tile (640 tokens, 5 heads: 9.5 -> 14 us).  Every mbarrier wait is bounded and reports through the error word.
+// of two sequences, 16 heads: 260 -> 143; one of 8192, 28 heads: 122 -> 77.  A grid that leaves SMs idle would pay the longer chain of a tile: it keeps the warp-MMA kernel
+// (qsa_attn_small.cu).  Every mbarrier wait is bounded and reports through the error word.
 constexpr int AF_THREADS = 192, AF_STAGES = 2;             // TMA warp, MMA warp, four warps of row threads
 constexpr int HALF_BYTES = 64 * 128, TILE_BYTES = 2 * HALF_BYTES;
 constexpr uint32_t COL_S = 0, COL_O = 64;
@@ -256,6 +260,12 @@ std::vector<at::Tensor> qsa_attn_fwd(const at::Tensor& q, const at::Tensor& k, c
   auto sel = selection_matrix(count, index, B, nb, q.options(), stream);
   auto o = at::empty({B, S, nq, 64}, q.options());
   auto lse = at::empty({B, nq, S}, q.options().dtype(at::kFloat));
+  // up to one CTA per SM the shorter chain wins, above it the tensor cores (times of both: qsa_attn_small.cu)
+  const int64_t ctas = (int64_t)B * nkv * ((nq / nkv + 1) / 2) * nb;
+  if (ctas <= kNumSMs) {
+    qsa_attn_fwd_small(q, k, v, v_tokens, sel, o, lse, scale);
+    return {o, lse, sel};
+  }
   const CUtensorMap tq = make_tmap_box(q.data_ptr(), 2, 64, (int64_t)B * nq * S, 1, 64, 0, 64, 128), tk = make_tmap_box(k.data_ptr(), 2, 64, (int64_t)B * nkv * S, 1, 64, 0, 64, 128),
                     tv = value_map(v, v_tokens);
   FwdArgs p{};
@@ -264,7 +274,7 @@ std::vector<at::Tensor> qsa_attn_fwd(const at::Tensor& q, const at::Tensor& k, c
   const int smem = (1 + AF_STAGES) * TILE_BYTES + 128 + list_bytes(nb);
   static bool cfg = false;
   if (!cfg) { allow_smem(qsa_attn_fwd_kernel); cfg = true; }
-  launch(qsa_attn_fwd_kernel, dim3(B * nkv * ((nq / nkv + 1) / 2), nb), AF_THREADS, smem, stream, tq, tk, tv, p);
+  launch(qsa_attn_fwd_kernel, dim3((unsigned)(ctas / nb), nb), AF_THREADS, smem, stream, tq, tk, tv, p);
   C10_CUDA_KERNEL_LAUNCH_CHECK();
   count_launch();
   return {o, lse, sel};

@@ -164,3 +164,34 @@ def test_indexer_weight_gradient_sees_more_than_bf16(ops, B, nb):  # noqa: F811
 @pytest.mark.parametrize("B,nb,NI", [(1, 1, 4), (1, 17, 3), (1, 37, 4), (3, 41, 2)])
 def test_first_query_grids(ops, B, nb, NI):  # noqa: F811
     first_query(ops, B, 64 * nb, NI)
+
+
+@gpu
+@pytest.mark.parametrize("nb,nq,nkv,pick", [(1, 1, 1, "dense"), (3, 5, 1, "dense"), (9, 11, 1, "gaps"), (37, 4, 1, "dense")])
+@pytest.mark.parametrize("tokens", [False, True])
+def test_block_attention_is_the_same_on_both_kernels(ops, nb, nq, nkv, pick, tokens):  # noqa: F811
+    """Up to one CTA per SM the warp-MMA kernel runs, above it the tensor-memory one: a sequence alone, and among copies that make the grid large, gives the
+    same bits.  Values as a transposed view too."""
+    S, copies = 64 * nb, 150
+    gen = torch.Generator(device="cuda").manual_seed(nb)
+    q, k, v = (torch.randn(1, h, S, 64, device="cuda", generator=gen).to(torch.bfloat16) for h in (nq, nkv, nkv))
+    count = index = None
+    if pick == "gaps":
+        index = torch.tensor([[j for j in range(nb) if j <= i and (i - j) % 3 == 0][::-1] + [0] * (i - i // 3 + nb - 1 - i) for i in range(nb)], dtype=torch.int32, device="cuda")[None]
+        count = torch.tensor([[i // 3 + 1 for i in range(nb)]], dtype=torch.int32, device="cuda")
+    lay = lambda t: t.transpose(1, 2).contiguous().transpose(1, 2) if tokens else t
+    many = lambda t: None if t is None else t.expand(copies, *t.shape[1:]).contiguous()
+    alone = ops.load().qsa_attn_fwd(q, k, lay(v), count, index, 0.125)
+    among = ops.load().qsa_attn_fwd(many(q), many(k), lay(many(v)), many(count), many(index), 0.125)
+    for a, b in zip(alone, among):
+        assert torch.equal(a[0], b[0]) and torch.equal(a[0], b[copies - 1])
+
+
+@gpu
+@pytest.mark.parametrize("B", [1, 150])
+def test_block_attention_refuses_unaligned_operands(ops, B):  # noqa: F811
+    flat = torch.randn(B * 64 * 64 + 1, device="cuda").to(torch.bfloat16)
+    q, odd = flat[:-1].view(B, 1, 64, 64), flat[1:].view(B, 1, 64, 64)
+    for operands in ((odd, q, q), (q, odd, q), (q, q, odd)):
+        with pytest.raises(RuntimeError):
+            ops.load().qsa_attn_fwd(*operands, None, None, 0.125)
