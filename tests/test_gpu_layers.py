@@ -1,12 +1,15 @@
 """Layer calls (one native call per pass) against the op-by-op path of the same hook: the same launches, so the same bits.
 
-The key and value gradients of the attention and the indexer's key gradient are added with fp32 atomics in both, and so are split weight
-gradients: these are compared to 1e-3 of their norm (one bf16 rounding of a sum whose order varies)."""
+Sums whose order varies are compared to 1e-3 of their norm (one bf16 rounding of such a sum): the key and value gradients of the attention and the
+indexer's key gradient (fp32 atomics), what is computed from them, the small parameters' gradients, and split weight gradients.  Where a gradient is added to a buffer, what was
+added is compared, not the sum, and the buffer's content is of the gradient's own size."""
 import pytest
 import torch
 
 pytestmark = pytest.mark.gpu
 HIDDEN, S = 64, 128
+# hidden width, tokens per sequence (an even, a single and an odd number of blocks), heads, KV heads, key and value heads of the delta rule
+SHAPES = {"even": (64, 128, 6, 2, 2, 6), "single": (192, 64, 5, 1, 3, 3), "odd": (128, 192, 4, 4, 1, 4)}
 
 
 @pytest.fixture(scope="module")
@@ -17,10 +20,11 @@ def modeling():
     return modeling
 
 
-def build(modeling, kind):
+def build(modeling, kind, shape="even"):
     from q38.presets import model_config
-    shape = dict(layers=4, hidden=HIDDEN, heads=6, kv_heads=2, lin_k_heads=2, lin_v_heads=6, experts=8, topk=2, moe_ffn=32, shared_ffn=32, ngram_rows=64)
-    cfg = model_config(shape, 512, S, bos_token_id=1, eos_token_id=2, pad_token_id=0)
+    hidden, seq, heads, kv_heads, k_heads, v_heads = SHAPES[shape]
+    cfg = model_config(dict(layers=4, hidden=hidden, heads=heads, kv_heads=kv_heads, lin_k_heads=k_heads, lin_v_heads=v_heads, experts=8, topk=2, moe_ffn=32, shared_ffn=32,
+                            ngram_rows=64), 512, seq, bos_token_id=1, eos_token_id=2, pad_token_id=0)
     torch.manual_seed(0)
     with torch.device("cuda"):
         if kind == "gdn":
@@ -30,11 +34,11 @@ def build(modeling, kind):
             torch.nn.init.normal_(module.experts.gate_up_proj, std=0.1)
             torch.nn.init.normal_(module.experts.down_proj, std=0.1)
         elif kind == "mhc":
-            module = torch.nn.ModuleDict(dict(mhc=modeling.MHC(HIDDEN), norm=modeling.Qwen3_8MoeRMSNorm(HIDDEN)))
+            module = torch.nn.ModuleDict(dict(mhc=modeling.MHC(hidden), norm=modeling.Qwen3_8MoeRMSNorm(hidden)))
         elif kind == "head":
-            module = torch.nn.Linear(HIDDEN, 512, bias=False)
+            module = torch.nn.Linear(hidden, 512, bias=False)
         else:
-            module = torch.nn.ModuleDict(dict(attn=modeling.Qwen3_8MoeAttention(cfg, 3), indexer=modeling.Indexer(HIDDEN, 4, 64)))
+            module = torch.nn.ModuleDict(dict(attn=modeling.Qwen3_8MoeAttention(cfg, 3), indexer=modeling.Indexer(hidden, 4, 64)))
     return module
 
 
@@ -47,8 +51,8 @@ def run(modeling, module, kind, x, target, parts):
         return [backend.mhc_post(module["mhc"], xin, link)]
     if kind == "head":
         from q38.losses import linear_cross_entropy
-        return [linear_cross_entropy(module.weight, x.reshape(-1, HIDDEN), target)]
-    cos, sin = modeling.rope_tables(torch.arange(S, device="cuda")[None], 16, 1e7, torch.float32)
+        return [linear_cross_entropy(module.weight, x.reshape(-1, x.shape[-1]), target)]
+    cos, sin = modeling.rope_tables(torch.arange(x.shape[1], device="cuda")[None], 16, 1e7, torch.float32)
     train = x.requires_grad or any(p.requires_grad for p in module.parameters())
     y, kl = modeling.qsa_attention(module["attn"], x, cos, sin, None if "plain" in kind else module["indexer"], 1, "dense" in kind, train and "kl" in kind)
     return [out for name, out in (("y", y), ("kl", kl)) if out is not None and name in parts and (not train or out.requires_grad)]
@@ -56,54 +60,83 @@ def run(modeling, module, kind, x, target, parts):
 
 KINDS = ["gdn", "moe", "mhc", "head", "qsa kl", "qsa kl dense", "qsa dense", "qsa", "qsa plain dense"]
 MODES = ["infer", "buffers", "fresh", "side stream", "frozen input", "frozen weights", "y alone", "kl alone"]
+CASES = [(mode, "even") for mode in MODES] + [(mode, shape) for shape in ("single", "odd") for mode in ("infer", "buffers", "fresh")]
+# results with sums whose order varies, besides weight gradients that are added to a buffer
+ANY_ORDER = {"gdn": ("conv1d.weight", "A_log", "dt_bias", "norm.weight"), "moe": (), "mhc": ("mhc.B.weight", "mhc.b_pre", "mhc.b_post", "mhc.b_res", "mhc.alphas", "norm.weight"), "head": (),
+             "qsa": ("dx", "attn.k_proj.weight", "attn.v_proj.weight", "attn.q_norm.weight", "attn.k_norm.weight", "indexer.wk.weight")}
+
+
+class Library:
+    """The kernel library, with the names of the operators that were called."""
+
+    def __init__(self, lib):
+        self.lib, self.called = lib, set()
+
+    def __getattr__(self, name):
+        self.called.add(name)
+        return getattr(self.lib, name)
 
 
 @pytest.mark.parametrize("kind", KINDS)
-@pytest.mark.parametrize("mode", MODES)
-def test_layer_call_matches_its_ops(modeling, kind, mode, monkeypatch):
+@pytest.mark.parametrize("mode,shape", CASES)
+def test_layer_call_matches_its_ops(modeling, kind, mode, shape, monkeypatch):
+    from q38.ops import backend as ops_backend
     from q38.ops.backend import WGRAD_STREAM
     if "alone" in mode and "kl" not in kind:
         pytest.skip("one output")
     backend = modeling.get_backend()
+    hidden, seq = SHAPES[shape][:2]
     gen = torch.Generator(device="cuda").manual_seed(1)
-    shape = (2, S, 4, HIDDEN) if kind == "mhc" else (2, S, HIDDEN)
-    x0 = torch.randn(shape, device="cuda", generator=gen)
+    x0 = torch.randn((2, seq, 4, hidden) if kind == "mhc" else (2, seq, hidden), device="cuda", generator=gen)
     x0 = x0 if kind == "mhc" else x0.to(torch.bfloat16)
-    target = torch.randint(0, 512, (2 * S,), device="cuda", generator=gen)
+    target = torch.randint(0, 512, (2 * seq,), device="cuda", generator=gen)
     parts = {"y alone": ("y",), "kl alone": ("kl",)}.get(mode, ("y", "kl"))
-    results = []
-    for native in (True, False):
-        module = build(modeling, kind)
-        if not native:
-            monkeypatch.setattr(backend, "native_layers", lambda hidden: False)
-        calls = []
-        if native and kind != "head":
-            from q38.ops import backend as ops_backend
-            lib = ops_backend.load()
-            monkeypatch.setattr(ops_backend, "load", lambda: calls.append(1) or lib)
+    op = {"gdn": "gdn_layer", "moe": "moe_layer", "mhc": "mhc_layer", "head": "linear_ce"}.get(kind, "qsa_layer")
+
+    def once(native, buffers):
+        """Outputs and gradients; `buffers`: what the gradient buffers hold before, by name."""
+        module = build(modeling, kind, shape)
+        library = Library(ops_backend.load())
         x = x0.clone().requires_grad_(mode not in ("infer", "frozen input"))
-        names = [n for n, _ in module.named_parameters()]
-        for i, p in enumerate(module.parameters()):
+        for i, (name, p) in enumerate(module.named_parameters()):
             p.requires_grad_(mode != "infer" and not (mode == "frozen weights" and i % 2))
-            if mode not in ("fresh", "infer") and p.requires_grad:
-                p.grad = torch.full_like(p, 0.25)
+            if name in buffers and p.requires_grad:
+                p.grad = buffers[name].clone()
         WGRAD_STREAM.enabled = mode == "side stream"
-        with torch.set_grad_enabled(mode != "infer"):
+        with monkeypatch.context() as patch, torch.set_grad_enabled(mode != "infer"):
+            patch.setattr(ops_backend, "load", lambda: library)
+            if not native:
+                patch.setattr(backend, "native_layers", lambda hidden: False)
             outs = run(modeling, module, kind, x, target, parts)
             if mode != "infer":
                 torch.autograd.backward(outs, [torch.ones_like(o) * 0.5 for o in outs])
                 WGRAD_STREAM.join()
         WGRAD_STREAM.enabled = False
-        if native and kind != "head":
-            assert len(calls) <= 4, "the op-by-op path ran"
-            monkeypatch.undo()
-        results.append([("out", o.detach()) for o in outs] + [("dx", x.grad)] + [(n, p.grad) for n, p in zip(names, module.parameters())])
-    for (name, got), (_, want) in zip(*results):
-        assert (got is None) == (want is None), name
-        if got is not None:
-            assert got.dtype == want.dtype and got.shape == want.shape
-            err = (got.double() - want.double()).norm() / want.double().norm().clamp_min(1e-30)
-            assert err <= (0 if name == "out" else 1e-3), (name, float(err))
+        used = {name for name in library.called if "_layer_" in name or name.startswith("linear_ce_")}
+        assert used == ({op + "_fwd"} | ({op + "_bwd"} if mode != "infer" else set()) if native else set())
+        added = {n: p.grad if n not in buffers or p.grad is None else p.grad - buffers[n] for n, p in module.named_parameters()}
+        return {**{f"out {i}": o.detach() for i, o in enumerate(outs)}, "dx": x.grad, **added}
+
+    buffers = {}
+    if mode not in ("infer", "fresh"):
+        own = once(False, {})
+        noise = lambda g: torch.randn(g.shape, device="cuda", generator=gen) * (g.double().pow(2).mean().sqrt().float() if bool(g.any()) else 1e-3)
+        buffers = {n: noise(torch.zeros_like(p) if own[n] is None else own[n]) for n, p in build(modeling, kind, shape).named_parameters()}
+    got, want = once(True, buffers), once(False, buffers)
+    assert got.keys() == want.keys()
+    for name in got:
+        a, b = got[name], want[name]
+        assert (a is None) == (b is None), name
+        if a is None:
+            continue
+        assert a.dtype == b.dtype and a.shape == b.shape
+        if buffers and name in buffers:
+            assert bool(b.any()) == (own[name] is not None and bool(own[name].any())), (name, "nothing was added")
+            if own[name] is not None:
+                assert (a.double() - own[name].double()).norm() <= 1e-3 * own[name].double().norm(), (name, "not the gradient that is returned without a buffer")
+        err = (a.double() - b.double()).norm() / b.double().norm().clamp_min(1e-30)
+        varies = name in ANY_ORDER[kind.split()[0]] or name in buffers
+        assert err <= (1e-3 if varies else 0), (name, float(err))
 
 
 def test_layer_call_under_activation_checkpointing(modeling):
