@@ -1,6 +1,6 @@
 // 64x64x64 bf16 tile products on the warp-level tensor-core path (mma.sync m16n8k16, fp32 accumulation) for kernels
-// whose chains of small dependent products are latency bound (the delta rule), and for block masses of sequence lengths that the
-// tcgen05 kernel does not take.  Four warps cooperate on one 64x64 output; warp w owns rows 16w..16w+15 and keeps them in registers.
+// whose chains of small dependent products are latency bound (the delta rule, the attention of a short prompt), and for block masses of sequence lengths
+// that the tcgen05 kernel does not take.  Four warps cooperate on one 64x64 output; warp w owns rows 16w..16w+15 and keeps them in registers.
 #pragma once
 #include "common.cuh"
 

@@ -186,7 +186,7 @@ at::Tensor qsa_indexer_fwd(const at::Tensor& qi, const at::Tensor& ki, const at:
   if (!cfg) { C10_CUDA_CHECK(cudaFuncSetAttribute(qsa_indexer_fwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, IF_SMEM)); cfg = true; }
   launch(qsa_indexer_fwd_kernel, dim3(B * Z, tiles), IF_THREADS, IF_SMEM, at::cuda::getCurrentCUDAStream(), tq, tk, p);
   C10_CUDA_KERNEL_LAUNCH_CHECK();
-  count_launch(2);
+  count_launch();
   return blse;
 }
 

@@ -164,7 +164,7 @@ __global__ void __launch_bounds__(32 * HP_WARPS, 4) qsa_headprep_bwd_kernel(cons
   }
 }
 
-// Enough CTAs to fill the chip several times over, few enough that a warp handles many rows (the backward adds one weight gradient per CTA).
+// As many CTAs as are resident at once, so that none waits for a second wave and a warp handles many rows (the backward adds one weight gradient per CTA).
 static unsigned headprep_grid(long long rows, int resident) { return (unsigned)std::max<long long>(1, std::min<long long>((rows + 4 * HP_WARPS - 1) / (4 * HP_WARPS), kNumSMs * resident)); }
 
 // The kernels read 16-byte pieces; a contiguous view that starts elsewhere is copied first.  Other strides go on to the checks as they are (a copy
