@@ -15,8 +15,8 @@
 // (fp32 adds of 32 x 32 boxes); query gradients are stored, or left in one slice per z that a small kernel adds in ascending order, so they have the same
 // bits in every run.
 //
-// Bound by the instructions per element (16 compute warps; rounding, masks and packing run at half rate), not by
-// the products.  Two warp-MMA passes with the scores formed twice stood here: four
+// Bound by the instructions per element (16 compute warps; rounding, masks and packing run at half rate; issue slots 43 % busy) and the writes of E's operand (shared memory
+// 46 %), not by the products (tensor pipe 26 %).  Two warp-MMA passes with the scores formed twice stood here: four
 // sequences of 4096 with four heads 405 -> 120 us, one 149 -> 70, one of 1024 tokens 33 -> 22.  dk goes before the unit's next scores in the queue and E
 // after them, so that compute warps wait for two products instead of four, and all sequences' longest query blocks start first.
 // With dI in one bf16 it took 98, 59 and 20 us (13 us of the difference are the second operand's stores, 7 its products, 2 the ring of two stages and the single key-gradient
