@@ -195,3 +195,41 @@ def test_block_attention_refuses_unaligned_operands(ops, B):  # noqa: F811
     for operands in ((odd, q, q), (q, odd, q), (q, q, odd)):
         with pytest.raises(RuntimeError):
             ops.load().qsa_attn_fwd(*operands, None, None, 0.125)
+
+
+@gpu
+@pytest.mark.parametrize("copies", [1, 60])
+@pytest.mark.parametrize("bad", [float("nan"), float("inf")])
+@pytest.mark.parametrize("where", ["query", "key", "value", "upstream"])
+def test_block_attention_keeps_bad_values_to_what_they_reach(ops, copies, bad, where):  # noqa: F811
+    """One element that is not finite, on both forward kernels (grids below and above one CTA per SM): what does not depend on it keeps its bits, although
+    tiles hold two heads, accumulators two gradients and blocks masked positions; what does shows it."""
+    B, nq, nkv, S, at = copies, 5, 1, 192, 70
+    gen = torch.Generator(device="cuda").manual_seed(3)
+    clean = {n: torch.randn(s, device="cuda", generator=gen).to(torch.bfloat16)
+             for n, s in dict(query=(B, nq, S, 64), key=(B, nkv, S, 64), value=(B, nkv, S, 64), upstream=(B, S, nq, 64)).items()}
+    dirty = dict(clean, **{where: clean[where].clone()})
+    if where == "upstream":
+        dirty[where][0, at, 1, 5] = bad
+    else:
+        dirty[where][0, 1 if where == "query" else 0, at, 5] = bad
+    results = []
+    for t in (clean, dirty):
+        o, lse, sel = ops.load().qsa_attn_fwd(t["query"], t["key"], t["value"], None, None, 0.125)
+        results.append((o, *ops.load().qsa_attn_bwd(t["query"], t["key"], t["value"], o, t["upstream"], lse, sel, 0.125)))
+    (o, dq, dk, dv), (o2, dq2, dk2, dv2) = results
+    one_row = where in ("query", "upstream")                             # else all heads' rows from the key's block on (hidden positions of it weigh zero times the bad value)
+    touched = torch.zeros(B, nq, S, dtype=torch.bool, device="cuda")
+    touched[0, 1 if one_row else slice(None), at if one_row else slice(at // 64 * 64, None)] = True
+    if where != "upstream":
+        assert torch.equal(o.transpose(1, 2)[~touched], o2.transpose(1, 2)[~touched]) and not o2[0, at, 1].isfinite().all()
+    else:
+        assert torch.equal(o, o2)
+    assert torch.equal(dq[~touched], dq2[~touched]) and not dq2[0, 1, at].isfinite().all()
+    last = (at // 64 + 1) * 64 if one_row else S                         # keys after the query's block get nothing from it
+    for a, b in ((dk, dk2), (dv, dv2)):
+        if copies > 1:
+            assert (a[1:].float() - b[1:].float()).norm() <= 4e-3 * a[1:].float().norm()
+        if last < S:
+            assert (a[0, :, last:].float() - b[0, :, last:].float()).norm() <= 4e-3 * a[0, :, last:].float().norm()
+    assert not dk2[0].isfinite().all()
